@@ -263,71 +263,23 @@ static int create(const fs_params* prm, Solver* s) {
 // F32 Poisson solve on (p32, div32): `iterations` sweeps or V-cycles
 // (_encodePoisson, solver.js:686-738)
 static void poisson_f32(Solver* s, int iterations, bool p_nonzero) {
-  const fs_params& P = s->prm;
-  const Grid& g = s->g;
-  float h2 = g.dx * g.dx;
-  if (P.pressure_solver == FS_PRESSURE_MULTIGRID) {
-    s->lev[0].x = s->p32;
-    s->lev[0].x2 = s->p32b;
-    for (int k = 0; k < iterations; k++) {
-      if (s->fused) mg_vcycle_fused(s, p_nonzero || k > 0);
-      else mg_vcycle(s);
-    }
-    s->p32 = s->lev[0].x;
-    s->p32b = s->lev[0].x2;
+  if (s->prm.pressure_solver != FS_PRESSURE_MULTIGRID) {
+    flat_sweeps(s, &s->p32, &s->p32b, s->div32, iterations, !p_nonzero);
     return;
-  } else if (P.pressure_solver == FS_PRESSURE_RED_BLACK) {
-    for (int k = 0; k < iterations; k++)
-      for (int colour = 0; colour < 2; colour++) {
-        if (!s->odd) {
-          launch_rb_half(s, s->p32, s->div32, s->p32, h2, colour, g.nx, g.ny);
-        } else {
-          launch_rb_half(s, s->p32, s->div32, s->p32b, h2, colour, g.nx, g.ny);
-          std::swap(s->p32, s->p32b);
-        }
-      }
-  } else {
-    for (int k = 0; k < iterations; k++) {
-      launch_jacobi(s, s->p32, s->div32, s->p32b, h2, g.nx, g.ny);
-      std::swap(s->p32, s->p32b);
-    }
   }
+  s->lev[0].x = s->p32;
+  s->lev[0].x2 = s->p32b;
+  for (int k = 0; k < iterations; k++) {
+    if (s->fused) mg_vcycle_fused(s, p_nonzero || k > 0);
+    else mg_vcycle(s);
+  }
+  s->p32 = s->lev[0].x;
+  s->p32b = s->lev[0].x2;
 }
 
-// correction solve of the MIXED mode: e32 from r32 starting at zero
+// correction solve of the MIXED mode with the flat solvers: e32 from r32 starting at zero
 static void correction_solve(Solver* s, int iterations) {
-  const fs_params& P = s->prm;
-  const Grid& g = s->g;
-  float h2 = g.dx * g.dx;
-  if (P.pressure_solver == FS_PRESSURE_MULTIGRID) {
-    s->lev[0].x = s->e32;
-    s->lev[0].x2 = s->e32b;
-    if (!s->fused) launch_fill(s, s->e32, 0.f, s->n);  // the fused cycle starts from zero itself
-    for (int k = 0; k < iterations; k++) {
-      if (s->fused) mg_vcycle_fused(s, k > 0);
-      else mg_vcycle(s);
-    }
-    s->e32 = s->lev[0].x;
-    s->e32b = s->lev[0].x2;
-    return;
-  }
-  launch_fill(s, s->e32, 0.f, s->n);
-  if (P.pressure_solver == FS_PRESSURE_RED_BLACK) {
-    for (int k = 0; k < iterations; k++)
-      for (int colour = 0; colour < 2; colour++) {
-        if (!s->odd) {
-          launch_rb_half(s, s->e32, s->r32, s->e32, h2, colour, g.nx, g.ny);
-        } else {
-          launch_rb_half(s, s->e32, s->r32, s->e32b, h2, colour, g.nx, g.ny);
-          std::swap(s->e32, s->e32b);
-        }
-      }
-  } else {
-    for (int k = 0; k < iterations; k++) {
-      launch_jacobi(s, s->e32, s->r32, s->e32b, h2, g.nx, g.ny);
-      std::swap(s->e32, s->e32b);
-    }
-  }
+  flat_sweeps(s, &s->e32, &s->e32b, s->r32, iterations, true);
 }
 
 // One cycle of the multigrid tolerance loop (both precisions):
@@ -452,7 +404,8 @@ static int pressure_solve(Solver* s, bool capture, bool defer = false, bool star
       launch_fill(s, s->pl, 0.f, s->n);
     }
   } else {
-    if (!P.warm_start) launch_fill(s, s->p32, 0.f, s->n);
+    // a fixed count of flat sweeps starts from zero by itself
+    if (!P.warm_start && (mg || tol)) launch_fill(s, s->p32, 0.f, s->n);
     if (tol) launch_absmax_residual32(s, s->p32, s->div32);
   }
   if (!tol) {
@@ -1172,7 +1125,7 @@ FS_API int fs_poisson_residual_after(fs_solver* h, int iterations, double dt, do
   if (!out || iterations < 0) return fail(s, FS_ERR_INVALID_ARGUMENT, "bad arguments");
   if (s->mixed) return fail(s, FS_ERR_UNSUPPORTED, "poisson_residual_after measures the F32 solver");
   launch_divergence<float, float>(s, s->u, s->v, s->div32);
-  launch_fill(s, s->p32, 0.f, s->n);
+  if (s->prm.pressure_solver == FS_PRESSURE_MULTIGRID) launch_fill(s, s->p32, 0.f, s->n);
   poisson_f32(s, iterations, false);
   launch_poisson_norms(s, s->p32, s->div32, s->g.dx * s->g.dx, s->g.dxd * s->g.dxd);
   int rc = check_launch(s);

@@ -257,6 +257,8 @@ void launch_df_to_f(Solver* s, const float* hi, const float* lo, float* x, int64
 void launch_jacobi(Solver* s, const float* p, const float* d, float* out, float h2, int nx, int ny);
 void launch_rb_half(Solver* s, const float* src, const float* d, float* dst, float h2, int colour,
                     int nx, int ny);
+// fs_flat.cu: `iterations` Jacobi / red-black sweeps on (*x, d), *x from 0 if zero
+void flat_sweeps(Solver* s, float** x, float** y, const float* d, int iterations, bool zero);
 void launch_residual(Solver* s, const float* x, const float* rhs, float* out, float h2, int n);
 void launch_restrict(Solver* s, const float* fine, float* coarse, int nc);
 void launch_prolong_add(Solver* s, const float* coarse, float* fine, int nf);
