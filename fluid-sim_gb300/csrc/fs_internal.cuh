@@ -301,7 +301,11 @@ bool mg_fused_supported(const Solver* s);
 int mg_tile(const Solver* s, int l);
 // tile side of level l of a batch size class of count members led by s0
 int mg_tile_class(const Solver* s0, int l, int count);
+// fs_bottom.cu: the first level of the bottom solve, and the solve from there
+// (hx: from the iterate in lev[lb].x; acc: added to the double-float pressure)
 int bottom_first_level(const Solver* s);
+void launch_bottom(Solver* s, int lb, bool hx, float* acc_h, float* acc_l);
+void launch_bottom_class(Solver* const* ms, int count, int lb, cudaStream_t st);
 // batched refinement cycle of one size class of a batch (fs_multigrid.cu, fs_pressure.cu)
 int mg_vcycle_class(Solver* const* ms, int count, cudaStream_t st);
 void launch_refine_class(Solver* const* ms, int count, cudaStream_t st);

@@ -10,10 +10,7 @@
 //               there (the valid region shrinks one ring per half-sweep), then
 //               the residual and its 2x2 restriction are formed; only the
 //               tile's x and the coarse right-hand side go back to HBM;
-//   k_mg_bottom one CTA runs every level <= 64 in shared memory: levels >= 32
-//               with the whole CTA, levels <= 16 (including the coarse
-//               sweeps, 40 by default) with one warp and __syncwarp between
-//               half-sweeps;
+//   k_mg_bottom one CTA runs every level <= 64 in shared memory (fs_bottom.cu);
 //   k_mg_up     per level n > 64: prolongation-add of the coarse correction on
 //               the tile plus a halo of 2*post, then the post-smoothing sweeps.
 //
@@ -29,6 +26,7 @@
 #include <string>
 #include <utility>
 
+#include "fs_async.cuh"
 #include "fs_df.cuh"
 #include "fs_internal.cuh"
 #include "fs_stencil.cuh"
@@ -47,21 +45,6 @@ __device__ __forceinline__ int wrap_n(int i, int n) {
 
 constexpr int kTileThreads = 256;  // threads of a tile kernel (32 x 8)
 
-// 4-byte asynchronous global -> shared copies (no register round trip, all of
-// a thread's copies in flight at once); wait_all before the barrier that
-// publishes them.
-__device__ __forceinline__ void cp_async4(float* sdst, const float* gsrc) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(sdst)),
-               "l"((size_t)__cvta_generic_to_global(gsrc))
-               : "memory");
-}
-// 16-byte form (both addresses 16-byte aligned), L2 only
-__device__ __forceinline__ void cp_async16(float* sdst, const float* gsrc) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(sdst)),
-               "l"((size_t)__cvta_generic_to_global(gsrc))
-               : "memory");
-}
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 __device__ __forceinline__ void prefetch_l2(const void* p) {
   asm volatile("prefetch.global.L2 [%0];" ::"l"((size_t)__cvta_generic_to_global(p)));
 }
@@ -640,454 +623,6 @@ __global__ void __launch_bounds__(256)
                         err, pfast);
 }
 
-// ---------------------------------------------------------------- bottom
-// Levels 0..count-1 of the bottom (each n <= 64), all in shared memory.  Per
-// level: x, rhs and, for odd n, a ping-pong partner (red-black on an odd
-// periodic grid reads cells of its own colour across the wrap, so the
-// reference's ping-pong result is kept).
-struct BottomLevels {
-  int count;
-  int n[8];
-  float h2[8];
-  int off_x[8], off_x2[8], off_r[8];  // float offsets into dynamic smem (-1: none)
-  float w;                            // relaxation factor of every sweep
-};
-
-// A thread group: the whole CTA, or warp 0 alone (levels <= 16).
-struct Group {
-  int tid, nthr;
-  bool warp;
-  __device__ __forceinline__ void sync() const {
-    if (warp) __syncwarp();
-    else __syncthreads();
-  }
-};
-
-__device__ __forceinline__ void bottom_smooth(float* sm, const BottomLevels& L, int l, int sweeps, Group G) {
-  const int n = L.n[l];
-  const float h2 = L.h2[l];
-  float* x = sm + L.off_x[l];
-  float* x2 = (n & 1) ? sm + L.off_x2[l] : nullptr;
-  const float* r = sm + L.off_r[l];
-  for (int s = 0; s < 2 * sweeps; s++) {
-    const int c = s & 1;
-    if (!(n & 1)) {
-      for (int k = G.tid; k < n * n; k += G.nthr) {
-        int j = k / n, i = k - j * n;
-        if (((i + j) & 1) != c) continue;
-        int im = i == 0 ? n - 1 : i - 1, ip = i + 1 == n ? 0 : i + 1;
-        int jm = j == 0 ? n - 1 : j - 1, jp = j + 1 == n ? 0 : j + 1;
-        x[k] = gs_update(x[k], x[j * n + im], x[j * n + ip], x[jm * n + i], x[jp * n + i], r[k], h2, L.w);
-      }
-    } else {
-      for (int k = G.tid; k < n * n; k += G.nthr) {
-        int j = k / n, i = k - j * n;
-        float cur = x[k];
-        if (((i + j) & 1) != c) { x2[k] = cur; continue; }
-        int im = i == 0 ? n - 1 : i - 1, ip = i + 1 == n ? 0 : i + 1;
-        int jm = j == 0 ? n - 1 : j - 1, jp = j + 1 == n ? 0 : j + 1;
-        x2[k] = gs_update(cur, x[j * n + im], x[j * n + ip], x[jm * n + i], x[jp * n + i], r[k], h2, L.w);
-      }
-      G.sync();
-      float* t = x; x = x2; x2 = t;  // two swaps per sweep: x is back in off_x at the end
-    }
-    G.sync();
-  }
-}
-
-__device__ __forceinline__ void bottom_restrict(float* sm, const BottomLevels& L, int l, Group G) {
-  const int n = L.n[l], nc = L.n[l + 1];
-  const float ih2 = inv_h2(L.h2[l]);
-  const float* x = sm + L.off_x[l];
-  const float* r = sm + L.off_r[l];
-  float* cr = sm + L.off_r[l + 1];
-  float* cx = sm + L.off_x[l + 1];
-  for (int k = G.tid; k < nc * nc; k += G.nthr) {
-    int cj = k / nc, ci = k - cj * nc;
-    float r4[4];
-    for (int q = 0; q < 4; q++) {
-      int i = 2 * ci + (q & 1), j = 2 * cj + (q >> 1);
-      int im = i == 0 ? n - 1 : i - 1, ip = i + 1 == n ? 0 : i + 1;
-      int jm = j == 0 ? n - 1 : j - 1, jp = j + 1 == n ? 0 : j + 1;
-      r4[q] = residual_at(x[j * n + i], x[j * n + im], x[j * n + ip], x[jm * n + i], x[jp * n + i], r[j * n + i], ih2);
-    }
-    cr[k] = restrict4(r4[0], r4[1], r4[2], r4[3]);
-    cx[k] = 0.f;
-  }
-  G.sync();
-}
-
-__device__ __forceinline__ void bottom_prolong(float* sm, const BottomLevels& L, int l, Group G) {
-  const int n = L.n[l], nc = L.n[l + 1];
-  float* x = sm + L.off_x[l];
-  const float* c = sm + L.off_x[l + 1];
-  for (int k = G.tid; k < n * n; k += G.nthr) {
-    int j = k / n, i = k - j * n;
-    int ci0 = (i & 1) ? (i >> 1) : (i >> 1) - 1;
-    int cj0 = (j & 1) ? (j >> 1) : (j >> 1) - 1;
-    float fx = (i & 1) ? 0.25f : 0.75f, fy = (j & 1) ? 0.25f : 0.75f;
-    int x0 = ci0 < 0 ? ci0 + nc : ci0, x1 = ci0 + 1 >= nc ? ci0 + 1 - nc : ci0 + 1;
-    int y0 = cj0 < 0 ? cj0 + nc : cj0, y1 = cj0 + 1 >= nc ? cj0 + 1 - nc : cj0 + 1;
-    x[k] = __fadd_rn(x[k], prolong_val(c[y0 * nc + x0], c[y0 * nc + x1], c[y1 * nc + x0], c[y1 * nc + x1], fx, fy));
-  }
-  G.sync();
-}
-
-__device__ __forceinline__ void mg_bottom_body(const float* __restrict__ rhs_top, float* __restrict__ x_top,
-                                               int has_x, const BottomLevels& L, int pre, int post, int coarse,
-                                               float* __restrict__ acc_h, float* __restrict__ acc_l) {
-  extern __shared__ float sm[];
-  const int tid = threadIdx.x;
-  const Group CTA{tid, (int)blockDim.x, false};
-  const Group W0{tid, 32, true};
-  {
-    // the top level's rhs (and iterate) by asynchronous copies, all in flight at once
-    const int n = L.n[0];
-    for (int k = tid; k < n * n; k += CTA.nthr) {
-      cp_async4(&sm[L.off_r[0] + k], rhs_top + k);
-      if (has_x) cp_async4(&sm[L.off_x[0] + k], x_top + k);
-      else sm[L.off_x[0] + k] = 0.f;
-    }
-  }
-  cp_async_wait_all();
-  __syncthreads();
-  // first level handled by warp 0 alone
-  int ls = 0;
-  while (ls < L.count && L.n[ls] > 16) ls++;
-  if (ls >= L.count) {
-    // every bottom level is a CTA level
-    for (int l = 0; l < L.count - 1; l++) {
-      bottom_smooth(sm, L, l, pre, CTA);
-      bottom_restrict(sm, L, l, CTA);
-    }
-    bottom_smooth(sm, L, L.count - 1, coarse, CTA);
-    for (int l = L.count - 2; l >= 0; l--) {
-      bottom_prolong(sm, L, l, CTA);
-      bottom_smooth(sm, L, l, post, CTA);
-    }
-  } else {
-    for (int l = 0; l < ls; l++) {
-      bottom_smooth(sm, L, l, pre, CTA);
-      bottom_restrict(sm, L, l, CTA);
-    }
-    if (tid < 32) {
-      for (int l = ls; l < L.count - 1; l++) {
-        bottom_smooth(sm, L, l, pre, W0);
-        bottom_restrict(sm, L, l, W0);
-      }
-      bottom_smooth(sm, L, L.count - 1, coarse, W0);
-      for (int l = L.count - 2; l >= ls; l--) {
-        bottom_prolong(sm, L, l, W0);
-        bottom_smooth(sm, L, l, post, W0);
-      }
-    }
-    __syncthreads();
-    for (int l = ls - 1; l >= 0; l--) {
-      bottom_prolong(sm, L, l, CTA);
-      bottom_smooth(sm, L, l, post, CTA);
-    }
-  }
-  {
-    const int n = L.n[0];
-    for (int k = tid; k < n * n; k += CTA.nthr) {
-      float e = sm[L.off_x[0] + k];
-      if (acc_h) {  // the whole hierarchy fits here: add the correction to the pressure
-        df p = df_add_f(df{acc_h[k], acc_l[k]}, e);
-        acc_h[k] = p.hi;
-        acc_l[k] = p.lo;
-      } else {
-        x_top[k] = e;
-      }
-    }
-  }
-}
-
-__global__ void __launch_bounds__(1024) k_mg_bottom(const float* __restrict__ rhs_top, float* __restrict__ x_top,
-                                                    int has_x, BottomLevels L, int pre, int post, int coarse,
-                                                    float* __restrict__ acc_h, float* __restrict__ acc_l) {
-  mg_bottom_body(rhs_top, x_top, has_x, L, pre, post, coarse, acc_h, acc_l);
-}
-
-// ------------------------------------------------ bottom, compile-time chains
-// The common cases: the bottom levels are N0, N0/2, ..., NMIN with every size
-// but the coarsest even and N0 <= 64 -- the power-of-two chains down to 8 and
-// the 48 -> 24 -> 12 chain of grids of 3 * 2^k cells -- all sizes known at
-// compile time, so cell indices use constant divisors.  Levels >= 32 run on
-// the whole CTA (256 threads), levels <= 16 -- including the coarse sweeps --
-// on warp 0 alone.  Same arithmetic (fs_stencil.cuh) and order as the generic
-// kernel above.
-struct BottomH2 {
-  float h2[4];
-  float w;  // relaxation factor of every sweep
-};
-
-template <int N>
-constexpr int ilog2() {
-  return N <= 1 ? 0 : 1 + ilog2<N / 2>();
-}
-// levels and floats of the chain N0, N0/2, ..., NMIN
-template <int N0, int NMIN>
-constexpr int chain_levels() {
-  return N0 == NMIN ? 1 : 1 + chain_levels<N0 / 2, NMIN>();
-}
-template <int N0, int NMIN>
-constexpr int chain_floats() {
-  return N0 == NMIN ? N0 * N0 : N0 * N0 + chain_floats<N0 / 2, NMIN>();
-}
-
-constexpr int kBottomThreads = 256;  // threads of the bottom-chain kernels
-
-template <int N, bool WARP>
-__device__ __forceinline__ void p2_sync() {
-  if (WARP) __syncwarp();
-  else __syncthreads();
-}
-
-// The chain's loops run a compile-time number of cells per thread (the CTA
-// has kBottomThreads threads, warp 0 has 32), fully unrolled, every result of
-// a phase computed before any is stored: the cells a phase writes are not
-// read in that phase (a colour's cells read only the other colour; restrict
-// and prolong write the other level's array, or the cell itself), so the
-// loads of a thread's cells are in flight together instead of waiting on the
-// stores of the cells before them.  The levels are latency-bound, one phase
-// between two barriers after another.
-template <int N, bool WARP>
-__device__ __forceinline__ void p2_smooth(float* x, const float* r, float h2, int sweeps, float w) {
-  constexpr int HALF = N / 2, NT = WARP ? 32 : kBottomThreads;
-  constexpr int CELLS = N * HALF, PER = (CELLS + NT - 1) / NT;
-  const int tid = WARP ? (int)(threadIdx.x & 31) : (int)threadIdx.x;
-  // When the threads cover whole rows of a colour (NT a multiple of N/2)
-  // and step an even number of rows, a thread's cells share their column and
-  // its neighbours' offsets: rows j0, j0 + RS, ...; only the first and last
-  // rows of the level wrap vertically.
-  constexpr bool ROWS = NT % HALF == 0 && (NT / HALF) % 2 == 0 && CELLS % NT == 0;
-  if constexpr (ROWS) {
-    constexpr int RS = NT / HALF;
-    const int j0 = tid / HALF, m = tid - j0 * HALF;
-    for (int s = 0; s < 2 * sweeps; s++) {
-      const int i = 2 * m + ((j0 + (s & 1)) & 1);
-      const int dl = i == 0 ? N - 1 : -1, dr = i + 1 == N ? 1 - N : 1;
-      float nv[PER];
-#pragma unroll
-      for (int u = 0; u < PER; u++) {
-        const int j = j0 + u * RS, k = j * N + i;
-        const int db = j == 0 ? (N - 1) * N : -N, dt = j + 1 == N ? -(N - 1) * N : N;
-        nv[u] = gs_update(x[k], x[k + dl], x[k + dr], x[k + db], x[k + dt], r[k], h2, w);
-      }
-#pragma unroll
-      for (int u = 0; u < PER; u++) x[(j0 + u * RS) * N + i] = nv[u];
-      p2_sync<N, WARP>();
-    }
-  } else {
-    for (int s = 0; s < 2 * sweeps; s++) {
-      const int c = s & 1;
-      float nv[PER];
-      int kk[PER];
-#pragma unroll
-      for (int u = 0; u < PER; u++) {
-        const int idx = tid + u * NT;
-        kk[u] = -1;
-        if (CELLS % NT == 0 || idx < CELLS) {
-          const int j = idx / HALF, m = idx - j * HALF;
-          const int i = 2 * m + ((j + c) & 1);
-          const int row = j * N, k = row + i;
-          const int rm = (j == 0 ? N - 1 : j - 1) * N, rp = (j + 1 == N ? 0 : j + 1) * N;
-          const int im = i == 0 ? N - 1 : i - 1, ip = i + 1 == N ? 0 : i + 1;
-          kk[u] = k;
-          nv[u] = gs_update(x[k], x[row + im], x[row + ip], x[rm + i], x[rp + i], r[k], h2, w);
-        }
-      }
-#pragma unroll
-      for (int u = 0; u < PER; u++)
-        if (CELLS % NT == 0 || kk[u] >= 0) x[kk[u]] = nv[u];
-      p2_sync<N, WARP>();
-    }
-  }
-}
-
-// residual of level N restricted into (cr, cx = 0) of level N/2
-template <int N, bool WARP>
-__device__ __forceinline__ void p2_restrict(const float* x, const float* r, float h2, float* cr, float* cx) {
-  constexpr int NC = N / 2, NT = WARP ? 32 : kBottomThreads, PER = (NC * NC + NT - 1) / NT;
-  const int tid = WARP ? (int)(threadIdx.x & 31) : (int)threadIdx.x;
-  const float ih2 = inv_h2(h2);
-  float rv[PER];
-  // threads covering whole coarse rows: a thread's blocks share their two
-  // fine columns and the columns' neighbour offsets; only the level's first
-  // and last fine rows wrap
-  constexpr bool ROWS = NT % NC == 0 && (NC * NC) % NT == 0;
-  if constexpr (ROWS) {
-    constexpr int RS = NT / NC;
-    const int cj0 = tid / NC, ci = tid - cj0 * NC;
-    const int i0 = 2 * ci;
-    const int dl0 = i0 == 0 ? N - 1 : -1, dr1 = i0 + 2 == N ? 1 - N : 1;  // left of column i0, right of i0 + 1
-#pragma unroll
-    for (int u = 0; u < PER; u++) {
-      const int j = 2 * (cj0 + u * RS), k0 = j * N + i0, k1 = k0 + N;
-      const int db = j == 0 ? (N - 1) * N : -N, dt = j + 2 == N ? -(N - 1) * N : N;  // below row j, above row j + 1
-      const float r00 = residual_at(x[k0], x[k0 + dl0], x[k0 + 1], x[k0 + db], x[k1], r[k0], ih2);
-      const float r10 = residual_at(x[k0 + 1], x[k0], x[k0 + 1 + dr1], x[k0 + 1 + db], x[k1 + 1], r[k0 + 1], ih2);
-      const float r01 = residual_at(x[k1], x[k1 + dl0], x[k1 + 1], x[k0], x[k1 + dt], r[k1], ih2);
-      const float r11 = residual_at(x[k1 + 1], x[k1], x[k1 + 1 + dr1], x[k0 + 1], x[k1 + 1 + dt], r[k1 + 1], ih2);
-      rv[u] = restrict4(r00, r10, r01, r11);
-    }
-#pragma unroll
-    for (int u = 0; u < PER; u++) {
-      const int k = (cj0 + u * RS) * NC + ci;
-      cr[k] = rv[u];
-      cx[k] = 0.f;
-    }
-  } else {
-#pragma unroll
-    for (int u = 0; u < PER; u++) {
-      const int k = tid + u * NT;
-      if ((NC * NC) % NT != 0 && k >= NC * NC) break;
-      const int cj = k / NC, ci = k - cj * NC;
-      float r4[4];
-#pragma unroll
-      for (int q = 0; q < 4; q++) {
-        const int i = 2 * ci + (q & 1), j = 2 * cj + (q >> 1);
-        const int row = j * N;
-        const int rm = (j == 0 ? N - 1 : j - 1) * N, rp = (j + 1 == N ? 0 : j + 1) * N;
-        const int im = i == 0 ? N - 1 : i - 1, ip = i + 1 == N ? 0 : i + 1;
-        r4[q] = residual_at(x[row + i], x[row + im], x[row + ip], x[rm + i], x[rp + i], r[row + i], ih2);
-      }
-      rv[u] = restrict4(r4[0], r4[1], r4[2], r4[3]);
-    }
-#pragma unroll
-    for (int u = 0; u < PER; u++) {
-      const int k = tid + u * NT;
-      if ((NC * NC) % NT != 0 && k >= NC * NC) break;
-      cr[k] = rv[u];
-      cx[k] = 0.f;
-    }
-  }
-  p2_sync<N, WARP>();
-}
-
-// x (level N) += bilinear prolongation of c (level N/2)
-template <int N, bool WARP>
-__device__ __forceinline__ void p2_prolong(float* x, const float* c) {
-  constexpr int NC = N / 2, NT = WARP ? 32 : kBottomThreads, PER = (N * N + NT - 1) / NT;
-  const int tid = WARP ? (int)(threadIdx.x & 31) : (int)threadIdx.x;
-  float pv[PER];
-  // threads covering whole rows with an even row step: a thread's cells share
-  // their column, its coarse columns and both weights; only the first and
-  // last rows wrap to the other edge of the coarse level
-  constexpr bool ROWS = NT % N == 0 && (NT / N) % 2 == 0 && (N * N) % NT == 0;
-  if constexpr (ROWS) {
-    constexpr int RS = NT / N;
-    const int j0 = tid / N, i = tid - j0 * N;
-    const int ci0 = (i & 1) ? (i >> 1) : (i >> 1) - 1;
-    const float fx = (i & 1) ? 0.25f : 0.75f, fy = (j0 & 1) ? 0.25f : 0.75f;
-    const int x0 = ci0 < 0 ? ci0 + NC : ci0, x1 = ci0 + 1 >= NC ? ci0 + 1 - NC : ci0 + 1;
-#pragma unroll
-    for (int u = 0; u < PER; u++) {
-      const int j = j0 + u * RS, k = j * N + i;
-      const int cj0 = (j & 1) ? (j >> 1) : (j >> 1) - 1;
-      const int y0 = (cj0 < 0 ? cj0 + NC : cj0) * NC, y1 = (cj0 + 1 >= NC ? cj0 + 1 - NC : cj0 + 1) * NC;
-      pv[u] = __fadd_rn(x[k], prolong_val(c[y0 + x0], c[y0 + x1], c[y1 + x0], c[y1 + x1], fx, fy));
-    }
-#pragma unroll
-    for (int u = 0; u < PER; u++) x[(j0 + u * RS) * N + i] = pv[u];
-  } else {
-#pragma unroll
-    for (int u = 0; u < PER; u++) {
-      const int k = tid + u * NT;
-      if ((N * N) % NT != 0 && k >= N * N) break;
-      const int j = k / N, i = k - j * N;
-      const int ci0 = (i & 1) ? (i >> 1) : (i >> 1) - 1;
-      const int cj0 = (j & 1) ? (j >> 1) : (j >> 1) - 1;
-      const float fx = (i & 1) ? 0.25f : 0.75f, fy = (j & 1) ? 0.25f : 0.75f;
-      const int x0 = ci0 < 0 ? ci0 + NC : ci0, x1 = ci0 + 1 >= NC ? ci0 + 1 - NC : ci0 + 1;
-      const int y0 = (cj0 < 0 ? cj0 + NC : cj0) * NC, y1 = (cj0 + 1 >= NC ? cj0 + 1 - NC : cj0 + 1) * NC;
-      pv[u] = __fadd_rn(x[k], prolong_val(c[y0 + x0], c[y0 + x1], c[y1 + x0], c[y1 + x1], fx, fy));
-    }
-#pragma unroll
-    for (int u = 0; u < PER; u++) {
-      const int k = tid + u * NT;
-      if ((N * N) % NT != 0 && k >= N * N) break;
-      x[k] = pv[u];
-    }
-  }
-  p2_sync<N, WARP>();
-}
-
-// sub-cycle from level N (chain level LVL, at float offset OFF of the chain's
-// x and rhs arrays) down to NMIN and back; levels <= 16 are called by warp 0
-// only.  Every level's arrays are the shared arrays plus a compile-time
-// offset, so all accesses compile as shared-memory accesses.
-template <int N, int NMIN, int LVL, int OFF>
-__device__ __forceinline__ void p2_cycle(float* sx, float* sr, const BottomH2& H, int pre, int post, int coarse) {
-  constexpr bool W = N <= 16;
-  float* const x = sx + OFF;
-  float* const r = sr + OFF;
-  if constexpr (N == NMIN) {
-    p2_smooth<N, W>(x, r, H.h2[LVL], coarse, H.w);
-  } else {
-    static_assert(N % 2 == 0, "every level above the coarsest is even");
-    constexpr int OFFC = OFF + N * N;
-    p2_smooth<N, W>(x, r, H.h2[LVL], pre, H.w);
-    p2_restrict<N, W>(x, r, H.h2[LVL], sr + OFFC, sx + OFFC);
-    if constexpr (!W && N / 2 <= 16) {
-      if (threadIdx.x < 32) p2_cycle<N / 2, NMIN, LVL + 1, OFFC>(sx, sr, H, pre, post, coarse);
-      __syncthreads();
-    } else {
-      p2_cycle<N / 2, NMIN, LVL + 1, OFFC>(sx, sr, H, pre, post, coarse);
-    }
-    p2_prolong<N, W>(x, sx + OFFC);
-    p2_smooth<N, W>(x, r, H.h2[LVL], post, H.w);
-  }
-}
-
-template <int N0, int NMIN>
-__device__ __forceinline__ void mg_bottom_chain_body(const float* __restrict__ rhs_top, float* __restrict__ x_top,
-                                                     int has_x, const BottomH2& H, int pre, int post, int coarse,
-                                                     float* __restrict__ acc_h, float* __restrict__ acc_l) {
-  constexpr int L = chain_levels<N0, NMIN>();
-  constexpr int SZ = chain_floats<N0, NMIN>();
-  static_assert(L <= 4 && NMIN % 2 == 0, "chains of at most four even levels");
-  // the chain's levels one after another, level 0 first
-  __shared__ __align__(16) float sx[SZ];
-  __shared__ __align__(16) float sr[SZ];
-  const int tid = threadIdx.x;
-  // level 0's rhs (and iterate): 16-byte asynchronous copies, all in flight at
-  // once (N0 is even, so N0^2 is a multiple of 4; the level arrays are
-  // cudaMalloc'd, 256-byte aligned)
-  static_assert((N0 * N0) % 4 == 0, "whole 16-byte groups");
-  for (int k = tid; k < N0 * N0 / 4; k += blockDim.x) {
-    cp_async16(sr + 4 * k, rhs_top + 4 * k);
-    if (has_x) cp_async16(sx + 4 * k, x_top + 4 * k);
-    else reinterpret_cast<float4*>(sx)[k] = make_float4(0.f, 0.f, 0.f, 0.f);
-  }
-  cp_async_wait_all();
-  __syncthreads();
-  if constexpr (N0 <= 16) {
-    if (tid < 32) p2_cycle<N0, NMIN, 0, 0>(sx, sr, H, pre, post, coarse);
-    __syncthreads();
-  } else {
-    p2_cycle<N0, NMIN, 0, 0>(sx, sr, H, pre, post, coarse);
-  }
-  for (int k = tid; k < N0 * N0; k += blockDim.x) {
-    float e = sx[k];
-    if (acc_h) {
-      df p = df_add_f(df{acc_h[k], acc_l[k]}, e);
-      acc_h[k] = p.hi;
-      acc_l[k] = p.lo;
-    } else {
-      x_top[k] = e;
-    }
-  }
-}
-
-template <int N0, int NMIN>
-__global__ void __launch_bounds__(kBottomThreads) k_mg_bottom_chain(const float* __restrict__ rhs_top,
-                                                         float* __restrict__ x_top, int has_x, BottomH2 H, int pre,
-                                                         int post, int coarse, float* __restrict__ acc_h,
-                                                         float* __restrict__ acc_l) {
-  mg_bottom_chain_body<N0, NMIN>(rhs_top, x_top, has_x, H, pre, post, coarse, acc_h, acc_l);
-}
-
 // ------------------------------------------------- batched (one size class)
 // The members of a batch with the same grid and multigrid settings run each
 // kernel of their refinement cycles as one launch, member = blockIdx.z, with
@@ -1128,16 +663,6 @@ struct UpTab {
   } m[kClassMax];
 };
 static_assert(sizeof(UpTab) + 64 <= 32764, "kernel parameter limit");
-struct BottomTab {
-  struct {
-    const float* rhs;
-    float* x;
-    float* acc_h;
-    float* acc_l;
-    const DevState* st;
-  } m[kClassMax];
-};
-
 template <int T, int H>
 __global__ void __launch_bounds__(256) k_mg_down_class(const __grid_constant__ DownTab tab, int n, float h2,
                                                        int pre, float w, int max_cycles) {
@@ -1157,21 +682,6 @@ __global__ void __launch_bounds__(256) k_mg_up_class(const __grid_constant__ UpT
   const CUtensorMap* tm = tab.tm[blockIdx.z];
   mg_up_body<T, H, ACC>(tile_smem(tile_dyn), a.rhs, a.xin, a.xout, a.xc, n, h2, post, a.ph, a.pl, w, &tm[0], &tm[1],
                         &tm[2], a.tma, &a.st->async_err);
-}
-
-template <int N0, int NMIN>
-__global__ void __launch_bounds__(kBottomThreads) k_mg_bottom_chain_class(const BottomTab tab, BottomH2 H, int pre, int post,
-                                                               int coarse, int max_cycles) {
-  const auto& a = tab.m[blockIdx.z];
-  if (!member_active(a.st, max_cycles)) return;
-  mg_bottom_chain_body<N0, NMIN>(a.rhs, a.x, 0, H, pre, post, coarse, a.acc_h, a.acc_l);
-}
-
-__global__ void __launch_bounds__(1024) k_mg_bottom_class(const BottomTab tab, BottomLevels L, int pre, int post,
-                                                          int coarse, int max_cycles) {
-  const auto& a = tab.m[blockIdx.z];
-  if (!member_active(a.st, max_cycles)) return;
-  mg_bottom_body(a.rhs, a.x, 0, L, pre, post, coarse, a.acc_h, a.acc_l);
 }
 
 // ------------------------------------------------------------------ host
@@ -1318,14 +828,6 @@ static void up(Solver* s, Level& L, const Level& C, float* acc_h, float* acc_l, 
   }
 }
 
-// first level of the bottom solve: every level from there down is <= 64
-int bottom_first_level(const Solver* s) {
-  int nl = (int)s->lev.size();
-  int lb = nl - 1;
-  while (lb > 0 && s->lev[lb - 1].n <= 64 && nl - (lb - 1) <= 8) lb--;
-  return lb;
-}
-
 // the fused cycle needs even tile levels, a bottom of <= 8 levels each <= 64,
 // and 1 <= pre, post <= 3
 bool mg_fused_supported(const Solver* s) {
@@ -1338,46 +840,6 @@ bool mg_fused_supported(const Solver* s) {
   for (size_t l = lb; l < s->lev.size(); l++)
     if (s->lev[l].n > 64) return false;
   return true;
-}
-
-static size_t bottom_layout(const Solver* s, BottomLevels* B) {
-  int lb = bottom_first_level(s);
-  int nl = (int)s->lev.size();
-  B->count = nl - lb;
-  B->w = (float)s->prm.relax;
-  int off = 0;
-  for (int k = 0; k < B->count; k++) {
-    const Level& L = s->lev[lb + k];
-    int m = L.n * L.n;
-    B->n[k] = L.n;
-    B->h2[k] = L.h2;
-    B->off_x[k] = off; off += m;
-    B->off_r[k] = off; off += m;
-    if (L.n & 1) { B->off_x2[k] = off; off += m; }
-    else B->off_x2[k] = -1;
-  }
-  // levels <= 64 hold at most 2 * (64^2 + 32^2 + ...) + 15^2 floats < 48 KB
-  return (size_t)off * sizeof(float);
-}
-
-// The compile-time chain kernel for the bottom levels from lb, identified by
-// its first size (64, 32, 16, 8 down to 8; 48, 24, 12 down to 12), or 0 when
-// the levels form another chain (odd sizes, other coarsest sizes).
-static int bottom_chain(const Solver* s, int lb) {
-  const std::vector<Level>& L = s->lev;
-  for (size_t k = lb; k + 1 < L.size(); k++)
-    if ((L[k].n & 1) || L[k + 1].n * 2 != L[k].n) return 0;
-  const int nb = L[lb].n, nmin = L.back().n;
-  if (nmin == 8 && (nb == 64 || nb == 32 || nb == 16 || nb == 8)) return nb;
-  if (nmin == 12 && (nb == 48 || nb == 24 || nb == 12)) return nb;
-  return 0;
-}
-
-static BottomH2 bottom_h2(const Solver* s, int lb) {
-  BottomH2 H{};
-  for (int k = 0; k < (int)s->lev.size() - lb && k < 4; k++) H.h2[k] = s->lev[lb + k].h2;
-  H.w = (float)s->prm.relax;
-  return H;
 }
 
 void mg_vcycle_fused(Solver* s, bool first_has_x, float* acc_h, float* acc_l) {
@@ -1406,38 +868,10 @@ void mg_vcycle_fused(Solver* s, bool first_has_x, float* acc_h, float* acc_l) {
       default: down<7>(s, L[l], L[l + 1], hx, f, cyc, xu); break;
     }
   }
-  int nb = L[lb].n;
-  bool hx = lb == 0 && first_has_x;
+  const bool hx = lb == 0 && first_has_x;
   float* bah = lb == 0 ? acc_h : nullptr;
   float* bal = lb == 0 ? acc_l : nullptr;
-  double bytes = (double)nb * nb * (hx ? 12.0 : 8.0);
-  // a chain of levels known at compile time: the specialised kernel
-  const int chain = bottom_chain(s, lb);
-  if (chain) {
-    const BottomH2 H = bottom_h2(s, lb);
-#define FS_CHAIN(N0, NM)                                                                                     \
-  FS_LAUNCH(s, "mg_bottom", bytes,                                                                           \
-            k_mg_bottom_chain<N0, NM><<<1, kBottomThreads, 0, s->stream>>>(L[lb].rhs, L[lb].x, hx ? 1 : 0, H,            \
-                                                                 P.mg_pre_smooth, P.mg_post_smooth,            \
-                                                                 P.mg_coarse_sweeps, bah, bal))
-    switch (chain) {
-      case 64: FS_CHAIN(64, 8); break;
-      case 32: FS_CHAIN(32, 8); break;
-      case 16: FS_CHAIN(16, 8); break;
-      case 8: FS_CHAIN(8, 8); break;
-      case 48: FS_CHAIN(48, 12); break;
-      case 24: FS_CHAIN(24, 12); break;
-      default: FS_CHAIN(12, 12); break;
-    }
-#undef FS_CHAIN
-  } else {
-    BottomLevels B;
-    size_t smem = bottom_layout(s, &B);
-    int threads = std::min(1024, std::max(32, ((nb * nb / 4 + 31) / 32) * 32));
-    FS_LAUNCH(s, "mg_bottom", bytes,
-              k_mg_bottom<<<1, threads, smem, s->stream>>>(L[lb].rhs, L[lb].x, hx ? 1 : 0, B, P.mg_pre_smooth,
-                                                           P.mg_post_smooth, P.mg_coarse_sweeps, bah, bal));
-  }
+  launch_bottom(s, lb, hx, bah, bal);
   for (int l = lb - 1; l >= 0; l--) {
     float* ah = l == 0 ? acc_h : nullptr;
     float* al = l == 0 ? acc_l : nullptr;
@@ -1564,36 +998,7 @@ int mg_vcycle_class(Solver* const* ms, int count, cudaStream_t st) {
       default: down_class<7>(ms, count, l, st); break;
     }
   }
-  const int nb = L[lb].n;
-  BottomTab tab{};
-  for (int i = 0; i < count; i++) {
-    Solver* s = ms[i];
-    tab.m[i] = {s->lev[lb].rhs, s->lev[lb].x, lb == 0 ? s->ph : nullptr, lb == 0 ? s->pl : nullptr, s->dev};
-  }
-  const int chain = bottom_chain(s0, lb);
-  if (chain) {
-    const BottomH2 H = bottom_h2(s0, lb);
-    const dim3 grid(1, 1, count);
-#define FS_CHAIN(N0, NM)                                                                                        \
-  k_mg_bottom_chain_class<N0, NM><<<grid, kBottomThreads, 0, st>>>(tab, H, P.mg_pre_smooth, P.mg_post_smooth,             \
-                                                         P.mg_coarse_sweeps, P.max_cycles)
-    switch (chain) {
-      case 64: FS_CHAIN(64, 8); break;
-      case 32: FS_CHAIN(32, 8); break;
-      case 16: FS_CHAIN(16, 8); break;
-      case 8: FS_CHAIN(8, 8); break;
-      case 48: FS_CHAIN(48, 12); break;
-      case 24: FS_CHAIN(24, 12); break;
-      default: FS_CHAIN(12, 12); break;
-    }
-#undef FS_CHAIN
-  } else {
-    BottomLevels B;
-    const size_t smem = bottom_layout(s0, &B);
-    const int threads = std::min(1024, std::max(32, ((nb * nb / 4 + 31) / 32) * 32));
-    k_mg_bottom_class<<<dim3(1, 1, count), threads, smem, st>>>(tab, B, P.mg_pre_smooth, P.mg_post_smooth,
-                                                                 P.mg_coarse_sweeps, P.max_cycles);
-  }
+  launch_bottom_class(ms, count, lb, st);
   launches++;
   for (int l = lb - 1; l >= 0; l--, launches++) {
     switch (P.mg_post_smooth) {
