@@ -38,6 +38,7 @@
 #include "fs_internal.cuh"
 #include "fs_reduce.cuh"
 #include "fs_tc.cuh"
+#include "fs_wgrad.cuh"
 
 namespace fs {
 namespace conv {
@@ -299,260 +300,6 @@ __global__ void k_loss_seed(const float* __restrict__ out, const float* __restri
   }
 }
 
-// ------------------------------------------ weight gradients on tcgen05
-// dW[co][ci][tap] = sum_p G[p][co] X[p + s_tap][ci] as a GEMM with K = pixels:
-// D[m][n] += sum_k A[m][k] B[n][k], rows m = tap * CIN + ci of the shifted
-// input X (A), n = co of the output gradient G (B), accumulated in TMEM over
-// every pixel a CTA visits.  Rows are packed nine taps deep, so M-blocks of
-// 128 rows cover 9 CIN rows (two blocks for 16 input channels, nine for 128);
-// a CTA owns NMB consecutive M-blocks (blockIdx.y picks the group) so that
-// its accumulators fit the 512 TMEM columns.  Both operands are NHWC bf16 in
-// global memory (channels contiguous); the CTA stages them K-major (pixels
-// contiguous per row) by transposing blocks of 8 pixels x 8 channels in
-// registers, into the no-swizzle core-matrix layout of fs_tc_gemm_check with
-// the 8-row groups 272 bytes apart (LBO 128, SBO 272): the 16 bytes of
-// padding per group put neighbouring threads' blocks 16 bytes apart modulo
-// 128, so the eight threads of one 128-bit store phase write eight different
-// bank quads (with SBO 256 every block starts on the same banks).  Per-CTA
-// partial sums (and the bias sums of G, by the CTAs of blockIdx.y == 0) go to
-// global memory; k_wgrad_reduce adds them in a fixed order, so the gradient
-// is deterministic.
-constexpr int kWgThreads = 512;  // 16 warps: staging parallelism (one CTA per SM by shared memory)
-constexpr int kWgTile = 128;  // pixels per K tile
-constexpr int kWgSBO = 272;   // bytes between consecutive 8-row groups of a staged operand
-
-template <int CIN, int COUT, int NMB>
-struct WgCfg {
-  static constexpr int MROWS = 9 * CIN;                    // rows of D
-  static constexpr int MBLK = (MROWS + 127) / 128;         // M-blocks in all
-  static constexpr int A_STEP = 16 * kWgSBO;               // one K step (16 pixels) of an M-block
-  static constexpr int A_MB = (kWgTile / 16) * A_STEP;      // one M-block
-  static constexpr int A_BYTES = NMB * A_MB;                // this CTA's A operand
-  static constexpr int B_STEP = (COUT / 8) * kWgSBO;
-  static constexpr int B_BYTES = (kWgTile / 16) * B_STEP;
-  static constexpr int R_BYTES = 3 * (kWgTile + 2) * (CIN / 8) * 16;  // three input rows of the tile, halo 1
-  static constexpr int GR_BYTES = kWgTile * (COUT / 8) * 16;          // the tile's output-gradient row
-  static constexpr int SMEM = A_BYTES + B_BYTES + R_BYTES + GR_BYTES + 128;  // + barrier, TMEM slot, flag
-  // row groups (tap, chunk) this CTA stages each tile; the rest of its M-blocks are zero padding
-  static constexpr int real_groups(int mb0) {
-    return 9 * (CIN / 8) - mb0 * 16 < NMB * 16 ? (9 * (CIN / 8) - mb0 * 16 > 0 ? 9 * (CIN / 8) - mb0 * 16 : 0)
-                                               : NMB * 16;
-  }
-  static constexpr int NCOL_USED = NMB * COUT;
-  static constexpr int NCOL = NCOL_USED <= 32    ? 32
-                              : NCOL_USED <= 64  ? 64
-                              : NCOL_USED <= 128 ? 128
-                              : NCOL_USED <= 256 ? 256
-                                                 : 512;
-  static_assert(NCOL_USED <= 512 && COUT % 16 == 0 && CIN % 8 == 0, "TMEM columns, channel counts");
-  static_assert(A_BYTES + B_BYTES + 3 * (kWgTile + 2) * (CIN / 8) * 16 + kWgTile * (COUT / 8) * 16 + 128 <= 227 * 1024,
-                "shared memory of one CTA");
-};
-
-// 8 rows of 8 bf16 (r[i] = pixel i, channels 0..7) -> t[c] = channel c, pixels 0..7
-__device__ __forceinline__ void transpose8x8(const uint4* r, uint4* t) {
-  const uint32_t* w = reinterpret_cast<const uint32_t*>(r);  // w[4 i + j]: pixel i, channels 2j, 2j+1
-  uint32_t* o = reinterpret_cast<uint32_t*>(t);               // o[4 c + j']: channel c, pixels 2j', 2j'+1
-#pragma unroll
-  for (int j = 0; j < 4; j++)
-#pragma unroll
-    for (int jp = 0; jp < 4; jp++) {
-      const uint32_t a = w[4 * (2 * jp) + j], b = w[4 * (2 * jp + 1) + j];
-      o[4 * (2 * j) + jp] = __byte_perm(a, b, 0x5410);
-      o[4 * (2 * j + 1) + jp] = __byte_perm(a, b, 0x7632);
-    }
-}
-
-// byte offset of the 8x8 block (rows 8g.., pixels 8q..) of a staged operand of R rows
-__device__ __forceinline__ int kmaj_block(int R, int g, int q) {
-  return (q >> 1) * ((R / 8) * kWgSBO) + g * kWgSBO + (q & 1) * 128;
-}
-
-// A tile is a segment of up to 128 pixels of one image row; its three input
-// rows (y - 1 .. y + 1, x0 - 1 .. x0 + 128, wrapped) are staged once with
-// coalesced loads, and the nine taps' shifted operands are transposed out of
-// that copy.  The next tile's rows are loaded while the previous tile's MMAs
-// run (the row copy is not an MMA operand).
-template <int CIN, int COUT, int NMB>
-__global__ void __launch_bounds__(kWgThreads) k_wgrad_tc(const uint4* __restrict__ X, const uint4* __restrict__ G,
-                                                         int B, int H, int W, float* __restrict__ part,
-                                                         float* __restrict__ bpart, int* __restrict__ err) {
-  using C = WgCfg<CIN, COUT, NMB>;
-  extern __shared__ __align__(128) unsigned char smem[];
-  unsigned char* sa = smem;
-  unsigned char* sb = smem + C::A_BYTES;
-  uint4* xr = reinterpret_cast<uint4*>(smem + C::A_BYTES + C::B_BYTES);  // [3][kWgTile + 2][KC]
-  uint4* gr = reinterpret_cast<uint4*>(smem + C::A_BYTES + C::B_BYTES + C::R_BYTES);  // [kWgTile][OC]
-  uint64_t* bar = reinterpret_cast<uint64_t*>(smem + C::A_BYTES + C::B_BYTES + C::R_BYTES + C::GR_BYTES);
-  uint32_t* tslot = reinterpret_cast<uint32_t*>(bar + 1);
-  int* failed = reinterpret_cast<int*>(bar + 2);
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int mb0 = blockIdx.y * NMB;  // first M-block of this CTA
-  const int ntx = (W + kWgTile - 1) / kWgTile;
-  const int64_t ntiles = (int64_t)B * H * ntx;
-  constexpr int KC = CIN / 8, OC = COUT / 8, RW = kWgTile + 2;
-  if (warp == 0) {
-    tc::tmem_alloc(tslot, C::NCOL);
-    tc::tmem_relinquish();
-    tc::fence_before_sync();
-  }
-  if (tid == 0) {
-    tc::mbar_init(bar, 1);
-    tc::mbar_fence_init();
-    *failed = 0;
-  }
-  __syncthreads();
-  tc::fence_after_sync();
-  const uint32_t taddr = *tslot;
-  const uint32_t sa_s = tc::smem_u32(sa), sb_s = tc::smem_u32(sb);
-  constexpr uint32_t IDESC = tc::idesc_bf16(128, COUT);
-  float bsum = 0.f;  // bias partial of output channel tid (tid < COUT, blockIdx.y == 0)
-  uint32_t phase = 0;
-  int issued = 0;
-  // the padding row groups of the last M-block are zero for every tile: written once
-  const int nreal = C::real_groups(mb0);
-  for (int k = tid; k < (kWgTile / 8) * (NMB * 16 - nreal); k += kWgThreads) {
-    const int q = k / (NMB * 16 - nreal), gl = nreal + (k - q * (NMB * 16 - nreal));
-    uint4* dst = reinterpret_cast<uint4*>(sa + (gl >> 4) * C::A_MB + kmaj_block(128, gl & 15, q));
-#pragma unroll
-    for (int c = 0; c < 8; c++) dst[c] = make_uint4(0, 0, 0, 0);
-  }
-  for (int64_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
-    const int xt = (int)(t % ntx);
-    const int64_t by = t / ntx;  // b * H + y
-    const int y = (int)(by % H);
-    const int64_t b = by / H;
-    const int x0 = xt * kWgTile;
-    // the tile's three input rows (the previous tile's transposes, the only
-    // readers, finished before the __syncthreads ahead of its MMAs)
-    for (int k = tid; k < 3 * RW * KC; k += kWgThreads) {
-      const int rc = k / KC, kc = k - rc * KC, r = rc / RW, c = rc - r * RW;
-      int gy = y - 1 + r, gx = x0 - 1 + c;
-      gy = gy < 0 ? gy + H : (gy >= H ? gy - H : gy);
-      gx = ((gx % W) + W) % W;
-      xr[k] = X[((b * H + gy) * W + gx) * KC + kc];
-    }
-    // and its output-gradient row (zero beyond the row's end)
-    for (int k = tid; k < kWgTile * OC; k += kWgThreads) {
-      const int x = x0 + k / OC;
-      gr[k] = x < W ? G[(by * W + x0) * OC + k] : make_uint4(0, 0, 0, 0);
-    }
-    if (issued) {
-      // the MMAs of the previous tile read the operand buffers
-      if (tid == 0 && !tc::mbar_wait(bar, phase)) *failed = 1;
-      phase ^= 1;
-    }
-    __syncthreads();
-    if (*failed) break;
-    // B: G[p][co] -> rows co, K = pixels, from the staged row
-    for (int k = tid; k < (kWgTile / 8) * OC; k += kWgThreads) {
-      const int q = k / OC, oc = k - q * OC;
-      uint4 r[8];
-#pragma unroll
-      for (int i = 0; i < 8; i++) r[i] = gr[(8 * q + i) * OC + oc];
-      uint4 tt[8];
-      transpose8x8(r, tt);
-      uint4* dst = reinterpret_cast<uint4*>(sb + kmaj_block(COUT, oc, q));
-#pragma unroll
-      for (int c = 0; c < 8; c++) dst[c] = tt[c];
-    }
-    // A: for each row group (tap, input chunk) of this CTA's M-blocks, the
-    // staged rows at the tap's shift -> rows ci, K = pixels; padding groups zero
-    for (int k = tid; k < (kWgTile / 8) * nreal; k += kWgThreads) {
-      const int q = k / nreal, gl = k - q * nreal;
-      const int gg = mb0 * 16 + gl;  // global row group, < 9 KC
-      const int tap = gg / KC, kc = gg - tap * KC;
-      const uint4* src = xr + ((tap / 3) * RW + 8 * q + (tap % 3)) * KC + kc;
-      uint4 r[8];
-#pragma unroll
-      for (int i = 0; i < 8; i++) r[i] = src[i * KC];
-      uint4 tt[8];
-      transpose8x8(r, tt);
-      const int blk = gl >> 4, g = gl & 15;  // M-block of this CTA, row group in it
-      uint4* dst = reinterpret_cast<uint4*>(sa + blk * C::A_MB + kmaj_block(128, g, q));
-#pragma unroll
-      for (int c = 0; c < 8; c++) dst[c] = tt[c];
-    }
-    tc::fence_async_smem();
-    __syncthreads();
-    tc::fence_after_sync();
-    if (tid == 0) {
-#pragma unroll 1
-      for (int j = 0; j < NMB; j++)
-#pragma unroll
-        for (int s = 0; s < kWgTile / 16; s++)
-          tc::mma_bf16(taddr + j * COUT, tc::sdesc(sa_s + j * C::A_MB + s * C::A_STEP, 128, kWgSBO),
-                       tc::sdesc(sb_s + s * C::B_STEP, 128, kWgSBO), IDESC, (issued || s > 0) ? 1u : 0u);
-      tc::mma_commit(bar);
-    }
-    issued = 1;
-    // bias partial: output channel tid sums its staged row (read only, like the MMAs)
-    if (blockIdx.y == 0 && tid < COUT) {
-#pragma unroll 4
-      for (int q = 0; q < kWgTile / 8; q++) {
-        const uint4 v = *reinterpret_cast<const uint4*>(sb + kmaj_block(COUT, tid >> 3, q) + (tid & 7) * 16);
-        const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&v);
-#pragma unroll
-        for (int e = 0; e < 4; e++) {
-          const float2 f = __bfloat1622float2(h[e]);
-          bsum += f.x + f.y;
-        }
-      }
-    }
-  }
-  if (tid == 0 && issued) {
-    if (!*failed) {
-      if (!tc::mbar_wait(bar, phase)) *failed = 1;
-    } else {
-      tc::mbar_wait(bar, phase, 1u << 20);  // let what was issued drain before the TMEM is released
-    }
-  }
-  if (tid == 0 && *failed) atomicExch(err, 1);
-  __syncthreads();
-  tc::fence_after_sync();
-  const int64_t cta = blockIdx.x;
-  if (!*failed) {
-    // warp w reads TMEM lanes 32 (w % 4) ..; the four warp groups share the
-    // (M-block, 16-column) chunks
-    const int m = 32 * (warp & 3) + lane, grp = warp >> 2;
-#pragma unroll 1
-    for (int jc = grp; jc < NMB * (COUT / 16); jc += kWgThreads / 128) {
-      const int j = jc / (COUT / 16), c0 = (jc - j * (COUT / 16)) * 16;
-      const int row = (mb0 + j) * 128 + m;
-      float v[16];
-      tc::tmem_ld16(taddr + ((uint32_t)(32 * (warp & 3)) << 16) + j * COUT + c0, v);
-      if (row < C::MROWS) {
-        float* dst = part + (cta * C::MROWS + row) * COUT + c0;
-#pragma unroll
-        for (int k = 0; k < 16; k++) dst[k] = issued ? v[k] : 0.f;
-      }
-    }
-    if (blockIdx.y == 0 && tid < COUT) bpart[cta * COUT + tid] = bsum;
-  }
-  tc::fence_before_sync();
-  __syncthreads();
-  if (warp == 0) tc::tmem_dealloc(taddr, C::NCOL);
-}
-
-// grad[off_w + OIHW] = sum over the P partials of row tap * cin + ci, column
-// co; grad[off_b + co] = sum of the bias partials
-__global__ void k_wgrad_reduce(const float* __restrict__ part, const float* __restrict__ bpart, int P, int cin,
-                               int cout, float* __restrict__ gw, float* __restrict__ gb) {
-  const int64_t mrows = 9 * (int64_t)cin, nw = mrows * cout;
-  GRID_STRIDE(e, nw + cout) {
-    float s = 0.f;
-    if (e < nw) {
-      for (int p = 0; p < P; p++) s += part[(int64_t)p * nw + e];
-      const int row = (int)(e / cout), co = (int)(e % cout), tap = row / cin, ci = row % cin;
-      gw[((int64_t)co * cin + ci) * 9 + tap] = s;
-    } else {
-      const int co = (int)(e - nw);
-      for (int p = 0; p < P; p++) s += bpart[(int64_t)p * cout + co];
-      gb[co] = s;
-    }
-  }
-}
-
 // ------------------------------------------------------------ parameters
 struct PackTable {
   int64_t off_w[NL], off_pk[NL];
@@ -721,46 +468,50 @@ static cudaError_t ensure_corr(Net* g, int64_t floats) {
   return cudaSuccess;
 }
 
-template <int CIN, int COUT, int NMB>
+template <int CIN, int COUT, int TY, int PX, int NDX>
 static cudaError_t wgrad_tc(const Ctx& c, int l, Buf xbuf, Buf gbuf, int B, int H, int W) {
-  using C = WgCfg<CIN, COUT, NMB>;
+  using C = WgCfg<CIN, COUT, TY, PX, NDX>;
   Net* g = c.g;
+  auto* kernel = k_wgrad_tc<CIN, COUT, TY, PX, NDX>;
   static std::atomic<uint64_t> attr{0};
   const uint64_t bit = 1ull << (g->device & 63);
   if (!(attr.load() & bit)) {
-    CK(cudaFuncSetAttribute(k_wgrad_tc<CIN, COUT, NMB>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM));
+    CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM));
     attr.fetch_or(bit);
   }
-  const int groups = (C::MBLK + NMB - 1) / NMB;
-  const int64_t ntiles = (int64_t)B * H * ((W + kWgTile - 1) / kWgTile);
-  const int P = (int)std::max<int64_t>(1, std::min<int64_t>(ntiles, 4 * 152 / groups));
+  // one wave: as many CTAs as the shared memory lets an SM hold, over the taps' groups
+  constexpr int per_sm = C::SMEM <= 110 * 1024 ? 2 : 1;
+  const int64_t ntiles = (int64_t)B * ((H + TY - 1) / TY) * ((W + PX - 1) / PX);
+  const int P = (int)std::max<int64_t>(1, std::min<int64_t>(ntiles, per_sm * 152 * NDX / 3));
   const int64_t nw = (int64_t)C::MROWS * COUT;
   CK(ensure_corr(g, (int64_t)P * (nw + COUT)));
   float* part = g->corr_part;
   float* bpart = part + (int64_t)P * nw;
   GL(c, "guess_wgrad", (double)(CIN + COUT) * 2 * B * H * W,
-     (k_wgrad_tc<CIN, COUT, NMB><<<dim3(P, groups), kWgThreads, C::SMEM, c.st>>>(
+     (kernel<<<dim3(P, 3 / NDX), kWgThreads + 32, C::SMEM, c.st>>>(
          reinterpret_cast<const uint4*>(g->buf[xbuf]), reinterpret_cast<const uint4*>(g->buf[gbuf]), B, H, W, part,
          bpart, g->err)));
   CK(cudaGetLastError());
   GL(c, "guess_wgrad_reduce", (double)P * (nw + COUT) * 4,
-     k_wgrad_reduce<<<blocks_for(nw + COUT), 256, 0, c.st>>>(part, bpart, P, CIN, COUT, g->grad + g->off_w[l],
-                                                            g->grad + g->off_b[l]));
+     k_wgrad_reduce<<<(int)((nw + COUT + 31) / 32), 256, 0, c.st>>>(part, bpart, P, CIN, COUT, g->grad + g->off_w[l],
+                                                                   g->grad + g->off_b[l]));
   return cudaGetLastError();
 }
 
-// the (c_in, c_out) pairs of the network, M-blocks per CTA
+// the (c_in, c_out) pairs of the network: rows and pixels of a tile (two stages
+// in shared memory, two CTAs an SM at the wide levels), horizontal taps per CTA
+// (one where three would not fit the 512 TMEM columns)
 static cudaError_t wgrad(const Ctx& c, int l, Buf xbuf, Buf gbuf, int B, int H, int W) {
   const int ci = kCI[l], co = kCO[l];
-#define FS_WG(a, b, nmb) \
-  if (ci == a && co == b) return wgrad_tc<a, b, nmb>(c, l, xbuf, gbuf, B, H, W);
-  FS_WG(16, 16, 2)
-  FS_WG(16, 32, 2)
-  FS_WG(32, 16, 3)
-  FS_WG(32, 64, 3)
-  FS_WG(64, 128, 3)
-  FS_WG(128, 64, 2)
-  FS_WG(64, 32, 3)
+#define FS_WG(a, b, ty, px, ndx) \
+  if (ci == a && co == b) return wgrad_tc<a, b, ty, px, ndx>(c, l, xbuf, gbuf, B, H, W);
+  FS_WG(16, 16, 4, 128, 3)
+  FS_WG(16, 32, 2, 128, 3)
+  FS_WG(32, 16, 2, 128, 3)
+  FS_WG(32, 64, 1, 128, 3)
+  FS_WG(64, 128, 1, 128, 1)
+  FS_WG(128, 64, 1, 64, 1)
+  FS_WG(64, 32, 1, 128, 3)
 #undef FS_WG
   return cudaErrorInvalidValue;
 }

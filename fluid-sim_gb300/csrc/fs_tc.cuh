@@ -3,7 +3,8 @@
 // described by shared-memory matrix descriptors, completion tracked by an
 // mbarrier, and every wait bounded.
 //
-// Layout used for both operands ("K-major, no swizzle"): the operand is a grid
+// Layout used for both operands ("K-major, no swizzle"; for the MN-major form see
+// idesc_bf16_mn): the operand is a grid
 // of core matrices of 8 rows x 16 bytes (8 bf16 along K), each stored as 128
 // contiguous bytes.  LBO is the byte distance between the two core matrices
 // that one K=16 MMA step reads along K; SBO is the distance between
@@ -41,6 +42,9 @@ __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
 }
 __device__ __forceinline__ void mbar_fence_init() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
 // non-blocking probe: has the phase of the given parity completed?
 __device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
   uint32_t ok;
@@ -95,6 +99,14 @@ __host__ __device__ constexpr uint32_t idesc_bf16(int M, int N) {
          | (1u << 10)                 // B format bf16
          | ((uint32_t)(N >> 3) << 17)  // N / 8
          | ((uint32_t)(M >> 4) << 24);  // M / 16
+}
+
+// The same with both operands MN-major: the 8 elements of a core matrix's 16-byte
+// row lie along M (N), its 8 rows along K; LBO is the distance between the
+// step's two core matrices along K, SBO between groups of 8 along M (N).  M = 64
+// leaves row m of D in lane 32 (m / 16) + m % 16.
+__host__ __device__ constexpr uint32_t idesc_bf16_mn(int M, int N) {
+  return idesc_bf16(M, N) | (1u << 15) | (1u << 16);
 }
 
 // D[tmem] (+)= A * B^T, issued by one thread
