@@ -34,18 +34,12 @@
 #include <vector>
 
 #include "../../include/fluid.h"
+#include "fs_conv.cuh"
 #include "fs_df.cuh"
 #include "fs_internal.cuh"
 #include "fs_reduce.cuh"
 #include "fs_tc.cuh"
 #include "fs_wgrad.cuh"
-
-namespace fs {
-namespace conv {
-cudaError_t conv3x3(int cin, int cout, int epi, const void* in, const void* w, const float* bias, void* out, int B,
-                    int H, int W, int* err, cudaStream_t st);
-}
-}  // namespace fs
 
 struct fs_guess;
 
@@ -62,13 +56,13 @@ enum { LA, LB, LC, LD, LE, LF, LG, LH, LI, LJ };
 // activation / gradient buffers: (level, channels)
 enum Buf {
   X0, A0, A0B, Q1, A1, Q2, A2, Q3, A3, F3, S2, G2, S1, H1, S0, I0,  // forward
-  GJ, DI0, DS0, DH1, DS1, DG2, DS2, DF3, DA3, DQ3, DQ2, DQ1, DA0,   // backward
+  GJ, DI0, DS0, DH1, DS1, DG2, DS2, DF3, DA3, DA0,  // backward
   NBUF
 };
 constexpr int kBufLevel[NBUF] = {0, 0, 0, 1, 1, 2, 2, 3, 3, 3, 2, 2, 1, 1, 0, 0,
-                                 0, 0, 0, 1, 1, 2, 2, 3, 3, 3, 2, 1, 0};
+                                 0, 0, 0, 1, 1, 2, 2, 3, 3, 0};
 constexpr int kBufCh[NBUF] = {16, 16, 16, 16, 32, 32, 64, 64, 128, 64, 64, 32, 32, 16, 16, 16,
-                              16, 16, 16, 16, 32, 32, 64, 64, 128, 64, 32, 16, 16};
+                              16, 16, 16, 16, 32, 32, 64, 64, 128, 16};
 
 
 struct Net {
@@ -100,15 +94,6 @@ static int64_t level_pixels(const Net* g, int B, int H, int W, int lev) {
 }
 
 // ------------------------------------------------------------ small kernels
-__device__ __forceinline__ void unpack8(uint4 q, float* f) {
-  const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&q);
-#pragma unroll
-  for (int k = 0; k < 4; k++) {
-    float2 t = __bfloat1622float2(h[k]);
-    f[2 * k] = t.x;
-    f[2 * k + 1] = t.y;
-  }
-}
 __device__ __forceinline__ uint4 pack8(const float* f) {
   uint4 q;
   __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&q);
@@ -120,73 +105,6 @@ __device__ __forceinline__ uint4 pack8(const float* f) {
 #define GRID_STRIDE(k, n) for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < (n); k += (int64_t)gridDim.x * blockDim.x)
 // element loops of the network's buffers (all below 2^31 elements, checked on the host)
 #define GRID_STRIDE32(k, n) for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < (n); k += gridDim.x * blockDim.x)
-
-// average 2x2 (out dims Ho x Wo); C8 = channels / 8
-__global__ void k_pool(const uint4* __restrict__ in, uint4* __restrict__ out, int B, int Ho, int Wo, int C8) {
-  const int n = B * Ho * Wo * C8;
-  GRID_STRIDE32(k, n) {
-    int c = k % C8, r = k / C8;
-    int x = r % Wo, t2 = r / Wo, y = t2 % Ho, b = t2 / Ho;
-    float s[8] = {}, t[8];
-#pragma unroll
-    for (int q = 0; q < 4; q++) {
-      int src = ((b * 2 * Ho + 2 * y + (q >> 1)) * 2 * Wo + 2 * x + (q & 1)) * C8 + c;
-      unpack8(in[src], t);
-#pragma unroll
-      for (int e = 0; e < 8; e++) s[e] += t[e];
-    }
-#pragma unroll
-    for (int e = 0; e < 8; e++) s[e] *= 0.25f;
-    out[k] = pack8(s);
-  }
-}
-
-// out = up(coarse) + skip (fine dims H x W), or, with scale != 0 and out == skip,
-// skip += scale * up(coarse)
-__global__ void k_upadd(const uint4* __restrict__ coarse, const uint4* skip, uint4* out, int B, int H, int W, int C8,
-                        float scale) {
-  const int n = B * H * W * C8;
-  GRID_STRIDE32(k, n) {
-    int c = k % C8, r = k / C8;
-    int x = r % W, t2 = r / W, y = t2 % H, b = t2 / H;
-    float a[8], s[8];
-    unpack8(coarse[((b * (H >> 1) + (y >> 1)) * (W >> 1) + (x >> 1)) * C8 + c], a);
-    unpack8(skip[k], s);
-#pragma unroll
-    for (int e = 0; e < 8; e++) s[e] = __fmaf_rn(scale, a[e], s[e]);
-    out[k] = pack8(s);
-  }
-}
-
-// coarse = sum over each 2x2 block of fine (the adjoint of nearest upsampling)
-__global__ void k_poolsum(const uint4* __restrict__ in, uint4* __restrict__ out, int B, int Ho, int Wo, int C8) {
-  const int n = B * Ho * Wo * C8;
-  GRID_STRIDE32(k, n) {
-    int c = k % C8, r = k / C8;
-    int x = r % Wo, t2 = r / Wo, y = t2 % Ho, b = t2 / Ho;
-    float s[8] = {}, t[8];
-#pragma unroll
-    for (int q = 0; q < 4; q++) {
-      int src = ((b * 2 * Ho + 2 * y + (q >> 1)) * 2 * Wo + 2 * x + (q & 1)) * C8 + c;
-      unpack8(in[src], t);
-#pragma unroll
-      for (int e = 0; e < 8; e++) s[e] += t[e];
-    }
-    out[k] = pack8(s);
-  }
-}
-
-// g = a > 0 ? g : 0 (the ReLU's derivative, from its output)
-__global__ void k_relu_mask(uint4* __restrict__ g, const uint4* __restrict__ a, int n8) {
-  GRID_STRIDE32(k, n8) {
-    float gv[8], av[8];
-    unpack8(g[k], gv);
-    unpack8(a[k], av);
-#pragma unroll
-    for (int e = 0; e < 8; e++) gv[e] = av[e] > 0.f ? gv[e] : 0.f;
-    g[k] = pack8(gv);
-  }
-}
 
 // sigma = RMS from a sum of squares (1 when it is 0), computed by one thread
 // of the block: FP64 runs at 1/54 of the FP32 rate on this part, so it is not
@@ -386,16 +304,15 @@ static cudaError_t ensure_capacity(Net* g, int B, int H, int W) {
   return cudaSuccess;
 }
 
-static cudaError_t conv(const Ctx& c, int l, bool transposed, const bf* in, void* out, int B, int H, int W, int epi) {
+static cudaError_t conv(const Ctx& c, int l, bool transposed, const bf* in, const conv::ConvOut& o, int flags, int B,
+                        int H, int W) {
   Net* g = c.g;
   const int ci = transposed ? kCO[l] : kCI[l], co = transposed ? kCI[l] : kCO[l];
   const bf* w = (transposed ? g->wpkT : g->wpk) + g->off_pk[l];
   const float* bias = transposed ? g->zero_bias : g->theta + g->off_b[l];
   cudaError_t e = cudaSuccess;
-  double flops = 2.0 * 9 * ci * co * B * H * W;
-  (void)flops;
   const double bytes = (double)(ci + co) * 2 * B * H * W;
-  GL(c, "guess_conv", bytes, e = conv::conv3x3(ci, co, epi, in, w, bias, out, B, H, W, g->err, c.st));
+  GL(c, "guess_conv", bytes, e = conv::conv3x3(ci, co, flags, in, w, bias, o, B, H, W, g->err, c.st));
   return e;
 }
 
@@ -405,57 +322,50 @@ static cudaError_t conv(const Ctx& c, int l, bool transposed, const bf* in, void
     if (_e != cudaSuccess) return _e;     \
   } while (0)
 
-static cudaError_t pool(const Ctx& c, Buf in, Buf out, int B, int H, int W, int lev_out) {
-  const int C8 = kBufCh[out] / 8, Ho = H >> lev_out, Wo = W >> lev_out;
-  int64_t n = (int64_t)B * Ho * Wo * C8;
-  GL(c, "guess_pool", n * 80.0,
-     k_pool<<<blocks_for(n), 256, 0, c.st>>>((const uint4*)c.g->buf[in], (uint4*)c.g->buf[out], B, Ho, Wo, C8));
-  return cudaGetLastError();
+using conv::ConvOut;
+
+// a plain layer: out (ReLU'd except the network's last, which is f32 planar)
+static ConvOut to(void* out) {
+  ConvOut o;
+  o.out = out;
+  return o;
 }
-static cudaError_t poolsum(const Ctx& c, Buf in, Buf out, int B, int H, int W, int lev_out) {
-  const int C8 = kBufCh[out] / 8, Ho = H >> lev_out, Wo = W >> lev_out;
-  int64_t n = (int64_t)B * Ho * Wo * C8;
-  GL(c, "guess_poolsum", n * 80.0,
-     k_poolsum<<<blocks_for(n), 256, 0, c.st>>>((const uint4*)c.g->buf[in], (uint4*)c.g->buf[out], B, Ho, Wo, C8));
-  return cudaGetLastError();
+// + the 2 x 2 sums times scale (0 where mask, if given, is not > 0)
+static ConvOut to_pool(void* out, void* pool, float scale, const void* mask = nullptr) {
+  ConvOut o = to(out);
+  o.pool = pool;
+  o.pool_scale = scale;
+  o.pool_mask = mask;
+  return o;
 }
-// out = up(coarse) * scale + skip at level lev (fine)
-static cudaError_t upadd(const Ctx& c, Buf coarse, Buf skip, Buf out, int B, int H, int W, int lev, float scale) {
-  const int C8 = kBufCh[out] / 8, Hf = H >> lev, Wf = W >> lev;
-  int64_t n = (int64_t)B * Hf * Wf * C8;
-  GL(c, "guess_upadd", n * 52.0,
-     k_upadd<<<blocks_for(n), 256, 0, c.st>>>((const uint4*)c.g->buf[coarse], (const uint4*)c.g->buf[skip],
-                                              (uint4*)c.g->buf[out], B, Hf, Wf, C8, scale));
-  return cudaGetLastError();
-}
-static cudaError_t relu_mask(const Ctx& c, Buf gbuf, Buf abuf, int B, int H, int W) {
-  int n8 = (int)(level_pixels(c.g, B, H, W, kBufLevel[gbuf]) * kBufCh[gbuf] / 8);
-  GL(c, "guess_relu_mask", n8 * 48.0,
-     k_relu_mask<<<blocks_for(n8), 256, 0, c.st>>>((uint4*)c.g->buf[gbuf], (const uint4*)c.g->buf[abuf], n8));
-  return cudaGetLastError();
+// + fine + scale * up(out) into up, on the next finer level (out may be null)
+static ConvOut to_up(void* out, void* up, const void* fine, float scale, const void* mask = nullptr) {
+  ConvOut o = to(out);
+  o.up = up;
+  o.fine = fine;
+  o.scale = scale;
+  o.up_mask = mask;
+  return o;
 }
 
-// the network on x0 (already in buf[X0]); result in g->out
+// the network on x0 (already in buf[X0]); result in g->out.  Pooling and the
+// upsampled skip sums are made by the epilogue of the layer before them.
 static cudaError_t forward(const Ctx& c, int B, int H, int W) {
+  using namespace conv;
   Net* g = c.g;
   bf** b = g->buf;
   const int Hl1 = H >> 1, Wl1 = W >> 1, Hl2 = H >> 2, Wl2 = W >> 2, Hl3 = H >> 3, Wl3 = W >> 3;
-  CK(conv(c, LA, false, b[X0], b[A0], B, H, W, 1));
-  CK(conv(c, LB, false, b[A0], b[A0B], B, H, W, 1));
-  CK(pool(c, A0B, Q1, B, H, W, 1));
-  CK(conv(c, LC, false, b[Q1], b[A1], B, Hl1, Wl1, 1));
-  CK(pool(c, A1, Q2, B, H, W, 2));
-  CK(conv(c, LD, false, b[Q2], b[A2], B, Hl2, Wl2, 1));
-  CK(pool(c, A2, Q3, B, H, W, 3));
-  CK(conv(c, LE, false, b[Q3], b[A3], B, Hl3, Wl3, 1));
-  CK(conv(c, LF, false, b[A3], b[F3], B, Hl3, Wl3, 1));
-  CK(upadd(c, F3, A2, S2, B, H, W, 2, 1.f));
-  CK(conv(c, LG, false, b[S2], b[G2], B, Hl2, Wl2, 1));
-  CK(upadd(c, G2, A1, S1, B, H, W, 1, 1.f));
-  CK(conv(c, LH, false, b[S1], b[H1], B, Hl1, Wl1, 1));
-  CK(upadd(c, H1, A0B, S0, B, H, W, 0, 1.f));
-  CK(conv(c, LI, false, b[S0], b[I0], B, H, W, 1));
-  CK(conv(c, LJ, false, b[I0], g->out, B, H, W, 2));
+  constexpr int R = kOutStore | kOutRelu;
+  CK(conv(c, LA, false, b[X0], to(b[A0]), R, B, H, W));
+  CK(conv(c, LB, false, b[A0], to_pool(b[A0B], b[Q1], 0.25f), R | kOutPool, B, H, W));
+  CK(conv(c, LC, false, b[Q1], to_pool(b[A1], b[Q2], 0.25f), R | kOutPool, B, Hl1, Wl1));
+  CK(conv(c, LD, false, b[Q2], to_pool(b[A2], b[Q3], 0.25f), R | kOutPool, B, Hl2, Wl2));
+  CK(conv(c, LE, false, b[Q3], to(b[A3]), R, B, Hl3, Wl3));
+  CK(conv(c, LF, false, b[A3], to_up(b[F3], b[S2], b[A2], 1.f), R | kOutUp, B, Hl3, Wl3));
+  CK(conv(c, LG, false, b[S2], to_up(b[G2], b[S1], b[A1], 1.f), R | kOutUp, B, Hl2, Wl2));
+  CK(conv(c, LH, false, b[S1], to_up(b[H1], b[S0], b[A0B], 1.f), R | kOutUp, B, Hl1, Wl1));
+  CK(conv(c, LI, false, b[S0], to(b[I0]), R, B, H, W));
+  CK(conv(c, LJ, false, b[I0], to(g->out), kOutPlanar, B, H, W));
   return cudaSuccess;
 }
 
@@ -518,6 +428,7 @@ static cudaError_t wgrad(const Ctx& c, int l, Buf xbuf, Buf gbuf, int B, int H, 
 
 // loss against target (f32 [B][H][W]) and the gradient of every parameter into g->grad
 static cudaError_t backward(const Ctx& c, const float* target, int B, int H, int W) {
+  using namespace conv;
   Net* g = c.g;
   bf** b = g->buf;
   const int64_t npix = (int64_t)H * W;
@@ -534,40 +445,33 @@ static cudaError_t backward(const Ctx& c, const float* target, int B, int H, int
      k_loss_seed<<<dim3(lb, B), 256, 0, c.st>>>(g->out, target, with_res ? g->res : nullptr, g->acc,
                                                 (uint4*)b[GJ], H, W, B, g->w_p, g->w_r));
   CK(cudaGetLastError());
+  // Each layer's weight gradient, then the gradient of its input; the ReLU
+  // masks, the gradients of the upsampled skip sums (2 x 2 sums) and of the
+  // pooling (a quarter of the coarse gradient, added) are made by the epilogue.
+  constexpr int M = kOutStore | kOutMask, P = kOutStore | kOutPool | kOutPoolMask, U = kOutUp | kOutUpMask;
+  auto masked = [&](Buf out, Buf act) {
+    ConvOut o = to(b[out]);
+    o.mask = b[act];
+    return o;
+  };
   CK(wgrad(c, LJ, I0, GJ, B, H, W));
-  CK(conv(c, LJ, true, b[GJ], b[DI0], B, H, W, 0));
-  CK(relu_mask(c, DI0, I0, B, H, W));
+  CK(conv(c, LJ, true, b[GJ], masked(DI0, I0), M, B, H, W));
   CK(wgrad(c, LI, S0, DI0, B, H, W));
-  CK(conv(c, LI, true, b[DI0], b[DS0], B, H, W, 0));
-  CK(poolsum(c, DS0, DH1, B, H, W, 1));
-  CK(relu_mask(c, DH1, H1, B, H, W));
+  CK(conv(c, LI, true, b[DI0], to_pool(b[DS0], b[DH1], 1.f, b[H1]), P, B, H, W));
   CK(wgrad(c, LH, S1, DH1, B, Hl1, Wl1));
-  CK(conv(c, LH, true, b[DH1], b[DS1], B, Hl1, Wl1, 0));
-  CK(poolsum(c, DS1, DG2, B, H, W, 2));
-  CK(relu_mask(c, DG2, G2, B, H, W));
+  CK(conv(c, LH, true, b[DH1], to_pool(b[DS1], b[DG2], 1.f, b[G2]), P, B, Hl1, Wl1));
   CK(wgrad(c, LG, S2, DG2, B, Hl2, Wl2));
-  CK(conv(c, LG, true, b[DG2], b[DS2], B, Hl2, Wl2, 0));
-  CK(poolsum(c, DS2, DF3, B, H, W, 3));
-  CK(relu_mask(c, DF3, F3, B, H, W));
+  CK(conv(c, LG, true, b[DG2], to_pool(b[DS2], b[DF3], 1.f, b[F3]), P, B, Hl2, Wl2));
   CK(wgrad(c, LF, A3, DF3, B, Hl3, Wl3));
-  CK(conv(c, LF, true, b[DF3], b[DA3], B, Hl3, Wl3, 0));
-  CK(relu_mask(c, DA3, A3, B, H, W));
+  CK(conv(c, LF, true, b[DF3], masked(DA3, A3), M, B, Hl3, Wl3));
   CK(wgrad(c, LE, Q3, DA3, B, Hl3, Wl3));
-  CK(conv(c, LE, true, b[DA3], b[DQ3], B, Hl3, Wl3, 0));
-  // da2 = ds2 + up(dq3) / 4, masked
-  CK(upadd(c, DQ3, DS2, DS2, B, H, W, 2, 0.25f));
-  CK(relu_mask(c, DS2, A2, B, H, W));
+  CK(conv(c, LE, true, b[DA3], to_up(nullptr, b[DS2], b[DS2], 0.25f, b[A2]), U, B, Hl3, Wl3));
   CK(wgrad(c, LD, Q2, DS2, B, Hl2, Wl2));
-  CK(conv(c, LD, true, b[DS2], b[DQ2], B, Hl2, Wl2, 0));
-  CK(upadd(c, DQ2, DS1, DS1, B, H, W, 1, 0.25f));
-  CK(relu_mask(c, DS1, A1, B, H, W));
+  CK(conv(c, LD, true, b[DS2], to_up(nullptr, b[DS1], b[DS1], 0.25f, b[A1]), U, B, Hl2, Wl2));
   CK(wgrad(c, LC, Q1, DS1, B, Hl1, Wl1));
-  CK(conv(c, LC, true, b[DS1], b[DQ1], B, Hl1, Wl1, 0));
-  CK(upadd(c, DQ1, DS0, DS0, B, H, W, 0, 0.25f));
-  CK(relu_mask(c, DS0, A0B, B, H, W));
+  CK(conv(c, LC, true, b[DS1], to_up(nullptr, b[DS0], b[DS0], 0.25f, b[A0B]), U, B, Hl1, Wl1));
   CK(wgrad(c, LB, A0, DS0, B, H, W));
-  CK(conv(c, LB, true, b[DS0], b[DA0], B, H, W, 0));
-  CK(relu_mask(c, DA0, A0, B, H, W));
+  CK(conv(c, LB, true, b[DS0], masked(DA0, A0), M, B, H, W));
   CK(wgrad(c, LA, X0, DA0, B, H, W));
   return cudaSuccess;
 }

@@ -66,6 +66,22 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint32
   return false;
 }
 
+// The same wait with the thread suspended between probes (a microsecond at
+// most, a second in all): for kernels whose warps wait on one another, where
+// spinning probes take the shared-memory issue slots of the warps that work.
+__device__ __forceinline__ bool mbar_wait_idle(uint64_t* bar, uint32_t parity) {
+  for (uint32_t k = 0; k < (1u << 20); k++) {
+    uint32_t ok;
+    asm volatile(
+        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n selp.u32 %0, 1, 0, p;\n}\n"
+        : "=r"(ok)
+        : "r"(smem_u32(bar)), "r"(parity), "r"(1000u)
+        : "memory");
+    if (ok) return true;
+  }
+  return false;
+}
+
 // -------------------------------------------------------------- TMA loads
 // one arrival on the barrier that also expects `bytes` of asynchronous copies
 __device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, uint32_t bytes) {
@@ -117,6 +133,24 @@ __device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t adesc, uint64
       " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d_tmem),
       "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
+}
+// The same called by a whole warp with warp-uniform arguments, issued by the lane
+// whose `leader` is not 0: the descriptors then stay in uniform registers, where
+// the instruction wants them (computed by one lane in a divergent branch they
+// are moved there one by one, ~70 cycles an MMA where the tensor core takes 32)
+__device__ __forceinline__ void mma_bf16_warp(uint32_t leader, uint32_t d_tmem, uint64_t adesc, uint64_t bdesc,
+                                              uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n .reg .pred p, q;\n setp.ne.b32 p, %4, 0;\n setp.ne.b32 q, %5, 0;\n"
+      " @q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d_tmem),
+      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(leader)
+      : "memory");
+}
+// 1 in one lane of the (converged) warp
+__device__ __forceinline__ uint32_t elect_one() {
+  uint32_t r;
+  asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(r));
+  return r;
 }
 // the mbarrier receives one arrival when every MMA this thread issued so far is done
 __device__ __forceinline__ void mma_commit(uint64_t* bar) {

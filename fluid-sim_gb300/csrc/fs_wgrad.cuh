@@ -75,6 +75,16 @@ __device__ __forceinline__ void wg_copy(uint32_t dst, const void* src, bool real
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(real ? 16 : 0) : "memory");
 }
 
+// i modulo n for i >= -n; a division only where the image is smaller than a tile
+__device__ __forceinline__ int wg_wrap(int i, int n) {
+  if (i < 0) return i + n;
+  if (i >= n) {
+    i -= n;
+    if (i >= n) i %= n;
+  }
+  return i;
+}
+
 // Warps 0 .. 7 stage tiles (and sum the bias gradient from their own copies),
 // warp 8 issues the MMAs; two stages, handed over by barriers: full[s] (the
 // staging threads' copies have landed) and done[s] (the MMAs that read them).
@@ -120,21 +130,18 @@ __global__ void __launch_bounds__(kWgThreads + 32, 1) k_wgrad_tc(const uint4* __
         const int xt = t % ntx, r = t / ntx, y0 = (r % nty) * TY, x0 = xt * PX;
         const int img = (r / nty) * H;
         const uint32_t sx = s0 + buf * C::STAGE, sg = sx + C::X_BYTES;
-        if (k >= 2 && !tc::mbar_wait(&done[buf], ((k - 2) >> 1) & 1)) *failed = 1;
+        if (k >= 2 && !tc::mbar_wait_idle(&done[buf], ((k - 2) >> 1) & 1)) *failed = 1;
         if (*failed) break;
         // columns x0 - 1 .. x0 + PX of rows y0 - 1 .. y0 + TY, wrapped
+        const uint4* rows[TY + 2];
+#pragma unroll
+        for (int row = 0; row < TY + 2; row++) rows[row] = X + (int64_t)(img + wg_wrap(y0 - 1 + row, H)) * (W * C::KC);
         for (int q = tid; q < C::RW * C::KC; q += kWgThreads) {
           const int kc = q % C::KC, px = q / C::KC;
-          int gx = x0 - 1 + px;
-          gx = gx < 0 ? gx + W : gx >= W ? gx % W : gx;
-          const uint4* col = X + gx * C::KC + kc;
+          const int col = wg_wrap(x0 - 1 + px, W) * C::KC + kc;
           const uint32_t dst = sx + kc * C::XP + px * 16;
 #pragma unroll
-          for (int row = 0; row < TY + 2; row++) {
-            int gy = y0 - 1 + row;
-            gy = gy < 0 ? gy + H : gy >= H ? gy % H : gy;
-            wg_copy(dst + row * C::KC * C::XP, col + (int64_t)(img + gy) * (W * C::KC), true);
-          }
+          for (int row = 0; row < TY + 2; row++) wg_copy(dst + row * C::KC * C::XP, rows[row] + col, true);
         }
         // and the tile's G, zeros beyond the image
 #pragma unroll
@@ -175,12 +182,16 @@ __global__ void __launch_bounds__(kWgThreads + 32, 1) k_wgrad_tc(const uint4* __
       }
     }
     asm volatile("cp.async.wait_all;" ::: "memory");
-  } else if (lane == 0) {
+  } else {
+    const uint32_t leader = tc::elect_one(), ta = __shfl_sync(0xffffffffu, taddr, 0);
     int k = 0;
     for (; k < mine; k++) {
       const int buf = k & 1;
-      if (!tc::mbar_wait(&full[buf], (k >> 1) & 1)) *failed = 1;
-      if (*failed) break;
+      const bool ok = tc::mbar_wait_idle(&full[buf], (k >> 1) & 1);
+      if (__any_sync(0xffffffffu, !ok || *failed)) {
+        *failed = 1;
+        break;
+      }
       tc::fence_after_sync();
       const uint32_t sx = s0 + buf * C::STAGE, sg = sx + C::X_BYTES;
       // the descriptors' address field counts 16-byte units
@@ -191,14 +202,16 @@ __global__ void __launch_bounds__(kWgThreads + 32, 1) k_wgrad_tc(const uint4* __
         for (int d = 0; d < NDX; d++)
 #pragma unroll
           for (int j = 0; j < C::MB; j++)
-            tc::mma_bf16(taddr + (d * C::MB + j) * C::NN, ad0 + 16 * j * (C::XP / 16) + s * 16 + d, bd0 + s * 16,
-                         tc::idesc_bf16_mn(j == C::MB - 1 ? C::LAST_M : 128, C::NN), (k > 0 || s > 0) ? 1u : 0u);
+            tc::mma_bf16_warp(leader, ta + (d * C::MB + j) * C::NN, ad0 + 16 * j * (C::XP / 16) + s * 16 + d,
+                              bd0 + s * 16, tc::idesc_bf16_mn(j == C::MB - 1 ? C::LAST_M : 128, C::NN),
+                              (k > 0 || s > 0) ? 1u : 0u);
       }
-      tc::mma_commit(&done[buf]);
+      if (leader) tc::mma_commit(&done[buf]);
+      __syncwarp();
     }
     // every MMA issued is done before the accumulators are read or released
     // (a commit covers all before it)
-    if (k > 0 && !tc::mbar_wait(&done[(k - 1) & 1], ((k - 1) >> 1) & 1)) *failed = 1;
+    if (k > 0 && !tc::mbar_wait_idle(&done[(k - 1) & 1], ((k - 1) >> 1) & 1)) *failed = 1;
   }
   __syncthreads();
   if (tid == 0 && *failed) atomicExch(err, 1);
