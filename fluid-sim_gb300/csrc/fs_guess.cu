@@ -119,103 +119,166 @@ __device__ __forceinline__ float block_sigma(const double* __restrict__ sumsq, i
   return sig;
 }
 
-// x0[p] = (div / sigma, mask, 0, ..., 0); sigma = 1 without a sum of squares
+// x0[p] = (div / sigma, mask, 0, ..., 0); sigma = 1 without a sum of squares.
+// A thread writes one half of a pixel, so that a warp's stores are one
+// contiguous run (a pixel per thread, 1024^2 x 4: 43 us; 27 us here, of which
+// 25 us for the bytes).
 __global__ void k_prep(const float* __restrict__ div, const float* __restrict__ mask, uint4* __restrict__ x0,
                        int npix, const double* __restrict__ sumsq, int64_t nnorm) {
   const float inv = sumsq ? 1.f / block_sigma(sumsq, nnorm) : 1.f;
-  GRID_STRIDE32(p, npix) {
-    float f[8] = {div[p] * inv, mask ? mask[p] : 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    float z[8] = {};
-    x0[2 * p] = pack8(f);
-    x0[2 * p + 1] = pack8(z);
+  GRID_STRIDE32(k, 2 * npix) {
+    uint4 v = make_uint4(0, 0, 0, 0);
+    if (!(k & 1)) {
+      const int p = k >> 1;
+      const float f[8] = {div[p] * inv, mask ? mask[p] : 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+      v = pack8(f);
+    }
+    x0[k] = v;
   }
+}
+
+// ---- The loss.  FP64 runs at 1/54 of the FP32 rate on this part, conversions
+// included, so these passes are bound by the number of FP64 instructions a cell
+// takes: the error of a cell is formed once and handed to its neighbours, and
+// f32 values are widened with integer instructions.  A warp walks down a strip
+// of kLossCols columns (lanes 0 and 31 hold its neighbours' columns) with the
+// three rows of the stencil in registers.  1024^2 x 4, mean + residual + seed:
+// 39 + 175 + 163 us with a thread per cell that converted every operand, 105 + 148 us
+// here (mean and residual in one pass).
+constexpr int kLossCols = 30, kLossWarps = 8;
+
+// (double)f by integer instructions where f is a normal number
+__device__ __forceinline__ double widen(float f) {
+  const uint32_t b = __float_as_uint(f);
+  if ((b << 1) - 0x01000000u >= 0xfe000000u) return (double)f;  // 0, subnormal, infinite, NaN
+  return __hiloint2double((int)((b & 0x80000000u) | (((b & 0x7fffffffu) >> 3) + 0x38000000u)), (int)(b << 29));
+}
+
+// the block's sum of s, on thread 0
+__device__ __forceinline__ double loss_block_sum(double s) {
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  __shared__ double sm[kLossWarps];
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = s;
+  __syncthreads();
+  double t = 0.0;
+  if (threadIdx.x == 0)
+    for (int w = 0; w < kLossWarps; w++) t += sm[w];
+  return t;
 }
 
 // per-sample sum of e = out - target -> acc[b]
-__global__ void k_loss_mean(const float* __restrict__ out, const float* __restrict__ tgt, double* __restrict__ acc,
-                            int64_t npix) {
+__global__ void __launch_bounds__(32 * kLossWarps)
+    k_loss_mean(const float* __restrict__ out, const float* __restrict__ tgt, double* __restrict__ acc, int64_t npix) {
   const int b = blockIdx.y;
   double s = 0.0;
   for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < npix; p += (int64_t)gridDim.x * blockDim.x)
-    s += (double)out[b * npix + p] - (double)tgt[b * npix + p];
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  __shared__ double sm[8];
-  if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = s;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double t = 0.0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); w++) t += sm[w];
-    atomicAdd(&acc[b], t);
-  }
+    s += widen(out[b * npix + p]) - widen(tgt[b * npix + p]);
+  const double t = loss_block_sum(s);
+  if (threadIdx.x == 0) atomicAdd(&acc[b], t);
 }
 
-__device__ __forceinline__ int64_t wrap_idx(int b, int y, int x, int H, int W) {
-  y = y < 0 ? y + H : (y >= H ? y - H : y);
-  x = x < 0 ? x + W : (x >= W ? x - W : x);
-  return ((int64_t)b * H + y) * W + x;
+// This warp's strip of image blockIdx.y: columns x0 .. x0 + 29, rows y0 .. y1 - 1;
+// x is this lane's column, wrapped.
+struct LossStrip {
+  int x0, x, y0, y1, lane;
+  bool any, store;  // the strip exists; this lane's column is one of its own
+};
+__device__ __forceinline__ LossStrip loss_strip(int H, int W, int rows) {
+  LossStrip t;
+  const int nx = (W + kLossCols - 1) / kLossCols, k = blockIdx.x * kLossWarps + (threadIdx.x >> 5);
+  t.lane = threadIdx.x & 31;
+  t.x0 = (k % nx) * kLossCols;
+  t.y0 = (k / nx) * rows;
+  t.y1 = min(t.y0 + rows, H);
+  t.any = t.y0 < H;
+  const int x = t.x0 + t.lane - 1;
+  t.store = t.lane >= 1 && t.lane <= kLossCols && x < W;
+  t.x = (x + W) % W;  // x <= W + 29: wrapped again where the image is narrower
+  return t;
+}
+// c's neighbours' sum and centre: left + right + above + below - 4 c
+__device__ __forceinline__ double lap5(double above, double c, double below) {
+  const double left = __shfl_up_sync(0xffffffffu, c, 1), right = __shfl_down_sync(0xffffffffu, c, 1);
+  return left + right + above + below - 4.0 * c;
 }
 
-// res = lap(out - target) (periodic 5-point, unscaled); w_r sum res^2 / (B N) into acc[B]
-__global__ void k_loss_res(const float* __restrict__ out, const float* __restrict__ tgt, float* __restrict__ res,
-                           double* __restrict__ acc, int H, int W, int B, double w_r) {
+// res = lap(out - target) (periodic 5-point, unscaled); sum of out - target into
+// acc[b], w_r sum res^2 / (B N) into acc[B]
+__global__ void __launch_bounds__(32 * kLossWarps)
+    k_loss_res(const float* __restrict__ out, const float* __restrict__ tgt, float* __restrict__ res,
+               double* __restrict__ acc, int H, int W, int B, int rows, double w_r) {
   const int b = blockIdx.y;
-  const int64_t npix = (int64_t)H * W;
-  double s = 0.0;
-  for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < npix; p += (int64_t)gridDim.x * blockDim.x) {
-    const int pi = (int)p, y = pi / W, x = pi - y * W;
-    auto e = [&](int yy, int xx) {
-      int64_t q = wrap_idx(b, yy, xx, H, W);
-      return (double)out[q] - (double)tgt[q];
+  const int64_t npix = (int64_t)H * W, base = b * npix;
+  const LossStrip t = loss_strip(H, W, rows);
+  double s = 0.0, m = 0.0;
+  if (t.any) {
+    auto e = [&](int y) {
+      const int64_t q = base + (int64_t)(y < 0 ? y + H : y >= H ? y - H : y) * W + t.x;
+      return widen(out[q]) - widen(tgt[q]);
     };
-    double r = e(y, x - 1) + e(y, x + 1) + e(y - 1, x) + e(y + 1, x) - 4.0 * e(y, x);
-    res[b * npix + p] = (float)r;
-    s += r * r;
+    double above = e(t.y0 - 1), c = e(t.y0);
+#pragma unroll 4
+    for (int y = t.y0; y < t.y1; y++) {
+      const double below = e(y + 1), r = lap5(above, c, below);
+      if (t.store) {
+        res[base + (int64_t)y * W + t.x] = (float)r;
+        s += r * r;
+        m += c;
+      }
+      above = c;
+      c = below;
+    }
   }
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  __shared__ double sm[8];
-  if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = s;
-  __syncthreads();
+  const double sum = loss_block_sum(s), err = loss_block_sum(m);
   if (threadIdx.x == 0) {
-    double t = 0.0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); w++) t += sm[w];
-    atomicAdd(&acc[B], w_r * t / ((double)B * npix));
+    atomicAdd(&acc[b], err);
+    atomicAdd(&acc[B], w_r * sum / ((double)B * npix));
   }
 }
 
 // seed gradient dL/dout = (w_p 2 (e - mean_b e) + w_r 2 lap(res)) / (B N) into
 // channel 0 of gJ; w_p sum (e - mean)^2 / (B N) into acc[B]
-__global__ void k_loss_seed(const float* __restrict__ out, const float* __restrict__ tgt,
-                            const float* __restrict__ res, double* __restrict__ acc, uint4* __restrict__ gJ, int H,
-                            int W, int B, double w_p, double w_r) {
+__global__ void __launch_bounds__(32 * kLossWarps)
+    k_loss_seed(const float* __restrict__ out, const float* __restrict__ tgt, const float* __restrict__ res,
+                double* __restrict__ acc, uint4* __restrict__ gJ, int H, int W, int B, int rows, double w_p,
+                double w_r) {
   const int b = blockIdx.y;
-  const int64_t npix = (int64_t)H * W;
+  const int64_t npix = (int64_t)H * W, base = b * npix;
   const double mean = acc[b] / (double)npix, scale = 2.0 / ((double)B * npix);
+  const LossStrip t = loss_strip(H, W, rows);
   double s = 0.0;
-  for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < npix; p += (int64_t)gridDim.x * blockDim.x) {
-    int64_t q = b * npix + p;
-    double ec = (double)out[q] - (double)tgt[q] - mean;
-    s += ec * ec;
-    double g = w_p * ec;
-    if (res) {
-      const int pi = (int)p, y = pi / W, x = pi - y * W;
-      double lr = (double)res[wrap_idx(b, y, x - 1, H, W)] + res[wrap_idx(b, y, x + 1, H, W)] +
-                  res[wrap_idx(b, y - 1, x, H, W)] + res[wrap_idx(b, y + 1, x, H, W)] - 4.0 * res[q];
-      g += w_r * lr;
+  if (t.any) {
+    auto row = [&](int y) {
+      return res ? widen(res[base + (int64_t)(y < 0 ? y + H : y >= H ? y - H : y) * W + t.x]) : 0.0;
+    };
+    double above = row(t.y0 - 1), c = row(t.y0);
+#pragma unroll 4
+    for (int y = t.y0; y < t.y1; y++) {
+      const int64_t q = base + (int64_t)y * W + t.x;
+      const double ec = widen(out[q]) - widen(tgt[q]) - mean;
+      double g = w_p * ec;
+      if (res) {
+        const double below = row(y + 1);
+        g += w_r * lap5(above, c, below);
+        above = c;
+        c = below;
+      }
+      if (t.store) s += ec * ec;
+      // the strip's pixels, 16 bytes a lane: channel 0 and zeros, zeros
+      const float f[8] = {(float)(scale * g), 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+      const uint32_t first = pack8(f).x;
+#pragma unroll
+      for (int half = 0; half < 2; half++) {
+        const int k = t.lane + 32 * half, px = k >> 1;
+        const uint32_t v = __shfl_sync(0xffffffffu, first, (px + 1) & 31);
+        if (px < kLossCols && t.x0 + px < W)
+          gJ[2 * (base + (int64_t)y * W + t.x0) + k] = make_uint4(k & 1 ? 0u : v, 0u, 0u, 0u);
+      }
     }
-    float f[8] = {(float)(scale * g), 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    float z[8] = {};
-    gJ[2 * q] = pack8(f);
-    gJ[2 * q + 1] = pack8(z);
   }
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  __shared__ double sm[8];
-  if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = s;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double t = 0.0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); w++) t += sm[w];
-    atomicAdd(&acc[B], w_p * t / ((double)B * npix));
-  }
+  const double sum = loss_block_sum(s);
+  if (threadIdx.x == 0) atomicAdd(&acc[B], w_p * sum / ((double)B * npix));
 }
 
 // ------------------------------------------------------------ parameters
@@ -348,9 +411,9 @@ static ConvOut to_up(void* out, void* up, const void* fine, float scale, const v
   return o;
 }
 
-// the network on x0 (already in buf[X0]); result in g->out.  Pooling and the
+// the network on x0 (already in buf[X0]); result in out (f32 [B][H][W]).  Pooling and the
 // upsampled skip sums are made by the epilogue of the layer before them.
-static cudaError_t forward(const Ctx& c, int B, int H, int W) {
+static cudaError_t forward(const Ctx& c, int B, int H, int W, float* out) {
   using namespace conv;
   Net* g = c.g;
   bf** b = g->buf;
@@ -365,7 +428,7 @@ static cudaError_t forward(const Ctx& c, int B, int H, int W) {
   CK(conv(c, LG, false, b[S2], to_up(b[G2], b[S1], b[A1], 1.f), R | kOutUp, B, Hl2, Wl2));
   CK(conv(c, LH, false, b[S1], to_up(b[H1], b[S0], b[A0B], 1.f), R | kOutUp, B, Hl1, Wl1));
   CK(conv(c, LI, false, b[S0], to(b[I0]), R, B, H, W));
-  CK(conv(c, LJ, false, b[I0], to(g->out), kOutPlanar, B, H, W));
+  CK(conv(c, LJ, false, b[I0], to(out), kOutPlanar, B, H, W));
   return cudaSuccess;
 }
 
@@ -434,16 +497,22 @@ static cudaError_t backward(const Ctx& c, const float* target, int B, int H, int
   const int64_t npix = (int64_t)H * W;
   const int Hl1 = H >> 1, Wl1 = W >> 1, Hl2 = H >> 2, Wl2 = W >> 2, Hl3 = H >> 3, Wl3 = W >> 3;
   CK(cudaMemsetAsync(g->acc, 0, sizeof(double) * (B + 1), c.st));
-  int lb = (int)((npix + 255) / 256);
-  if (lb > 256) lb = 256;
-  GL(c, "guess_loss", npix * B * 8.0, k_loss_mean<<<dim3(lb, B), 256, 0, c.st>>>(g->out, target, g->acc, npix));
   const bool with_res = g->w_r != 0.0;
+  // rows of a strip: long ones read their two extra rows less often, short ones
+  // give small images more warps
+  const int64_t cols = (W + kLossCols - 1) / kLossCols;
+  const int rows = B * cols * (H / 32) >= 152 * 16 ? 32 : 8;
+  const dim3 lb((unsigned)((cols * ((H + rows - 1) / rows) + kLossWarps - 1) / kLossWarps), B);
   if (with_res)
     GL(c, "guess_loss", npix * B * 12.0,
-       k_loss_res<<<dim3(lb, B), 256, 0, c.st>>>(g->out, target, g->res, g->acc, H, W, B, g->w_r));
+       k_loss_res<<<lb, 32 * kLossWarps, 0, c.st>>>(g->out, target, g->res, g->acc, H, W, B, rows, g->w_r));
+  else
+    GL(c, "guess_loss", npix * B * 8.0,
+       k_loss_mean<<<dim3((unsigned)std::min<int64_t>((npix + 255) / 256, 256), B), 32 * kLossWarps, 0, c.st>>>(
+           g->out, target, g->acc, npix));
   GL(c, "guess_loss", npix * B * 40.0,
-     k_loss_seed<<<dim3(lb, B), 256, 0, c.st>>>(g->out, target, with_res ? g->res : nullptr, g->acc,
-                                                (uint4*)b[GJ], H, W, B, g->w_p, g->w_r));
+     k_loss_seed<<<lb, 32 * kLossWarps, 0, c.st>>>(g->out, target, with_res ? g->res : nullptr, g->acc,
+                                                   (uint4*)b[GJ], H, W, B, rows, g->w_p, g->w_r));
   CK(cudaGetLastError());
   // Each layer's weight gradient, then the gradient of its input; the ReLU
   // masks, the gradients of the upsampled skip sums (2 x 2 sums) and of the
@@ -608,7 +677,7 @@ int guess_enqueue(Solver* s, fs_guess* handle, int f) {
   FS_LAUNCH(s, "guess_prep", (double)npn * 40,
             guess::k_prep<<<guess::blocks_for(npn), 256, 0, s->stream>>>(g->gin, g->gmask, (uint4*)g->buf[guess::X0],
                                                                          npn, gsum, npn));
-  cudaError_t e = guess::forward(c, 1, Hn, Wn);
+  cudaError_t e = guess::forward(c, 1, Hn, Wn, g->out);
   if (e != cudaSuccess) return fail_status(s, FS_ERR_CUDA, std::string("pressure guess: ") + cudaGetErrorString(e));
   FS_LAUNCH(s, "guess_out", (double)s->n * 8,
             k_guess_out<<<guess::blocks_for(s->n), 256, 0, s->stream>>>(
@@ -855,9 +924,7 @@ extern "C" FS_API int fs_guess_predict(fs_guess* h, const float* d_div, const fl
   const int64_t np = (int64_t)B * H * W;
   k_prep<<<blocks_for(np), 256, 0, g->stream>>>(d_div, d_mask, (uint4*)g->buf[X0], np, nullptr, 1);
   g->launches++;
-  if ((e = forward(c, B, H, W)) != cudaSuccess) return gcuda(g, e, "fs_guess_predict");
-  e = cudaMemcpyAsync(d_out, g->out, np * 4, cudaMemcpyDeviceToDevice, g->stream);
-  if (e != cudaSuccess) return gcuda(g, e, "fs_guess_predict");
+  if ((e = forward(c, B, H, W, d_out)) != cudaSuccess) return gcuda(g, e, "fs_guess_predict");
   return read_err(g, "fs_guess_predict");
 }
 
@@ -873,7 +940,7 @@ static int loss_grad_impl(Net* g, const float* d_div, const float* d_mask, const
   const int64_t np = (int64_t)B * H * W;
   k_prep<<<blocks_for(np), 256, 0, g->stream>>>(d_div, d_mask, (uint4*)g->buf[X0], np, nullptr, 1);
   g->launches++;
-  if ((e = forward(c, B, H, W)) != cudaSuccess) return gcuda(g, e, who);
+  if ((e = forward(c, B, H, W, g->out)) != cudaSuccess) return gcuda(g, e, who);
   if ((e = backward(c, d_tgt, B, H, W)) != cudaSuccess) return gcuda(g, e, who);
   if (loss) {
     e = cudaMemcpyAsync(loss, g->acc + B, 8, cudaMemcpyDeviceToHost, g->stream);
