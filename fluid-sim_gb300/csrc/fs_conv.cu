@@ -226,11 +226,8 @@ __device__ __forceinline__ int wrap_near(int i, int n) {
   return i;
 }
 
+// through L1: past it (.cg) the wide layers took 5 .. 10% longer
 __device__ __forceinline__ void copy16(uint32_t dst, const void* src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
-}
-// through L1, for when another copy takes the other half of the 32-byte sector
-__device__ __forceinline__ void copy16_l1(uint32_t dst, const void* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
 
@@ -368,15 +365,12 @@ __global__ void __launch_bounds__(kThreads, (Per<F, Cfg<CIN, COUT, TY, NS, D>>::
           dst[r - R0] = s0 + q * C::ROW;
         }
         for (int q = st; q < kTW * C::KC; q += kStage) {
-          // 16 channels: pixel by pixel through L1 (contiguous in shared memory);
-          // more: a pixel's chunks on neighbouring threads (contiguous in global)
+          // 16 channels: a chunk of neighbouring pixels on neighbouring threads; more:
+          // a pixel's chunks on neighbouring threads
           const int xx = C::KC == 2 ? q % kTW : q / C::KC, kc = C::KC == 2 ? q / kTW : q % C::KC;
           const int col = wrap_near(t.x0 - 1 + xx, W) * C::KC + kc, off = kc * C::PLANE + xx * 16;
 #pragma unroll
-          for (int r = 0; r < TY + 2 - R0; r++) {
-            if (C::KC == 2) copy16_l1(dst[r] + off, src[r] + col);
-            else copy16(dst[r] + off, src[r] + col);
-          }
+          for (int r = 0; r < TY + 2 - R0; r++) copy16(dst[r] + off, src[r] + col);
         }
       };
       if (t.first) rows(std::integral_constant<int, 0>());

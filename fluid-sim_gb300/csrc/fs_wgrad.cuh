@@ -20,8 +20,7 @@
 // (288 8 x 8 blocks per 128 pixels at 16 channels), 478 us for 16 -> 16 channels
 // at 1024^2 x 4.  The same layout with one MMA per row and horizontal tap took
 // 151 us (a 64 x 16 x 16 MMA occupies the tensor core for 32 cycles, a 128 x 64 x
-// 16 one hardly more); this one takes 121 us (268 MB read, 40 us of HBM time) and
-// is bound by the latency of its copies.
+// 16 one hardly more); this one takes 62 us (268 MB read, 40 us of HBM time).
 //
 // The last M block of a layer may have rows beyond (TY + 2) CIN: its descriptor
 // runs on into whatever the stage holds there, and those rows of D are not
@@ -70,9 +69,11 @@ struct WgCfg {
   static_assert(kWgThreads % OC == 0, "a bias thread keeps its channels");
 };
 
-// a 16-byte asynchronous copy, or 16 zero bytes
+// A 16-byte asynchronous copy, or 16 zero bytes.  Through L1 (.ca): past it
+// (.cg), whichever way lanes are dealt to pixels and chunks, these kernels were
+// much slower (16 -> 16 channels 100 .. 119 us, 62 us here; 64 -> 32 52, 35 here).
 __device__ __forceinline__ void wg_copy(uint32_t dst, const void* src, bool real) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(real ? 16 : 0) : "memory");
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(real ? 16 : 0) : "memory");
 }
 
 // i modulo n for i >= -n; a division only where the image is smaller than a tile
@@ -123,7 +124,7 @@ __global__ void __launch_bounds__(kWgThreads + 32, 1) k_wgrad_tc(const uint4* __
   if (warp < kWgThreads / 32) {
     // the G copies of this thread: channel chunk goc, pixels gpx, gpx + GS, ...
     constexpr int GS = kWgThreads / C::OC;
-    const int goc = tid % C::OC, gpx = tid / C::OC;
+    const int goc = C::OC == 2 ? tid / GS : tid % C::OC, gpx = C::OC == 2 ? tid % GS : tid / C::OC;
     for (int k = 0; k <= mine; k++) {
       if (k < mine) {
         const int t = blockIdx.x + k * gridDim.x, buf = k & 1;
@@ -136,12 +137,21 @@ __global__ void __launch_bounds__(kWgThreads + 32, 1) k_wgrad_tc(const uint4* __
         const uint4* rows[TY + 2];
 #pragma unroll
         for (int row = 0; row < TY + 2; row++) rows[row] = X + (int64_t)(img + wg_wrap(y0 - 1 + row, H)) * (W * C::KC);
-        for (int q = tid; q < C::RW * C::KC; q += kWgThreads) {
-          const int kc = q % C::KC, px = q / C::KC;
+        auto column = [&](int px, int kc) {
           const int col = wg_wrap(x0 - 1 + px, W) * C::KC + kc;
           const uint32_t dst = sx + kc * C::XP + px * 16;
 #pragma unroll
           for (int row = 0; row < TY + 2; row++) wg_copy(dst + row * C::KC * C::XP, rows[row] + col, true);
+        };
+        if constexpr (C::KC == 2) {
+          // 16 channels: a chunk of neighbouring pixels on neighbouring threads (80 us with
+          // the other order)
+          static_assert(kWgThreads == 2 * PX, "one column a thread");
+          column(tid % PX, tid / PX);
+          if (tid % PX < 2) column(PX + tid % PX, tid / PX);
+        } else {
+          // a pixel's chunks on neighbouring threads
+          for (int q = tid; q < C::RW * C::KC; q += kWgThreads) column(q / C::KC, q % C::KC);
         }
         // and the tile's G, zeros beyond the image
 #pragma unroll
@@ -256,9 +266,13 @@ __global__ void __launch_bounds__(kWgThreads + 32, 1) k_wgrad_tc(const uint4* __
       const int tap = k / (CIN * COUT), r = k - tap * (CIN * COUT), dy = tap / NDX, d = tap - dy * NDX;
       part[((int64_t)blockIdx.x * 9 + dy * 3 + dx0 + d) * CIN * COUT + r] = mine > 0 ? acc[k] : 0.f;
     }
-    if (blockIdx.y == 0 && tid < COUT) {  // thread t holds channels 8 (t % OC) .. of its pixels
+    if (blockIdx.y == 0 && tid < COUT) {  // the threads that hold these channels, in order
       float s = 0.f;
-      for (int k = tid / 8; k < kWgThreads; k += C::OC) s += fold[k * 8 + tid % 8];
+      if (C::OC == 2) {
+        for (int k = 0; k < kWgThreads / 2; k++) s += fold[(tid / 8 * (kWgThreads / 2) + k) * 8 + tid % 8];
+      } else {
+        for (int k = tid / 8; k < kWgThreads; k += C::OC) s += fold[k * 8 + tid % 8];
+      }
       bpart[(int64_t)blockIdx.x * COUT + tid] = s;
     }
   }
