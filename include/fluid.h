@@ -469,9 +469,10 @@ FS_API int fs_convergence_record(fs_solver* s, int64_t* steps, int64_t* failed_s
  * keeps the fastest that still meets pressure_tol; the state, dye, time and
  * pressure are restored afterwards.  No reference counterpart. */
 FS_API int fs_autotune(fs_solver* s, double dt, int32_t nsteps, int32_t* pre, int32_t* post, double* ms_per_step);
-/* Tile sides (16, 32 or 64 cells) of the fused multigrid kernels of each tile
- * level (the levels above the bottom solve); 0 = the built-in rule (64 where
- * that gives >= 1024 CTAs, else 32 where that gives >= 256, else 16).  A side
+/* Tile side classes (16, 32 or 64: the larger, the larger the regions) of the
+ * fused multigrid kernels of each tile level (the levels above the bottom
+ * solve); 0 = the built-in rule (64 for levels of more than 1984 cells a side,
+ * else 32 for more than 480, else 16).  A side
  * larger than half its level is not used there (the built-in rule applies;
  * fs_get_mg_tiles reports the side in use).  The tiles give the same values
  * whatever their size, so they change only the speed. */
