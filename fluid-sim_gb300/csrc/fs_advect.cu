@@ -91,15 +91,15 @@ __device__ __forceinline__ void trace(const TV* __restrict__ u, const TV* __rest
 }
 
 // ------------------------------------------------------ tiled advection
-// The advection kernels are gather-bound: a MacCormack step takes about 20
-// bilinear samples per cell.  A CTA stages its 32x16-cell tile of each field
+// A MacCormack step takes about 20 bilinear samples per cell.  A CTA stages its 32x16-cell tile of each field
 // it samples, plus a halo of 4 cells, in shared memory.  When the largest
 // displacement any trace of the tile can reach is at most 3 cells (checked
 // once per CTA on the staged velocities, below) every sample lies in the
-// staged block and is read from there unchecked; otherwise each sample is
-// checked and one whose four cells leave the block falls back to the wrapped
-// global read.  The arithmetic of the three ways is the same, so the results
-// are too.
+// staged block and is read from there unchecked, two cells a thread at once
+// (advect_pair, combine_pair); otherwise each sample is checked and one whose
+// four cells leave the block falls back to the wrapped global read.  (Checked
+// samples may round a departure offset differently, by how the compiler
+// contracts it.)
 constexpr int kTX = 32, kTY = 16, kHalo = 4;
 constexpr int kSW = kTX + 2 * kHalo, kSH = kTY + 2 * kHalo;
 // largest |u| dt/dx (cells) for which every trace stays in the staged block:
@@ -125,7 +125,6 @@ __device__ __forceinline__ void lerp_rows(float a, float b, float c, float d, fl
       : "f"(a), "f"(b), "f"(c), "f"(d), "f"(fx));
 }
 
-template <bool FAST>
 struct TileView {
   const float* sm;  // kSH x kSW staged block
   int oi, oj;       // global (unwrapped) index of the block's element (0, 0)
@@ -141,7 +140,7 @@ struct TileView {
     const float fx = ox - fo, fy = oy - go;
     const int li = bi + (int)fo - oi, lj = bj + (int)go - oj;
     float a, b, c, d;
-    if (FAST || ((unsigned)li < (unsigned)(kSW - 1) && (unsigned)lj < (unsigned)(kSH - 1))) {
+    if ((unsigned)li < (unsigned)(kSW - 1) && (unsigned)lj < (unsigned)(kSH - 1)) {
       const float* p = sm + lj * kSW + li;
       a = p[0]; b = p[1]; c = p[kSW]; d = p[kSW + 1];
     } else {
@@ -162,8 +161,7 @@ struct TileView {
 };
 
 // RK2 midpoint backward trace (src/cpu/advect.js:46-54, shaders.js:117-122) in cells
-template <bool FAST>
-__device__ __forceinline__ void trace_t(const TileView<FAST>& u, const TileView<FAST>& v, int i, int j, Home h,
+__device__ __forceinline__ void trace_t(const TileView& u, const TileView& v, int i, int j, Home h,
                                         float cx, float cy, float& dX, float& dY) {
   const float u1 = u.sample(i, j, h.ux, h.uy);
   const float v1 = v.sample(i, j, h.vx, h.vy);
@@ -178,11 +176,9 @@ __device__ __forceinline__ void trace_t(const TileView<FAST>& u, const TileView<
 // forward pass: the face's own component at the home point sits on a grid
 // point (offsets 0, 0), where the bilinear sample equals the stored value for
 // every finite field, so it is passed in (own, read from the staged block)
-// instead of sampled.  Forward kernel 55.4 -> 53.0 us at 2048^2; in the
-// combine kernel the same change measured slower (59.9 -> 63.3 us), which
-// keeps trace_t.
-template <bool FAST, bool UFACE>
-__device__ __forceinline__ void trace_face(const TileView<FAST>& u, const TileView<FAST>& v, int i, int j,
+// instead of sampled.
+template <bool UFACE>
+__device__ __forceinline__ void trace_face(const TileView& u, const TileView& v, int i, int j,
                                            float own, float cx, float cy, float& dX, float& dY) {
   const Home h = UFACE ? home_u() : home_v();
   const float u1 = UFACE ? own : u.sample(i, j, h.ux, h.uy);
@@ -226,7 +222,12 @@ __device__ __forceinline__ void stage_tiles(float* const (&sm)[F], const float* 
 __device__ __forceinline__ uint32_t smem_absmax_bits(const float* sm) {
   const int tid = threadIdx.y * blockDim.x + threadIdx.x, nthr = blockDim.x * blockDim.y;
   uint32_t m = 0;
-  for (int k = tid; k < kSW * kSH; k += nthr) m = max(m, __float_as_uint(fabsf(sm[k])));
+  static_assert(kSW * kSH % 4 == 0, "whole float4 groups");
+  for (int k = tid; k < kSW * kSH / 4; k += nthr) {
+    const float4 x = reinterpret_cast<const float4*>(sm)[k];
+    m = max(max(m, __float_as_uint(fabsf(x.x))), __float_as_uint(fabsf(x.y)));
+    m = max(max(m, __float_as_uint(fabsf(x.z))), __float_as_uint(fabsf(x.w)));
+  }
   return m;
 }
 
@@ -248,10 +249,10 @@ __device__ __forceinline__ bool tma_stage(float* const (&sm)[F], const CUtensorM
 #pragma unroll
     for (int q = 0; q < F; q++) tc::tma_load_2d(sm[q], tm[q], oi, oj, bar);
   }
-  const bool ok = __syncthreads_and(tc::mbar_wait(bar, 0)) != 0;
+  const bool ok = __syncthreads_and(tc::mbar_wait_idle(bar, 0)) != 0;
   if (!ok) {
     if (tid == 0) atomicExch(err, 1);
-    tc::mbar_wait(bar, 0);
+    tc::mbar_wait_idle(bar, 0);
   }
   return ok;
 }
@@ -262,13 +263,132 @@ __device__ __forceinline__ bool fast_tile(float umax, float vmax, float cx, floa
   return __syncthreads_and(ok) != 0;
 }
 
+// ------------------------------------------------ a fast tile, two rows at once
+// Both kernels are bound by the number of instructions they issue (2048^2: 83%
+// of the issue slots taken, 320 instructions a cell, 34 of them shared loads).
+// A thread of a fast tile has two cells, 8 rows apart: their coordinates,
+// weights and interpolations are computed in pairs by packed f32x2 multiply-adds
+// (sm_100 and later), the same roundings per cell as the scalar code after
+// contraction.  The floor of an offset x (|x| < 2^22) is taken by adding 1.5 *
+// 2^23, rounded down, which leaves the integer in the sum's low bits; row and
+// column are joined by one multiply-add in that form.  With waits for the TMA
+// copies that do not spin (they took issue slots too), 4096^2: forward 175 -> 152
+// us, combine 195 -> 160 us, of which the bytes are 79 us and 99 us.
+struct F2 {
+  unsigned long long v;
+};
+__device__ __forceinline__ F2 f2(float a, float b) {
+  F2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ F2 f2(float a) { return f2(a, a); }
+__device__ __forceinline__ void split(F2 a, float& x, float& y) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(a.v));
+}
+__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
+  F2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+  return r;
+}
+__device__ __forceinline__ F2 sub2(F2 a, F2 b) { return fma2(b, f2(-1.f), a); }
+__device__ __forceinline__ F2 add2_down(F2 a, F2 b) {
+  float x, y, u, v;
+  split(a, x, y);
+  split(b, u, v);
+  return f2(__fadd_rd(x, u), __fadd_rd(y, v));
+}
+// top = a + (b - a) fx, bot = c + (d - c) fx, top + (bot - top) fy
+__device__ __forceinline__ F2 lerp2(F2 a, F2 b, F2 c, F2 d, F2 fx, F2 fy) {
+  const F2 top = fma2(sub2(b, a), fx, a), bot = fma2(sub2(d, c), fx, c);
+  return fma2(sub2(bot, top), fy, top);
+}
+
+// a staged block seen from this thread's two cells: sm points at the upper of
+// them, the other is kPair words on
+constexpr int kPair = 8 * kSW;
+struct PairView {
+  const float* sm;
+  __device__ __forceinline__ F2 at(int k) const { return f2(sm[k], sm[k + kPair]); }
+  // sample halfway between four cells, the first k words from the home cell
+  __device__ __forceinline__ F2 half(int k) const {
+    return lerp2(at(k), at(k + 1), at(k + kSW), at(k + kSW + 1), f2(0.5f), f2(0.5f));
+  }
+  template <bool RANGE = false>
+  __device__ __forceinline__ F2 sample(F2 ox, F2 oy, float* lo = nullptr, float* hi = nullptr) const {
+    const F2 magic = f2(12582912.f);
+    const F2 mx = add2_down(ox, magic), my = add2_down(oy, magic);
+    const F2 go = sub2(my, magic);
+    const F2 fx = sub2(ox, sub2(mx, magic)), fy = sub2(oy, go);
+    float i0, i1;
+    split(fma2(go, f2((float)kSW), mx), i0, i1);
+    const float* p = sm + (__float_as_int(i0) - 0x4b400000);
+    const float* q = sm + (__float_as_int(i1) - 0x4b400000) + kPair;
+    const float a0 = p[0], b0 = p[1], c0 = p[kSW], d0 = p[kSW + 1];
+    const float a1 = q[0], b1 = q[1], c1 = q[kSW], d1 = q[kSW + 1];
+    if (RANGE) {
+      lo[0] = fminf(fminf(a0, b0), fminf(c0, d0));
+      hi[0] = fmaxf(fmaxf(a0, b0), fmaxf(c0, d0));
+      lo[1] = fminf(fminf(a1, b1), fminf(c1, d1));
+      hi[1] = fmaxf(fmaxf(a1, b1), fmaxf(c1, d1));
+    }
+    return lerp2(f2(a0, a1), f2(b0, b1), f2(c0, c1), f2(d0, d1), fx, fy);
+  }
+};
+
+// offsets of the departure point on the face's own grid.  A face's own
+// component at home is the stored value (the sample at offsets 0, 0).
+template <bool UFACE>
+__device__ __forceinline__ void trace_pair(const PairView& u, const PairView& v, float cx, float cy, F2& dx, F2& dy) {
+  const Home h = UFACE ? home_u() : home_v();
+  const F2 u1 = UFACE ? u.at(0) : u.half(-kSW), v1 = UFACE ? v.half(-1) : v.at(0);
+  const F2 hx = f2(-0.5f * cx), hy = f2(-0.5f * cy);
+  const F2 u2 = u.sample(fma2(hx, u1, f2(h.ux)), fma2(hy, v1, f2(h.uy)));
+  const F2 v2 = v.sample(fma2(hx, u1, f2(h.vx)), fma2(hy, v1, f2(h.vy)));
+  dx = fma2(f2(-cx), u2, f2(0.f));
+  dy = fma2(f2(-cy), v2, f2(0.f));
+}
+
+__device__ __forceinline__ void advect_pair(const float* su, const float* sv, float* __restrict__ ou,
+                                            float* __restrict__ ov, int nx, int ny, int ti, int tj, float cx, float cy,
+                                            float* __restrict__ bounds) {
+  const int i = ti + threadIdx.x, j = tj + threadIdx.y;
+  if (i >= nx || j >= ny) return;
+  const int lc = (threadIdx.y + kHalo) * kSW + threadIdx.x + kHalo;
+  const PairView U{su + lc}, V{sv + lc};
+  const int64_t n = (int64_t)nx * ny, c = (int64_t)j * nx + i, c1 = c + 8 * (int64_t)nx;
+  const bool two = j + 8 < ny;
+  F2 dx, dy;
+  float r0, r1, lo[2], hi[2];
+#pragma unroll
+  for (int k = 0; k < 2; k++) {
+    if (k == 0) trace_pair<true>(U, V, cx, cy, dx, dy);
+    else trace_pair<false>(U, V, cx, cy, dx, dy);
+    float* o = k == 0 ? ou : ov;
+    const PairView& F = k == 0 ? U : V;
+    if (bounds) {
+      split(F.sample<true>(dx, dy, lo, hi), r0, r1);
+      float* b = bounds + 2 * k * n;
+      b[c] = lo[0];
+      b[n + c] = hi[0];
+      if (two) {
+        b[c1] = lo[1];
+        b[n + c1] = hi[1];
+      }
+    } else {
+      split(F.sample(dx, dy), r0, r1);
+    }
+    o[c] = r0;
+    if (two) o[c1] = r1;
+  }
+}
+
 // ADVECT_VELOCITY: each component traced from its own face (shaders.js:126-146).
 // With bounds != nullptr (the forward pass of MacCormack) the min and max of
 // the four cells each sample read -- the limiter's range, src/cpu/advect.js
 // :104-111 -- are written too, planes (lo_u, hi_u, lo_v, hi_v), so the combine
 // pass does not trace forward again.
-template <bool FAST>
-__device__ __forceinline__ void advect_rows(const TileView<FAST>& U, const TileView<FAST>& V, float* __restrict__ ou,
+__device__ __forceinline__ void advect_rows(const TileView& U, const TileView& V, float* __restrict__ ou,
                                             float* __restrict__ ov, int nx, int ny, int ti, int tj, float cx,
                                             float cy, float* __restrict__ bounds) {
   const Home hu = home_u(), hv = home_v();
@@ -281,17 +401,17 @@ __device__ __forceinline__ void advect_rows(const TileView<FAST>& U, const TileV
     const int64_t c = (int64_t)j * nx + i;
     const int lc = (r + kHalo) * kSW + threadIdx.x + kHalo;  // this cell in the staged block
     float dX, dY, lo, hi;
-    trace_face<FAST, true>(U, V, i, j, U.sm[lc], cx, cy, dX, dY);
+    trace_face<true>(U, V, i, j, U.sm[lc], cx, cy, dX, dY);
     if (bounds) {
-      ou[c] = U.template sample<true>(i, j, hu.ux + dX, hu.uy + dY, &lo, &hi);
+      ou[c] = U.sample<true>(i, j, hu.ux + dX, hu.uy + dY, &lo, &hi);
       bounds[c] = lo;
       bounds[n + c] = hi;
     } else {
       ou[c] = U.sample(i, j, hu.ux + dX, hu.uy + dY);
     }
-    trace_face<FAST, false>(U, V, i, j, V.sm[lc], cx, cy, dX, dY);
+    trace_face<false>(U, V, i, j, V.sm[lc], cx, cy, dX, dY);
     if (bounds) {
-      ov[c] = V.template sample<true>(i, j, hv.vx + dX, hv.vy + dY, &lo, &hi);
+      ov[c] = V.sample<true>(i, j, hv.vx + dX, hv.vy + dY, &lo, &hi);
       bounds[2 * n + c] = lo;
       bounds[3 * n + c] = hi;
     } else {
@@ -326,10 +446,9 @@ __global__ void __launch_bounds__(256) k_advect_sl_t(const float* __restrict__ u
     }
   }
   if (fast_tile(umax, vmax, cx, cy)) {
-    const TileView<true> U{su, oi, oj, u, nx, ny}, V{sv, oi, oj, v, nx, ny};
-    advect_rows(U, V, ou, ov, nx, ny, ti, tj, cx, cy, bounds);
+    advect_pair(su, sv, ou, ov, nx, ny, ti, tj, cx, cy, bounds);
   } else {
-    const TileView<false> U{su, oi, oj, u, nx, ny}, V{sv, oi, oj, v, nx, ny};
+    const TileView U{su, oi, oj, u, nx, ny}, V{sv, oi, oj, v, nx, ny};
     advect_rows(U, V, ou, ov, nx, ny, ti, tj, cx, cy, bounds);
   }
 }
@@ -337,9 +456,8 @@ __global__ void __launch_bounds__(256) k_advect_sl_t(const float* __restrict__ u
 // MACCORMACK: the backward pass (ADVECT_FIELD_BY with -dt) is evaluated inside
 // the combine kernel at the single point it is needed, then the correction
 // limited to the forward pass's range (shaders.js:187-231, src/cpu/advect.js:149-185).
-template <bool FAST>
-__device__ __forceinline__ void combine_rows(const TileView<FAST>& U, const TileView<FAST>& V,
-                                             const TileView<FAST>& FU, const TileView<FAST>& FV,
+__device__ __forceinline__ void combine_rows(const TileView& U, const TileView& V,
+                                             const TileView& FU, const TileView& FV,
                                              const float* __restrict__ bounds, float* __restrict__ ou,
                                              float* __restrict__ ov, int nx, int ny, int ti, int tj, float cx,
                                              float cy) {
@@ -367,6 +485,35 @@ __device__ __forceinline__ void combine_rows(const TileView<FAST>& U, const Tile
     cv = cv < lov ? lov : cv > hiv ? hiv : cv;
     ou[c] = cu;
     ov[c] = cv;
+  }
+}
+
+__device__ __forceinline__ void combine_pair(const float* su, const float* sv, const float* sfu, const float* sfv,
+                                             const float* __restrict__ bounds, float* __restrict__ ou,
+                                             float* __restrict__ ov, int nx, int ny, int ti, int tj, float cx,
+                                             float cy) {
+  const int i = ti + threadIdx.x, j = tj + threadIdx.y;
+  if (i >= nx || j >= ny) return;
+  const int lc = (threadIdx.y + kHalo) * kSW + threadIdx.x + kHalo;
+  const PairView U{su + lc}, V{sv + lc};
+  const int64_t n = (int64_t)nx * ny, c = (int64_t)j * nx + i, c1 = c + 8 * (int64_t)nx;
+  const bool two = j + 8 < ny;
+#pragma unroll
+  for (int k = 0; k < 2; k++) {
+    const float* b = bounds + 2 * k * n;
+    const float lo0 = __ldg(b + c), hi0 = __ldg(b + n + c);
+    const float lo1 = two ? __ldg(b + c1) : 0.f, hi1 = two ? __ldg(b + n + c1) : 0.f;
+    const PairView& own = k == 0 ? U : V;
+    const PairView F{(k == 0 ? sfu : sfv) + lc};
+    F2 dx, dy;
+    // backward: trace with -dt
+    if (k == 0) trace_pair<true>(U, V, -cx, -cy, dx, dy);
+    else trace_pair<false>(U, V, -cx, -cy, dx, dy);
+    float r0, r1;
+    split(fma2(f2(0.5f), sub2(own.at(0), F.sample(dx, dy)), F.at(0)), r0, r1);
+    float* o = k == 0 ? ou : ov;
+    o[c] = r0 < lo0 ? lo0 : r0 > hi0 ? hi0 : r0;
+    if (two) o[c1] = r1 < lo1 ? lo1 : r1 > hi1 ? hi1 : r1;
   }
 }
 
@@ -399,12 +546,10 @@ __global__ void __launch_bounds__(256) k_mc_combine_t(const float* __restrict__ 
     }
   }
   if (fast_tile(umax, vmax, cx, cy)) {
-    const TileView<true> U{su, oi, oj, u, nx, ny}, V{sv, oi, oj, v, nx, ny};
-    const TileView<true> FU{sfu, oi, oj, fu, nx, ny}, FV{sfv, oi, oj, fv, nx, ny};
-    combine_rows(U, V, FU, FV, bounds, ou, ov, nx, ny, ti, tj, cx, cy);
+    combine_pair(su, sv, sfu, sfv, bounds, ou, ov, nx, ny, ti, tj, cx, cy);
   } else {
-    const TileView<false> U{su, oi, oj, u, nx, ny}, V{sv, oi, oj, v, nx, ny};
-    const TileView<false> FU{sfu, oi, oj, fu, nx, ny}, FV{sfv, oi, oj, fv, nx, ny};
+    const TileView U{su, oi, oj, u, nx, ny}, V{sv, oi, oj, v, nx, ny};
+    const TileView FU{sfu, oi, oj, fu, nx, ny}, FV{sfv, oi, oj, fv, nx, ny};
     combine_rows(U, V, FU, FV, bounds, ou, ov, nx, ny, ti, tj, cx, cy);
   }
 }
@@ -449,10 +594,9 @@ __global__ void __launch_bounds__(256) k_advect_sl_class(const AdvTab tab, int n
     stage_tiles<2>(sm, f, oi, oj, nx, ny, umax, vmax);
   }
   if (fast_tile(umax, vmax, a.cx, a.cy)) {
-    const TileView<true> U{su, oi, oj, a.u, nx, ny}, V{sv, oi, oj, a.v, nx, ny};
-    advect_rows(U, V, a.ou, a.ov, nx, ny, ti, tj, a.cx, a.cy, a.bounds);
+    advect_pair(su, sv, a.ou, a.ov, nx, ny, ti, tj, a.cx, a.cy, a.bounds);
   } else {
-    const TileView<false> U{su, oi, oj, a.u, nx, ny}, V{sv, oi, oj, a.v, nx, ny};
+    const TileView U{su, oi, oj, a.u, nx, ny}, V{sv, oi, oj, a.v, nx, ny};
     advect_rows(U, V, a.ou, a.ov, nx, ny, ti, tj, a.cx, a.cy, a.bounds);
   }
 }
@@ -472,12 +616,10 @@ __global__ void __launch_bounds__(256) k_mc_combine_class(const AdvTab tab, int 
     stage_tiles<4>(sm, f, oi, oj, nx, ny, umax, vmax);
   }
   if (fast_tile(umax, vmax, a.cx, a.cy)) {
-    const TileView<true> U{su, oi, oj, a.u, nx, ny}, V{sv, oi, oj, a.v, nx, ny};
-    const TileView<true> FU{sfu, oi, oj, a.fu, nx, ny}, FV{sfv, oi, oj, a.fv, nx, ny};
-    combine_rows(U, V, FU, FV, a.bounds, a.ou, a.ov, nx, ny, ti, tj, a.cx, a.cy);
+    combine_pair(su, sv, sfu, sfv, a.bounds, a.ou, a.ov, nx, ny, ti, tj, a.cx, a.cy);
   } else {
-    const TileView<false> U{su, oi, oj, a.u, nx, ny}, V{sv, oi, oj, a.v, nx, ny};
-    const TileView<false> FU{sfu, oi, oj, a.fu, nx, ny}, FV{sfv, oi, oj, a.fv, nx, ny};
+    const TileView U{su, oi, oj, a.u, nx, ny}, V{sv, oi, oj, a.v, nx, ny};
+    const TileView FU{sfu, oi, oj, a.fu, nx, ny}, FV{sfv, oi, oj, a.fv, nx, ny};
     combine_rows(U, V, FU, FV, a.bounds, a.ou, a.ov, nx, ny, ti, tj, a.cx, a.cy);
   }
 }
