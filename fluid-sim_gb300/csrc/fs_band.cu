@@ -80,8 +80,8 @@ struct ModeCoef {
 };
 
 // Mode m of this step: wave numbers and the two complex coefficients.  Every
-// block of the column kernel regenerates the list (at most kMaxBandModes
-// modes), so no block waits for another.
+// block of the column kernel regenerates the modes it adds, so no block waits
+// for another.
 __device__ void band_mode(int kind, int m, uint32_t step, uint64_t seed, double kf, double width, double s,
                           const int2* __restrict__ lattice, ModeCoef* out) {
   double kx, ky, A, phi;
@@ -120,20 +120,37 @@ __device__ void band_mode(int kind, int m, uint32_t step, uint64_t seed, double 
 }
 
 // grid (ceil(nx / 256), 2K+1): column sums G_q(i) for ky = q - K, the modes
-// added in the order of their index (deterministic run to run)
+// added in the order of their index (deterministic run to run).  A mode's
+// coefficients take some 150 FP64 instructions, at 1/54 of the FP32 rate, which
+// is all this kernel costs: the GAUSSIAN modes of one ky are a run of the
+// lattice, and only those are made (the 24 of the other kind carry their ky in
+// the draw).  1024^2, kf = 9 +- 1: 14 -> 10 us, one chain of them.
 __global__ void __launch_bounds__(256)
     k_band_columns(int kind, int M, int K, const DevState* __restrict__ st, uint64_t seed, double kf, double width,
                    double s, const int2* __restrict__ lattice, const float2* __restrict__ ex_u,
                    const float2* __restrict__ ex_v, float2* __restrict__ gu, float2* __restrict__ gv, int nx) {
   __shared__ ModeCoef modes[kMaxBandModes];
+  __shared__ int first, last;
   const int q = blockIdx.y - K;
   const uint32_t step = (uint32_t)st->band_step;
-  for (int m = threadIdx.x; m < M; m += blockDim.x) band_mode(kind, m, step, seed, kf, width, s, lattice, modes + m);
+  if (threadIdx.x == 0) {
+    first = kind == FS_BAND_REFERENCE ? 0 : M;
+    last = kind == FS_BAND_REFERENCE ? M - 1 : -1;
+  }
+  __syncthreads();
+  for (int m = threadIdx.x; m < M; m += blockDim.x) {
+    if (kind != FS_BAND_REFERENCE) {
+      if (lattice[m].y != q) continue;
+      atomicMin(&first, m);
+      atomicMax(&last, m);
+    }
+    band_mode(kind, m, step, seed, kf, width, s, lattice, modes + m);
+  }
   __syncthreads();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nx) return;
   float2 au = make_float2(0.f, 0.f), av = make_float2(0.f, 0.f);
-  for (int m = 0; m < M; m++) {
+  for (int m = first; m <= last; m++) {
     const ModeCoef& c = modes[m];
     if (c.ky != q || c.kx < -K || c.kx > K) continue;
     const float2 eu = __ldg(ex_u + (size_t)(c.kx + K) * nx + i), ev = __ldg(ex_v + (size_t)(c.kx + K) * nx + i);
@@ -147,25 +164,79 @@ __global__ void __launch_bounds__(256)
 }
 
 // u = (u + Re sum_q G_q(i) e^{i q y_j}) * damp, in place; the first thread of
-// the grid advances the step counter (no block of this kernel reads it)
+// the grid advances the step counter (no block of this kernel reads it).  A
+// block stages the sums of its 64 columns and the phases of its 32 rows, 32 ky at
+// a time, a thread has four rows of two columns: a cell a thread loaded four
+// table entries from L1 for four multiply-adds.  1024^2, 23 values of ky: 31 ->
+// 12 us.
+constexpr int kBandRows = 4, kBandTX = 64, kBandTY = 8 * kBandRows, kBandQ = 32;
+struct BandStage {
+  float2 gu[kBandQ][kBandTX], gv[kBandQ][kBandTX], eu[kBandQ][kBandTY], ev[kBandQ][kBandTY];
+};
 __global__ void __launch_bounds__(256)
     k_band_apply(float* __restrict__ u, float* __restrict__ v, int nx, int ny, int K,
                  const float2* __restrict__ gu, const float2* __restrict__ gv, const float2* __restrict__ ey_u,
                  const float2* __restrict__ ey_v, float damp, DevState* __restrict__ st) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
-  if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0 && threadIdx.y == 0) st->band_step += 1;
-  if (i >= nx || j >= ny) return;
-  float fu = 0.f, fv = 0.f;
+  extern __shared__ __align__(16) unsigned char band_smem[];
+  BandStage& t = *reinterpret_cast<BandStage*>(band_smem);
+  const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * 32 + tx;
+  const int i0 = blockIdx.x * kBandTX, j0 = blockIdx.y * kBandTY;
+  if (blockIdx.x == 0 && blockIdx.y == 0 && tid == 0) st->band_step += 1;
+  float uc[kBandRows][2], vc[kBandRows][2];
+#pragma unroll
+  for (int r = 0; r < kBandRows; r++)
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+      const int64_t c = (int64_t)min(j0 + ty * kBandRows + r, ny - 1) * nx + min(i0 + tx + 32 * k, nx - 1);
+      uc[r][k] = u[c];
+      vc[r][k] = v[c];
+    }
+  float fu[kBandRows][2] = {}, fv[kBandRows][2] = {};
   const int nq = 2 * K + 1;
-  for (int q = 0; q < nq; q++) {
-    const float2 a = __ldg(gu + (size_t)q * nx + i), b = __ldg(ey_u + (size_t)q * ny + j);
-    const float2 c = __ldg(gv + (size_t)q * nx + i), d = __ldg(ey_v + (size_t)q * ny + j);
-    fu = fmaf(a.x, b.x, fmaf(-a.y, b.y, fu));
-    fv = fmaf(c.x, d.x, fmaf(-c.y, d.y, fv));
+  for (int q0 = 0; q0 < nq; q0 += kBandQ) {
+    const int nb = min(kBandQ, nq - q0);
+    if (q0 > 0) __syncthreads();
+#pragma unroll 4
+    for (int q = tid / kBandTX; q < nb; q += 256 / kBandTX) {
+      const int c = tid % kBandTX, i = min(i0 + c, nx - 1);
+      t.gu[q][c] = __ldg(gu + (size_t)(q0 + q) * nx + i);
+      t.gv[q][c] = __ldg(gv + (size_t)(q0 + q) * nx + i);
+    }
+#pragma unroll 4
+    for (int q = tid / kBandTY; q < nb; q += 256 / kBandTY) {
+      const int r = tid % kBandTY, j = min(j0 + r, ny - 1);
+      t.eu[q][r] = __ldg(ey_u + (size_t)(q0 + q) * ny + j);
+      t.ev[q][r] = __ldg(ey_v + (size_t)(q0 + q) * ny + j);
+    }
+    __syncthreads();
+#pragma unroll 4
+    for (int q = 0; q < nb; q++) {
+      const float2 a[2] = {t.gu[q][tx], t.gu[q][tx + 32]}, c[2] = {t.gv[q][tx], t.gv[q][tx + 32]};
+#pragma unroll
+      for (int r = 0; r < kBandRows; r += 2) {
+        // the phases of two rows
+        const float4 b = *reinterpret_cast<const float4*>(&t.eu[q][ty * kBandRows + r]);
+        const float4 d = *reinterpret_cast<const float4*>(&t.ev[q][ty * kBandRows + r]);
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+          fu[r][k] = fmaf(a[k].x, b.x, fmaf(-a[k].y, b.y, fu[r][k]));
+          fv[r][k] = fmaf(c[k].x, d.x, fmaf(-c[k].y, d.y, fv[r][k]));
+          fu[r + 1][k] = fmaf(a[k].x, b.z, fmaf(-a[k].y, b.w, fu[r + 1][k]));
+          fv[r + 1][k] = fmaf(c[k].x, d.z, fmaf(-c[k].y, d.w, fv[r + 1][k]));
+        }
+      }
+    }
   }
-  const int64_t c = (int64_t)j * nx + i;
-  u[c] = (u[c] + fu) * damp;
-  v[c] = (v[c] + fv) * damp;
+#pragma unroll
+  for (int r = 0; r < kBandRows; r++)
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+      const int i = i0 + tx + 32 * k, j = j0 + ty * kBandRows + r;
+      if (i >= nx || j >= ny) continue;
+      const int64_t c = (int64_t)j * nx + i;
+      u[c] = (uc[r][k] + fu[r][k]) * damp;
+      v[c] = (vc[r][k] + fv[r][k]) * damp;
+    }
 }
 
 void free_band(Band* b) {
@@ -253,6 +324,8 @@ int band_set(Solver* s, const fs_band* p) {
   return FS_OK;
 }
 
+static_assert(sizeof(BandStage) <= 48 * 1024, "no opt-in to larger dynamic shared memory");
+
 void launch_band(Solver* s, float* u, float* v, float dt) {
   Band* b = static_cast<Band*>(s->band);
   const Grid& g = s->g;
@@ -264,7 +337,8 @@ void launch_band(Solver* s, float* u, float* v, float dt) {
                 b->kind, b->M, b->K, s->dev, b->seed, b->kf, b->width, scale, b->lattice, b->ex_u, b->ex_v, b->gu,
                 b->gv, g.nx));
   FS_LAUNCH(s, "band_apply", (double)s->n * 16,
-            k_band_apply<<<grid2d(g.nx, g.ny, dim3(32, 8)), dim3(32, 8), 0, s->stream>>>(
+            k_band_apply<<<dim3((g.nx + kBandTX - 1) / kBandTX, (g.ny + kBandTY - 1) / kBandTY), dim3(32, 8),
+                         sizeof(BandStage), s->stream>>>(
                 u, v, g.nx, g.ny, b->K, b->gu, b->gv, b->ey_u, b->ey_v, damp, s->dev));
 }
 
