@@ -286,10 +286,10 @@ static void correction_solve(Solver* s, int iterations) {
 //   F32:   one V-cycle on (p32, div32) from the current p [+ max|div - lap p|]
 //   MIXED: one V-cycle on (r32 -> e) from zero, p += e (double-float), then
 //          r = d - lap p -> r32 and max|r|.
-// The fused F32 cycle always reads p (the zero-initial-guess shortcut would
-// change the kernel sequence from the first cycle to the next, which a
-// replayed loop body cannot do); reading a zero p gives the same bits.
-static void mg_cycle(Solver* s, bool residual) {
+// The fused F32 cycle reads p, except (zero) in the first cycle of a fixed count
+// that starts from zero; inside a captured loop the kernels cannot change from
+// the first cycle to the next, and reading a zero p gives the same bits.
+static void mg_cycle(Solver* s, bool residual, bool zero = false) {
   if (s->mixed) {
     s->lev[0].x = s->e32;
     s->lev[0].x2 = s->e32b;
@@ -307,7 +307,7 @@ static void mg_cycle(Solver* s, bool residual) {
   }
   s->lev[0].x = s->p32;
   s->lev[0].x2 = s->p32b;
-  if (s->fused) mg_vcycle_fused(s, true);
+  if (s->fused) mg_vcycle_fused(s, true, nullptr, nullptr, zero);
   else mg_vcycle(s);
   s->p32 = s->lev[0].x;
   s->p32b = s->lev[0].x2;
@@ -404,15 +404,15 @@ static int pressure_solve(Solver* s, bool capture, bool defer = false, bool star
       launch_fill(s, s->pl, 0.f, s->n);
     }
   } else {
-    // a fixed count of flat sweeps starts from zero by itself
-    if (!P.warm_start && (mg || tol)) launch_fill(s, s->p32, 0.f, s->n);
+    // a fixed count of flat sweeps or fused cycles starts from zero by itself
+    if (!P.warm_start && (tol || (mg && (!s->fused || iters == 0)))) launch_fill(s, s->p32, 0.f, s->n);
     if (tol) launch_absmax_residual32(s, s->p32, s->div32);
   }
   if (!tol) {
     if (mg) {
       for (int k = 0; k < iters; k++) {
         s->mg_cycle_index = k;
-        mg_cycle(s, false);
+        mg_cycle(s, false, k == 0 && !P.warm_start && !s->guess);
       }
       s->mg_cycle_index = -1;
     } else if (s->mixed) {
@@ -456,21 +456,25 @@ static int pressure_solve(Solver* s, bool capture, bool defer = false, bool star
 }
 
 // divergence of (wu, wv) -> solve -> state velocity = w - grad p
-static int project_finish(Solver* s, const float* wu, const float* wv) {
-  if (s->mixed) launch_subgrad_df(s, wu, nullptr, wv, nullptr, s->ph, s->pl, s->u, s->ulo, s->v, s->vlo);
-  else launch_subtract_gradient_f32(s, wu, wv, s->p32, s->u, s->v);
+static int project_finish(Solver* s, const float* wu, const float* wv, const StepFinish& fin = {}) {
+  if (s->mixed) launch_subgrad_df(s, wu, nullptr, wv, nullptr, s->ph, s->pl, s->u, s->ulo, s->v, s->vlo, fin);
+  else launch_subtract_gradient_f32(s, wu, wv, s->p32, s->u, s->v, fin);
   return check_launch(s);
 }
 
+static StepFinish step_end(const Solver* s, double dt) { return {s->dev, dt, s->stats_on_device ? 1 : 0}; }
+
+// step_dt: the projection ends a step.
 // defer: stop after the start of the pressure solve (see pressure_solve)
-static int project_from(Solver* s, const float* wu, const float* wv, bool capture, bool defer = false) {
+static int project_from(Solver* s, const float* wu, const float* wv, bool capture, bool defer = false,
+                        const double* step_dt = nullptr) {
   const bool start = s->mixed && !s->guess && !s->prm.warm_start;
   if (start) launch_div_start(s, wu, wv);
   else if (s->mixed) launch_div_df(s, wu, nullptr, wv, nullptr, s->dh, s->dl);
   else launch_divergence<float, float>(s, wu, wv, s->div32);
   int rc = pressure_solve(s, capture, defer, start);
   if (defer) return rc;
-  int rc2 = project_finish(s, wu, wv);
+  int rc2 = project_finish(s, wu, wv, step_dt ? step_end(s, *step_dt) : StepFinish{});
   return rc ? rc : rc2;
 }
 
@@ -503,7 +507,7 @@ static int enqueue_step(Solver* s, double dt, bool capture, StepSplit* split = n
   if (s->n_modes > 0) launch_forcing(s, cu, cv, fdt);
   if (s->channel_on) launch_channel(s, cu, cv);
   if (!s->disks.empty()) launch_solids(s, cu, cv, fdt, false);
-  int rc = project_from(s, cu, cv, capture, split != nullptr);
+  int rc = project_from(s, cu, cv, capture, split != nullptr, &dt);
   if (split) {
     split->wu = cu;
     split->wv = cv;
@@ -511,14 +515,12 @@ static int enqueue_step(Solver* s, double dt, bool capture, StepSplit* split = n
   }
   // dye through the now divergence-free field (solver.js:516, 577-586)
   if (s->dye) launch_advect_dye(s, fdt);
-  launch_step_finish(s, dt);
   return rc;
 }
 
 static int enqueue_step_back(Solver* s, double dt, const StepSplit& split) {
-  int rc = project_finish(s, split.wu, split.wv);
+  int rc = project_finish(s, split.wu, split.wv, step_end(s, dt));
   if (s->dye) launch_advect_dye(s, (float)dt);
-  launch_step_finish(s, dt);
   return rc;
 }
 
@@ -1703,7 +1705,7 @@ static int batch_build(fs_batch* b, const double* dt) {
       const int nproj = launch_front_project_class(ms.data(), count, wu.data(), wv.data(), cdt.data(), cs);
       rc = capture_class_loop(b, b->classes[c], cs, b->d_iters + c, 2);
       if (rc == FS_OK) launch_back_class(ms.data(), count, wu.data(), wv.data(), cdt.data(), cs);
-      class_fixed += (ms[0]->prm.advection == FS_ADVECT_MACCORMACK ? 2 : 1) + (ms[0]->prm.nu > 0 ? 1 : 0) + nproj + 2;
+      class_fixed += (ms[0]->prm.advection == FS_ADVECT_MACCORMACK ? 2 : 1) + (ms[0]->prm.nu > 0 ? 1 : 0) + nproj + 1;
       if (rc == FS_OK && cudaGetLastError() != cudaSuccess) rc = bfail(b, FS_ERR_CUDA, "batch: class launch failed");
       if (rc == FS_OK && cudaEventRecord(b->class_done[c], cs) != cudaSuccess) rc = FS_ERR_CUDA;
       if (rc == FS_OK && cudaStreamWaitEvent(b->stream, b->class_done[c], 0) != cudaSuccess) rc = FS_ERR_CUDA;

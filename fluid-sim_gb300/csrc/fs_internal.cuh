@@ -244,13 +244,21 @@ void launch_band(Solver* s, float* u, float* v, float dt);
 // fs_pressure.cu
 template <class TV, class TD>
 void launch_divergence(Solver* s, const TV* u, const TV* v, TD* d);
+// the step's end, done along with its gradient subtraction (st == nullptr: none)
+struct StepFinish {
+  DevState* st = nullptr;
+  double dt = 0;
+  int track = 0;  // the step's tolerance loop ran on the device: add to the record
+};
 void launch_subtract_gradient_f32(Solver* s, const float* wu, const float* wv, const float* p,
-                                  float* ou, float* ov);
+                                  float* ou, float* ov,
+                                  const StepFinish& fin = {});
 // double-float (MIXED) variants; lo planes of the input velocity may be nullptr
 void launch_div_df(Solver* s, const float* uh, const float* ul, const float* vh, const float* vl, float* dh,
                    float* dl);
 void launch_subgrad_df(Solver* s, const float* wuh, const float* wul, const float* wvh, const float* wvl,
-                       const float* ph, const float* pl, float* uh, float* ul, float* vh, float* vl);
+                       const float* ph, const float* pl, float* uh, float* ul, float* vh, float* vl,
+                       const StepFinish& fin = {});
 void launch_d_to_df(Solver* s, const double* x, float* hi, float* lo, int64_t n);
 void launch_df_to_d(Solver* s, const float* hi, const float* lo, double* x, int64_t n);
 void launch_df_to_f(Solver* s, const float* hi, const float* lo, float* x, int64_t n);
@@ -285,7 +293,6 @@ void launch_absmax_residual32(Solver* s, const float* p, const float* d);
 // tolerance loop state on the device (fs_pressure.cu)
 void launch_cond_init(Solver* s, cudaGraphConditionalHandle h, bool graph);
 void launch_cond_step(Solver* s, cudaGraphConditionalHandle h, bool graph);
-void launch_step_finish(Solver* s, double dt);
 void launch_poisson_norms(Solver* s, const float* p, const float* d, float h2f, double h2);
 void launch_convert(Solver* s, const void* src, int src_f64, void* dst, int dst_f64, int64_t n);
 
@@ -295,7 +302,8 @@ void launch_convert(Solver* s, const void* src, int src_f64, void* dst, int dst_
 void mg_vcycle(Solver* s);
 // acc_h/acc_l != nullptr: the level-0 up kernel adds its correction to the
 // double-float pressure (acc_h, acc_l) in place instead of writing lev[0].x2
-void mg_vcycle_fused(Solver* s, bool first_has_x, float* acc_h = nullptr, float* acc_l = nullptr);
+// zero (with first_has_x): the iterate is zero and is not read
+void mg_vcycle_fused(Solver* s, bool first_has_x, float* acc_h = nullptr, float* acc_l = nullptr, bool zero = false);
 bool mg_fused_supported(const Solver* s);
 // tile side of the kernels of level l (an override or the built-in rule)
 int mg_tile(const Solver* s, int l);

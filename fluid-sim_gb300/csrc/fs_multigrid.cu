@@ -164,25 +164,26 @@ static dim3 region_grid(int n, int members = 1) {
 // cyc: the loop's cycle count on the device that decides (nullptr: the host
 // knows this is the first cycle)
 template <int T, int H>
-static void down_t(Solver* s, Level& L, const Level& C, bool has_x, int first, const int* cyc, bool x_unused) {
+static void down_t(Solver* s, Level& L, const Level& C, bool has_x, bool zero, int first, const int* cyc,
+                   bool x_unused) {
   typedef typename RegionOf<T, H>::R R;
-  double bytes = (double)L.n * L.n * (has_x ? 12.0 : 8.0) + (double)C.n * C.n * 4.0;
+  double bytes = (double)L.n * L.n * (has_x && !zero ? 12.0 : 8.0) + (double)C.n * C.n * 4.0;
   // a first cycle the host knows is profiled under its own name
   const std::string name = level_name(s, L, "mg_down") + (first >= 0 && !cyc ? "_first" : "");
   FS_LAUNCH(s, name.c_str(), bytes,
             k_mg_down<R><<<region_grid<R>(L.n), R::THREADS, 0, s->stream>>>(
-                L.rhs, has_x ? L.x : nullptr, has_x ? L.x2 : L.x, C.rhs, L.n, L.h2, s->prm.mg_pre_smooth,
+                L.rhs, has_x && !zero ? L.x : nullptr, has_x ? L.x2 : L.x, C.rhs, L.n, L.h2, s->prm.mg_pre_smooth,
                 (float)s->prm.relax, cyc, first < s->prm.mg_pre_smooth ? first : s->prm.mg_pre_smooth,
                 x_unused ? 1 : 0));
   if (has_x) std::swap(L.x, L.x2);
 }
 
 template <int H>
-static void down(Solver* s, Level& L, const Level& C, bool has_x, int first, const int* cyc, bool x_unused) {
+static void down(Solver* s, Level& L, const Level& C, bool has_x, bool zero, int first, const int* cyc, bool x_unused) {
   switch (region_side(L.n, mg_tile(s, (int)(&L - s->lev.data())))) {
-    case 64: down_t<64, H>(s, L, C, has_x, first, cyc, x_unused); break;
-    case 32: down_t<32, H>(s, L, C, has_x, first, cyc, x_unused); break;
-    default: down_t<16, H>(s, L, C, has_x, first, cyc, x_unused); break;
+    case 64: down_t<64, H>(s, L, C, has_x, zero, first, cyc, x_unused); break;
+    case 32: down_t<32, H>(s, L, C, has_x, zero, first, cyc, x_unused); break;
+    default: down_t<16, H>(s, L, C, has_x, zero, first, cyc, x_unused); break;
   }
 }
 
@@ -231,7 +232,7 @@ bool mg_fused_supported(const Solver* s) {
   return true;
 }
 
-void mg_vcycle_fused(Solver* s, bool first_has_x, float* acc_h, float* acc_l) {
+void mg_vcycle_fused(Solver* s, bool first_has_x, float* acc_h, float* acc_l, bool zero) {
   std::vector<Level>& L = s->lev;
   const int lb = bottom_first_level(s);
   const fs_params& P = s->prm;
@@ -252,12 +253,12 @@ void mg_vcycle_fused(Solver* s, bool first_has_x, float* acc_h, float* acc_l) {
     const int f = l == 0 ? fpre : -1;
     const bool xu = l == 0 && fpost == 0;  // the first cycle's up kernel reads no iterate here
     switch (P.mg_pre_smooth) {
-      case 1: down<3>(s, L[l], L[l + 1], hx, f, cyc, xu); break;
-      case 2: down<5>(s, L[l], L[l + 1], hx, f, cyc, xu); break;
-      default: down<7>(s, L[l], L[l + 1], hx, f, cyc, xu); break;
+      case 1: down<3>(s, L[l], L[l + 1], hx, zero && l == 0, f, cyc, xu); break;
+      case 2: down<5>(s, L[l], L[l + 1], hx, zero && l == 0, f, cyc, xu); break;
+      default: down<7>(s, L[l], L[l + 1], hx, zero && l == 0, f, cyc, xu); break;
     }
   }
-  const bool hx = lb == 0 && first_has_x;
+  const bool hx = lb == 0 && first_has_x && !zero;
   float* bah = lb == 0 ? acc_h : nullptr;
   float* bal = lb == 0 ? acc_l : nullptr;
   launch_bottom(s, lb, hx, bah, bal);

@@ -50,11 +50,32 @@ void launch_divergence(Solver* s, const TV* u, const TV* v, TD* d) {
 }
 template void launch_divergence<float, float>(Solver*, const float*, const float*, float*);
 
+// end of a step: the time, and (track: the step's tolerance loop ran on the
+// device) the record of every projection -- how many, how many failed, the
+// worst final residual -- that the per-projection statistics overwrite
+__device__ __forceinline__ void finish_step(DevState* st, double dt, int track) {
+  st->t += dt;
+  if (track) {
+    st->rec_steps += 1;
+    if (!st->converged) st->rec_failed += 1;
+    const double m = isfinite(st->res_max) ? st->res_max : INFINITY;
+    if (!(m <= st->rec_worst)) st->rec_worst = m;
+  }
+}
+// done by one thread of the gradient subtraction, which no kernel of the step
+// that reads the state follows: a kernel of its own cost 4 us a step
+__device__ __forceinline__ void finish_step(const StepFinish& f) {
+  if (f.st && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0 && threadIdx.y == 0)
+    finish_step(f.st, f.dt, f.track);
+}
+
 // ------------------------------------------------------ gradient subtraction
 // u -= (p_i - p_{i-1})/dx, v -= (p_j - p_{j-1})/dy (grid.js:209-218)
 __global__ void __launch_bounds__(256)
     k_subgrad_f32(const float* __restrict__ wu, const float* __restrict__ wv, const float* __restrict__ p,
-                  float* __restrict__ ou, float* __restrict__ ov, int nx, int ny, float idx, float idy) {
+                  float* __restrict__ ou, float* __restrict__ ov, int nx, int ny, float idx, float idy,
+                  const StepFinish fin) {
+  finish_step(fin);
   int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
   if (i >= nx || j >= ny) return;
   int im = i == 0 ? nx - 1 : i - 1, jm = j == 0 ? ny - 1 : j - 1;
@@ -65,11 +86,11 @@ __global__ void __launch_bounds__(256)
 }
 
 void launch_subtract_gradient_f32(Solver* s, const float* wu, const float* wv, const float* p,
-                                  float* ou, float* ov) {
+                                  float* ou, float* ov, const StepFinish& fin) {
   const Grid& g = s->g;
   FS_LAUNCH(s, "subtract_gradient", (double)s->n * 20,
             k_subgrad_f32<<<grid2d(g.nx, g.ny, kBlock), kBlock, 0, s->stream>>>(wu, wv, p, ou, ov, g.nx,
-                                                                                g.ny, g.idx, g.idy));
+                                                                                g.ny, g.idx, g.idy, fin));
 }
 // ----------------------------------------------------------------- smoothers
 // damped Jacobi, relaxation factor w (shaders.js:302-325)
@@ -416,7 +437,8 @@ __global__ void __launch_bounds__(256)
     k_subgrad4_df(const float* __restrict__ wuh, const float* __restrict__ wul, const float* __restrict__ wvh,
                   const float* __restrict__ wvl, const float* __restrict__ ph, const float* __restrict__ pl,
                   float* __restrict__ uh, float* __restrict__ ul, float* __restrict__ vh, float* __restrict__ vl,
-                  int nx, int ny, df idx, df idy) {
+                  int nx, int ny, df idx, df idy, const StepFinish fin) {
+  finish_step(fin);
   subgrad4_body(wuh, wul, wvh, wvl, ph, pl, uh, ul, vh, vl, nx, ny, idx, idy);
 }
 
@@ -424,20 +446,22 @@ __global__ void __launch_bounds__(256)
     k_subgrad_df(const float* __restrict__ wuh, const float* __restrict__ wul, const float* __restrict__ wvh,
                  const float* __restrict__ wvl, const float* __restrict__ ph, const float* __restrict__ pl,
                  float* __restrict__ uh, float* __restrict__ ul, float* __restrict__ vh, float* __restrict__ vl,
-                 int nx, int ny, df idx, df idy) {
+                 int nx, int ny, df idx, df idy, const StepFinish fin) {
+  finish_step(fin);
   subgrad_df_body(wuh, wul, wvh, wvl, ph, pl, uh, ul, vh, vl, nx, ny, idx, idy);
 }
 
 void launch_subgrad_df(Solver* s, const float* wuh, const float* wul, const float* wvh, const float* wvl,
-                       const float* ph, const float* pl, float* uh, float* ul, float* vh, float* vl) {
+                       const float* ph, const float* pl, float* uh, float* ul, float* vh, float* vl,
+                       const StepFinish& fin) {
   const Grid& g = s->g;
   FS_LAUNCH(s, "subtract_gradient", (double)s->n * ((wul ? 16 : 8) + 8 + 16),
             if (g.nx % 4 == 0) {
               k_subgrad4_df<<<grid2d(g.nx / 4, g.ny, kBlock), kBlock, 0, s->stream>>>(
-                  wuh, wul, wvh, wvl, ph, pl, uh, ul, vh, vl, g.nx, g.ny, df_host(g.idxd), df_host(g.idyd));
+                  wuh, wul, wvh, wvl, ph, pl, uh, ul, vh, vl, g.nx, g.ny, df_host(g.idxd), df_host(g.idyd), fin);
             } else {
               k_subgrad_df<<<grid2d(g.nx, g.ny, kBlock), kBlock, 0, s->stream>>>(
-                  wuh, wul, wvh, wvl, ph, pl, uh, ul, vh, vl, g.nx, g.ny, df_host(g.idxd), df_host(g.idyd));
+                  wuh, wul, wvh, wvl, ph, pl, uh, ul, vh, vl, g.nx, g.ny, df_host(g.idxd), df_host(g.idyd), fin);
             });
 }
 
@@ -770,21 +794,6 @@ __global__ void k_cond(cudaGraphConditionalHandle h, int use_handle, const doubl
   if (use_handle) cudaGraphSetConditional(h, again ? 1u : 0u);
 }
 
-// end of a step: the time, and (track: the step's tolerance loop ran on the
-// device) the record of every projection -- how many, how many failed, the
-// worst final residual -- that the per-projection statistics overwrite
-__device__ __forceinline__ void finish_step(DevState* st, double dt, int track) {
-  st->t += dt;
-  if (track) {
-    st->rec_steps += 1;
-    if (!st->converged) st->rec_failed += 1;
-    const double m = isfinite(st->res_max) ? st->res_max : INFINITY;
-    if (!(m <= st->rec_worst)) st->rec_worst = m;
-  }
-}
-
-__global__ void k_step_finish(DevState* __restrict__ st, double dt, int track) { finish_step(st, dt, track); }
-
 void launch_cond_init(Solver* s, cudaGraphConditionalHandle h, bool graph) {
   FS_LAUNCH(s, "cond", 0.0,
             k_cond<<<1, 1, 0, s->stream>>>(h, graph ? 1 : 0, s->red_out, s->dev, dev_tol(s),
@@ -795,11 +804,6 @@ void launch_cond_step(Solver* s, cudaGraphConditionalHandle h, bool graph) {
             k_cond<<<1, 1, 0, s->stream>>>(h, graph ? 1 : 0, s->red_out, s->dev, dev_tol(s),
                                            s->prm.max_cycles, 0));
 }
-void launch_step_finish(Solver* s, double dt) {
-  FS_LAUNCH(s, "step_finish", 0.0,
-            k_step_finish<<<1, 1, 0, s->stream>>>(s->dev, dt, s->stats_on_device ? 1 : 0));
-}
-
 // ------------------------------------------- batched refinement bookkeeping
 // One size class of a batch (see fs_multigrid.cu): the refinement residual of
 // every member still in its loop as one launch (member = blockIdx.z, each with
@@ -902,8 +906,8 @@ void launch_cond_class(Solver* const* ms, int count, cudaStream_t st, cudaGraphC
 // ---- the rest of a plain class member's step, batched: the divergence of the
 // (advected, diffused) velocity, the initial residual from zero pressure, the
 // zeroed pressure, and after the loop the gradient subtraction and the step
-// finish (k_div_df, k_refine_init with zero_p, launch_fill, k_subgrad_df,
-// k_step_finish, one launch each for the whole class)
+// finish (k_div_df, k_refine_init with zero_p, launch_fill, k_subgrad_df, one
+// launch each for the whole class)
 struct ProjTab {
   struct {
     const float* wu;  // the velocity the projection reads
@@ -949,15 +953,11 @@ __global__ void __launch_bounds__(256) k_div_start_class(const ProjTab tab, int 
 
 __global__ void __launch_bounds__(256) k_subgrad_class(const ProjTab tab, int nx, int ny) {
   const auto& a = tab.m[blockIdx.z];
+  finish_step(StepFinish{a.st, a.dt, 1});
   if ((nx & 3) == 0)
     subgrad4_body(a.wu, nullptr, a.wv, nullptr, a.ph, a.pl, a.uh, a.ul, a.vh, a.vl, nx, ny, a.idx, a.idy);
   else
     subgrad_df_body(a.wu, nullptr, a.wv, nullptr, a.ph, a.pl, a.uh, a.ul, a.vh, a.vl, nx, ny, a.idx, a.idy);
-}
-
-__global__ void k_finish_class(const ProjTab tab, int count) {
-  const int z = threadIdx.x;
-  if (z < count) finish_step(tab.m[z].st, tab.m[z].dt, 1);
 }
 
 static ProjTab proj_tab(Solver* const* ms, int count, const float* const* wu, const float* const* wv,
@@ -1002,7 +1002,6 @@ void launch_back_class(Solver* const* ms, int count, const float* const* wu, con
   dim3 g2 = grid2d(g.nx % 4 == 0 ? g.nx / 4 : g.nx, g.ny, kBlock);  // four cells per thread when nx % 4 == 0
   g2.z = count;
   k_subgrad_class<<<g2, kBlock, 0, st>>>(tab, g.nx, g.ny);
-  k_finish_class<<<1, kClassMax, 0, st>>>(tab, count);
 }
 
 
