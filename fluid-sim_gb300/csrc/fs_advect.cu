@@ -427,6 +427,7 @@ __global__ void __launch_bounds__(256) k_advect_sl_t(const float* __restrict__ u
                                                      float cx, float cy, float* __restrict__ bounds,
                                                      const __grid_constant__ CUtensorMap tm_u,
                                                      const __grid_constant__ CUtensorMap tm_v, int tma, int* err) {
+  pdl_wait();
   __shared__ __align__(128) float su[kSW * kSH];
   __shared__ __align__(128) float sv[kSW * kSH];
   __shared__ uint64_t bar;
@@ -525,6 +526,7 @@ __global__ void __launch_bounds__(256) k_mc_combine_t(const float* __restrict__ 
                                                       const __grid_constant__ CUtensorMap tm_v,
                                                       const __grid_constant__ CUtensorMap tm_fu,
                                                       const __grid_constant__ CUtensorMap tm_fv, int tma, int* err) {
+  pdl_wait();
   __shared__ __align__(128) float su[kSW * kSH];
   __shared__ __align__(128) float sv[kSW * kSH];
   __shared__ __align__(128) float sfu[kSW * kSH];
@@ -700,7 +702,7 @@ void launch_advect_mc<float>(Solver* s, const float* u, const float* v, float* f
             k_advect_sl_t<<<tile_grid(g), kBlock, 0, s->stream>>>(u, v, fu, fv, g.nx, g.ny, cx, cy, s->mc_bounds, tu,
                                                                   tv, tma, &s->dev->async_err));
   FS_LAUNCH(s, "mc_combine", (double)s->n * 40,
-            k_mc_combine_t<<<tile_grid(g), kBlock, 0, s->stream>>>(u, v, fu, fv, s->mc_bounds, ou, ov, g.nx, g.ny,
+            launch_dependent(true, k_mc_combine_t, tile_grid(g), kBlock, 0, s->stream, u, v, fu, fv, s->mc_bounds, ou, ov, g.nx, g.ny,
                                                                    cx, cy, tu, tv, tfu, tfv, tma,
                                                                    &s->dev->async_err));
 }
@@ -760,12 +762,14 @@ __device__ __forceinline__ void diffuse4_body(const float* __restrict__ u, const
 __global__ void __launch_bounds__(256) k_diffuse4(const float* __restrict__ u, const float* __restrict__ v,
                                                   float* __restrict__ ou, float* __restrict__ ov,
                                                   int nx, int ny, float a, float b) {
+  pdl_wait();
   diffuse4_body(u, v, ou, ov, nx, ny, a, b);
 }
 
 __global__ void __launch_bounds__(256) k_diffuse(const float* __restrict__ u, const float* __restrict__ v,
                                                  float* __restrict__ ou, float* __restrict__ ov,
                                                  int nx, int ny, float a, float b) {
+  pdl_wait();
   diffuse_body(u, v, ou, ov, nx, ny, a, b);
 }
 
@@ -775,9 +779,9 @@ void launch_diffuse(Solver* s, const float* u, const float* v, float* ou, float*
   float b = (float)(s->prm.nu * dt / (g.dyd * g.dyd));
   FS_LAUNCH(s, "diffuse", (double)s->n * 16,
             if (g.nx % 4 == 0) {
-              k_diffuse4<<<grid2d(g.nx / 4, g.ny, kBlock), kBlock, 0, s->stream>>>(u, v, ou, ov, g.nx, g.ny, a, b);
+              launch_dependent(true, k_diffuse4, grid2d(g.nx / 4, g.ny, kBlock), kBlock, 0, s->stream, u, v, ou, ov, g.nx, g.ny, a, b);
             } else {
-              k_diffuse<<<grid2d(g.nx, g.ny, kBlock), kBlock, 0, s->stream>>>(u, v, ou, ov, g.nx, g.ny, a, b);
+              launch_dependent(true, k_diffuse, grid2d(g.nx, g.ny, kBlock), kBlock, 0, s->stream, u, v, ou, ov, g.nx, g.ny, a, b);
             });
 }
 
@@ -848,12 +852,6 @@ __global__ void __launch_bounds__(256) k_forcing(float* __restrict__ u, float* _
   __syncthreads();
   const float drift = s_drift;
   float fu[R] = {}, fv[R] = {}, uc[R], vc[R];
-#pragma unroll
-  for (int r = 0; r < R; r++) {
-    const int64_t c = (int64_t)min(j0 + r, ny - 1) * nx + min(i, nx - 1);
-    uc[r] = u[c];
-    vc[r] = v[c];
-  }
   for (int k0 = 0; k0 < m; k0 += kForceM) {
     const int nm = min(kForceM, m - k0);
     if (k0 > 0) __syncthreads();
@@ -871,6 +869,15 @@ __global__ void __launch_bounds__(256) k_forcing(float* __restrict__ u, float* _
         const int f = (r - 64) / kForceTY, c = (r - 64) - f * kForceTY;
         sincosf(ky * ((blockIdx.y * kForceTY + c + (f ? 0.f : 0.5f)) * dy), &sn, &cs);
         ey[f][k][c] = make_float2(cs, sn);
+      }
+    }
+    if (k0 == 0) {  // the tables need nothing of the launch ahead
+      pdl_wait();
+#pragma unroll
+      for (int r = 0; r < R; r++) {
+        const int64_t c = (int64_t)min(j0 + r, ny - 1) * nx + min(i, nx - 1);
+        uc[r] = u[c];
+        vc[r] = v[c];
       }
     }
     __syncthreads();
@@ -899,7 +906,7 @@ void launch_forcing(Solver* s, float* u, float* v, float dt) {
   float scale = (float)(s->amp * dt / sqrt((double)s->n_modes));
   float damp = (float)exp(-s->drag * dt);
   FS_LAUNCH(s, "forcing", (double)s->n * 16,
-            k_forcing<<<dim3((g.nx + 31) / 32, (g.ny + kForceTY - 1) / kForceTY), kBlock, 0, s->stream>>>(
+            launch_dependent(true, k_forcing, dim3((g.nx + 31) / 32, (g.ny + kForceTY - 1) / kForceTY), kBlock, 0, s->stream, 
                 u, v, s->modes, s->n_modes, g.nx, g.ny, g.dx, g.dy, scale, damp, s->drift, s->dev));
 }
 
@@ -1095,6 +1102,7 @@ __device__ __forceinline__ Home home_c() { return {0.5f, 0.f, 0.f, 0.5f}; }
 __global__ void __launch_bounds__(256) k_advect_dye(const float* __restrict__ u, const float* __restrict__ v,
                                                     const float4* __restrict__ q, float4* __restrict__ out, int nx,
                                                     int ny, float cx, float cy, float keep) {
+  pdl_wait();
   int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
   if (i >= nx || j >= ny) return;
   float dX, dY;
@@ -1117,7 +1125,7 @@ void launch_advect_dye(Solver* s, float dt) {
   const Grid& g = s->g;
   dim3 b(32, 8);
   FS_LAUNCH(s, "advect_dye", (double)s->n * 40,
-            k_advect_dye<<<grid2d(g.nx, g.ny, b), b, 0, s->stream>>>(
+            launch_dependent(true, k_advect_dye, grid2d(g.nx, g.ny, b), b, 0, s->stream, 
                 s->u, s->v, static_cast<const float4*>(s->dye), static_cast<float4*>(s->dye2), g.nx, g.ny,
                 (float)(dt * g.idxd), (float)(dt * g.idyd), (float)(1.0 - s->prm.dye_fade)));
   // the next step reads s->dye again: copy back (a captured step cannot swap pointers)

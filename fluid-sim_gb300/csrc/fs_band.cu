@@ -147,8 +147,7 @@ __global__ void __launch_bounds__(256)
     band_mode(kind, m, step, seed, kf, width, s, lattice, modes + m);
   }
   __syncthreads();
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nx) return;
+  const int i = min((int)(blockIdx.x * blockDim.x + threadIdx.x), nx - 1);
   float2 au = make_float2(0.f, 0.f), av = make_float2(0.f, 0.f);
   for (int m = first; m <= last; m++) {
     const ModeCoef& c = modes[m];
@@ -159,6 +158,7 @@ __global__ void __launch_bounds__(256)
     av.x = fmaf(c.cv.x, ev.x, fmaf(-c.cv.y, ev.y, av.x));
     av.y = fmaf(c.cv.x, ev.y, fmaf(c.cv.y, ev.x, av.y));
   }
+  pdl_wait();  // the sums need nothing of the launch ahead
   gu[(size_t)blockIdx.y * nx + i] = au;
   gv[(size_t)blockIdx.y * nx + i] = av;
 }
@@ -181,16 +181,17 @@ __global__ void __launch_bounds__(256)
   BandStage& t = *reinterpret_cast<BandStage*>(band_smem);
   const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * 32 + tx;
   const int i0 = blockIdx.x * kBandTX, j0 = blockIdx.y * kBandTY;
-  if (blockIdx.x == 0 && blockIdx.y == 0 && tid == 0) st->band_step += 1;
   float uc[kBandRows][2], vc[kBandRows][2];
 #pragma unroll
   for (int r = 0; r < kBandRows; r++)
 #pragma unroll
     for (int k = 0; k < 2; k++) {
       const int64_t c = (int64_t)min(j0 + ty * kBandRows + r, ny - 1) * nx + min(i0 + tx + 32 * k, nx - 1);
-      uc[r][k] = u[c];
+      uc[r][k] = u[c];  // complete before the column sums began
       vc[r][k] = v[c];
     }
+  pdl_wait();
+  if (blockIdx.x == 0 && blockIdx.y == 0 && tid == 0) st->band_step += 1;
   float fu[kBandRows][2] = {}, fv[kBandRows][2] = {};
   const int nq = 2 * K + 1;
   for (int q0 = 0; q0 < nq; q0 += kBandQ) {
@@ -333,12 +334,12 @@ void launch_band(Solver* s, float* u, float* v, float dt) {
   const float damp = b->drag > 0 ? (float)exp(-b->drag * (double)dt) : 1.f;
   const int nq = 2 * b->K + 1;
   FS_LAUNCH(s, "band_columns", (double)nq * g.nx * 32,
-            k_band_columns<<<dim3((g.nx + 255) / 256, nq), 256, 0, s->stream>>>(
+            launch_dependent(true, k_band_columns, dim3((g.nx + 255) / 256, nq), dim3(256), 0, s->stream, 
                 b->kind, b->M, b->K, s->dev, b->seed, b->kf, b->width, scale, b->lattice, b->ex_u, b->ex_v, b->gu,
                 b->gv, g.nx));
   FS_LAUNCH(s, "band_apply", (double)s->n * 16,
-            k_band_apply<<<dim3((g.nx + kBandTX - 1) / kBandTX, (g.ny + kBandTY - 1) / kBandTY), dim3(32, 8),
-                         sizeof(BandStage), s->stream>>>(
+            launch_dependent(true, k_band_apply, dim3((g.nx + kBandTX - 1) / kBandTX, (g.ny + kBandTY - 1) / kBandTY),
+                             dim3(32, 8), sizeof(BandStage), s->stream, 
                 u, v, g.nx, g.ny, b->K, b->gu, b->gv, b->ey_u, b->ey_v, damp, s->dev));
 }
 

@@ -182,6 +182,7 @@ __device__ __forceinline__ void mg_bottom_body(const float* __restrict__ rhs_top
 __global__ void __launch_bounds__(1024) k_mg_bottom(const float* __restrict__ rhs_top, float* __restrict__ x_top,
                                                     int has_x, BottomLevels L, int pre, int post, int coarse,
                                                     float* __restrict__ acc_h, float* __restrict__ acc_l) {
+  pdl_wait();
   mg_bottom_body(rhs_top, x_top, has_x, L, pre, post, coarse, acc_h, acc_l);
 }
 
@@ -702,6 +703,7 @@ template <int N0, int NMIN>
 __global__ void __launch_bounds__(kBottomThreads)
     k_mg_bottom_chain(const float* __restrict__ rhs_top, float* __restrict__ x_top, int has_x, BottomH2 H, int pre,
                       int post, int coarse, float* __restrict__ acc_h, float* __restrict__ acc_l) {
+  pdl_wait();
   mg_bottom_chain_body<N0, NMIN>(rhs_top, x_top, has_x, H, pre, post, coarse, acc_h, acc_l);
 }
 
@@ -803,7 +805,7 @@ void launch_bottom(Solver* s, int lb, bool hx, float* acc_h, float* acc_l) {
 #define FS_CASE(N0, NM)                                                                                          \
   case N0:                                                                                                       \
     FS_LAUNCH(s, "mg_bottom", bytes,                                                                             \
-              k_mg_bottom_chain<N0, NM><<<1, kBottomThreads, 0, s->stream>>>(                                    \
+              launch_dependent(true, k_mg_bottom_chain<N0, NM>, dim3(1), dim3(kBottomThreads), 0, s->stream,                                     \
                   L[lb].rhs, L[lb].x, hx ? 1 : 0, H, P.mg_pre_smooth, P.mg_post_smooth, P.mg_coarse_sweeps,      \
                   acc_h, acc_l));                                                                                \
     return;
@@ -814,7 +816,7 @@ void launch_bottom(Solver* s, int lb, bool hx, float* acc_h, float* acc_l) {
   const size_t smem = bottom_layout(s, &B);
   const int threads = std::min(1024, std::max(32, ((nb * nb / 4 + 31) / 32) * 32));
   FS_LAUNCH(s, "mg_bottom", bytes,
-            k_mg_bottom<<<1, threads, smem, s->stream>>>(L[lb].rhs, L[lb].x, hx ? 1 : 0, B, P.mg_pre_smooth,
+            launch_dependent(true, k_mg_bottom, dim3(1), dim3(threads), smem, s->stream, L[lb].rhs, L[lb].x, hx ? 1 : 0, B, P.mg_pre_smooth,
                                                          P.mg_post_smooth, P.mg_coarse_sweeps, acc_h, acc_l));
 }
 

@@ -67,6 +67,7 @@ struct Bands {
 __global__ void __launch_bounds__(256)
     k_channel(float* __restrict__ u, float* __restrict__ v, int nx, int ny, float dx, float dy, ChannelDev c,
               float w, Bands b) {
+  pdl_wait();
   int i, j;
   const int blk = blockIdx.x;
   if (blk < b.na) {
@@ -157,7 +158,7 @@ void launch_channel(Solver* s, float* u, float* v) {
   // algorithmic bytes: u, v read and written on the cells of the two bands
   const double cells = (double)b.nw * g.nx + (double)b.nf * (g.ny - b.nw);
   FS_LAUNCH(s, "channel", 16.0 * cells,
-            k_channel<<<b.na + nb, dim3(32, 8), 0, s->stream>>>(u, v, g.nx, g.ny, g.dx, g.dy, d, (float)w, b));
+            launch_dependent(true, k_channel, dim3(b.na + nb), dim3(32, 8), 0, s->stream, u, v, g.nx, g.ny, g.dx, g.dy, d, (float)w, b));
 }
 
 }  // namespace fs

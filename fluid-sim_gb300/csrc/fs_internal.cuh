@@ -213,6 +213,34 @@ void prof_end(Solver* s, int slot, cudaEvent_t a);
     if ((S)->profiling) fs::prof_end((S), _slot, _ev);                   \
   } while (0)
 
+// Programmatic dependent launch: with dependent, a kernel may start while the one
+// ahead of it in the stream finishes, and calls pdl_wait before it reads or
+// overwrites anything of the step.  Every kernel waits first and lets the next
+// one start then, so that the launch before the one ahead is complete when a
+// kernel starts, and at most one waits beside the one that runs (the other
+// order piled waiting kernels up and made the V-cycles slower by up to 10%).
+// Steps without and with: 512^2 multigrid 116.8 -> 110.7 us, 192^2 mixed 145.6 -> 131.4,
+// 576^2 147.5 -> 129.2, 1024^2 forced 309.9 -> 297.8, 4096^2 2374 -> 2307.
+template <class... P, class... A>
+inline cudaError_t launch_dependent(bool dependent, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem,
+                                    cudaStream_t st, A&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute pdl = {};
+  pdl.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  pdl.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &pdl;
+  cfg.numAttrs = dependent ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+__device__ __forceinline__ void pdl_wait() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;");
+}
+
 inline dim3 grid2d(int nx, int ny, dim3 b) { return dim3((nx + b.x - 1) / b.x, (ny + b.y - 1) / b.y); }
 
 // failed step captures after which a handle refuses to capture again

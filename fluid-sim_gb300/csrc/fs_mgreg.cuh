@@ -20,6 +20,7 @@
 
 #include "fs_df.cuh"
 #include "fs_flat.cuh"
+#include "fs_internal.cuh"
 #include "fs_stencil.cuh"
 
 namespace fs {
@@ -189,6 +190,12 @@ __device__ __forceinline__ void mg_up_reg(const float* __restrict__ rhs, const f
   // column 2 i + 1 columns i, i + 1 (weight 1/4 on i + 1); likewise the rows
   // (PROLONG, multigrid.js:99-131: sample at ((i+1/2)/2 - 1/2, (j+1/2)/2 - 1/2)).
   const int nc = n >> 1, gc = t.gx >> 1, jc = (t.yl >> 1) - 1;
+  // the iterate and the rhs were complete before the launch ahead of this one began
+  if (!zero) {
+    t.load(t.p, xin, n);
+    t.load(t.d, rhs, n);
+  }
+  pdl_wait();
   float cv[CR][CC], side[CR];
   const int gs = flat_wrap(t.lane == 0 ? gc - 1 : gc + CC, nc);
 #pragma unroll
@@ -201,10 +208,6 @@ __device__ __forceinline__ void mg_up_reg(const float* __restrict__ rhs, const f
       cv[k][0] = __ldg(row + gc);
     }
     side[k] = t.lane == 0 || t.lane == 31 ? __ldg(row + gs) : 0.f;
-  }
-  if (!zero) {
-    t.load(t.p, xin, n);
-    t.load(t.d, rhs, n);
   }
   float m0[CPL], m1[CPL];  // the two coarse rows before, interpolated to the fine columns
 #pragma unroll

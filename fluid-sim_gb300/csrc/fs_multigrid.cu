@@ -34,6 +34,7 @@ __global__ void __launch_bounds__(R::THREADS, R::CTAS)
     k_mg_down(const float* __restrict__ rhs, const float* __restrict__ xin, float* __restrict__ xout,
                   float* __restrict__ crhs, int n, float h2, int pre, float w, const int* first_cycle, int first_pre,
                   int first_x_unused) {
+  pdl_wait();
   // the first cycle of a projection may run fewer sweeps on this level
   // (fs_params mg_first_pre, at most pre): first_pre >= 0 applies it, inside
   // a captured loop only while the loop's cycle count is still 0;
@@ -171,7 +172,7 @@ static void down_t(Solver* s, Level& L, const Level& C, bool has_x, bool zero, i
   // a first cycle the host knows is profiled under its own name
   const std::string name = level_name(s, L, "mg_down") + (first >= 0 && !cyc ? "_first" : "");
   FS_LAUNCH(s, name.c_str(), bytes,
-            k_mg_down<R><<<region_grid<R>(L.n), R::THREADS, 0, s->stream>>>(
+            launch_dependent(true, k_mg_down<R>, region_grid<R>(L.n), dim3(R::THREADS), 0, s->stream, 
                 L.rhs, has_x && !zero ? L.x : nullptr, has_x ? L.x2 : L.x, C.rhs, L.n, L.h2, s->prm.mg_pre_smooth,
                 (float)s->prm.relax, cyc, first < s->prm.mg_pre_smooth ? first : s->prm.mg_pre_smooth,
                 x_unused ? 1 : 0));
@@ -195,14 +196,14 @@ static void up_t(Solver* s, Level& L, const Level& C, float* acc_h, float* acc_l
   if (acc_h) {
     typedef typename RegionOf<T, H, true>::R R;
     FS_LAUNCH(s, first >= 0 && !cyc ? "mg_up_acc_first" : "mg_up_acc", bytes,
-              k_mg_up<R, true><<<region_grid<R>(L.n), R::THREADS, 0, s->stream>>>(
+              launch_dependent(true, k_mg_up<R, true>, region_grid<R>(L.n), dim3(R::THREADS), 0, s->stream, 
                   L.rhs, L.x, nullptr, C.x, L.n, L.h2, s->prm.mg_post_smooth, (float)s->prm.relax, acc_h, acc_l, cyc,
                   fp, x_zero ? 1 : 0));
     return;
   }
   typedef typename RegionOf<T, H>::R R;
   FS_LAUNCH(s, level_name(s, L, "mg_up").c_str(), bytes,
-            k_mg_up<R, false><<<region_grid<R>(L.n), R::THREADS, 0, s->stream>>>(
+            launch_dependent(true, k_mg_up<R, false>, region_grid<R>(L.n), dim3(R::THREADS), 0, s->stream, 
                 L.rhs, L.x, L.x2, C.x, L.n, L.h2, s->prm.mg_post_smooth, (float)s->prm.relax, nullptr, nullptr, cyc,
                 fp, x_zero ? 1 : 0));
   std::swap(L.x, L.x2);

@@ -30,6 +30,7 @@ __device__ __forceinline__ int wrapm(int i, int n) { return i < 0 ? i + n : (i >
 template <class TV, class TD>
 __global__ void __launch_bounds__(256) k_divergence(const TV* __restrict__ u, const TV* __restrict__ v,
                                                     TD* __restrict__ d, int nx, int ny, TD idx, TD idy) {
+  pdl_wait();
   int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
   if (i >= nx || j >= ny) return;
   int ip = i + 1 == nx ? 0 : i + 1, jp = j + 1 == ny ? 0 : j + 1;
@@ -45,7 +46,7 @@ void launch_divergence(Solver* s, const TV* u, const TV* v, TD* d) {
   TD ix = sizeof(TD) == 8 ? (TD)g.idxd : (TD)g.idx;
   TD iy = sizeof(TD) == 8 ? (TD)g.idyd : (TD)g.idy;
   FS_LAUNCH(s, "divergence", (double)s->n * (2 * sizeof(TV) + sizeof(TD)),
-            k_divergence<TV, TD><<<grid2d(g.nx, g.ny, kBlock), kBlock, 0, s->stream>>>(u, v, d, g.nx,
+            launch_dependent(true, k_divergence<TV, TD>, grid2d(g.nx, g.ny, kBlock), kBlock, 0, s->stream, u, v, d, g.nx,
                                                                                         g.ny, ix, iy));
 }
 template void launch_divergence<float, float>(Solver*, const float*, const float*, float*);
@@ -75,6 +76,7 @@ __global__ void __launch_bounds__(256)
     k_subgrad_f32(const float* __restrict__ wu, const float* __restrict__ wv, const float* __restrict__ p,
                   float* __restrict__ ou, float* __restrict__ ov, int nx, int ny, float idx, float idy,
                   const StepFinish fin) {
+  pdl_wait();
   finish_step(fin);
   int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
   if (i >= nx || j >= ny) return;
@@ -89,7 +91,7 @@ void launch_subtract_gradient_f32(Solver* s, const float* wu, const float* wv, c
                                   float* ou, float* ov, const StepFinish& fin) {
   const Grid& g = s->g;
   FS_LAUNCH(s, "subtract_gradient", (double)s->n * 20,
-            k_subgrad_f32<<<grid2d(g.nx, g.ny, kBlock), kBlock, 0, s->stream>>>(wu, wv, p, ou, ov, g.nx,
+            launch_dependent(true, k_subgrad_f32, grid2d(g.nx, g.ny, kBlock), kBlock, 0, s->stream, wu, wv, p, ou, ov, g.nx,
                                                                                 g.ny, g.idx, g.idy, fin));
 }
 // ----------------------------------------------------------------- smoothers
@@ -357,6 +359,7 @@ __global__ void __launch_bounds__(256)
     k_div_start4(const float* __restrict__ wu, const float* __restrict__ wv, float* __restrict__ dh,
                  float* __restrict__ dl, float* __restrict__ ph, float* __restrict__ pl, float* __restrict__ r32,
                  int nx, int ny, df idx, df idy, RedCtx ctx) {
+  pdl_wait();
   div_start4_body(wu, wv, dh, dl, ph, pl, r32, nx, ny, idx, idy, ctx);
 }
 
@@ -364,6 +367,7 @@ __global__ void __launch_bounds__(256)
     k_div_df(const float* __restrict__ uh, const float* __restrict__ ul, const float* __restrict__ vh,
              const float* __restrict__ vl, float* __restrict__ dh, float* __restrict__ dl, int nx, int ny, df idx,
              df idy) {
+  pdl_wait();
   div_df_body(uh, ul, vh, vl, dh, dl, nx, ny, idx, idy);
 }
 
@@ -371,7 +375,7 @@ void launch_div_df(Solver* s, const float* uh, const float* ul, const float* vh,
                    float* dl) {
   const Grid& g = s->g;
   FS_LAUNCH(s, "divergence", (double)s->n * ((ul ? 16 : 8) + 8),
-            k_div_df<<<grid2d(g.nx, g.ny, kBlock), kBlock, 0, s->stream>>>(
+            launch_dependent(true, k_div_df, grid2d(g.nx, g.ny, kBlock), kBlock, 0, s->stream, 
                 uh, ul, vh, vl, dh, dl, g.nx, g.ny, df_host(g.idxd), df_host(g.idyd)));
 }
 
@@ -438,6 +442,7 @@ __global__ void __launch_bounds__(256)
                   const float* __restrict__ wvl, const float* __restrict__ ph, const float* __restrict__ pl,
                   float* __restrict__ uh, float* __restrict__ ul, float* __restrict__ vh, float* __restrict__ vl,
                   int nx, int ny, df idx, df idy, const StepFinish fin) {
+  pdl_wait();
   finish_step(fin);
   subgrad4_body(wuh, wul, wvh, wvl, ph, pl, uh, ul, vh, vl, nx, ny, idx, idy);
 }
@@ -447,6 +452,7 @@ __global__ void __launch_bounds__(256)
                  const float* __restrict__ wvl, const float* __restrict__ ph, const float* __restrict__ pl,
                  float* __restrict__ uh, float* __restrict__ ul, float* __restrict__ vh, float* __restrict__ vl,
                  int nx, int ny, df idx, df idy, const StepFinish fin) {
+  pdl_wait();
   finish_step(fin);
   subgrad_df_body(wuh, wul, wvh, wvl, ph, pl, uh, ul, vh, vl, nx, ny, idx, idy);
 }
@@ -457,10 +463,10 @@ void launch_subgrad_df(Solver* s, const float* wuh, const float* wul, const floa
   const Grid& g = s->g;
   FS_LAUNCH(s, "subtract_gradient", (double)s->n * ((wul ? 16 : 8) + 8 + 16),
             if (g.nx % 4 == 0) {
-              k_subgrad4_df<<<grid2d(g.nx / 4, g.ny, kBlock), kBlock, 0, s->stream>>>(
+              launch_dependent(true, k_subgrad4_df, grid2d(g.nx / 4, g.ny, kBlock), kBlock, 0, s->stream, 
                   wuh, wul, wvh, wvl, ph, pl, uh, ul, vh, vl, g.nx, g.ny, df_host(g.idxd), df_host(g.idyd), fin);
             } else {
-              k_subgrad_df<<<grid2d(g.nx, g.ny, kBlock), kBlock, 0, s->stream>>>(
+              launch_dependent(true, k_subgrad_df, grid2d(g.nx, g.ny, kBlock), kBlock, 0, s->stream, 
                   wuh, wul, wvh, wvl, ph, pl, uh, ul, vh, vl, g.nx, g.ny, df_host(g.idxd), df_host(g.idyd), fin);
             });
 }
@@ -556,6 +562,7 @@ __global__ void __launch_bounds__(256)
     k_refine_init(const float* __restrict__ dh, const float* __restrict__ dl, const float* __restrict__ ph,
                   const float* __restrict__ pl, float* __restrict__ r32, int nx, int ny, LapScale ks,
                   int zero_p, RedCtx ctx) {
+  pdl_wait();
   refine_init_body(dh, dl, ph, pl, r32, nx, ny, ks, zero_p, ctx);
 }
 
@@ -639,6 +646,7 @@ __global__ void __launch_bounds__(256, 5)
     k_refine_init4(const float* __restrict__ dh, const float* __restrict__ dl, const float* __restrict__ ph,
                    const float* __restrict__ pl, float* __restrict__ r32, int nx, int ny, LapScale ks, RedCtx ctx,
                    CondFold cf) {
+  pdl_wait();
   refine_init4_body(dh, dl, ph, pl, r32, nx, ny, ks, ctx, cf);
 }
 
@@ -699,10 +707,10 @@ bool launch_refine_init(Solver* s, const float* dh, const float* dl, const float
                                      : CondFold{};
   FS_LAUNCH(s, "refine_init", (double)s->n * (zero_p ? 12 : 20),
             if (quad) {
-              k_refine_init4<<<refine4_grid(s, g.nx / 4, g.ny), kBlock, 0, s->stream>>>(
+              launch_dependent(true, k_refine_init4, refine4_grid(s, g.nx / 4, g.ny), kBlock, 0, s->stream, 
                   dh, dl, ph, pl, r32, g.nx, g.ny, lap_scale(g), red_ctx(s, s->red_out), cf);
             } else {
-              k_refine_init<<<red_grid2(g.nx, g.ny), kBlock, 0, s->stream>>>(
+              launch_dependent(true, k_refine_init, red_grid2(g.nx, g.ny), kBlock, 0, s->stream, 
                   dh, dl, ph, pl, r32, g.nx, g.ny, lap_scale(g), zero_p ? 1 : 0, red_ctx(s, s->red_out));
             });
   return cf.on != 0;
@@ -720,7 +728,7 @@ void launch_div_start(Solver* s, const float* wu, const float* wv) {
     return;
   }
   FS_LAUNCH(s, "div_start", (double)s->n * 28,
-            k_div_start4<<<red_grid2(g.nx / 4, g.ny), kBlock, 0, s->stream>>>(
+            launch_dependent(true, k_div_start4, red_grid2(g.nx / 4, g.ny), kBlock, 0, s->stream, 
                 wu, wv, s->dh, s->dl, s->ph, s->pl, s->r32, g.nx, g.ny, df_host(g.idxd), df_host(g.idyd),
                 red_ctx(s, s->red_out)));
 }
