@@ -584,6 +584,7 @@ struct DiffTab {
 };
 
 __global__ void __launch_bounds__(256) k_advect_sl_class(const AdvTab tab, int nx, int ny) {
+  pdl_wait();
   const auto& a = tab.m[blockIdx.z];
   __shared__ __align__(128) float su[kSW * kSH];
   __shared__ __align__(128) float sv[kSW * kSH];
@@ -604,6 +605,7 @@ __global__ void __launch_bounds__(256) k_advect_sl_class(const AdvTab tab, int n
 }
 
 __global__ void __launch_bounds__(256) k_mc_combine_class(const AdvTab tab, int nx, int ny) {
+  pdl_wait();
   const auto& a = tab.m[blockIdx.z];
   __shared__ __align__(128) float su[kSW * kSH];
   __shared__ __align__(128) float sv[kSW * kSH];
@@ -786,6 +788,7 @@ void launch_diffuse(Solver* s, const float* u, const float* v, float* ou, float*
 }
 
 __global__ void __launch_bounds__(256) k_diffuse_class(const DiffTab tab, int nx, int ny) {
+  pdl_wait();
   const auto& a = tab.m[blockIdx.z];
   if ((nx & 3) == 0) diffuse4_body(a.u, a.v, a.ou, a.ov, nx, ny, a.a, a.b);
   else diffuse_body(a.u, a.v, a.ou, a.ov, nx, ny, a.a, a.b);
@@ -812,7 +815,7 @@ void launch_front_advect_class(Solver* const* ms, int count, const double* dts, 
   dim3 grid = tile_grid(g);
   grid.z = count;
   k_advect_sl_class<<<grid, kBlock, 0, st>>>(fwd, g.nx, g.ny);
-  if (mc) k_mc_combine_class<<<grid, kBlock, 0, st>>>(comb, g.nx, g.ny);
+  if (mc) launch_dependent(true, k_mc_combine_class, grid, kBlock, 0, st, comb, g.nx, g.ny);
   if (s0->prm.nu > 0) {
     DiffTab dt{};
     for (int i = 0; i < count; i++) {
@@ -823,7 +826,7 @@ void launch_front_advect_class(Solver* const* ms, int count, const double* dts, 
     }
     dim3 g2 = grid2d(g.nx % 4 == 0 ? g.nx / 4 : g.nx, g.ny, kBlock);  // four cells per thread when nx % 4 == 0
     g2.z = count;
-    k_diffuse_class<<<g2, kBlock, 0, st>>>(dt, g.nx, g.ny);
+    launch_dependent(true, k_diffuse_class, g2, kBlock, 0, st, dt, g.nx, g.ny);
   }
 }
 

@@ -727,6 +727,7 @@ struct BottomTab {
 template <int N0, int NMIN>
 __global__ void __launch_bounds__(kBottomThreads)
     k_mg_bottom_chain_class(const BottomTab tab, BottomH2 H, int pre, int post, int coarse, int max_cycles) {
+  pdl_wait();
   const auto& a = tab.m[blockIdx.z];
   if (!member_active(a.st, max_cycles)) return;
   mg_bottom_chain_body<N0, NMIN>(a.rhs, a.x, 0, H, pre, post, coarse, a.acc_h, a.acc_l);
@@ -734,6 +735,7 @@ __global__ void __launch_bounds__(kBottomThreads)
 
 __global__ void __launch_bounds__(1024) k_mg_bottom_class(const BottomTab tab, BottomLevels L, int pre, int post,
                                                           int coarse, int max_cycles) {
+  pdl_wait();
   const auto& a = tab.m[blockIdx.z];
   if (!member_active(a.st, max_cycles)) return;
   mg_bottom_body(a.rhs, a.x, 0, L, pre, post, coarse, a.acc_h, a.acc_l);
@@ -834,7 +836,7 @@ void launch_bottom_class(Solver* const* ms, int count, int lb, cudaStream_t st) 
   switch (bottom_chain(s0, lb)) {
 #define FS_CASE(N0, NM)                                                                                        \
   case N0:                                                                                                     \
-    k_mg_bottom_chain_class<N0, NM><<<grid, kBottomThreads, 0, st>>>(tab, H, P.mg_pre_smooth, P.mg_post_smooth, \
+    launch_dependent(true, k_mg_bottom_chain_class<N0, NM>, dim3(grid), dim3(kBottomThreads), 0, st, tab, H, P.mg_pre_smooth, P.mg_post_smooth, \
                                                                      P.mg_coarse_sweeps, P.max_cycles);         \
     return;
     FS_CHAINS(FS_CASE)
@@ -843,7 +845,7 @@ void launch_bottom_class(Solver* const* ms, int count, int lb, cudaStream_t st) 
   BottomLevels B;
   const size_t smem = bottom_layout(s0, &B);
   const int threads = std::min(1024, std::max(32, ((nb * nb / 4 + 31) / 32) * 32));
-  k_mg_bottom_class<<<grid, threads, smem, st>>>(tab, B, P.mg_pre_smooth, P.mg_post_smooth, P.mg_coarse_sweeps,
+  launch_dependent(true, k_mg_bottom_class, dim3(grid), dim3(threads), smem, st, tab, B, P.mg_pre_smooth, P.mg_post_smooth, P.mg_coarse_sweeps,
                                                  P.max_cycles);
 }
 

@@ -31,9 +31,10 @@ struct ConvOut {
   float scale = 1.f;
 };
 
-// images of B x H x W pixels; the flag combinations the network uses
+// images of B x H x W pixels; the flag combinations the network uses.  dependent:
+// the launch may start while the one ahead of it finishes, which has not written w
 cudaError_t conv3x3(int cin, int cout, int flags, const void* in, const void* w, const float* bias, const ConvOut& o,
-                    int B, int H, int W, int* err, cudaStream_t st);
+                    int B, int H, int W, int* err, cudaStream_t st, bool dependent = false);
 
 }  // namespace conv
 }  // namespace fs

@@ -9,7 +9,8 @@
 // a region shares with its neighbours are computed by each of them (2.6x the
 // useful cells for the 64 x 64 region at 12, 1.9x for the 128 x 64 one),
 // which the idle issue slots pay for.  The same solves, captured: 18.5 us,
-// 43 us and 37 us.
+// 43 us and 37 us; with the first launch of a solve a dependent one too, steps of
+// these sizes take 32.6 -> 29.8, 84.5 -> 81.6 and 46.6 -> 45.6 us.
 #include <algorithm>
 #include <utility>
 
@@ -33,10 +34,10 @@ static void flat_t(Solver* s, float** x, float** y, const float* d, int n, float
     pdl.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     pdl.val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = &pdl;
-    cfg.numAttrs = done > 0 ? 1 : 0;
+    cfg.numAttrs = 1;
     FS_LAUNCH(s, MODE == kFlatJacobi ? "jacobi" : "red_black", (double)s->n * (zero ? 8 : 12),
               cudaLaunchKernelEx(&cfg, k_flat<CPL, RPW, NW, H, MODE>, (const float*)*x, d, *y, g.nx, g.ny, h2,
-                                 (float)s->prm.relax, now, done & 1, zero ? 1 : 0));
+                                 (float)s->prm.relax, now, done & 1, zero ? 1 : 0, done == 0 ? 1 : 0));
     zero = false;
     std::swap(*x, *y);
   }

@@ -110,14 +110,13 @@ __device__ __forceinline__ void flat_all_rows(float (&p)[RPW][CPL], const float 
 // k <= H sweeps (half-sweeps of colours c0, c0 + 1, ...) of (p, d) into o; zero:
 // p is taken as 0 and not read.
 //
-// The launches of one solve after the first are programmatic dependents: a
-// CTA may start while the launch before it, which writes p and reads o, still
-// runs, loads d (which no launch of the solve writes) and then waits for that
-// launch to complete.  The first is an ordinary launch, so the right-hand side
-// is complete when any of them starts.
+// The launches are programmatic dependents: a CTA may start while the launch
+// before it, which writes p and reads o, still runs, loads d (which no launch of
+// the solve writes, except that the one ahead of the first may) and then waits
+// for that launch to complete before it lets the next one start.
 template <int CPL, int RPW, int NW, int H, int MODE>
 __global__ void __launch_bounds__(NW * 32) k_flat(const float* p, const float* __restrict__ d, float* o, int nx, int ny,
-                                                  float h2, float w, int k, int c0, int zero) {
+                                                  float h2, float w, int k, int c0, int zero, int first) {
   using F = FlatTile<CPL, RPW, NW, H>;
   typedef typename FlatVec<CPL>::T V;
   static_assert(MODE != kFlatRbOdd || RPW * CPL <= 32, "one mask bit per cell");
@@ -127,6 +126,7 @@ __global__ void __launch_bounds__(NW * 32) k_flat(const float* p, const float* _
   const int xl = x0 + lane * CPL, yl = y0 + warp * RPW;
   const bool vec = nx % CPL == 0;  // a lane's columns never straddle the wrap
   float pv[RPW][CPL], dv[RPW][CPL];
+  if (first) asm volatile("griddepcontrol.wait;" ::: "memory");
   uint32_t odd = 0;  // bit r * CPL + c: the parity of the cell's wrapped indices
   int gx[CPL];
 #pragma unroll
@@ -147,8 +147,8 @@ __global__ void __launch_bounds__(NW * 32) k_flat(const float* p, const float* _
       if (MODE == kFlatRbOdd) odd |= (uint32_t)((gx[c] + gy) & 1) << (r * CPL + c);
     }
   }
-  asm volatile("griddepcontrol.launch_dependents;");
   asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;");
   if (!zero) {
 #pragma unroll
     for (int r = 0; r < RPW; r++) {

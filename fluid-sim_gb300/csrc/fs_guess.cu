@@ -243,6 +243,7 @@ __global__ void __launch_bounds__(32 * kLossWarps)
     k_loss_seed(const float* __restrict__ out, const float* __restrict__ tgt, const float* __restrict__ res,
                 double* __restrict__ acc, uint4* __restrict__ gJ, int H, int W, int B, int rows, double w_p,
                 double w_r) {
+  pdl_wait();
   const int b = blockIdx.y;
   const int64_t npix = (int64_t)H * W, base = b * npix;
   const double mean = acc[b] / (double)npix, scale = 2.0 / ((double)B * npix);
@@ -375,7 +376,7 @@ static cudaError_t conv(const Ctx& c, int l, bool transposed, const bf* in, cons
   const float* bias = transposed ? g->zero_bias : g->theta + g->off_b[l];
   cudaError_t e = cudaSuccess;
   const double bytes = (double)(ci + co) * 2 * B * H * W;
-  GL(c, "guess_conv", bytes, e = conv::conv3x3(ci, co, flags, in, w, bias, o, B, H, W, g->err, c.st));
+  GL(c, "guess_conv", bytes, e = conv::conv3x3(ci, co, flags, in, w, bias, o, B, H, W, g->err, c.st, true));
   return e;
 }
 
@@ -452,6 +453,7 @@ static cudaError_t wgrad_tc(const Ctx& c, int l, Buf xbuf, Buf gbuf, int B, int 
     CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM));
     attr.fetch_or(bit);
   }
+  // (ordinary launches: as dependent ones these two made the backward pass 2% slower)
   // one wave: as many CTAs as the shared memory lets an SM hold, over the taps' groups
   constexpr int per_sm = C::SMEM <= 110 * 1024 ? 2 : 1;
   const int64_t ntiles = (int64_t)B * ((H + TY - 1) / TY) * ((W + PX - 1) / PX);
@@ -511,8 +513,8 @@ static cudaError_t backward(const Ctx& c, const float* target, int B, int H, int
        k_loss_mean<<<dim3((unsigned)std::min<int64_t>((npix + 255) / 256, 256), B), 32 * kLossWarps, 0, c.st>>>(
            g->out, target, g->acc, npix));
   GL(c, "guess_loss", npix * B * 40.0,
-     k_loss_seed<<<lb, 32 * kLossWarps, 0, c.st>>>(g->out, target, with_res ? g->res : nullptr, g->acc,
-                                                   (uint4*)b[GJ], H, W, B, rows, g->w_p, g->w_r));
+     launch_dependent(true, k_loss_seed, lb, dim3(32 * kLossWarps), 0, c.st, g->out, target,
+                      with_res ? g->res : nullptr, g->acc, (uint4*)b[GJ], H, W, B, rows, g->w_p, g->w_r));
   CK(cudaGetLastError());
   // Each layer's weight gradient, then the gradient of its input; the ReLU
   // masks, the gradients of the upsampled skip sums (2 x 2 sums) and of the

@@ -93,6 +93,7 @@ static_assert(sizeof(UpTab) + 64 <= 32764, "kernel parameter limit");
 template <class R>
 __global__ void __launch_bounds__(R::THREADS, R::CTAS)
     k_mg_down_class(const __grid_constant__ DownTab tab, int n, float h2, int pre, float w, int max_cycles) {
+  pdl_wait();
   const auto& a = tab.m[blockIdx.z];
   if (!member_active(a.st, max_cycles)) return;
   mg_down_reg<R>(a.rhs, nullptr, a.xout, a.crhs, n, h2, pre, w);
@@ -102,7 +103,10 @@ template <class R, bool ACC>
 __global__ void __launch_bounds__(R::THREADS, R::CTAS)
     k_mg_up_class(const __grid_constant__ UpTab tab, int n, float h2, int post, float w, int max_cycles) {
   const auto& a = tab.m[blockIdx.z];
-  if (!member_active(a.st, max_cycles)) return;
+  if (!member_active(a.st, max_cycles)) {  // (the loop state was set before the cycle began)
+    pdl_wait();
+    return;
+  }
   mg_up_reg<R, ACC>(a.rhs, a.xin, a.xout, a.xc, n, h2, post, w, a.ph, a.pl, false);
 }
 
@@ -291,7 +295,7 @@ static void down_class_t(Solver* const* ms, int count, int l, cudaStream_t st) {
     Level& L = ms[i]->lev[l];
     tab.m[i] = {L.rhs, L.x, ms[i]->lev[l + 1].rhs, ms[i]->dev};
   }
-  k_mg_down_class<R><<<region_grid<R>(L0.n, count), R::THREADS, 0, st>>>(
+  launch_dependent(true, k_mg_down_class<R>, region_grid<R>(L0.n, count), dim3(R::THREADS), 0, st,
       tab, L0.n, L0.h2, ms[0]->prm.mg_pre_smooth, (float)ms[0]->prm.relax, ms[0]->prm.max_cycles);
 }
 
@@ -330,7 +334,7 @@ static void up_class_t(Solver* const* ms, int count, int l, cudaStream_t st) {
     tab.m[i] = {L.rhs, L.x, ACC ? nullptr : L.x2, s->lev[l + 1].x, ACC ? s->ph : nullptr, ACC ? s->pl : nullptr, s->dev};
     if (!ACC) std::swap(L.x, L.x2);
   }
-  k_mg_up_class<R, ACC><<<region_grid<R>(L0.n, count), R::THREADS, 0, st>>>(
+  launch_dependent(true, k_mg_up_class<R, ACC>, region_grid<R>(L0.n, count), dim3(R::THREADS), 0, st,
       tab, L0.n, L0.h2, ms[0]->prm.mg_post_smooth, (float)ms[0]->prm.relax, ms[0]->prm.max_cycles);
 }
 

@@ -843,6 +843,7 @@ struct CondTab {
 
 __global__ void __launch_bounds__(256, 5) k_refine_class(const RefineTab tab, int nx, int ny, LapScale ks,
                                                       int max_cycles, int quad) {
+  pdl_wait();
   const auto& a = tab.m[blockIdx.z];
   if (!member_in_loop(a.st, max_cycles)) return;
   if (quad) refine_init4_body(a.dh, a.dl, a.ph, a.pl, a.r32, nx, ny, ks, a.ctx, CondFold{});
@@ -855,6 +856,7 @@ __global__ void __launch_bounds__(256, 5) k_refine_class(const RefineTab tab, in
 __global__ void __launch_bounds__(kClassMax) k_cond_class(const CondTab tab, int count, int max_cycles,
                                                           cudaGraphConditionalHandle h, int init,
                                                           long long* iterations) {
+  pdl_wait();
   const int z = threadIdx.x;
   int again = 0;
   if (z < count) {
@@ -901,14 +903,14 @@ void launch_refine_class(Solver* const* ms, int count, cudaStream_t st) {
   const bool quad = g.nx % 4 == 0;
   dim3 grid = quad ? red_grid2(g.nx / 4, g.ny) : red_grid2(g.nx, g.ny);
   grid.z = count;
-  k_refine_class<<<grid, kBlock, 0, st>>>(tab, g.nx, g.ny, lap_scale(g), s0->prm.max_cycles, quad ? 1 : 0);
+  launch_dependent(true, k_refine_class, grid, kBlock, 0, st, tab, g.nx, g.ny, lap_scale(g), s0->prm.max_cycles, quad ? 1 : 0);
 }
 
 void launch_cond_class(Solver* const* ms, int count, cudaStream_t st, cudaGraphConditionalHandle h, int init,
                        long long* iterations) {
   CondTab tab{};
   for (int i = 0; i < count; i++) tab.m[i] = {ms[i]->red_out, ms[i]->dev, dev_tol(ms[i])};
-  k_cond_class<<<1, kClassMax, 0, st>>>(tab, count, ms[0]->prm.max_cycles, h, init, iterations);
+  launch_dependent(true, k_cond_class, dim3(1), dim3(kClassMax), 0, st, tab, count, ms[0]->prm.max_cycles, h, init, iterations);
 }
 
 // ---- the rest of a plain class member's step, batched: the divergence of the
@@ -937,16 +939,19 @@ struct ProjTab {
 };
 
 __global__ void __launch_bounds__(256) k_div_class(const ProjTab tab, int nx, int ny) {
+  pdl_wait();
   const auto& a = tab.m[blockIdx.z];
   div_df_body(a.wu, nullptr, a.wv, nullptr, a.dh, a.dl, nx, ny, a.idx, a.idy);
 }
 
 __global__ void __launch_bounds__(256) k_refine_zero_class(const ProjTab tab, int nx, int ny, LapScale ks) {
+  pdl_wait();
   const auto& a = tab.m[blockIdx.z];
   refine_init_body(a.dh, a.dl, a.ph, a.pl, a.r32, nx, ny, ks, 1, a.ctx);
 }
 
 __global__ void k_zero_p_class(const ProjTab tab, int64_t n) {
+  pdl_wait();
   const auto& a = tab.m[blockIdx.z];
   for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < n; k += (int64_t)gridDim.x * blockDim.x) {
     a.ph[k] = 0.f;
@@ -955,11 +960,13 @@ __global__ void k_zero_p_class(const ProjTab tab, int64_t n) {
 }
 
 __global__ void __launch_bounds__(256) k_div_start_class(const ProjTab tab, int nx, int ny) {
+  pdl_wait();
   const auto& a = tab.m[blockIdx.z];
   div_start4_body(a.wu, a.wv, a.dh, a.dl, a.ph, a.pl, a.r32, nx, ny, a.idx, a.idy, a.ctx);
 }
 
 __global__ void __launch_bounds__(256) k_subgrad_class(const ProjTab tab, int nx, int ny) {
+  pdl_wait();
   const auto& a = tab.m[blockIdx.z];
   finish_step(StepFinish{a.st, a.dt, 1});
   if ((nx & 3) == 0)
@@ -989,16 +996,16 @@ int launch_front_project_class(Solver* const* ms, int count, const float* const*
   if (g.nx % 4 == 0) {  // all three in one pass
     dim3 gq = red_grid2(g.nx / 4, g.ny);
     gq.z = count;
-    k_div_start_class<<<gq, kBlock, 0, st>>>(tab, g.nx, g.ny);
+    launch_dependent(true, k_div_start_class, gq, kBlock, 0, st, tab, g.nx, g.ny);
     return 1;
   }
   dim3 g2 = grid2d(g.nx, g.ny, kBlock);
   g2.z = count;
-  k_div_class<<<g2, kBlock, 0, st>>>(tab, g.nx, g.ny);
+  launch_dependent(true, k_div_class, g2, kBlock, 0, st, tab, g.nx, g.ny);
   dim3 gr = red_grid2(g.nx, g.ny);
   gr.z = count;
-  k_refine_zero_class<<<gr, kBlock, 0, st>>>(tab, g.nx, g.ny, lap_scale(g));
-  k_zero_p_class<<<dim3(fill_blocks(ms[0]->n), 1, count), 256, 0, st>>>(tab, ms[0]->n);
+  launch_dependent(true, k_refine_zero_class, gr, kBlock, 0, st, tab, g.nx, g.ny, lap_scale(g));
+  launch_dependent(true, k_zero_p_class, dim3(fill_blocks(ms[0]->n), 1, count), dim3(256), 0, st, tab, ms[0]->n);
   return 3;
 }
 
@@ -1009,7 +1016,7 @@ void launch_back_class(Solver* const* ms, int count, const float* const* wu, con
   const ProjTab tab = proj_tab(ms, count, wu, wv, dts);
   dim3 g2 = grid2d(g.nx % 4 == 0 ? g.nx / 4 : g.nx, g.ny, kBlock);  // four cells per thread when nx % 4 == 0
   g2.z = count;
-  k_subgrad_class<<<g2, kBlock, 0, st>>>(tab, g.nx, g.ny);
+  launch_dependent(true, k_subgrad_class, g2, kBlock, 0, st, tab, g.nx, g.ny);
 }
 
 
