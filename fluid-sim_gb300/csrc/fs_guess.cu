@@ -143,7 +143,7 @@ __global__ void k_prep(const float* __restrict__ div, const float* __restrict__ 
 // f32 values are widened with integer instructions.  A warp walks down a strip
 // of kLossCols columns (lanes 0 and 31 hold its neighbours' columns) with the
 // three rows of the stencil in registers.  1024^2 x 4, mean + residual + seed:
-// 39 + 175 + 163 us with a thread per cell that converted every operand, 105 + 148 us
+// 39 + 175 + 163 us with a thread per cell that converted every operand, 105 + 67 us
 // here (mean and residual in one pass).
 constexpr int kLossCols = 30, kLossWarps = 8;
 
@@ -238,7 +238,10 @@ __global__ void __launch_bounds__(32 * kLossWarps)
 }
 
 // seed gradient dL/dout = (w_p 2 (e - mean_b e) + w_r 2 lap(res)) / (B N) into
-// channel 0 of gJ; w_p sum (e - mean)^2 / (B N) into acc[B]
+// channel 0 of gJ; w_p sum (e - mean)^2 / (B N) into acc[B].  The loss is summed
+// in f64; the gradient, which is rounded to bf16, is formed in double-float (48
+// bits) on the FP32 pipe, in f64 where a value is too large for it or not finite
+// (the loss: 3 f64 instructions a cell, 11 with the gradient in f64, 148 us).
 __global__ void __launch_bounds__(32 * kLossWarps)
     k_loss_seed(const float* __restrict__ out, const float* __restrict__ tgt, const float* __restrict__ res,
                 double* __restrict__ acc, uint4* __restrict__ gJ, int H, int W, int B, int rows, double w_p,
@@ -247,27 +250,43 @@ __global__ void __launch_bounds__(32 * kLossWarps)
   const int b = blockIdx.y;
   const int64_t npix = (int64_t)H * W, base = b * npix;
   const double mean = acc[b] / (double)npix, scale = 2.0 / ((double)B * npix);
+  const df meanf = df_neg(df_from_d(mean)), wp = df_from_d(scale * w_p), wr = df_from_d(scale * w_r);
+  const bool dfok = fabs(mean) < 1e30 && scale * w_p < 1e6 && scale * w_r < 1e6;
   const LossStrip t = loss_strip(H, W, rows);
   double s = 0.0;
   if (t.any) {
     auto row = [&](int y) {
-      return res ? widen(res[base + (int64_t)(y < 0 ? y + H : y >= H ? y - H : y) * W + t.x]) : 0.0;
+      return res ? res[base + (int64_t)(y < 0 ? y + H : y >= H ? y - H : y) * W + t.x] : 0.f;
     };
-    double above = row(t.y0 - 1), c = row(t.y0);
+    float above = row(t.y0 - 1), c = row(t.y0);
 #pragma unroll 4
     for (int y = t.y0; y < t.y1; y++) {
       const int64_t q = base + (int64_t)y * W + t.x;
-      const double ec = widen(out[q]) - widen(tgt[q]) - mean;
-      double g = w_p * ec;
-      if (res) {
-        const double below = row(y + 1);
-        g += w_r * lap5(above, c, below);
-        above = c;
-        c = below;
-      }
+      const float o = out[q], g0 = tgt[q], below = row(y + 1);
+      const float left = __shfl_up_sync(0xffffffffu, c, 1), right = __shfl_down_sync(0xffffffffu, c, 1);
+      const double ec = widen(o) - widen(g0) - mean;
       if (t.store) s += ec * ec;
+      float g;
+      const float size = ((fabsf(o) + fabsf(g0)) + (fabsf(above) + fabsf(below))) + ((fabsf(left) + fabsf(right)) + fabsf(c));
+      if (dfok && size < 1e30f) {
+        df v = df_mul(df_add(two_sum(o, -g0), meanf), wp);
+        if (res) {
+          const df a = two_sum(left, right), d = two_sum(a.hi, above), e = two_sum(d.hi, below);
+          df l = two_sum(e.hi, -4.f * c);
+          l.lo = l.lo + ((a.lo + d.lo) + e.lo);
+          v = df_add(v, df_mul(fast_two_sum(l.hi, l.lo), wr));
+        }
+        g = df_to_f(v);
+      } else {
+        double v = w_p * ec;
+        if (res)
+          v += w_r * ((double)left + (double)right + (double)above + (double)below - 4.0 * (double)c);
+        g = (float)(scale * v);
+      }
+      above = c;
+      c = below;
       // the strip's pixels, 16 bytes a lane: channel 0 and zeros, zeros
-      const float f[8] = {(float)(scale * g), 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+      const float f[8] = {g, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
       const uint32_t first = pack8(f).x;
 #pragma unroll
       for (int half = 0; half < 2; half++) {

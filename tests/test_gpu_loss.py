@@ -31,3 +31,27 @@ def test_loss_value(fs, shape, weights):
     assert abs(loss - ref) <= 2e-11 * ref, (loss, ref)
     assert torch.isfinite(grad).all()
     g.close()
+
+
+@pytest.mark.parametrize("size", [1e25, 1e29, 1e31])
+def test_large_targets(fs, size):
+    """Either side of the size (1e30) above which the gradient is formed in
+    float64: against targets of 1 the gradient of this loss, which then hardly
+    depends on the network's output, scales with the targets."""
+    B, H, W = 1, 24, 40
+    rng = np.random.default_rng(5)
+    div, tgt = rng.standard_normal((2, B, H, W)).astype(np.float32)
+    tgt *= np.float32(1e6)
+    mask = np.zeros_like(div)
+    g = fs.PressureGuess(seed=31)
+    g.set_loss(0.1, 1.0)
+    f = np.float32(2.0) ** int(np.log2(size / 1e6))  # a power of two: the same significands
+    loss, grad = g.loss_grad(div, mask, tgt)
+    grad = grad.cpu().numpy().astype(np.float64)
+    loss_f, grad_f = g.loss_grad(div, mask, tgt * f)
+    grad_f = grad_f.cpu().numpy().astype(np.float64) / float(f)
+    # the output is 1e-6 of the targets: so is the difference of the errors; the
+    # bf16 rounding of a few seeds goes the other way (1e-6 of them by 2^-9)
+    assert abs(loss_f / float(f) ** 2 - loss) <= 1e-5 * loss
+    assert np.linalg.norm(grad_f - grad) <= 1e-3 * np.linalg.norm(grad)
+    g.close()
