@@ -19,6 +19,7 @@
 #include <vector>
 
 #include "fs_internal.cuh"
+#include "fs_stencil.cuh"
 #include "fs_tc.cuh"
 
 namespace fs {
@@ -707,16 +708,6 @@ void launch_advect_mc<float>(Solver* s, const float* u, const float* v, float* f
             launch_dependent(true, k_mc_combine_t, tile_grid(g), kBlock, 0, s->stream, u, v, fu, fv, s->mc_bounds, ou, ov, g.nx, g.ny,
                                                                    cx, cy, tu, tv, tfu, tfv, tma,
                                                                    &s->dev->async_err));
-}
-
-// DIFFUSE (shaders.js:401-425; src/cpu/solver.js:56-68 operand order)
-// c + a (l + r - 2c) + b (bo + t - 2c) with every rounding spelled out, in
-// the order of DIFFUSE (shaders.js:420), so that the one-cell and the
-// four-cell forms (and the batched kernels) round identically
-__device__ __forceinline__ float diffuse_cell(float c, float l, float r, float bo, float t, float a, float b) {
-  const float c2 = __fmul_rn(2.f, c);
-  return __fadd_rn(__fadd_rn(c, __fmul_rn(a, __fsub_rn(__fadd_rn(l, r), c2))),
-                   __fmul_rn(b, __fsub_rn(__fadd_rn(bo, t), c2)));
 }
 
 __device__ __forceinline__ void diffuse_body(const float* __restrict__ u, const float* __restrict__ v,

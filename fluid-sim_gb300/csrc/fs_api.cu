@@ -464,12 +464,14 @@ static int project_finish(Solver* s, const float* wu, const float* wv, const Ste
 
 static StepFinish step_end(const Solver* s, double dt) { return {s->dev, dt, s->stats_on_device ? 1 : 0}; }
 
-// step_dt: the projection ends a step.
+// step_dt: the projection ends a step; diffuse: (wu, wv) is to be made by diffusion.
 // defer: stop after the start of the pressure solve (see pressure_solve)
 static int project_from(Solver* s, const float* wu, const float* wv, bool capture, bool defer = false,
-                        const double* step_dt = nullptr) {
+                        const double* step_dt = nullptr, bool diffuse = false) {
   const bool start = s->mixed && !s->guess && !s->prm.warm_start;
-  if (start) launch_div_start(s, wu, wv);
+  if (diffuse && s->mixed) launch_diffuse_start(s, s->wu, s->wv, s->tu, s->tv, (float)*step_dt);
+  else if (diffuse) launch_diffuse_div(s, s->wu, s->wv, s->tu, s->tv, (float)*step_dt);
+  else if (start) launch_div_start(s, wu, wv);
   else if (s->mixed) launch_div_df(s, wu, nullptr, wv, nullptr, s->dh, s->dl);
   else launch_divergence<float, float>(s, wu, wv, s->div32);
   int rc = pressure_solve(s, capture, defer, start);
@@ -499,15 +501,16 @@ static int enqueue_step(Solver* s, double dt, bool capture, StepSplit* split = n
   float fdt = (float)dt;
   advect_into(s, fdt, s->wu, s->wv);
   float *cu = s->wu, *cv = s->wv;
+  const bool fused = diffuse_fused(s);  // made by project_from
   if (s->prm.nu > 0) {
-    launch_diffuse(s, cu, cv, s->tu, s->tv, fdt);
+    if (!fused) launch_diffuse(s, cu, cv, s->tu, s->tv, fdt);
     cu = s->tu; cv = s->tv;
   }
   if (s->band) launch_band(s, cu, cv, fdt);
   if (s->n_modes > 0) launch_forcing(s, cu, cv, fdt);
   if (s->channel_on) launch_channel(s, cu, cv);
   if (!s->disks.empty()) launch_solids(s, cu, cv, fdt, false);
-  int rc = project_from(s, cu, cv, capture, split != nullptr, &dt);
+  int rc = project_from(s, cu, cv, capture, split != nullptr, &dt, fused);
   if (split) {
     split->wu = cu;
     split->wv = cv;

@@ -312,6 +312,19 @@ bool launch_refine_init(Solver* s, const float* dh, const float* dl, const float
 bool box_tmap(Solver* s, const float* f, int nx, int ny, int bw, int bh, CUtensorMap* out);
 // divergence + zero-pressure residual + zeroed pressure in one pass (MIXED)
 void launch_div_start(Solver* s, const float* wu, const float* wv);
+// DIFFUSE in the same pass as the divergence (F32) or the start of a MIXED solve
+// from zero pressure
+void launch_diffuse_div(Solver* s, const float* u, const float* v, float* ou, float* ov, float dt);
+void launch_diffuse_start(Solver* s, const float* u, const float* v, float* ou, float* ov, float dt);
+// a step's diffusion goes with its divergence: nothing comes between the two, and
+// the solve starts from that divergence (kernel_variant 1 runs them one by one).
+// A launch and 8 bytes a cell less: a pass of 192^2 mixed steps 1021 -> 1005 us, of
+// 4096^2 8327 -> 8265.  (A batch's class kernels stay apart: fused they were 1%
+// slower.)
+inline bool diffuse_fused(const Solver* s) {
+  return s->prm.kernel_variant == 0 && s->prm.nu > 0 && s->g.nx % 4 == 0 && !s->band && s->n_modes == 0 &&
+         !s->channel_on && s->disks.empty() && !(s->mixed && (s->guess || s->prm.warm_start));
+}
 void launch_refine_update(Solver* s, const float* ph, const float* pl, const float* e, const float* dh,
                           const float* dl, float* poh, float* pol, float* r32);
 // reductions (results land in s->red_out)

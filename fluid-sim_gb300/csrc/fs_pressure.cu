@@ -40,6 +40,64 @@ __global__ void __launch_bounds__(256) k_divergence(const TV* __restrict__ u, co
   d[c] = (uR - uL) * idx + (vT - vB) * idy;
 }
 
+// The faces a thread's four cells (j, i0 ..) take their divergence from.  The
+// diffused ones are made from the velocity before diffusion (DIFFUSE of the same
+// step, diffuse_cell): the four cells' own, and the right and upper neighbours'
+// again, which another thread makes and stores.
+struct FaceQuad {
+  float4 u, v, t;  // u and v at row j, v at row j + 1
+  float ur;        // u right of the quad
+};
+__device__ __forceinline__ float4 diffuse_quad(const float* __restrict__ row, float4 c, float4 b, float4 t, int il,
+                                               int ir, float ax, float ay) {
+  const float l = __ldg(row + il), r = __ldg(row + ir);
+  return {diffuse_cell(c.x, l, c.y, b.x, t.x, ax, ay), diffuse_cell(c.y, c.x, c.z, b.y, t.y, ax, ay),
+          diffuse_cell(c.z, c.y, c.w, b.z, t.z, ax, ay), diffuse_cell(c.w, c.z, r, b.w, t.w, ax, ay)};
+}
+__device__ __forceinline__ FaceQuad diffused_faces(const float* __restrict__ u, const float* __restrict__ v, int nx,
+                                                   int ny, int i0, int j, float ax, float ay) {
+  const int jm = j == 0 ? ny - 1 : j - 1, jp = j + 1 == ny ? 0 : j + 1, jq = jp + 1 == ny ? 0 : jp + 1;
+  const int il = i0 == 0 ? nx - 1 : i0 - 1, ir = i0 + 4 == nx ? 0 : i0 + 4;
+  const int64_t r = (int64_t)j * nx, rm = (int64_t)jm * nx, rp = (int64_t)jp * nx, rq = (int64_t)jq * nx;
+  auto quad = [&](const float* f, int64_t row) { return __ldg(reinterpret_cast<const float4*>(f + row + i0)); };
+  const float4 um = quad(u, rm), uc = quad(u, r), up = quad(u, rp);
+  const float4 vm = quad(v, rm), vc = quad(v, r), vp = quad(v, rp), vq = quad(v, rq);
+  FaceQuad f;
+  f.u = diffuse_quad(u + r, uc, um, up, il, ir, ax, ay);
+  f.v = diffuse_quad(v + r, vc, vm, vp, il, ir, ax, ay);
+  f.t = diffuse_quad(v + rp, vp, vc, vq, il, ir, ax, ay);
+  f.ur = diffuse_cell(__ldg(u + r + ir), uc.w, __ldg(u + r + (ir + 1)), __ldg(u + rm + ir), __ldg(u + rp + ir), ax, ay);
+  return f;
+}
+
+// DIFFUSE and the divergence of its result in one pass (nx a multiple of 4)
+__global__ void __launch_bounds__(256)
+    k_diffuse_div4(const float* __restrict__ u, const float* __restrict__ v, float* __restrict__ ou,
+                   float* __restrict__ ov, float* __restrict__ d, int nx, int ny, float ax, float ay, float idx,
+                   float idy) {
+  pdl_wait();
+  const int q = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
+  if (q >= (nx >> 2) || j >= ny) return;
+  const int64_t c = (int64_t)j * nx + 4 * q;
+  const FaceQuad f = diffused_faces(u, v, nx, ny, 4 * q, j, ax, ay);
+  *reinterpret_cast<float4*>(ou + c) = f.u;
+  *reinterpret_cast<float4*>(ov + c) = f.v;
+  // as k_divergence's is contracted
+  auto div = [&](float uL, float uR, float vB, float vT) {
+    return __fmaf_rn(__fsub_rn(uR, uL), idx, __fmul_rn(__fsub_rn(vT, vB), idy));
+  };
+  *reinterpret_cast<float4*>(d + c) = {div(f.u.x, f.u.y, f.v.x, f.t.x), div(f.u.y, f.u.z, f.v.y, f.t.y),
+                                       div(f.u.z, f.u.w, f.v.z, f.t.z), div(f.u.w, f.ur, f.v.w, f.t.w)};
+}
+
+void launch_diffuse_div(Solver* s, const float* u, const float* v, float* ou, float* ov, float dt) {
+  const Grid& g = s->g;
+  const float ax = (float)(s->prm.nu * dt / (g.dxd * g.dxd)), ay = (float)(s->prm.nu * dt / (g.dyd * g.dyd));
+  FS_LAUNCH(s, "diffuse_divergence", (double)s->n * 20,
+            launch_dependent(true, k_diffuse_div4, grid2d(g.nx / 4, g.ny, kBlock), kBlock, 0, s->stream, u, v, ou, ov,
+                             s->div32, g.nx, g.ny, ax, ay, g.idx, g.idy));
+}
+
 template <class TV, class TD>
 void launch_divergence(Solver* s, const TV* u, const TV* v, TD* d) {
   const Grid& g = s->g;
@@ -321,11 +379,18 @@ __device__ __forceinline__ df div_f32_faces(float uc, float ur, float vc, float 
 // arithmetic per cell.  Four consecutive cells per thread (nx a multiple of
 // 4), so a thread keeps five 16-byte loads in flight; tiles of 32 quads x 8
 // rows walked by the capped reduction grid.
+// With DIFFUSE, (wu, wv) is the velocity before diffusion and the diffused one goes
+// to (ou, ov) in the same pass.
+struct DiffuseOut {
+  float *ou, *ov;
+  float ax, ay;
+};
+template <bool DIFFUSE>
 __device__ __forceinline__ void div_start4_body(const float* __restrict__ wu, const float* __restrict__ wv,
                                                 float* __restrict__ dh, float* __restrict__ dl,
                                                 float* __restrict__ ph, float* __restrict__ pl,
                                                 float* __restrict__ r32, int nx, int ny, df idx, df idy,
-                                                const RedCtx& ctx) {
+                                                const RedCtx& ctx, const DiffuseOut& o = {}) {
   float m = 0.f;
   const int nq = nx >> 2;
   for (int ty = blockIdx.y, nty = (ny + 7) >> 3; ty < nty; ty += gridDim.y)
@@ -335,10 +400,19 @@ __device__ __forceinline__ void div_start4_body(const float* __restrict__ wu, co
       const int i0 = q << 2;
       const int jp = j + 1 == ny ? 0 : j + 1, ir = i0 + 4 == nx ? 0 : i0 + 4;
       const int64_t r = (int64_t)j * nx;
-      const float4 u4 = __ldg(reinterpret_cast<const float4*>(wu + r + i0));
-      const float4 v4 = __ldg(reinterpret_cast<const float4*>(wv + r + i0));
-      const float4 t4 = __ldg(reinterpret_cast<const float4*>(wv + (int64_t)jp * nx + i0));
-      const float ur = __ldg(wu + r + ir);
+      FaceQuad f;
+      if constexpr (DIFFUSE) {
+        f = diffused_faces(wu, wv, nx, ny, i0, j, o.ax, o.ay);
+        *reinterpret_cast<float4*>(o.ou + r + i0) = f.u;
+        *reinterpret_cast<float4*>(o.ov + r + i0) = f.v;
+      } else {
+        f.u = __ldg(reinterpret_cast<const float4*>(wu + r + i0));
+        f.v = __ldg(reinterpret_cast<const float4*>(wv + r + i0));
+        f.t = __ldg(reinterpret_cast<const float4*>(wv + (int64_t)jp * nx + i0));
+        f.ur = __ldg(wu + r + ir);
+      }
+      const float4 u4 = f.u, v4 = f.v, t4 = f.t;
+      const float ur = f.ur;
       const df d0 = div_f32_faces(u4.x, u4.y, v4.x, t4.x, idx, idy);
       const df d1 = div_f32_faces(u4.y, u4.z, v4.y, t4.y, idx, idy);
       const df d2 = div_f32_faces(u4.z, u4.w, v4.z, t4.z, idx, idy);
@@ -360,7 +434,15 @@ __global__ void __launch_bounds__(256)
                  float* __restrict__ dl, float* __restrict__ ph, float* __restrict__ pl, float* __restrict__ r32,
                  int nx, int ny, df idx, df idy, RedCtx ctx) {
   pdl_wait();
-  div_start4_body(wu, wv, dh, dl, ph, pl, r32, nx, ny, idx, idy, ctx);
+  div_start4_body<false>(wu, wv, dh, dl, ph, pl, r32, nx, ny, idx, idy, ctx);
+}
+
+__global__ void __launch_bounds__(256)
+    k_diffuse_start4(const float* __restrict__ wu, const float* __restrict__ wv, float* __restrict__ dh,
+                     float* __restrict__ dl, float* __restrict__ ph, float* __restrict__ pl, float* __restrict__ r32,
+                     int nx, int ny, df idx, df idy, RedCtx ctx, const DiffuseOut o) {
+  pdl_wait();
+  div_start4_body<true>(wu, wv, dh, dl, ph, pl, r32, nx, ny, idx, idy, ctx, o);
 }
 
 __global__ void __launch_bounds__(256)
@@ -716,6 +798,16 @@ bool launch_refine_init(Solver* s, const float* dh, const float* dl, const float
   return cf.on != 0;
 }
 
+// the same with the step's diffusion in front, (u, v) -> (ou, ov) (nx a multiple of 4)
+void launch_diffuse_start(Solver* s, const float* u, const float* v, float* ou, float* ov, float dt) {
+  const Grid& g = s->g;
+  const DiffuseOut o = {ou, ov, (float)(s->prm.nu * dt / (g.dxd * g.dxd)), (float)(s->prm.nu * dt / (g.dyd * g.dyd))};
+  FS_LAUNCH(s, "diffuse_start", (double)s->n * 36,
+            launch_dependent(true, k_diffuse_start4, red_grid2(g.nx / 4, g.ny), kBlock, 0, s->stream, u, v, s->dh, s->dl,
+                             s->ph, s->pl, s->r32, g.nx, g.ny, df_host(g.idxd), df_host(g.idyd),
+                             red_ctx(s, s->red_out), o));
+}
+
 // the start of a MIXED solve from zero pressure (k_div_start4; nx a multiple
 // of 4, else the divergence, the zero-pressure residual and two fills)
 void launch_div_start(Solver* s, const float* wu, const float* wv) {
@@ -962,7 +1054,7 @@ __global__ void k_zero_p_class(const ProjTab tab, int64_t n) {
 __global__ void __launch_bounds__(256) k_div_start_class(const ProjTab tab, int nx, int ny) {
   pdl_wait();
   const auto& a = tab.m[blockIdx.z];
-  div_start4_body(a.wu, a.wv, a.dh, a.dl, a.ph, a.pl, a.r32, nx, ny, a.idx, a.idy, a.ctx);
+  div_start4_body<false>(a.wu, a.wv, a.dh, a.dl, a.ph, a.pl, a.r32, nx, ny, a.idx, a.idy, a.ctx);
 }
 
 __global__ void __launch_bounds__(256) k_subgrad_class(const ProjTab tab, int nx, int ny) {

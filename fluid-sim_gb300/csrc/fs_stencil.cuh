@@ -53,4 +53,14 @@ __device__ __forceinline__ float restrict4(float r00, float r10, float r01, floa
   return __fmul_rn(__fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(0.f, r00), r10), r01), r11), 0.25f);
 }
 
+// DIFFUSE (shaders.js:401-425; src/cpu/solver.js:56-68 operand order)
+// c + a (l + r - 2c) + b (bo + t - 2c) with every rounding spelled out, in
+// the order of DIFFUSE (shaders.js:420), so that the one-cell and the
+// four-cell forms (and the batched kernels) round identically
+__device__ __forceinline__ float diffuse_cell(float c, float l, float r, float bo, float t, float a, float b) {
+  const float c2 = __fmul_rn(2.f, c);
+  return __fadd_rn(__fadd_rn(c, __fmul_rn(a, __fsub_rn(__fadd_rn(l, r), c2))),
+                   __fmul_rn(b, __fsub_rn(__fadd_rn(bo, t), c2)));
+}
+
 }  // namespace fs
