@@ -232,28 +232,37 @@ __device__ __forceinline__ uint32_t smem_absmax_bits(const float* sm) {
   return m;
 }
 
-// TMA staging of F kSH x kSW blocks (tiles whose block lies inside the grid):
-// thread 0 arms the barrier and issues the copies, every thread waits (bounded).
-// Returns false on every thread if the wait gave up (after waiting once more
-// for the copies in flight and raising *err); the caller then skips the tile.
-template <int F>
-__device__ __forceinline__ bool tma_stage(float* const (&sm)[F], const CUtensorMap* const (&tm)[F], int oi, int oj,
-                                          uint64_t* bar, int* err) {
+// TMA staging of NT blocks of F kSH x kSW fields each, one barrier a block (blocks
+// inside the grid only: in[t]): thread 0 arms the barriers and issues all copies;
+// tma_landed waits (bounded) for block t.  False on every thread if the wait gave
+// up, after waiting once more for the copies in flight and raising *err; the
+// caller then skips its tiles.
+template <int F, int NT>
+__device__ __forceinline__ void tma_issue(float (*const (&sm)[F])[kSW * kSH], const CUtensorMap* const (&tm)[F], int oi,
+                                          int oj, const bool (&in)[NT], uint64_t* bar) {
   const int tid = threadIdx.y * blockDim.x + threadIdx.x;
   if (tid == 0) {
-    tc::mbar_init(bar, 1);
+#pragma unroll
+    for (int t = 0; t < NT; t++) tc::mbar_init(&bar[t], 1);
     tc::mbar_fence_init();
   }
   __syncthreads();
-  if (tid == 0) {
-    tc::mbar_arrive_expect_tx(bar, (uint32_t)(F * kSW * kSH * sizeof(float)));
+  if (tid != 0) return;
 #pragma unroll
-    for (int q = 0; q < F; q++) tc::tma_load_2d(sm[q], tm[q], oi, oj, bar);
+  for (int t = 0; t < NT; t++) {
+    if (!in[t]) continue;
+    tc::mbar_arrive_expect_tx(&bar[t], (uint32_t)(F * kSW * kSH * sizeof(float)));
+#pragma unroll
+    for (int q = 0; q < F; q++) tc::tma_load_2d(sm[q][t], tm[q], oi, oj + t * kTY, &bar[t]);
   }
-  const bool ok = __syncthreads_and(tc::mbar_wait_idle(bar, 0)) != 0;
+}
+template <int NT>
+__device__ __forceinline__ bool tma_landed(int t, const bool (&in)[NT], uint64_t* bar, int* err) {
+  const bool ok = __syncthreads_and(tc::mbar_wait_idle(&bar[t], 0)) != 0;
   if (!ok) {
-    if (tid == 0) atomicExch(err, 1);
-    tc::mbar_wait_idle(bar, 0);
+    if (threadIdx.x == 0 && threadIdx.y == 0) atomicExch(err, 1);
+    for (int k = t; k < NT; k++)
+      if (in[k]) tc::mbar_wait_idle(&bar[k], 0);
   }
   return ok;
 }
@@ -273,8 +282,9 @@ __device__ __forceinline__ bool fast_tile(float umax, float vmax, float cx, floa
 // contraction.  The floor of an offset x (|x| < 2^22) is taken by adding 1.5 *
 // 2^23, rounded down, which leaves the integer in the sum's low bits; row and
 // column are joined by one multiply-add in that form.  With waits for the TMA
-// copies that do not spin (they took issue slots too), 4096^2: forward 175 -> 152
-// us, combine 195 -> 160 us, of which the bytes are 79 us and 99 us.
+// copies that do not spin (they took issue slots too), 4096^2: forward 175 -> 151
+// us, combine 195 -> 174 us (with two tiles staged at once, tiles_per_cta, 137 and
+// 158), of which the bytes are 79 us and 99 us.
 struct F2 {
   unsigned long long v;
 };
@@ -423,35 +433,46 @@ __device__ __forceinline__ void advect_rows(const TileView& U, const TileView& V
 
 // Tiles whose staged block lies inside the grid are staged by TMA when the
 // tensor maps are valid (tma != 0); the others by the wrapped loads.
+template <int NT>
 __global__ void __launch_bounds__(256) k_advect_sl_t(const float* __restrict__ u, const float* __restrict__ v,
                                                      float* __restrict__ ou, float* __restrict__ ov, int nx, int ny,
                                                      float cx, float cy, float* __restrict__ bounds,
                                                      const __grid_constant__ CUtensorMap tm_u,
                                                      const __grid_constant__ CUtensorMap tm_v, int tma, int* err) {
   pdl_wait();
-  __shared__ __align__(128) float su[kSW * kSH];
-  __shared__ __align__(128) float sv[kSW * kSH];
-  __shared__ uint64_t bar;
-  const int ti = blockIdx.x * kTX, tj = blockIdx.y * kTY;
-  const int oi = ti - kHalo, oj = tj - kHalo;
-  float umax, vmax;
+  __shared__ __align__(128) float su[NT][kSW * kSH];
+  __shared__ __align__(128) float sv[NT][kSW * kSH];
+  __shared__ uint64_t bar[NT];
+  const int ti = blockIdx.x * kTX, oi = ti - kHalo, oj = blockIdx.y * NT * kTY - kHalo;
+  bool in[NT];
+#pragma unroll
+  for (int t = 0; t < NT; t++)
+    in[t] = tma && oi >= 0 && oj + t * kTY >= 0 && oi + kSW <= nx && oj + t * kTY + kSH <= ny;
   {
-    float* const sm[2] = {su, sv};
-    if (tma && oi >= 0 && oj >= 0 && oi + kSW <= nx && oj + kSH <= ny) {
-      const CUtensorMap* const tm[2] = {&tm_u, &tm_v};
-      if (!tma_stage<2>(sm, tm, oi, oj, &bar, err)) return;
-      umax = __uint_as_float(smem_absmax_bits(su));
-      vmax = __uint_as_float(smem_absmax_bits(sv));
-    } else {
-      const float* const f[2] = {u, v};
-      stage_tiles<2>(sm, f, oi, oj, nx, ny, umax, vmax);
-    }
+    float(*const sm[2])[kSW * kSH] = {su, sv};
+    const CUtensorMap* const tm[2] = {&tm_u, &tm_v};
+    tma_issue<2, NT>(sm, tm, oi, oj, in, bar);
   }
-  if (fast_tile(umax, vmax, cx, cy)) {
-    advect_pair(su, sv, ou, ov, nx, ny, ti, tj, cx, cy, bounds);
-  } else {
-    const TileView U{su, oi, oj, u, nx, ny}, V{sv, oi, oj, v, nx, ny};
-    advect_rows(U, V, ou, ov, nx, ny, ti, tj, cx, cy, bounds);
+#pragma unroll
+  for (int t = 0; t < NT; t++) {
+    const int tj = (blockIdx.y * NT + t) * kTY;
+    if (tj >= ny) break;
+    float umax, vmax;
+    if (in[t]) {
+      if (!tma_landed<NT>(t, in, bar, err)) return;
+      umax = __uint_as_float(smem_absmax_bits(su[t]));
+      vmax = __uint_as_float(smem_absmax_bits(sv[t]));
+    } else {
+      float* const sm[2] = {su[t], sv[t]};
+      const float* const f[2] = {u, v};
+      stage_tiles<2>(sm, f, oi, tj - kHalo, nx, ny, umax, vmax);
+    }
+    if (fast_tile(umax, vmax, cx, cy)) {
+      advect_pair(su[t], sv[t], ou, ov, nx, ny, ti, tj, cx, cy, bounds);
+    } else {
+      const TileView U{su[t], oi, tj - kHalo, u, nx, ny}, V{sv[t], oi, tj - kHalo, v, nx, ny};
+      advect_rows(U, V, ou, ov, nx, ny, ti, tj, cx, cy, bounds);
+    }
   }
 }
 
@@ -519,6 +540,7 @@ __device__ __forceinline__ void combine_pair(const float* su, const float* sv, c
   }
 }
 
+template <int NT>
 __global__ void __launch_bounds__(256) k_mc_combine_t(const float* __restrict__ u, const float* __restrict__ v,
                                                       const float* __restrict__ fu, const float* __restrict__ fv,
                                                       const float* __restrict__ bounds, float* __restrict__ ou,
@@ -528,32 +550,42 @@ __global__ void __launch_bounds__(256) k_mc_combine_t(const float* __restrict__ 
                                                       const __grid_constant__ CUtensorMap tm_fu,
                                                       const __grid_constant__ CUtensorMap tm_fv, int tma, int* err) {
   pdl_wait();
-  __shared__ __align__(128) float su[kSW * kSH];
-  __shared__ __align__(128) float sv[kSW * kSH];
-  __shared__ __align__(128) float sfu[kSW * kSH];
-  __shared__ __align__(128) float sfv[kSW * kSH];
-  __shared__ uint64_t bar;
-  const int ti = blockIdx.x * kTX, tj = blockIdx.y * kTY;
-  const int oi = ti - kHalo, oj = tj - kHalo;
-  float umax, vmax;
+  __shared__ __align__(128) float su[NT][kSW * kSH];
+  __shared__ __align__(128) float sv[NT][kSW * kSH];
+  __shared__ __align__(128) float sfu[NT][kSW * kSH];
+  __shared__ __align__(128) float sfv[NT][kSW * kSH];
+  __shared__ uint64_t bar[NT];
+  const int ti = blockIdx.x * kTX, oi = ti - kHalo, oj = blockIdx.y * NT * kTY - kHalo;
+  bool in[NT];
+#pragma unroll
+  for (int t = 0; t < NT; t++)
+    in[t] = tma && oi >= 0 && oj + t * kTY >= 0 && oi + kSW <= nx && oj + t * kTY + kSH <= ny;
   {
-    float* const sm[4] = {su, sv, sfu, sfv};
-    if (tma && oi >= 0 && oj >= 0 && oi + kSW <= nx && oj + kSH <= ny) {
-      const CUtensorMap* const tm[4] = {&tm_u, &tm_v, &tm_fu, &tm_fv};
-      if (!tma_stage<4>(sm, tm, oi, oj, &bar, err)) return;
-      umax = __uint_as_float(smem_absmax_bits(su));
-      vmax = __uint_as_float(smem_absmax_bits(sv));
-    } else {
-      const float* const f[4] = {u, v, fu, fv};
-      stage_tiles<4>(sm, f, oi, oj, nx, ny, umax, vmax);
-    }
+    float(*const sm[4])[kSW * kSH] = {su, sv, sfu, sfv};
+    const CUtensorMap* const tm[4] = {&tm_u, &tm_v, &tm_fu, &tm_fv};
+    tma_issue<4, NT>(sm, tm, oi, oj, in, bar);
   }
-  if (fast_tile(umax, vmax, cx, cy)) {
-    combine_pair(su, sv, sfu, sfv, bounds, ou, ov, nx, ny, ti, tj, cx, cy);
-  } else {
-    const TileView U{su, oi, oj, u, nx, ny}, V{sv, oi, oj, v, nx, ny};
-    const TileView FU{sfu, oi, oj, fu, nx, ny}, FV{sfv, oi, oj, fv, nx, ny};
-    combine_rows(U, V, FU, FV, bounds, ou, ov, nx, ny, ti, tj, cx, cy);
+#pragma unroll
+  for (int t = 0; t < NT; t++) {
+    const int tj = (blockIdx.y * NT + t) * kTY;
+    if (tj >= ny) break;
+    float umax, vmax;
+    if (in[t]) {
+      if (!tma_landed<NT>(t, in, bar, err)) return;
+      umax = __uint_as_float(smem_absmax_bits(su[t]));
+      vmax = __uint_as_float(smem_absmax_bits(sv[t]));
+    } else {
+      float* const sm[4] = {su[t], sv[t], sfu[t], sfv[t]};
+      const float* const f[4] = {u, v, fu, fv};
+      stage_tiles<4>(sm, f, oi, tj - kHalo, nx, ny, umax, vmax);
+    }
+    if (fast_tile(umax, vmax, cx, cy)) {
+      combine_pair(su[t], sv[t], sfu[t], sfv[t], bounds, ou, ov, nx, ny, ti, tj, cx, cy);
+    } else {
+      const TileView U{su[t], oi, tj - kHalo, u, nx, ny}, V{sv[t], oi, tj - kHalo, v, nx, ny};
+      const TileView FU{sfu[t], oi, tj - kHalo, fu, nx, ny}, FV{sfv[t], oi, tj - kHalo, fv, nx, ny};
+      combine_rows(U, V, FU, FV, bounds, ou, ov, nx, ny, ti, tj, cx, cy);
+    }
   }
 }
 
@@ -631,7 +663,16 @@ __global__ void __launch_bounds__(256) k_mc_combine_class(const AdvTab tab, int 
 
 static const dim3 kBlock(32, 8);
 
-static dim3 tile_grid(const Grid& g) { return dim3((g.nx + kTX - 1) / kTX, (g.ny + kTY - 1) / kTY); }
+static dim3 tile_grid(const Grid& g, int nt = 1) {
+  return dim3((g.nx + kTX - 1) / kTX, (g.ny + nt * kTY - 1) / (nt * kTY));
+}
+
+// Tiles a CTA stages at once, one above the other: with two the copies of the
+// second are in flight while the first is worked on (4096^2: forward 151 -> 137
+// us, combine 174 -> 158; three 142 and 164).  Below 2048^2, where that leaves few
+// CTAs an SM, one is as fast (1024^2 303.4 us a step against 304.1) or faster
+// (512^2 110.7 against 118.9).
+static int tiles_per_cta(const Grid& g) { return (int64_t)g.nx * g.ny >= 4000000 ? 2 : 1; }
 
 
 
@@ -689,7 +730,7 @@ void launch_advect_sl<float>(Solver* s, const float* u, const float* v, float* o
   CUtensorMap tu{}, tv{};
   const int tma = tile_tmap(s, u, &tu) && tile_tmap(s, v, &tv) ? 1 : 0;
   FS_LAUNCH(s, "advect_sl", (double)s->n * 16,
-            k_advect_sl_t<<<tile_grid(g), kBlock, 0, s->stream>>>(u, v, ou, ov, g.nx, g.ny, cx, cy, nullptr, tu, tv,
+            (tiles_per_cta(g) == 2 ? k_advect_sl_t<2> : k_advect_sl_t<1>)<<<tile_grid(g, tiles_per_cta(g)), kBlock, 0, s->stream>>>(u, v, ou, ov, g.nx, g.ny, cx, cy, nullptr, tu, tv,
                                                                   tma, &s->dev->async_err));
 }
 
@@ -702,10 +743,11 @@ void launch_advect_mc<float>(Solver* s, const float* u, const float* v, float* f
   const int tma =
       tile_tmap(s, u, &tu) && tile_tmap(s, v, &tv) && tile_tmap(s, fu, &tfu) && tile_tmap(s, fv, &tfv) ? 1 : 0;
   FS_LAUNCH(s, "advect_sl", (double)s->n * 32,
-            k_advect_sl_t<<<tile_grid(g), kBlock, 0, s->stream>>>(u, v, fu, fv, g.nx, g.ny, cx, cy, s->mc_bounds, tu,
+            (tiles_per_cta(g) == 2 ? k_advect_sl_t<2> : k_advect_sl_t<1>)<<<tile_grid(g, tiles_per_cta(g)), kBlock, 0, s->stream>>>(u, v, fu, fv, g.nx, g.ny, cx, cy, s->mc_bounds, tu,
                                                                   tv, tma, &s->dev->async_err));
   FS_LAUNCH(s, "mc_combine", (double)s->n * 40,
-            launch_dependent(true, k_mc_combine_t, tile_grid(g), kBlock, 0, s->stream, u, v, fu, fv, s->mc_bounds, ou, ov, g.nx, g.ny,
+            launch_dependent(true, tiles_per_cta(g) == 2 ? k_mc_combine_t<2> : k_mc_combine_t<1>,
+                             tile_grid(g, tiles_per_cta(g)), kBlock, 0, s->stream, u, v, fu, fv, s->mc_bounds, ou, ov, g.nx, g.ny,
                                                                    cx, cy, tu, tv, tfu, tfv, tma,
                                                                    &s->dev->async_err));
 }

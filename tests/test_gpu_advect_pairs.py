@@ -30,3 +30,26 @@ def test_rolled_field(fs, ny, nx, scheme, precision):
         for f, r in zip(advect(np.roll(u, roll, (0, 1)), np.roll(v, roll, (0, 1))), ref):
             np.testing.assert_array_equal(f, np.roll(r, roll, (0, 1)))
     s.destroy()
+
+
+def test_two_tiles_per_cta(fs):
+    """Large grids stage two tiles a CTA: an odd number of tile rows, edge tiles
+    beside inner ones and a last tile cut in both directions, rolled."""
+    ny, nx = 2040, 2052
+    rng = np.random.default_rng(1)
+    u, v = rng.uniform(-1.0, 1.0, (2, ny, nx))
+    for scheme in ("semi-lagrangian", "maccormack"):
+        s = fs.GPUFluidSolver(nx=nx, ny=ny, lx=2 * np.pi * nx / ny, ly=2 * np.pi, advection=scheme,
+                              pressure_iterations=0)
+        dt = 2.5 * 2 * np.pi / ny
+
+        def advect(a, b):
+            s.upload_velocity(a, b)
+            s.run_stage("advect", dt)
+            return [f.reshape(ny, nx) for f in s.read_velocity()]
+
+        ref = advect(u, v)
+        roll = (17, 41)
+        for f, r in zip(advect(np.roll(u, roll, (0, 1)), np.roll(v, roll, (0, 1))), ref):
+            np.testing.assert_array_equal(f, np.roll(r, roll, (0, 1)))
+        s.destroy()
