@@ -25,10 +25,6 @@
 
 namespace fs {
 
-__device__ __forceinline__ void prefetch_l2(const void* p) {
-  asm volatile("prefetch.global.L2 [%0];" ::"l"((size_t)__cvta_generic_to_global(p)));
-}
-
 // H rings: 2 pre + 1 (down) or 2 post (up)
 template <int CPL_, int RPW_, int NW_, int H>
 struct MgRegion {
@@ -83,6 +79,21 @@ struct MgCells {
     return lane * R::CPL >= R::HX && lane * R::CPL < R::RW - R::HX && xl < n;
   }
 };
+
+// two fields of the region that the CTA `ahead` launches on will load, into L2: a
+// 128-byte line per thread and field
+template <class R>
+__device__ __forceinline__ void prefetch_region(int n, int ahead, const float* f, const float* g) {
+  const int b = blockIdx.y * gridDim.x + blockIdx.x + ahead;
+  if (b >= (int)(gridDim.x * gridDim.y)) return;
+  constexpr int LINES = R::RW / 32;
+  for (int k = threadIdx.x; k < LINES * R::RH; k += R::THREADS) {
+    const int x = flat_wrap((b % gridDim.x) * R::TW - R::HX + (k % LINES) * 32, n);
+    const int y = flat_wrap((int)(b / gridDim.x) * R::TH - R::HY + k / LINES, n);
+    prefetch_l2(f + (int64_t)y * n + x);
+    prefetch_l2(g + (int64_t)y * n + x);
+  }
+}
 
 // xin == nullptr: the level starts from zero.  xout == xin is not allowed (the
 // halo of a tile is another tile's interior).
@@ -163,7 +174,8 @@ __device__ __forceinline__ void mg_restrict_rhs(const float* __restrict__ rhs, f
 // (0 + P = P, and a -0 from P gives the same pressure sum as +0).  With ACC the
 // tile's correction is added to the double-float pressure (ph, pl) in place
 // instead of being written to xout: a cell is read and written by its own tile.
-template <class R, bool ACC>
+// AHEAD > 0: the CTA fetches a later one's iterate and rhs into L2.
+template <class R, bool ACC, int AHEAD>
 __device__ __forceinline__ void mg_up_reg(const float* __restrict__ rhs, const float* __restrict__ xin,
                                           float* __restrict__ xout, const float* __restrict__ xc, int n, float h2,
                                           int post, float w, float* __restrict__ ph, float* __restrict__ pl,
@@ -196,6 +208,7 @@ __device__ __forceinline__ void mg_up_reg(const float* __restrict__ rhs, const f
     t.load(t.d, rhs, n);
   }
   pdl_wait();
+  if (AHEAD > 0 && !zero) prefetch_region<R>(n, AHEAD, xin, rhs);
   float cv[CR][CC], side[CR];
   const int gs = flat_wrap(t.lane == 0 ? gc - 1 : gc + CC, nc);
 #pragma unroll

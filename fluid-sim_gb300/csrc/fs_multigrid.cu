@@ -17,7 +17,7 @@
 // The tiles are fs_mgreg.cuh's.  With the tile in shared memory instead (64 x 64,
 // a TMA copy per field) each update took five shared-memory loads and a store,
 // which bound the kernels: level 0 of 4096^2, down 62 us and up into the
-// pressure 80 us, against 36 us and 75 us here (22 us and 62 us of HBM time).
+// pressure 80 us, against 36 us and 70 us here (22 us and 62 us of HBM time).
 // The per-cell arithmetic is fs_stencil.cuh, shared with the one-pass-per-
 // operation kernels, so the fused cycle reproduces them bit for bit.
 #include <string>
@@ -46,7 +46,7 @@ __global__ void __launch_bounds__(R::THREADS, R::CTAS)
   else mg_down_reg<R>(rhs, xin, xout, crhs, n, h2, pre, w);
 }
 
-template <class R, bool ACC>
+template <class R, bool ACC, int AHEAD>
 __global__ void __launch_bounds__(R::THREADS, R::CTAS)
     k_mg_up(const float* __restrict__ rhs, const float* __restrict__ xin, float* __restrict__ xout,
                 const float* __restrict__ xc, int n, float h2, int post, float w, float* __restrict__ ph,
@@ -55,7 +55,7 @@ __global__ void __launch_bounds__(R::THREADS, R::CTAS)
   // sweeps, so the iterate is zero
   const bool first = first_post >= 0 && (!first_cycle || *first_cycle == 0);
   if (first) post = first_post;
-  mg_up_reg<R, ACC>(rhs, xin, xout, xc, n, h2, post, w, ph, pl, ACC && first && post == 0 && first_x_zero);
+  mg_up_reg<R, ACC, AHEAD>(rhs, xin, xout, xc, n, h2, post, w, ph, pl, ACC && first && post == 0 && first_x_zero);
 }
 
 // ------------------------------------------------- batched (one size class)
@@ -107,7 +107,7 @@ __global__ void __launch_bounds__(R::THREADS, R::CTAS)
     pdl_wait();
     return;
   }
-  mg_up_reg<R, ACC>(a.rhs, a.xin, a.xout, a.xc, n, h2, post, w, a.ph, a.pl, false);
+  mg_up_reg<R, ACC, 0>(a.rhs, a.xin, a.xout, a.xc, n, h2, post, w, a.ph, a.pl, false);
 }
 
 // ------------------------------------------------------------------ host
@@ -160,6 +160,12 @@ static std::string level_name(const Solver* s, const Level& L, const char* base)
   return std::string(base) + "_l" + std::to_string(&L - s->lev.data());
 }
 
+// CTAs between the one whose region an up kernel's CTA fetches into L2 and itself:
+// two an SM ahead, on levels whose fields L2 does not hold (4096^2: 71 us with it, 75
+// without, the pressure fetched as well 77; the down kernel is not bound by its
+// loads; at 2048^2 it only costs, 563 against 560 us a step)
+constexpr int kAheadFrom = 2896;
+
 template <class R>
 static dim3 region_grid(int n, int members = 1) {
   return dim3((n + R::TW - 1) / R::TW, (n + R::TH - 1) / R::TH, members);
@@ -200,14 +206,14 @@ static void up_t(Solver* s, Level& L, const Level& C, float* acc_h, float* acc_l
   if (acc_h) {
     typedef typename RegionOf<T, H, true>::R R;
     FS_LAUNCH(s, first >= 0 && !cyc ? "mg_up_acc_first" : "mg_up_acc", bytes,
-              launch_dependent(true, k_mg_up<R, true>, region_grid<R>(L.n), dim3(R::THREADS), 0, s->stream, 
+              launch_dependent(true, (L.n >= kAheadFrom && T == 64 ? k_mg_up<R, true, T == 64 ? 304 : 0> : k_mg_up<R, true, 0>), region_grid<R>(L.n), dim3(R::THREADS), 0, s->stream, 
                   L.rhs, L.x, nullptr, C.x, L.n, L.h2, s->prm.mg_post_smooth, (float)s->prm.relax, acc_h, acc_l, cyc,
                   fp, x_zero ? 1 : 0));
     return;
   }
   typedef typename RegionOf<T, H>::R R;
   FS_LAUNCH(s, level_name(s, L, "mg_up").c_str(), bytes,
-            launch_dependent(true, k_mg_up<R, false>, region_grid<R>(L.n), dim3(R::THREADS), 0, s->stream, 
+            launch_dependent(true, (L.n >= kAheadFrom && T == 64 ? k_mg_up<R, false, T == 64 ? 304 : 0> : k_mg_up<R, false, 0>), region_grid<R>(L.n), dim3(R::THREADS), 0, s->stream, 
                 L.rhs, L.x, L.x2, C.x, L.n, L.h2, s->prm.mg_post_smooth, (float)s->prm.relax, nullptr, nullptr, cyc,
                 fp, x_zero ? 1 : 0));
   std::swap(L.x, L.x2);

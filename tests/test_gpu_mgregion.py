@@ -67,3 +67,11 @@ def test_batch_equals_single_solver(fs, n, count):
             one.step(1e-3)
         for x, y in zip(batch.members[k].read_velocity(), one.read_velocity()):
             assert np.array_equal(x, y)
+
+
+@pytest.mark.parametrize("precision", ["f32", "mixed"])
+def test_level_that_fetches_ahead(fs, precision):
+    """Levels of 2896 cells on fetch a later region into L2."""
+    kw = dict(pressure_iterations=1, precision=precision)
+    for x, y in zip(run(fs, 3072, 0, **kw), run(fs, 3072, 1, **kw)):
+        assert np.array_equal(x, y)
