@@ -680,8 +680,7 @@ static int tiles_per_cta(const Grid& g) { return (int64_t)g.nx * g.ny >= 4000000
 
 
 
-// Tensor maps of f32 planes for the TMA-staged tiles (the advection tiles'
-// kSW x kSH box here, the multigrid tile boxes in fs_multigrid.cu), kept per
+// Tensor maps of f32 planes for the TMA-staged tiles' kSW x kSH boxes, kept per
 // device pointer, plane and box.  TMA needs the row pitch and the box width
 // multiples of 16 bytes (nx % 4 == 0) and a 16-byte-aligned base; otherwise,
 // or if the CUDA driver lacks the encoder, every tile uses wrapped loads.

@@ -105,7 +105,7 @@ struct Solver {
 
   std::vector<Level> lev;
   int tile_level[16] = {};  // tile side of each tile level's kernels; 0 = the built-in rule
-  // TMA tensor maps of the staged fields (advection, multigrid tiles), by
+  // TMA tensor maps of the staged fields (advection tiles), by
   // device pointer, plane and box (box_tmap, fs_advect.cu)
   struct Tmap {
     const void* p;
