@@ -5,7 +5,7 @@
 // costs, ~4.5 us in a stream and ~2.5 us of it on the GPU, where the sweep
 // itself needs well under 1 us: 40 Jacobi sweeps took 170 us at 256^2 and 250
 // us at 1280 x 720, 40 red-black sweeps 340 us at 333 x 500.  k_flat runs up
-// to 12 sweeps or half-sweeps per launch on a region in registers; the cells
+// to 12 sweeps or half-sweeps per launch (20 on small grids) on a region in registers; the cells
 // a region shares with its neighbours are computed by each of them (2.6x the
 // useful cells for the 64 x 64 region at 12, 1.9x for the 128 x 64 one),
 // which the idle issue slots pay for.  The same solves, captured: 18.5 us,
@@ -51,9 +51,21 @@ static void flat_t(Solver* s, float** x, float** y, const float* d, int n, float
 // 512^2, 53.1 / 90.1 against 38.9 / 55.3 at 1000^2.
 constexpr int64_t kFlatLarge = 200000;
 
+// Does a solve of n sweeps have at most one CTA an SM if up to H go into a launch
+// of the small region?  Fewer, deeper launches pay while they fit the chip: steps
+// with 40 Jacobi / red-black sweeps at H = 12, 16, 20: 256^2 29.6 / 39.9, 27.7 /
+// 36.0, 26.1 / 34.5 us (121 CTAs); 384^2 31.7 / 42.0, 29.7 / 38.1, 35.5 / 48.3 (256
+// CTAs at 20); 440^2 33.9 / 44.2, 39.9 / 52.3, 46.6 / 65.9 (182 at 16).
+static bool flat_fits(const Solver* s, int n, int H) {
+  const int launches = (n + H - 1) / H, k = (n + launches - 1) / launches, tw = 64 - 2 * H, th = 64 - 2 * k;
+  return (int64_t)((s->g.nx + tw - 1) / tw) * ((s->g.ny + th - 1) / th) <= 152;
+}
+
 template <int MODE>
 static void flat_mode(Solver* s, float** x, float** y, const float* d, int n, float h2, bool zero) {
   if (s->n >= kFlatLarge) flat_t<4, 8, 8, 12, MODE>(s, x, y, d, n, h2, zero);
+  else if (flat_fits(s, n, 20)) flat_t<2, 4, 16, 20, MODE>(s, x, y, d, n, h2, zero);
+  else if (flat_fits(s, n, 16)) flat_t<2, 4, 16, 16, MODE>(s, x, y, d, n, h2, zero);
   else flat_t<2, 4, 16, 12, MODE>(s, x, y, d, n, h2, zero);
 }
 

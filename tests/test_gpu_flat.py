@@ -54,3 +54,21 @@ def test_non_finite_right_hand_side_spreads_alike(fs, solver):
         out.append(s.read_field("pressure"))
         s.destroy()
     assert np.array_equal(out[0], out[1], equal_nan=True)
+
+
+@pytest.mark.parametrize("solver", ["jacobi", "red-black"])
+@pytest.mark.parametrize("nx,ny", [(24, 24), (23, 48), (256, 256), (264, 265), (384, 384), (416, 352)])
+def test_launch_depths_equal_one_pass_per_sweep(fs, nx, ny, solver):
+    """20, 16 and 12 sweeps a launch, by the CTAs that they make of the grid."""
+    out = []
+    for variant in (0, 1):
+        rng = np.random.default_rng(nx * 1000 + ny)
+        u, v = rng.standard_normal((2, ny, nx))
+        s = fs.GPUFluidSolver(nx=nx, ny=ny, lx=float(nx), ly=float(ny), pressure_solver=solver, pressure_iterations=40,
+                              kernel_variant=variant)
+        s.upload_velocity(u, v)
+        s.run_stage("divergence", 0.01)
+        s.run_stage("pressure", 0.01)
+        out.append(s.read_field("pressure"))
+        s.destroy()
+    assert np.array_equal(out[0], out[1])
