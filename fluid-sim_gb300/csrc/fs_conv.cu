@@ -96,7 +96,9 @@ struct Cfg {
   static constexpr int W_BYTES = align128(9 * WTAP);
   static constexpr int NACC = TY * NS;                       // columns of one accumulator set
   static constexpr int NCOL = 2 * NACC <= 32 ? 32 : 2 * NACC <= 64 ? 64 : 2 * NACC <= 128 ? 128 : 2 * NACC <= 256 ? 256 : 512;
-  static constexpr int SMEM = RING + W_BYTES + 256;          // + barriers and the TMEM slot
+  // + 128 bytes of barriers and the TMEM slot, and this CTA's biases (which the caller
+  // aligns to a word only: the epilogue reads them four at a time from here)
+  static constexpr int SMEM = RING + W_BYTES + 128 + align128(NS * 4);
   // CTAs of one SM: shared memory, TMEM columns and what is worth having
   static constexpr int BY_SMEM = 226 * 1024 / (SMEM + 1024), BY_TMEM = 512 / NCOL;
   static constexpr int FIT = BY_SMEM < BY_TMEM ? BY_SMEM : BY_TMEM, PER_SM = FIT < 2 ? FIT : 2;
@@ -105,6 +107,7 @@ struct Cfg {
   static constexpr int EROWS = BY_CHUNK ? TY : TY / 2;
   static_assert(CIN % 16 == 0 && NS % 16 == 0 && NS <= 256 && COUT % NS == 0, "channel counts");
   static_assert(2 * NACC <= 512 && PER_SM >= 1 && SMEM <= 227 * 1024, "TMEM columns, shared memory");
+  static_assert(8 * (2 * (D + 1) + 4) + 12 <= 128, "barriers, TMEM slot and flag");
 };
 
 // CTAs per SM: one where the epilogue holds 64 registers of loads in flight
@@ -300,6 +303,7 @@ __global__ void __launch_bounds__(kThreads, (Per<F, Cfg<CIN, COUT, TY, NS, D>>::
   uint64_t* taken = ready + 2;                                      // the set is read back
   uint32_t* tslot = reinterpret_cast<uint32_t*>(taken + 2);
   volatile int* failed = reinterpret_cast<volatile int*>(tslot + 2);
+  float* sbias = reinterpret_cast<float*>(wbuf + C::W_BYTES + 128);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int n0 = blockIdx.y * NS;  // first output channel
   if (warp == 0) {
@@ -325,11 +329,12 @@ __global__ void __launch_bounds__(kThreads, (Per<F, Cfg<CIN, COUT, TY, NS, D>>::
     const int blk = k / NS, co = k - blk * NS;
     copy16(tc::smem_u32(wbuf) + k * 16, wpk + blk * COUT + n0 + co);
   }
+  if (tid < ((F & kOutPlanar) ? 1 : NS)) sbias[tid] = bias[n0 + tid];
   asm volatile("cp.async.wait_all;" ::: "memory");
   tc::fence_async_smem();
   __syncthreads();
   tc::fence_after_sync();
-  pdl_wait();  // the weights were written long before the launch ahead
+  pdl_wait();  // the weights and biases were written long before the launch ahead
   const uint32_t taddr = *tslot, s0 = tc::smem_u32(smem), w0 = tc::smem_u32(wbuf);
   Walk<TY, C::NR> t(strips);
 
@@ -462,12 +467,12 @@ __global__ void __launch_bounds__(kThreads, (Per<F, Cfg<CIN, COUT, TY, NS, D>>::
             tc::mbar_arrive(&taken[set]);
           }
           if constexpr ((F & kOutPlanar) != 0) {
-            if (in_image) reinterpret_cast<float*>(o.out)[((int64_t)t.b * H + y) * W + x] = v[0] + __ldg(bias);
+            if (in_image) reinterpret_cast<float*>(o.out)[((int64_t)t.b * H + y) * W + x] = v[0] + sbias[0];
           } else {
             Px16 w;
 #pragma unroll
             for (int e = 0; e < 16; e += 4) {
-              const float4 bv = __ldg(reinterpret_cast<const float4*>(bias + n0 + c0 + e));
+              const float4 bv = *reinterpret_cast<const float4*>(sbias + c0 + e);
               v[e] += bv.x, v[e + 1] += bv.y, v[e + 2] += bv.z, v[e + 3] += bv.w;
             }
 #pragma unroll

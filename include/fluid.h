@@ -351,8 +351,10 @@ FS_API int fs_max_divergence_noalloc(const float* d_u, const float* d_v, int32_t
  * [ky*3+kx][ci/8][co][ci%8].  epilogue 0: bf16 out, 1: bf16 out after ReLU,
  * 2: f32 planar [b][y][x] of output channel 0 only (c_out must be 16).
  * Instantiated channel pairs: 16->16, 16->32, 32->16, 32->64, 64->32,
- * 64->128, 128->64.  Buffers 16-byte aligned; device pointers; enqueued on
- * `stream`.  *d_err is set to 1 if a tensor-core completion wait timed out. */
+ * 64->128, 128->64.  Image and weight buffers 16-byte aligned (else invalid
+ * argument), d_bias any f32 pointer (epilogue 2 reads its first value only);
+ * device pointers; enqueued on `stream`.  *d_err is set to 1 if a tensor-core
+ * completion wait timed out. */
 FS_API int fs_conv3x3_bf16(const void* d_in, const void* d_wpacked, const float* d_bias, void* d_out, int32_t batch,
                            int32_t h, int32_t w, int32_t c_in, int32_t c_out, int32_t epilogue, int32_t* d_err,
                            void* stream);
