@@ -32,7 +32,7 @@ __device__ __forceinline__ int wrap_idx(int i, int n) {
 
 template <class T>
 __device__ __forceinline__ float ld(const T* __restrict__ a, int64_t k) {
-  return (float)__ldg(a + k);
+  return (float)a[k];
 }
 
 // Bilinear sample at (bi + ox, bj + oy) in the field's own index space
@@ -149,7 +149,7 @@ struct TileView {
       const int i1 = i0 + 1 == nx ? 0 : i0 + 1;
       const int j1 = j0 + 1 == ny ? 0 : j0 + 1;
       const int64_t r0 = (int64_t)j0 * nx, r1 = (int64_t)j1 * nx;
-      a = __ldg(g + r0 + i0); b = __ldg(g + r0 + i1); c = __ldg(g + r1 + i0); d = __ldg(g + r1 + i1);
+      a = g[r0 + i0]; b = g[r0 + i1]; c = g[r1 + i0]; d = g[r1 + i1];
     }
     if (RANGE) {
       *lo = fminf(fminf(a, b), fminf(c, d));
@@ -208,7 +208,7 @@ __device__ __forceinline__ void stage_tiles(float* const (&sm)[F], const float* 
       const int k = lj * kSW + li;
 #pragma unroll
       for (int q = 0; q < F; q++) {
-        const float x = __ldg(f[q] + row + gi);
+        const float x = f[q][row + gi];
         sm[q][k] = x;
         if (q == 0) mu = max(mu, __float_as_uint(fabsf(x)));
         if (q == 1) mv = max(mv, __float_as_uint(fabsf(x)));
@@ -434,7 +434,7 @@ __device__ __forceinline__ void advect_rows(const TileView& U, const TileView& V
 // Tiles whose staged block lies inside the grid are staged by TMA when the
 // tensor maps are valid (tma != 0); the others by the wrapped loads.
 template <int NT>
-__global__ void __launch_bounds__(256) k_advect_sl_t(const float* __restrict__ u, const float* __restrict__ v,
+__global__ void __launch_bounds__(256) k_advect_sl_t(const float* u, const float* v,
                                                      float* __restrict__ ou, float* __restrict__ ov, int nx, int ny,
                                                      float cx, float cy, float* __restrict__ bounds,
                                                      const __grid_constant__ CUtensorMap tm_u,
@@ -493,8 +493,8 @@ __device__ __forceinline__ void combine_rows(const TileView& U, const TileView& 
     if (j >= ny) break;
     const int64_t c = (int64_t)j * nx + i;
     const int lc = (r + kHalo) * kSW + threadIdx.x + kHalo;  // this cell in the staged block
-    const float lou = __ldg(bounds + c), hiu = __ldg(bounds + n + c);
-    const float lov = __ldg(bounds + 2 * n + c), hiv = __ldg(bounds + 3 * n + c);
+    const float lou = bounds[c], hiu = bounds[n + c];
+    const float lov = bounds[2 * n + c], hiv = bounds[3 * n + c];
     float dX, dY;
     // u component
     trace_t(U, V, i, j, hu, -cx, -cy, dX, dY);  // backward: trace with -dt
@@ -524,8 +524,8 @@ __device__ __forceinline__ void combine_pair(const float* su, const float* sv, c
 #pragma unroll
   for (int k = 0; k < 2; k++) {
     const float* b = bounds + 2 * k * n;
-    const float lo0 = __ldg(b + c), hi0 = __ldg(b + n + c);
-    const float lo1 = two ? __ldg(b + c1) : 0.f, hi1 = two ? __ldg(b + n + c1) : 0.f;
+    const float lo0 = b[c], hi0 = b[n + c];
+    const float lo1 = two ? b[c1] : 0.f, hi1 = two ? b[n + c1] : 0.f;
     const PairView& own = k == 0 ? U : V;
     const PairView F{(k == 0 ? sfu : sfv) + lc};
     F2 dx, dy;
@@ -541,10 +541,10 @@ __device__ __forceinline__ void combine_pair(const float* su, const float* sv, c
 }
 
 template <int NT>
-__global__ void __launch_bounds__(256) k_mc_combine_t(const float* __restrict__ u, const float* __restrict__ v,
-                                                      const float* __restrict__ fu, const float* __restrict__ fv,
-                                                      const float* __restrict__ bounds, float* __restrict__ ou,
-                                                      float* __restrict__ ov, int nx, int ny, float cx, float cy,
+__global__ void __launch_bounds__(256) k_mc_combine_t(const float* u, const float* v, const float* fu,
+                                                      const float* fv, const float* bounds,
+                                                      float* __restrict__ ou, float* __restrict__ ov, int nx, int ny,
+                                                      float cx, float cy,
                                                       const __grid_constant__ CUtensorMap tm_u,
                                                       const __grid_constant__ CUtensorMap tm_v,
                                                       const __grid_constant__ CUtensorMap tm_fu,
@@ -763,20 +763,18 @@ __device__ __forceinline__ void diffuse_body(const float* __restrict__ u, const 
   int im = i == 0 ? nx - 1 : i - 1, ip = i + 1 == nx ? 0 : i + 1;
   int jm = j == 0 ? ny - 1 : j - 1, jp = j + 1 == ny ? 0 : j + 1;
   int64_t r = (int64_t)j * nx, rm = (int64_t)jm * nx, rp = (int64_t)jp * nx;
-  ou[r + i] = diffuse_cell(__ldg(u + r + i), __ldg(u + r + im), __ldg(u + r + ip), __ldg(u + rm + i),
-                           __ldg(u + rp + i), a, b);
-  ov[r + i] = diffuse_cell(__ldg(v + r + i), __ldg(v + r + im), __ldg(v + r + ip), __ldg(v + rm + i),
-                           __ldg(v + rp + i), a, b);
+  ou[r + i] = diffuse_cell(u[r + i], u[r + im], u[r + ip], u[rm + i], u[rp + i], a, b);
+  ov[r + i] = diffuse_cell(v[r + i], v[r + im], v[r + ip], v[rm + i], v[rp + i], a, b);
 }
 
 // Four consecutive cells per thread (nx a multiple of 4): float4 loads of the
 // three rows, the group's outer left and right neighbours as scalars.
 __device__ __forceinline__ void diffuse4_one(const float* __restrict__ f, float* __restrict__ o, int64_t r,
                                              int64_t rm, int64_t rp, int i0, int il, int ir, float a, float b) {
-  const float4 c = __ldg(reinterpret_cast<const float4*>(f + r + i0));
-  const float4 bo = __ldg(reinterpret_cast<const float4*>(f + rm + i0));
-  const float4 t = __ldg(reinterpret_cast<const float4*>(f + rp + i0));
-  const float l = __ldg(f + r + il), rr = __ldg(f + r + ir);
+  const float4 c = *reinterpret_cast<const float4*>(f + r + i0);
+  const float4 bo = *reinterpret_cast<const float4*>(f + rm + i0);
+  const float4 t = *reinterpret_cast<const float4*>(f + rp + i0);
+  const float l = f[r + il], rr = f[r + ir];
   float4 out;
   out.x = diffuse_cell(c.x, l, c.y, bo.x, t.x, a, b);
   out.y = diffuse_cell(c.y, c.x, c.z, bo.y, t.y, a, b);
@@ -797,16 +795,14 @@ __device__ __forceinline__ void diffuse4_body(const float* __restrict__ u, const
   diffuse4_one(v, ov, r, rm, rp, i0, il, ir, a, b);
 }
 
-__global__ void __launch_bounds__(256) k_diffuse4(const float* __restrict__ u, const float* __restrict__ v,
-                                                  float* __restrict__ ou, float* __restrict__ ov,
-                                                  int nx, int ny, float a, float b) {
+__global__ void __launch_bounds__(256) k_diffuse4(const float* u, const float* v, float* __restrict__ ou,
+                                                  float* __restrict__ ov, int nx, int ny, float a, float b) {
   pdl_wait();
   diffuse4_body(u, v, ou, ov, nx, ny, a, b);
 }
 
-__global__ void __launch_bounds__(256) k_diffuse(const float* __restrict__ u, const float* __restrict__ v,
-                                                 float* __restrict__ ou, float* __restrict__ ov,
-                                                 int nx, int ny, float a, float b) {
+__global__ void __launch_bounds__(256) k_diffuse(const float* u, const float* v, float* __restrict__ ou,
+                                                 float* __restrict__ ov, int nx, int ny, float a, float b) {
   pdl_wait();
   diffuse_body(u, v, ou, ov, nx, ny, a, b);
 }
@@ -877,10 +873,9 @@ void launch_front_advect_class(Solver* const* ms, int count, const double* dts, 
 // cosine, a square root and two divisions a mode and cell were all this kernel's
 // time.  512^2, 16 modes: 16 -> 6 us.
 constexpr int kForceTY = 32, kForceM = 8;
-__global__ void __launch_bounds__(256) k_forcing(float* __restrict__ u, float* __restrict__ v,
-                                                 const float* __restrict__ modes, int m, int nx,
-                                                 int ny, float dx, float dy, float scale, float damp,
-                                                 double drift_rate, const DevState* __restrict__ st) {
+__global__ void __launch_bounds__(256) k_forcing(float* u, float* v, const float* __restrict__ modes,
+                                                 int m, int nx, int ny, float dx, float dy, float scale,
+                                                 float damp, double drift_rate, const DevState* __restrict__ st) {
   // [mode][cell], u's and v's; the columns' x: weight cos, weight sin
   __shared__ float2 ex[2][kForceM][32], ey[2][kForceM][kForceTY];
   __shared__ float s_drift;
@@ -1138,9 +1133,8 @@ void launch_solids(Solver* s, float* u, float* v, float dt, bool record_impulse)
 // (i+1/2, j) and v-grid index (i, j+1/2).
 __device__ __forceinline__ Home home_c() { return {0.5f, 0.f, 0.f, 0.5f}; }
 
-__global__ void __launch_bounds__(256) k_advect_dye(const float* __restrict__ u, const float* __restrict__ v,
-                                                    const float4* __restrict__ q, float4* __restrict__ out, int nx,
-                                                    int ny, float cx, float cy, float keep) {
+__global__ void __launch_bounds__(256) k_advect_dye(const float* u, const float* v, const float4* q,
+                                                    float4* __restrict__ out, int nx, int ny, float cx, float cy, float keep) {
   pdl_wait();
   int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
   if (i >= nx || j >= ny) return;

@@ -128,7 +128,7 @@ __device__ void band_mode(int kind, int m, uint32_t step, uint64_t seed, double 
 __global__ void __launch_bounds__(256)
     k_band_columns(int kind, int M, int K, const DevState* __restrict__ st, uint64_t seed, double kf, double width,
                    double s, const int2* __restrict__ lattice, const float2* __restrict__ ex_u,
-                   const float2* __restrict__ ex_v, float2* __restrict__ gu, float2* __restrict__ gv, int nx) {
+                   const float2* __restrict__ ex_v, float2* gu, float2* gv, int nx) {
   __shared__ ModeCoef modes[kMaxBandModes];
   __shared__ int first, last;
   const int q = blockIdx.y - K;
@@ -175,7 +175,7 @@ struct BandStage {
 };
 __global__ void __launch_bounds__(256)
     k_band_apply(float* __restrict__ u, float* __restrict__ v, int nx, int ny, int K,
-                 const float2* __restrict__ gu, const float2* __restrict__ gv, const float2* __restrict__ ey_u,
+                 const float2* gu, const float2* gv, const float2* __restrict__ ey_u,
                  const float2* __restrict__ ey_v, float damp, DevState* __restrict__ st) {
   extern __shared__ __align__(16) unsigned char band_smem[];
   BandStage& t = *reinterpret_cast<BandStage*>(band_smem);
@@ -200,8 +200,8 @@ __global__ void __launch_bounds__(256)
 #pragma unroll 4
     for (int q = tid / kBandTX; q < nb; q += 256 / kBandTX) {
       const int c = tid % kBandTX, i = min(i0 + c, nx - 1);
-      t.gu[q][c] = __ldg(gu + (size_t)(q0 + q) * nx + i);
-      t.gv[q][c] = __ldg(gv + (size_t)(q0 + q) * nx + i);
+      t.gu[q][c] = gu[(size_t)(q0 + q) * nx + i];
+      t.gv[q][c] = gv[(size_t)(q0 + q) * nx + i];
     }
 #pragma unroll 4
     for (int q = tid / kBandTY; q < nb; q += 256 / kBandTY) {

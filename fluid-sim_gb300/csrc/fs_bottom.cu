@@ -179,9 +179,9 @@ __device__ __forceinline__ void mg_bottom_body(const float* __restrict__ rhs_top
   }
 }
 
-__global__ void __launch_bounds__(1024) k_mg_bottom(const float* __restrict__ rhs_top, float* __restrict__ x_top,
-                                                    int has_x, BottomLevels L, int pre, int post, int coarse,
-                                                    float* __restrict__ acc_h, float* __restrict__ acc_l) {
+__global__ void __launch_bounds__(1024) k_mg_bottom(const float* rhs_top, float* x_top, int has_x,
+                                                    BottomLevels L, int pre, int post, int coarse, float* acc_h,
+                                                    float* acc_l) {
   pdl_wait();
   mg_bottom_body(rhs_top, x_top, has_x, L, pre, post, coarse, acc_h, acc_l);
 }
@@ -701,8 +701,8 @@ __device__ __forceinline__ void mg_bottom_chain_body(const float* __restrict__ r
 
 template <int N0, int NMIN>
 __global__ void __launch_bounds__(kBottomThreads)
-    k_mg_bottom_chain(const float* __restrict__ rhs_top, float* __restrict__ x_top, int has_x, BottomH2 H, int pre,
-                      int post, int coarse, float* __restrict__ acc_h, float* __restrict__ acc_l) {
+    k_mg_bottom_chain(const float* rhs_top, float* x_top, int has_x, BottomH2 H, int pre, int post, int coarse,
+                      float* acc_h, float* acc_l) {
   pdl_wait();
   mg_bottom_chain_body<N0, NMIN>(rhs_top, x_top, has_x, H, pre, post, coarse, acc_h, acc_l);
 }

@@ -65,8 +65,7 @@ struct Bands {
 };
 
 __global__ void __launch_bounds__(256)
-    k_channel(float* __restrict__ u, float* __restrict__ v, int nx, int ny, float dx, float dy, ChannelDev c,
-              float w, Bands b) {
+    k_channel(float* u, float* v, int nx, int ny, float dx, float dy, ChannelDev c, float w, Bands b) {
   pdl_wait();
   int i, j;
   const int blk = blockIdx.x;

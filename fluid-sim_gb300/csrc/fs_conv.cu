@@ -135,7 +135,7 @@ struct Px16 {
 };
 __device__ __forceinline__ Px16 load16(const void* base, int64_t px, int channels, int c0) {
   const uint4* p = reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(base) + px * channels + c0);
-  const uint4 a = __ldg(p), b = __ldg(p + 1);
+  const uint4 a = p[0], b = p[1];
   return Px16{{a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w}};
 }
 __device__ __forceinline__ void store16(void* base, int64_t px, int channels, int c0, const Px16& v) {
@@ -215,7 +215,7 @@ __device__ __forceinline__ void pool16(const ConvOut& o, const Px16& r0, const P
   if (!store) return;
   const int64_t at = ((b * (H >> 1) + (y >> 1)) * (int64_t)(W >> 1) + (x >> 1)) * channels + c0 + 8 * odd;
   if (F & kOutPoolMask) {
-    const uint4 a = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(o.pool_mask) + at));
+    const uint4 a = *reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(o.pool_mask) + at);
     out[0] = relu_mask(out[0], a.x);
     out[1] = relu_mask(out[1], a.y);
     out[2] = relu_mask(out[2], a.z);
@@ -290,7 +290,7 @@ struct Walk {
 
 template <int CIN, int COUT, int TY, int NS, int D, int F>
 __global__ void __launch_bounds__(kThreads, (Per<F, Cfg<CIN, COUT, TY, NS, D>>::SM))
-    k_conv3x3(const uint4* __restrict__ in, const uint4* __restrict__ wpk,
+    k_conv3x3(const uint4* in, const uint4* __restrict__ wpk,
                                                          const float* __restrict__ bias, const ConvOut o,
                                                          const Strips strips, int H, int W, int* __restrict__ err) {
   using C = Cfg<CIN, COUT, TY, NS, D>;

@@ -12,12 +12,40 @@
 // 43 us and 37 us; with the first launch of a solve a dependent one too, steps of
 // these sizes take 32.6 -> 29.8, 84.5 -> 81.6 and 46.6 -> 45.6 us.
 #include <algorithm>
+#include <atomic>
 #include <utility>
 
 #include "fs_flat.cuh"
 #include "fs_internal.cuh"
 
 namespace fs {
+
+constexpr int kFlatSMs = 152;
+
+// Dynamic shared memory that leaves room for one CTA an SM only.  A launch of the
+// small region with at most one CTA an SM asks for it: its CTAs are placed while the
+// kernel ahead still holds some SMs, and where registers leave room for three an SM
+// two of them can share one and take twice the time.  Whether they do depends on
+// what else runs: eight steps at 256^2 with the velocity copied in and out 312 us,
+// 247 us with the limit (64 KB, two an SM: 318); steps alone at 256^2, red-black, 35.8
+// -> 34.1 us; from 16^2 to 446^2 no size is slower.  Launches with more CTAs than SMs
+// need the room: 8000 x 24 with 40 sweeps 43.7 -> 48.4 us a step.
+constexpr int kFlatAlone = 100 * 1024;
+
+template <int CPL, int RPW, int NW, int H, int MODE>
+static int flat_alone_bytes(int device) {
+  static std::atomic<uint64_t> set{0};  // the limit is an attribute of the function on each device
+  const uint64_t bit = 1ull << (device & 63);
+  if (!(set.load() & bit)) {
+    if (cudaFuncSetAttribute(k_flat<CPL, RPW, NW, H, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, kFlatAlone) !=
+        cudaSuccess) {
+      cudaGetLastError();
+      return 0;
+    }
+    set.fetch_or(bit);
+  }
+  return kFlatAlone;
+}
 
 template <int CPL, int RPW, int NW, int H, int MODE>
 static void flat_t(Solver* s, float** x, float** y, const float* d, int n, float h2, bool zero) {
@@ -30,6 +58,8 @@ static void flat_t(Solver* s, float** x, float** y, const float* d, int n, float
     cfg.gridDim = dim3((g.nx + F::TW - 1) / F::TW, (g.ny + F::RH - 2 * now - 1) / (F::RH - 2 * now));
     cfg.blockDim = dim3(NW * 32);
     cfg.stream = s->stream;
+    if (RPW == 4 && (int64_t)cfg.gridDim.x * cfg.gridDim.y <= kFlatSMs)
+      cfg.dynamicSmemBytes = flat_alone_bytes<CPL, RPW, NW, H, MODE>(s->device);
     cudaLaunchAttribute pdl = {};
     pdl.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     pdl.val.programmaticStreamSerializationAllowed = 1;
@@ -58,7 +88,7 @@ constexpr int64_t kFlatLarge = 200000;
 // CTAs at 20); 440^2 33.9 / 44.2, 39.9 / 52.3, 46.6 / 65.9 (182 at 16).
 static bool flat_fits(const Solver* s, int n, int H) {
   const int launches = (n + H - 1) / H, k = (n + launches - 1) / launches, tw = 64 - 2 * H, th = 64 - 2 * k;
-  return (int64_t)((s->g.nx + tw - 1) / tw) * ((s->g.ny + th - 1) / th) <= 152;
+  return (int64_t)((s->g.nx + tw - 1) / tw) * ((s->g.ny + th - 1) / th) <= kFlatSMs;
 }
 
 template <int MODE>

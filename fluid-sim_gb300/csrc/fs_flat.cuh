@@ -115,7 +115,7 @@ __device__ __forceinline__ void flat_all_rows(float (&p)[RPW][CPL], const float 
 // the solve writes, except that the one ahead of the first may) and then waits
 // for that launch to complete before it lets the next one start.
 template <int CPL, int RPW, int NW, int H, int MODE>
-__global__ void __launch_bounds__(NW * 32) k_flat(const float* p, const float* __restrict__ d, float* o, int nx, int ny,
+__global__ void __launch_bounds__(NW * 32) k_flat(const float* p, const float* d, float* o, int nx, int ny,
                                                   float h2, float w, int k, int c0, int zero, int first) {
   using F = FlatTile<CPL, RPW, NW, H>;
   typedef typename FlatVec<CPL>::T V;
@@ -136,10 +136,10 @@ __global__ void __launch_bounds__(NW * 32) k_flat(const float* p, const float* _
     const int gy = flat_wrap(yl + r, ny);
     const float* row = d + (int64_t)gy * nx;
     if (vec) {
-      *reinterpret_cast<V*>(dv[r]) = __ldg(reinterpret_cast<const V*>(row + gx[0]));
+      *reinterpret_cast<V*>(dv[r]) = *reinterpret_cast<const V*>(row + gx[0]);
     } else {
 #pragma unroll
-      for (int c = 0; c < CPL; c++) dv[r][c] = __ldg(row + gx[c]);
+      for (int c = 0; c < CPL; c++) dv[r][c] = row[gx[c]];
     }
 #pragma unroll
     for (int c = 0; c < CPL; c++) {

@@ -243,8 +243,8 @@ __global__ void __launch_bounds__(32 * kLossWarps)
 // bits) on the FP32 pipe, in f64 where a value is too large for it or not finite
 // (the loss: 3 f64 instructions a cell, 11 with the gradient in f64, 148 us).
 __global__ void __launch_bounds__(32 * kLossWarps)
-    k_loss_seed(const float* __restrict__ out, const float* __restrict__ tgt, const float* __restrict__ res,
-                double* __restrict__ acc, uint4* __restrict__ gJ, int H, int W, int B, int rows, double w_p,
+    k_loss_seed(const float* __restrict__ out, const float* __restrict__ tgt, const float* res,
+                double* acc, uint4* __restrict__ gJ, int H, int W, int B, int rows, double w_p,
                 double w_r) {
   pdl_wait();
   const int b = blockIdx.y;

@@ -219,6 +219,14 @@ void prof_end(Solver* s, int slot, cudaEvent_t a);
 // one start then, so that the launch before the one ahead is complete when a
 // kernel starts, and at most one waits beside the one that runs (the other
 // order piled waiting kernels up and made the V-cycles slower by up to 10%).
+// A dependent kernel is alive while the one ahead still writes, so what that one
+// may write is read by plain loads through pointers that are not __restrict__:
+// ld.global.nc (which __ldg is, and a load through const __restrict__ becomes) is for
+// data nothing writes during the kernel, and the compiler need not keep a load
+// through a pointer nothing else may reach behind the wait.  Tables, and fields that
+// were complete before the launch ahead began, may stay as they are
+// (tests/test_dependent_loads.py lists them).  The passes take what they took: four
+// 1024^2 forced steps 1954 -> 1951 us, 2048^2 channel 4184 -> 4144.
 // Steps without and with: 512^2 multigrid 116.8 -> 110.7 us, 192^2 mixed 145.6 -> 131.4,
 // 576^2 147.5 -> 129.2, 1024^2 forced 309.9 -> 297.8, 4096^2 2374 -> 2307.
 template <class... P, class... A>

@@ -48,10 +48,10 @@ struct MgCells {
     yl = blockIdx.y * R::TH - R::HY + warp * R::RPW;
     gx = flat_wrap(xl, n);  // n is a multiple of CPL: a lane's columns do not straddle the wrap
   }
-  __device__ __forceinline__ void load(float (&a)[R::RPW][R::CPL], const float* __restrict__ f, int n) const {
+  __device__ __forceinline__ void load(float (&a)[R::RPW][R::CPL], const float* f, int n) const {
 #pragma unroll
     for (int r = 0; r < R::RPW; r++)
-      *reinterpret_cast<V*>(a[r]) = __ldg(reinterpret_cast<const V*>(f + (int64_t)flat_wrap(yl + r, n) * n + gx));
+      *reinterpret_cast<V*>(a[r]) = *reinterpret_cast<const V*>(f + (int64_t)flat_wrap(yl + r, n) * n + gx);
   }
   // the rows above and below the thread's, from the neighbouring warps
   typedef float Edge[R::NW][2][R::RW];
@@ -163,8 +163,8 @@ __device__ __forceinline__ void mg_restrict_rhs(const float* __restrict__ rhs, f
     const int gci = blockIdx.x * (R::TW / 2) + ci, gcj = blockIdx.y * (R::TH / 2) + cj;
     if (gci >= nc || gcj >= nc) continue;
     const float* q = rhs + (int64_t)(2 * gcj) * n + 2 * gci;
-    const float2 q0 = __ldg(reinterpret_cast<const float2*>(q));
-    const float2 q1 = __ldg(reinterpret_cast<const float2*>(q + n));
+    const float2 q0 = *reinterpret_cast<const float2*>(q);
+    const float2 q1 = *reinterpret_cast<const float2*>(q + n);
     crhs[(int64_t)gcj * nc + gci] = restrict4(q0.x, q0.y, q1.x, q1.y);
   }
 }
@@ -177,7 +177,7 @@ __device__ __forceinline__ void mg_restrict_rhs(const float* __restrict__ rhs, f
 // AHEAD > 0: the CTA fetches a later one's iterate and rhs into L2.
 template <class R, bool ACC, int AHEAD>
 __device__ __forceinline__ void mg_up_reg(const float* __restrict__ rhs, const float* __restrict__ xin,
-                                          float* __restrict__ xout, const float* __restrict__ xc, int n, float h2,
+                                          float* __restrict__ xout, const float* xc, int n, float h2,
                                           int post, float w, float* __restrict__ ph, float* __restrict__ pl,
                                           bool zero) {
   constexpr int CPL = R::CPL, RPW = R::RPW, CC = CPL / 2, CR = RPW / 2 + 2;
@@ -215,12 +215,12 @@ __device__ __forceinline__ void mg_up_reg(const float* __restrict__ rhs, const f
   for (int k = 0; k < CR; k++) {
     const float* row = xc + (int64_t)flat_wrap(jc + k, nc) * nc;
     if (CC == 2) {
-      const float2 q = __ldg(reinterpret_cast<const float2*>(row + gc));
+      const float2 q = *reinterpret_cast<const float2*>(row + gc);
       cv[k][0] = q.x, cv[k][CC - 1] = q.y;
     } else {
-      cv[k][0] = __ldg(row + gc);
+      cv[k][0] = row[gc];
     }
-    side[k] = t.lane == 0 || t.lane == 31 ? __ldg(row + gs) : 0.f;
+    side[k] = t.lane == 0 || t.lane == 31 ? row[gs] : 0.f;
   }
   float m0[CPL], m1[CPL];  // the two coarse rows before, interpolated to the fine columns
 #pragma unroll

@@ -31,7 +31,7 @@ namespace fs {
 
 template <class R>
 __global__ void __launch_bounds__(R::THREADS, R::CTAS)
-    k_mg_down(const float* __restrict__ rhs, const float* __restrict__ xin, float* __restrict__ xout,
+    k_mg_down(const float* rhs, const float* xin, float* __restrict__ xout,
                   float* __restrict__ crhs, int n, float h2, int pre, float w, const int* first_cycle, int first_pre,
                   int first_x_unused) {
   pdl_wait();
@@ -49,7 +49,7 @@ __global__ void __launch_bounds__(R::THREADS, R::CTAS)
 template <class R, bool ACC, int AHEAD>
 __global__ void __launch_bounds__(R::THREADS, R::CTAS)
     k_mg_up(const float* __restrict__ rhs, const float* __restrict__ xin, float* __restrict__ xout,
-                const float* __restrict__ xc, int n, float h2, int post, float w, float* __restrict__ ph,
+                const float* xc, int n, float h2, int post, float w, float* __restrict__ ph,
                 float* __restrict__ pl, const int* first_cycle, int first_post, int first_x_zero) {
   // as k_mg_down; first_x_zero: that cycle's down kernel on this level ran no
   // sweeps, so the iterate is zero

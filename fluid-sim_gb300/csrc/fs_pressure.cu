@@ -28,7 +28,7 @@ __device__ __forceinline__ int wrapm(int i, int n) { return i < 0 ? i + n : (i >
 // ------------------------------------------------------------- divergence
 // (uR - uL)/dx + (vT - vB)/dy at cell centres (grid.js:191-206)
 template <class TV, class TD>
-__global__ void __launch_bounds__(256) k_divergence(const TV* __restrict__ u, const TV* __restrict__ v,
+__global__ void __launch_bounds__(256) k_divergence(const TV* u, const TV* v,
                                                     TD* __restrict__ d, int nx, int ny, TD idx, TD idy) {
   pdl_wait();
   int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
@@ -50,7 +50,7 @@ struct FaceQuad {
 };
 __device__ __forceinline__ float4 diffuse_quad(const float* __restrict__ row, float4 c, float4 b, float4 t, int il,
                                                int ir, float ax, float ay) {
-  const float l = __ldg(row + il), r = __ldg(row + ir);
+  const float l = row[il], r = row[ir];
   return {diffuse_cell(c.x, l, c.y, b.x, t.x, ax, ay), diffuse_cell(c.y, c.x, c.z, b.y, t.y, ax, ay),
           diffuse_cell(c.z, c.y, c.w, b.z, t.z, ax, ay), diffuse_cell(c.w, c.z, r, b.w, t.w, ax, ay)};
 }
@@ -59,20 +59,20 @@ __device__ __forceinline__ FaceQuad diffused_faces(const float* __restrict__ u, 
   const int jm = j == 0 ? ny - 1 : j - 1, jp = j + 1 == ny ? 0 : j + 1, jq = jp + 1 == ny ? 0 : jp + 1;
   const int il = i0 == 0 ? nx - 1 : i0 - 1, ir = i0 + 4 == nx ? 0 : i0 + 4;
   const int64_t r = (int64_t)j * nx, rm = (int64_t)jm * nx, rp = (int64_t)jp * nx, rq = (int64_t)jq * nx;
-  auto quad = [&](const float* f, int64_t row) { return __ldg(reinterpret_cast<const float4*>(f + row + i0)); };
+  auto quad = [&](const float* f, int64_t row) { return *reinterpret_cast<const float4*>(f + row + i0); };
   const float4 um = quad(u, rm), uc = quad(u, r), up = quad(u, rp);
   const float4 vm = quad(v, rm), vc = quad(v, r), vp = quad(v, rp), vq = quad(v, rq);
   FaceQuad f;
   f.u = diffuse_quad(u + r, uc, um, up, il, ir, ax, ay);
   f.v = diffuse_quad(v + r, vc, vm, vp, il, ir, ax, ay);
   f.t = diffuse_quad(v + rp, vp, vc, vq, il, ir, ax, ay);
-  f.ur = diffuse_cell(__ldg(u + r + ir), uc.w, __ldg(u + r + (ir + 1)), __ldg(u + rm + ir), __ldg(u + rp + ir), ax, ay);
+  f.ur = diffuse_cell(u[r + ir], uc.w, u[r + (ir + 1)], u[rm + ir], u[rp + ir], ax, ay);
   return f;
 }
 
 // DIFFUSE and the divergence of its result in one pass (nx a multiple of 4)
 __global__ void __launch_bounds__(256)
-    k_diffuse_div4(const float* __restrict__ u, const float* __restrict__ v, float* __restrict__ ou,
+    k_diffuse_div4(const float* u, const float* v, float* __restrict__ ou,
                    float* __restrict__ ov, float* __restrict__ d, int nx, int ny, float ax, float ay, float idx,
                    float idy) {
   pdl_wait();
@@ -131,7 +131,7 @@ __device__ __forceinline__ void finish_step(const StepFinish& f) {
 // ------------------------------------------------------ gradient subtraction
 // u -= (p_i - p_{i-1})/dx, v -= (p_j - p_{j-1})/dy (grid.js:209-218)
 __global__ void __launch_bounds__(256)
-    k_subgrad_f32(const float* __restrict__ wu, const float* __restrict__ wv, const float* __restrict__ p,
+    k_subgrad_f32(const float* wu, const float* wv, const float* p,
                   float* __restrict__ ou, float* __restrict__ ov, int nx, int ny, float idx, float idy,
                   const StepFinish fin) {
   pdl_wait();
@@ -140,9 +140,9 @@ __global__ void __launch_bounds__(256)
   if (i >= nx || j >= ny) return;
   int im = i == 0 ? nx - 1 : i - 1, jm = j == 0 ? ny - 1 : j - 1;
   int64_t c = (int64_t)j * nx + i;
-  float pc = __ldg(p + c);
-  ou[c] = __ldg(wu + c) - (pc - __ldg(p + (int64_t)j * nx + im)) * idx;
-  ov[c] = __ldg(wv + c) - (pc - __ldg(p + (int64_t)jm * nx + i)) * idy;
+  float pc = p[c];
+  ou[c] = wu[c] - (pc - p[(int64_t)j * nx + im]) * idx;
+  ov[c] = wv[c] - (pc - p[(int64_t)jm * nx + i]) * idy;
 }
 
 void launch_subtract_gradient_f32(Solver* s, const float* wu, const float* wv, const float* p,
@@ -358,10 +358,10 @@ __device__ __forceinline__ void div_df_body(const float* __restrict__ uh, const 
   if (i >= nx || j >= ny) return;
   int ip = i + 1 == nx ? 0 : i + 1, jp = j + 1 == ny ? 0 : j + 1;
   int64_t c = (int64_t)j * nx + i, cr = (int64_t)j * nx + ip, ct = (int64_t)jp * nx + i;
-  df du = two_diff(__ldg(uh + cr), __ldg(uh + c));
-  df dv = two_diff(__ldg(vh + ct), __ldg(vh + c));
-  if (ul) du = df_add(du, two_diff(__ldg(ul + cr), __ldg(ul + c)));
-  if (vl) dv = df_add(dv, two_diff(__ldg(vl + ct), __ldg(vl + c)));
+  df du = two_diff(uh[cr], uh[c]);
+  df dv = two_diff(vh[ct], vh[c]);
+  if (ul) du = df_add(du, two_diff(ul[cr], ul[c]));
+  if (vl) dv = df_add(dv, two_diff(vl[ct], vl[c]));
   df d = df_add(df_mul(du, idx), df_mul(dv, idy));
   dh[c] = d.hi;
   dl[c] = d.lo;
@@ -406,10 +406,10 @@ __device__ __forceinline__ void div_start4_body(const float* __restrict__ wu, co
         *reinterpret_cast<float4*>(o.ou + r + i0) = f.u;
         *reinterpret_cast<float4*>(o.ov + r + i0) = f.v;
       } else {
-        f.u = __ldg(reinterpret_cast<const float4*>(wu + r + i0));
-        f.v = __ldg(reinterpret_cast<const float4*>(wv + r + i0));
-        f.t = __ldg(reinterpret_cast<const float4*>(wv + (int64_t)jp * nx + i0));
-        f.ur = __ldg(wu + r + ir);
+        f.u = *reinterpret_cast<const float4*>(wu + r + i0);
+        f.v = *reinterpret_cast<const float4*>(wv + r + i0);
+        f.t = *reinterpret_cast<const float4*>(wv + (int64_t)jp * nx + i0);
+        f.ur = wu[r + ir];
       }
       const float4 u4 = f.u, v4 = f.v, t4 = f.t;
       const float ur = f.ur;
@@ -430,7 +430,7 @@ __device__ __forceinline__ void div_start4_body(const float* __restrict__ wu, co
 }
 
 __global__ void __launch_bounds__(256)
-    k_div_start4(const float* __restrict__ wu, const float* __restrict__ wv, float* __restrict__ dh,
+    k_div_start4(const float* wu, const float* wv, float* __restrict__ dh,
                  float* __restrict__ dl, float* __restrict__ ph, float* __restrict__ pl, float* __restrict__ r32,
                  int nx, int ny, df idx, df idy, RedCtx ctx) {
   pdl_wait();
@@ -438,7 +438,7 @@ __global__ void __launch_bounds__(256)
 }
 
 __global__ void __launch_bounds__(256)
-    k_diffuse_start4(const float* __restrict__ wu, const float* __restrict__ wv, float* __restrict__ dh,
+    k_diffuse_start4(const float* wu, const float* wv, float* __restrict__ dh,
                      float* __restrict__ dl, float* __restrict__ ph, float* __restrict__ pl, float* __restrict__ r32,
                      int nx, int ny, df idx, df idy, RedCtx ctx, const DiffuseOut o) {
   pdl_wait();
@@ -446,8 +446,8 @@ __global__ void __launch_bounds__(256)
 }
 
 __global__ void __launch_bounds__(256)
-    k_div_df(const float* __restrict__ uh, const float* __restrict__ ul, const float* __restrict__ vh,
-             const float* __restrict__ vl, float* __restrict__ dh, float* __restrict__ dl, int nx, int ny, df idx,
+    k_div_df(const float* uh, const float* ul, const float* vh,
+             const float* vl, float* __restrict__ dh, float* __restrict__ dl, int nx, int ny, df idx,
              df idy) {
   pdl_wait();
   div_df_body(uh, ul, vh, vl, dh, dl, nx, ny, idx, idy);
@@ -471,11 +471,11 @@ __device__ __forceinline__ void subgrad_df_body(const float* __restrict__ wuh, c
   if (i >= nx || j >= ny) return;
   int im = i == 0 ? nx - 1 : i - 1, jm = j == 0 ? ny - 1 : j - 1;
   int64_t c = (int64_t)j * nx + i, cl = (int64_t)j * nx + im, cb = (int64_t)jm * nx + i;
-  df pc = {__ldg(ph + c), __ldg(pl + c)};
-  df gx = df_mul(df_sub(pc, df{__ldg(ph + cl), __ldg(pl + cl)}), idx);
-  df gy = df_mul(df_sub(pc, df{__ldg(ph + cb), __ldg(pl + cb)}), idy);
-  df wu = {__ldg(wuh + c), wul ? __ldg(wul + c) : 0.f};
-  df wv = {__ldg(wvh + c), wvl ? __ldg(wvl + c) : 0.f};
+  df pc = {ph[c], pl[c]};
+  df gx = df_mul(df_sub(pc, df{ph[cl], pl[cl]}), idx);
+  df gy = df_mul(df_sub(pc, df{ph[cb], pl[cb]}), idy);
+  df wu = {wuh[c], wul ? wul[c] : 0.f};
+  df wv = {wvh[c], wvl ? wvl[c] : 0.f};
   df u = df_sub(wu, gx), v = df_sub(wv, gy);
   uh[c] = u.hi; ul[c] = u.lo;
   vh[c] = v.hi; vl[c] = v.lo;
@@ -494,16 +494,16 @@ __device__ __forceinline__ void subgrad4_body(const float* __restrict__ wuh, con
   if (q >= (nx >> 2) || j >= ny) return;
   const int i0 = q << 2, il = i0 == 0 ? nx - 1 : i0 - 1, jm = j == 0 ? ny - 1 : j - 1;
   const int64_t c = (int64_t)j * nx + i0, cb = (int64_t)jm * nx + i0, cl = (int64_t)j * nx + il;
-  const float4 h = __ldg(reinterpret_cast<const float4*>(ph + c));
-  const float4 l = __ldg(reinterpret_cast<const float4*>(pl + c));
-  const float4 hb = __ldg(reinterpret_cast<const float4*>(ph + cb));
-  const float4 lb = __ldg(reinterpret_cast<const float4*>(pl + cb));
-  const float4 uw = __ldg(reinterpret_cast<const float4*>(wuh + c));
-  const float4 vw = __ldg(reinterpret_cast<const float4*>(wvh + c));
+  const float4 h = *reinterpret_cast<const float4*>(ph + c);
+  const float4 l = *reinterpret_cast<const float4*>(pl + c);
+  const float4 hb = *reinterpret_cast<const float4*>(ph + cb);
+  const float4 lb = *reinterpret_cast<const float4*>(pl + cb);
+  const float4 uw = *reinterpret_cast<const float4*>(wuh + c);
+  const float4 vw = *reinterpret_cast<const float4*>(wvh + c);
   const float4 z = {0.f, 0.f, 0.f, 0.f};
-  const float4 uwl = wul ? __ldg(reinterpret_cast<const float4*>(wul + c)) : z;
-  const float4 vwl = wvl ? __ldg(reinterpret_cast<const float4*>(wvl + c)) : z;
-  const df pw = {__ldg(ph + cl), __ldg(pl + cl)};
+  const float4 uwl = wul ? *reinterpret_cast<const float4*>(wul + c) : z;
+  const float4 vwl = wvl ? *reinterpret_cast<const float4*>(wvl + c) : z;
+  const df pw = {ph[cl], pl[cl]};
   const df p0 = {h.x, l.x}, p1 = {h.y, l.y}, p2 = {h.z, l.z}, p3 = {h.w, l.w};
   const df u0 = df_sub(df{uw.x, uwl.x}, df_mul(df_sub(p0, pw), idx));
   const df u1 = df_sub(df{uw.y, uwl.y}, df_mul(df_sub(p1, p0), idx));
@@ -520,8 +520,8 @@ __device__ __forceinline__ void subgrad4_body(const float* __restrict__ wuh, con
 }
 
 __global__ void __launch_bounds__(256)
-    k_subgrad4_df(const float* __restrict__ wuh, const float* __restrict__ wul, const float* __restrict__ wvh,
-                  const float* __restrict__ wvl, const float* __restrict__ ph, const float* __restrict__ pl,
+    k_subgrad4_df(const float* wuh, const float* wul, const float* wvh,
+                  const float* wvl, const float* ph, const float* pl,
                   float* __restrict__ uh, float* __restrict__ ul, float* __restrict__ vh, float* __restrict__ vl,
                   int nx, int ny, df idx, df idy, const StepFinish fin) {
   pdl_wait();
@@ -530,8 +530,8 @@ __global__ void __launch_bounds__(256)
 }
 
 __global__ void __launch_bounds__(256)
-    k_subgrad_df(const float* __restrict__ wuh, const float* __restrict__ wul, const float* __restrict__ wvh,
-                 const float* __restrict__ wvl, const float* __restrict__ ph, const float* __restrict__ pl,
+    k_subgrad_df(const float* wuh, const float* wul, const float* wvh,
+                 const float* wvl, const float* ph, const float* pl,
                  float* __restrict__ uh, float* __restrict__ ul, float* __restrict__ vh, float* __restrict__ vl,
                  int nx, int ny, df idx, df idy, const StepFinish fin) {
   pdl_wait();
@@ -621,7 +621,7 @@ __device__ __forceinline__ void refine_init_body(const float* __restrict__ dh, c
     int i = tx * 32 + threadIdx.x, j = ty * 8 + threadIdx.y;
     if (i < nx && j < ny) {
       int64_t r = (int64_t)j * nx, c = r + i;
-      df d = {__ldg(dh + c), __ldg(dl + c)};
+      df d = {dh[c], dl[c]};
       float rf;
       if (zero_p) {
         rf = df_to_f(d);
@@ -629,9 +629,9 @@ __device__ __forceinline__ void refine_init_body(const float* __restrict__ dh, c
         int im = i == 0 ? nx - 1 : i - 1, ip = i + 1 == nx ? 0 : i + 1;
         int jm = j == 0 ? ny - 1 : j - 1, jp = j + 1 == ny ? 0 : j + 1;
         int64_t cl = r + im, cr = r + ip, cb = (int64_t)jm * nx + i, ct = (int64_t)jp * nx + i;
-        rf = residual_df(d, df{__ldg(ph + c), __ldg(pl + c)}, df{__ldg(ph + cl), __ldg(pl + cl)},
-                         df{__ldg(ph + cr), __ldg(pl + cr)}, df{__ldg(ph + cb), __ldg(pl + cb)},
-                         df{__ldg(ph + ct), __ldg(pl + ct)}, ks);
+        rf = residual_df(d, df{ph[c], pl[c]}, df{ph[cl], pl[cl]},
+                         df{ph[cr], pl[cr]}, df{ph[cb], pl[cb]},
+                         df{ph[ct], pl[ct]}, ks);
       }
       r32[c] = rf;
       m = fmaxf(m, absnanf(rf));
@@ -641,8 +641,8 @@ __device__ __forceinline__ void refine_init_body(const float* __restrict__ dh, c
 }
 
 __global__ void __launch_bounds__(256)
-    k_refine_init(const float* __restrict__ dh, const float* __restrict__ dl, const float* __restrict__ ph,
-                  const float* __restrict__ pl, float* __restrict__ r32, int nx, int ny, LapScale ks,
+    k_refine_init(const float* dh, const float* dl, const float* ph,
+                  const float* pl, float* __restrict__ r32, int nx, int ny, LapScale ks,
                   int zero_p, RedCtx ctx) {
   pdl_wait();
   refine_init_body(dh, dl, ph, pl, r32, nx, ny, ks, zero_p, ctx);
@@ -701,15 +701,15 @@ __device__ __forceinline__ void refine_init4_body(const float* __restrict__ dh, 
       const int jm = j == 0 ? ny - 1 : j - 1, jp = j + 1 == ny ? 0 : j + 1;
       const int64_t r = (int64_t)j * nx, rm = (int64_t)jm * nx, rp = (int64_t)jp * nx;
       const int il = i0 == 0 ? nx - 1 : i0 - 1, ir = i0 + 4 == nx ? 0 : i0 + 4;
-      const float4 ch = __ldg(reinterpret_cast<const float4*>(ph + r + i0));
-      const float4 cl = __ldg(reinterpret_cast<const float4*>(pl + r + i0));
-      const float4 bh = __ldg(reinterpret_cast<const float4*>(ph + rm + i0));
-      const float4 bl = __ldg(reinterpret_cast<const float4*>(pl + rm + i0));
-      const float4 th = __ldg(reinterpret_cast<const float4*>(ph + rp + i0));
-      const float4 tl = __ldg(reinterpret_cast<const float4*>(pl + rp + i0));
-      const float4 d4h = __ldg(reinterpret_cast<const float4*>(dh + r + i0));
-      const float4 d4l = __ldg(reinterpret_cast<const float4*>(dl + r + i0));
-      const df lft = {__ldg(ph + r + il), __ldg(pl + r + il)}, rgt = {__ldg(ph + r + ir), __ldg(pl + r + ir)};
+      const float4 ch = *reinterpret_cast<const float4*>(ph + r + i0);
+      const float4 cl = *reinterpret_cast<const float4*>(pl + r + i0);
+      const float4 bh = *reinterpret_cast<const float4*>(ph + rm + i0);
+      const float4 bl = *reinterpret_cast<const float4*>(pl + rm + i0);
+      const float4 th = *reinterpret_cast<const float4*>(ph + rp + i0);
+      const float4 tl = *reinterpret_cast<const float4*>(pl + rp + i0);
+      const float4 d4h = *reinterpret_cast<const float4*>(dh + r + i0);
+      const float4 d4l = *reinterpret_cast<const float4*>(dl + r + i0);
+      const df lft = {ph[r + il], pl[r + il]}, rgt = {ph[r + ir], pl[r + ir]};
       const df c0 = {ch.x, cl.x}, c1 = {ch.y, cl.y}, c2 = {ch.z, cl.z}, c3 = {ch.w, cl.w};
       float4 out;
       out.x = residual_df(df{d4h.x, d4l.x}, c0, lft, c1, df{bh.x, bl.x}, df{th.x, tl.x}, ks);
@@ -725,8 +725,8 @@ __device__ __forceinline__ void refine_init4_body(const float* __restrict__ dh, 
 }
 
 __global__ void __launch_bounds__(256, 5)
-    k_refine_init4(const float* __restrict__ dh, const float* __restrict__ dl, const float* __restrict__ ph,
-                   const float* __restrict__ pl, float* __restrict__ r32, int nx, int ny, LapScale ks, RedCtx ctx,
+    k_refine_init4(const float* dh, const float* dl, const float* ph,
+                   const float* pl, float* __restrict__ r32, int nx, int ny, LapScale ks, RedCtx ctx,
                    CondFold cf) {
   pdl_wait();
   refine_init4_body(dh, dl, ph, pl, r32, nx, ny, ks, ctx, cf);
