@@ -143,7 +143,7 @@ __global__ void k_prep(const float* __restrict__ div, const float* __restrict__ 
 // f32 values are widened with integer instructions.  A warp walks down a strip
 // of kLossCols columns (lanes 0 and 31 hold its neighbours' columns) with the
 // three rows of the stencil in registers.  1024^2 x 4, mean + residual + seed:
-// 39 + 175 + 163 us with a thread per cell that converted every operand, 105 + 67 us
+// 39 + 175 + 163 us with a thread per cell that converted every operand, 105 + 68 us
 // here (mean and residual in one pass).
 constexpr int kLossCols = 30, kLossWarps = 8;
 
@@ -238,10 +238,18 @@ __global__ void __launch_bounds__(32 * kLossWarps)
 }
 
 // seed gradient dL/dout = (w_p 2 (e - mean_b e) + w_r 2 lap(res)) / (B N) into
-// channel 0 of gJ; w_p sum (e - mean)^2 / (B N) into acc[B].  The loss is summed
-// in f64; the gradient, which is rounded to bf16, is formed in double-float (48
-// bits) on the FP32 pipe, in f64 where a value is too large for it or not finite
-// (the loss: 3 f64 instructions a cell, 11 with the gradient in f64, 148 us).
+// channel 0 of gJ; w_p sum (e - mean)^2 / (B N) into acc[B].  Both are formed in f64,
+// the gradient then rounded to f32 and bf16.  That takes 11 f64 instructions a cell
+// (148 us at 1024^2 x 4), 8 of them for the gradient, so a cell's gradient is formed
+// in double-float (48 bits) on the FP32 pipe first, with a bound on its distance from
+// the f64 value: with u = 2^-24 the sums of f32 values are exact but for 10 u^2 of
+// their terms, a product or a sum of two double-floats adds 3 to 7 u^2, the rounding
+// of the mean and the weights u^2, and the f64 value itself is within 2^-49 of the
+// exact one -- together less than 24 u^2 of the terms, 2^-42 of them (64 u^2) with room
+// to spare.  Where every value within that bound rounds to the same f32, that is the
+// f64 value's rounding too; where not (next to a rounding boundary, or after heavy
+// cancellation), and where values or products leave the range in which those bounds
+// hold, the cell is done in f64.  66 us without the bound, 68 us with it.
 __global__ void __launch_bounds__(32 * kLossWarps)
     k_loss_seed(const float* __restrict__ out, const float* __restrict__ tgt, const float* res,
                 double* acc, uint4* __restrict__ gJ, int H, int W, int B, int rows, double w_p,
@@ -251,7 +259,10 @@ __global__ void __launch_bounds__(32 * kLossWarps)
   const int64_t npix = (int64_t)H * W, base = b * npix;
   const double mean = acc[b] / (double)npix, scale = 2.0 / ((double)B * npix);
   const df meanf = df_neg(df_from_d(mean)), wp = df_from_d(scale * w_p), wr = df_from_d(scale * w_r);
-  const bool dfok = fabs(mean) < 1e30 && scale * w_p < 1e6 && scale * w_r < 1e6;
+  // weights whose double-float halves are normal numbers, and products of f32 range
+  auto in_range = [](double k) { return k == 0.0 || (k > 1e-28 && k < 1e6); };
+  const bool dfok = fabs(mean) < 1e30 && in_range(scale * w_p) && in_range(scale * w_r);
+  const float mabs = fabsf(meanf.hi), bound_p = 0x1p-42f * wp.hi, bound_r = res ? 0x1p-42f * wr.hi : 0.f;
   const LossStrip t = loss_strip(H, W, rows);
   double s = 0.0;
   if (t.any) {
@@ -267,8 +278,12 @@ __global__ void __launch_bounds__(32 * kLossWarps)
       const double ec = widen(o) - widen(g0) - mean;
       if (t.store) s += ec * ec;
       float g;
-      const float size = ((fabsf(o) + fabsf(g0)) + (fabsf(above) + fabsf(below))) + ((fabsf(left) + fabsf(right)) + fabsf(c));
-      if (dfok && size < 1e30f) {
+      const float size_e = fabsf(o) + fabsf(g0);
+      const float size_l = (fabsf(above) + fabsf(below)) + (fabsf(left) + fabsf(right)) + 4.f * fabsf(c);
+      const float bound = bound_p * (size_e + mabs) + bound_r * size_l;
+      // (above 1e-36 no product's error term is lost to underflow)
+      bool done = dfok && size_e + size_l < 1e30f && bound > 1e-36f;
+      if (done) {
         df v = df_mul(df_add(two_sum(o, -g0), meanf), wp);
         if (res) {
           const df a = two_sum(left, right), d = two_sum(a.hi, above), e = two_sum(d.hi, below);
@@ -276,8 +291,10 @@ __global__ void __launch_bounds__(32 * kLossWarps)
           l.lo = l.lo + ((a.lo + d.lo) + e.lo);
           v = df_add(v, df_mul(fast_two_sum(l.hi, l.lo), wr));
         }
-        g = df_to_f(v);
-      } else {
+        g = __fadd_rn(v.hi, __fadd_rn(v.lo, bound));
+        done = g == __fadd_rn(v.hi, __fsub_rn(v.lo, bound));
+      }
+      if (!done) {
         double v = w_p * ec;
         if (res)
           v += w_r * ((double)left + (double)right + (double)above + (double)below - 4.0 * (double)c);
