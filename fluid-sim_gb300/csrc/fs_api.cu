@@ -1356,6 +1356,7 @@ FS_API int fs_autotune_tiles(fs_solver* h, double dt, int32_t nsteps, int32_t* t
     for (int t : {start, 64, 32, 16}) {
       if (t == start && here < 1e300) continue;
       s->tile_level[l] = t;
+      if (mg_tile(s, l) != t) continue;  // not used on this level
       double per = 0;
       rc = tune_time(T, dt, nsteps, &per, &e);
       if (rc != FS_OK || e != cudaSuccess) break;
@@ -2000,6 +2001,7 @@ static int batch_autotune(fs_batch* b, const double* dt, int32_t nsteps, int wha
       int pick = start;
       for (int t : {64, 32, 16}) {
         for (int i : c.idx) b->members[i]->s.tile_level[l] = t;
+        if (mg_tile_class(lead, l, (int)c.idx.size()) != t) continue;  // not used on this level
         double per = 0;
         rc = time_batch(&per);
         if (rc != FS_OK || e != cudaSuccess) break;

@@ -141,19 +141,16 @@ static int tile_for(int n) {
   return 16;
 }
 
-// A side T serves a level of n cells only if T <= n / 2 (16 always: tile
-// levels have n > 64).
-static bool tile_fits(int t, int n) { return t == 16 || 2 * t <= n; }
+// A side T serves a level of n cells only if T <= n / 2 and its regions' four columns
+// a lane divide the level; side 16, with two columns a lane, serves every tile level (n
+// > 64 and even; n = 2 mod 4 only as the last above an odd bottom level, so n <= 126).
+static bool tile_fits(int t, int n) { return t == 16 || (n % 4 == 0 && 2 * t <= n); }
 
 int mg_tile(const Solver* s, int l) {
   const int n = s->lev[l].n;
   if (l >= 0 && l < 16 && s->tile_level[l] && tile_fits(s->tile_level[l], n)) return s->tile_level[l];
   return tile_for(n);
 }
-
-// a level of n = 2 mod 4 cells (the last above an odd bottom level, so n <= 126)
-// needs two columns a lane
-static int region_side(int n, int t) { return n % 4 ? 16 : t; }
 
 // profile name of a tile kernel: one entry per level ("mg_down_l0", ...)
 static std::string level_name(const Solver* s, const Level& L, const char* base) {
@@ -191,7 +188,7 @@ static void down_t(Solver* s, Level& L, const Level& C, bool has_x, bool zero, i
 
 template <int H>
 static void down(Solver* s, Level& L, const Level& C, bool has_x, bool zero, int first, const int* cyc, bool x_unused) {
-  switch (region_side(L.n, mg_tile(s, (int)(&L - s->lev.data())))) {
+  switch (mg_tile(s, (int)(&L - s->lev.data()))) {
     case 64: down_t<64, H>(s, L, C, has_x, zero, first, cyc, x_unused); break;
     case 32: down_t<32, H>(s, L, C, has_x, zero, first, cyc, x_unused); break;
     default: down_t<16, H>(s, L, C, has_x, zero, first, cyc, x_unused); break;
@@ -222,7 +219,7 @@ static void up_t(Solver* s, Level& L, const Level& C, float* acc_h, float* acc_l
 template <int H>
 static void up(Solver* s, Level& L, const Level& C, float* acc_h, float* acc_l, int first, const int* cyc,
                bool x_zero) {
-  switch (region_side(L.n, mg_tile(s, (int)(&L - s->lev.data())))) {
+  switch (mg_tile(s, (int)(&L - s->lev.data()))) {
     case 64: up_t<64, H>(s, L, C, acc_h, acc_l, first, cyc, x_zero); break;
     case 32: up_t<32, H>(s, L, C, acc_h, acc_l, first, cyc, x_zero); break;
     default: up_t<16, H>(s, L, C, acc_h, acc_l, first, cyc, x_zero); break;
@@ -322,7 +319,7 @@ int mg_tile_class(const Solver* s0, int l, int count) { return tile_for_class(s0
 
 template <int H>
 static void down_class(Solver* const* ms, int count, int l, cudaStream_t st) {
-  switch (region_side(ms[0]->lev[l].n, tile_for_class(ms[0], l, count))) {
+  switch (tile_for_class(ms[0], l, count)) {
     case 64: down_class_t<64, H>(ms, count, l, st); break;
     case 32: down_class_t<32, H>(ms, count, l, st); break;
     default: down_class_t<16, H>(ms, count, l, st); break;
@@ -347,7 +344,7 @@ static void up_class_t(Solver* const* ms, int count, int l, cudaStream_t st) {
 template <int H>
 static void up_class(Solver* const* ms, int count, int l, cudaStream_t st) {
   const bool acc = l == 0;
-  switch (region_side(ms[0]->lev[l].n, tile_for_class(ms[0], l, count))) {
+  switch (tile_for_class(ms[0], l, count)) {
     case 64: acc ? up_class_t<64, H, true>(ms, count, l, st) : up_class_t<64, H, false>(ms, count, l, st); break;
     case 32: acc ? up_class_t<32, H, true>(ms, count, l, st) : up_class_t<32, H, false>(ms, count, l, st); break;
     default: acc ? up_class_t<16, H, true>(ms, count, l, st) : up_class_t<16, H, false>(ms, count, l, st); break;

@@ -475,14 +475,15 @@ FS_API int fs_autotune(fs_solver* s, double dt, int32_t nsteps, int32_t* pre, in
  * fused multigrid kernels of each tile level (the levels above the bottom
  * solve); 0 = the built-in rule (64 for levels of more than 1984 cells a side,
  * else 32 for more than 480, else 16).  A side
- * larger than half its level is not used there (the built-in rule applies;
+ * larger than half its level is not used there, nor are 32 and 64 on a level
+ * whose cells a side are no multiple of 4 (the built-in rule applies;
  * fs_get_mg_tiles reports the side in use).  The tiles give the same values
  * whatever their size, so they change only the speed. */
 FS_API int fs_set_mg_tiles(fs_solver* s, const int32_t* tiles, int32_t count);
 /* the sides in use, one per tile level (*count = number of tile levels) */
 FS_API int fs_get_mg_tiles(fs_solver* s, int32_t* tiles, int32_t cap, int32_t* count);
-/* Greedy per level: every tile level tries 64, 32 and 16 (the others fixed),
- * each timed over nsteps steps from the same saved state; keeps the fastest.
+/* Greedy per level: every tile level tries those of 64, 32 and 16 that would be
+ * used there (the others fixed), each timed over nsteps steps from the same saved state; keeps the fastest.
  * The state and time are restored; tiles_out gets the picks (0 = rule kept). */
 FS_API int fs_autotune_tiles(fs_solver* s, double dt, int32_t nsteps, int32_t* tiles_out, int32_t cap,
                              int32_t* count, double* ms_per_step);
