@@ -52,20 +52,6 @@ __device__ __forceinline__ float bilerp(const T* __restrict__ f, int nx, int ny,
   return top + (bot - top) * fy;
 }
 
-// Range of the four cells a bilinear sample at (bi+ox, bj+oy) reads
-// (src/cpu/advect.js:104-111).
-template <class T>
-__device__ __forceinline__ void bounds4(const T* __restrict__ f, int nx, int ny, int bi, int bj,
-                                        float ox, float oy, float& lo, float& hi) {
-  int i0 = wrap_idx(bi + (int)floorf(ox), nx), j0 = wrap_idx(bj + (int)floorf(oy), ny);
-  int i1 = i0 + 1 == nx ? 0 : i0 + 1;
-  int j1 = j0 + 1 == ny ? 0 : j0 + 1;
-  int64_t r0 = (int64_t)j0 * nx, r1 = (int64_t)j1 * nx;
-  float a = ld(f, r0 + i0), b = ld(f, r0 + i1), c = ld(f, r1 + i0), d = ld(f, r1 + i1);
-  lo = fminf(fminf(a, b), fminf(c, d));
-  hi = fmaxf(fmaxf(a, b), fmaxf(c, d));
-}
-
 // Sample offsets of the u and v grids relative to a home point.  u lives at
 // (i, j+1/2), v at (i+1/2, j) (src/core/grid.js:99-105).  A point at home +
 // (dX, dY) cells has u-grid index (hux + dX, huy + dY) etc.
@@ -678,12 +664,10 @@ static dim3 tile_grid(const Grid& g, int nt = 1) {
 // (512^2 110.7 against 118.9).
 static int tiles_per_cta(const Grid& g) { return (int64_t)g.nx * g.ny >= 4000000 ? 2 : 1; }
 
-
-
-// Tensor maps of f32 planes for the TMA-staged tiles' kSW x kSH boxes, kept per
-// device pointer, plane and box.  TMA needs the row pitch and the box width
-// multiples of 16 bytes (nx % 4 == 0) and a 16-byte-aligned base; otherwise,
-// or if the CUDA driver lacks the encoder, every tile uses wrapped loads.
+// Tensor maps of the solver's f32 planes for the TMA-staged tiles' kSW x kSH boxes,
+// kept per device pointer.  TMA needs the row pitch a multiple of 16 bytes (nx % 4 ==
+// 0) and a 16-byte-aligned base; otherwise, or if the CUDA driver lacks the encoder,
+// every tile uses wrapped loads.
 static PFN_cuTensorMapEncodeTiled_v12000 tmap_encoder() {
   static PFN_cuTensorMapEncodeTiled_v12000 fn = [] {
     void* p = nullptr;
@@ -696,11 +680,12 @@ static PFN_cuTensorMapEncodeTiled_v12000 tmap_encoder() {
   return fn;
 }
 
-bool box_tmap(Solver* s, const float* f, int nx, int ny, int bw, int bh, CUtensorMap* out) {
-  if (nx % 4 != 0 || bw % 4 != 0 || ((uintptr_t)f & 15) != 0 || nx < bw || ny < bh || bw > 256 || bh > 256)
-    return false;
+static bool tile_tmap(Solver* s, const float* f, CUtensorMap* out) {
+  static_assert(kSW % 4 == 0 && kSW <= 256 && kSH <= 256, "TMA box");
+  const int nx = s->g.nx, ny = s->g.ny;
+  if (nx % 4 != 0 || ((uintptr_t)f & 15) != 0 || nx < kSW || ny < kSH) return false;
   for (const auto& e : s->tmaps)
-    if (e.p == f && e.nx == nx && e.ny == ny && e.bw == bw && e.bh == bh) {
+    if (e.p == f) {
       *out = e.m;
       return true;
     }
@@ -708,10 +693,9 @@ bool box_tmap(Solver* s, const float* f, int nx, int ny, int bw, int bh, CUtenso
   if (!enc) return false;
   Solver::Tmap e;
   e.p = f;
-  e.nx = nx; e.ny = ny; e.bw = bw; e.bh = bh;
   const cuuint64_t dims[2] = {(cuuint64_t)nx, (cuuint64_t)ny};
   const cuuint64_t pitch[1] = {(cuuint64_t)nx * sizeof(float)};
-  const cuuint32_t box[2] = {(cuuint32_t)bw, (cuuint32_t)bh};
+  const cuuint32_t box[2] = {(cuuint32_t)kSW, (cuuint32_t)kSH};
   const cuuint32_t estr[2] = {1, 1};
   if (enc(&e.m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float*>(f), dims, pitch, box, estr,
           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
@@ -720,10 +704,6 @@ bool box_tmap(Solver* s, const float* f, int nx, int ny, int bw, int bh, CUtenso
   s->tmaps.push_back(e);
   *out = e.m;
   return true;
-}
-
-static bool tile_tmap(Solver* s, const float* f, CUtensorMap* out) {
-  return box_tmap(s, f, s->g.nx, s->g.ny, kSW, kSH, out);
 }
 
 template <>

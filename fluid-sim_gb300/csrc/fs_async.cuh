@@ -14,12 +14,6 @@ __device__ __forceinline__ void cp_async4(float* sdst, const float* gsrc) {
                "l"((size_t)__cvta_generic_to_global(gsrc))
                : "memory");
 }
-// 16-byte form (both addresses 16-byte aligned), L2 only
-__device__ __forceinline__ void cp_async16(float* sdst, const float* gsrc) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(sdst)),
-               "l"((size_t)__cvta_generic_to_global(gsrc))
-               : "memory");
-}
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 }  // namespace fs

@@ -105,11 +105,9 @@ struct Solver {
 
   std::vector<Level> lev;
   int tile_level[16] = {};  // tile side of each tile level's kernels; 0 = the built-in rule
-  // TMA tensor maps of the staged fields (advection tiles), by
-  // device pointer, plane and box (box_tmap, fs_advect.cu)
+  // TMA tensor maps of the staged fields (advection tiles), by device pointer
   struct Tmap {
     const void* p;
-    int nx, ny, bw, bh;
     CUtensorMap m;
   };
   std::vector<Tmap> tmaps;
@@ -311,7 +309,6 @@ void launch_residual(Solver* s, const float* x, const float* rhs, float* out, fl
 void launch_restrict(Solver* s, const float* fine, float* coarse, int nc);
 void launch_prolong_add(Solver* s, const float* coarse, float* fine, int nf);
 void launch_fill(Solver* s, float* x, float value, int64_t n);
-void launch_fill64(Solver* s, double* x, double value, int64_t n);
 // mixed-precision refinement (double-float pressure and divergence)
 // cond (a captured tolerance loop's handle): the residual kernel also does
 // the loop's step bookkeeping and sets the condition when it can (returns
@@ -321,7 +318,6 @@ bool launch_refine_init(Solver* s, const float* dh, const float* dl, const float
 // TMA tensor map of a row-major f32 plane nx x ny (pitch nx) with a bw x bh
 // box, cached per solver; false when TMA cannot copy it (nx % 4 != 0, an
 // unaligned base, a box larger than the plane, no encoder in the CUDA driver)
-bool box_tmap(Solver* s, const float* f, int nx, int ny, int bw, int bh, CUtensorMap* out);
 // divergence + zero-pressure residual + zeroed pressure in one pass (MIXED)
 void launch_div_start(Solver* s, const float* wu, const float* wv);
 // DIFFUSE in the same pass as the divergence (F32) or the start of a MIXED solve

@@ -254,19 +254,12 @@ __global__ void k_fill(float* x, float v, int64_t n) {
   for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < n; k += (int64_t)gridDim.x * blockDim.x)
     x[k] = v;
 }
-__global__ void k_fill64(double* x, double v, int64_t n) {
-  for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < n; k += (int64_t)gridDim.x * blockDim.x)
-    x[k] = v;
-}
 static int fill_blocks(int64_t n) {
   int64_t b = (n + 255) / 256;
   return (int)(b < 152 * 16 ? b : 152 * 16);
 }
 void launch_fill(Solver* s, float* x, float value, int64_t n) {
   FS_LAUNCH(s, "fill", (double)n * 4, k_fill<<<fill_blocks(n), 256, 0, s->stream>>>(x, value, n));
-}
-void launch_fill64(Solver* s, double* x, double value, int64_t n) {
-  FS_LAUNCH(s, "fill", (double)n * 8, k_fill64<<<fill_blocks(n), 256, 0, s->stream>>>(x, value, n));
 }
 
 // Reduction kernels walk 32x8-cell tiles with a capped 1-D grid, so the
