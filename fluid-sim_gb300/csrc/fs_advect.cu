@@ -78,15 +78,15 @@ __device__ __forceinline__ void trace(const TV* __restrict__ u, const TV* __rest
 }
 
 // ------------------------------------------------------ tiled advection
-// A MacCormack step takes about 20 bilinear samples per cell.  A CTA stages its 32x16-cell tile of each field
-// it samples, plus a halo of 4 cells, in shared memory.  When the largest
-// displacement any trace of the tile can reach is at most 3 cells (checked
-// once per CTA on the staged velocities, below) every sample lies in the
-// staged block and is read from there unchecked, two cells a thread at once
-// (advect_pair, combine_pair); otherwise each sample is checked and one whose
-// four cells leave the block falls back to the wrapped global read.  (Checked
-// samples may round a departure offset differently, by how the compiler
-// contracts it.)
+// A MacCormack step takes about 20 bilinear samples per cell.  A CTA stages its
+// 32x16-cell tile of each field it samples, plus a halo of 4 cells, in shared
+// memory.  When the largest displacement any trace of the tile can reach is at
+// most 3 cells (checked once per CTA on the staged velocities, below) every
+// sample lies in the staged block and is read from there unchecked, two cells a
+// thread at once (advect_pair, combine_pair); otherwise each sample is checked
+// and one whose four cells leave the block falls back to the wrapped global
+// read.  (Checked samples may round a departure offset differently, by how the
+// compiler contracts it.)
 constexpr int kTX = 32, kTY = 16, kHalo = 4;
 constexpr int kSW = kTX + 2 * kHalo, kSH = kTY + 2 * kHalo;
 // largest |u| dt/dx (cells) for which every trace stays in the staged block:
@@ -551,7 +551,8 @@ __global__ void __launch_bounds__(256) k_mc_combine_t(const float* u, const floa
     const CUtensorMap* const tm[4] = {&tm_u, &tm_v, &tm_fu, &tm_fv};
     tma_issue<4, NT>(sm, tm, oi, oj, in, bar);
   }
-  if (NT > 1) {  // large grids: the limiter's ranges into L2 meanwhile (4096^2 158 -> 154 us), a line a row, tile and plane
+  if (NT > 1) {
+    // large grids: the limiter's ranges into L2 meanwhile (4096^2 158 -> 154 us), a line a row, tile and plane
     const int k = threadIdx.y * 32 + threadIdx.x, q = k / (NT * kTY), j = blockIdx.y * NT * kTY + k % (NT * kTY);
     if (q < 4 && j < ny) prefetch_l2(bounds + (int64_t)q * nx * ny + (int64_t)j * nx + ti);
   }
@@ -712,9 +713,11 @@ void launch_advect_sl<float>(Solver* s, const float* u, const float* v, float* o
   float cx = (float)((double)dt / g.dxd), cy = (float)((double)dt / g.dyd);
   CUtensorMap tu{}, tv{};
   const int tma = tile_tmap(s, u, &tu) && tile_tmap(s, v, &tv) ? 1 : 0;
+  const int nt = tiles_per_cta(g);
+  auto* forward = nt == 2 ? k_advect_sl_t<2> : k_advect_sl_t<1>;
   FS_LAUNCH(s, "advect_sl", (double)s->n * 16,
-            (tiles_per_cta(g) == 2 ? k_advect_sl_t<2> : k_advect_sl_t<1>)<<<tile_grid(g, tiles_per_cta(g)), kBlock, 0, s->stream>>>(u, v, ou, ov, g.nx, g.ny, cx, cy, nullptr, tu, tv,
-                                                                  tma, &s->dev->async_err));
+            forward<<<tile_grid(g, nt), kBlock, 0, s->stream>>>(u, v, ou, ov, g.nx, g.ny, cx, cy, nullptr, tu, tv, tma,
+                                                                &s->dev->async_err));
 }
 
 template <>
@@ -725,14 +728,15 @@ void launch_advect_mc<float>(Solver* s, const float* u, const float* v, float* f
   CUtensorMap tu{}, tv{}, tfu{}, tfv{};
   const int tma =
       tile_tmap(s, u, &tu) && tile_tmap(s, v, &tv) && tile_tmap(s, fu, &tfu) && tile_tmap(s, fv, &tfv) ? 1 : 0;
+  const int nt = tiles_per_cta(g);
+  auto* forward = nt == 2 ? k_advect_sl_t<2> : k_advect_sl_t<1>;
+  auto* combine = nt == 2 ? k_mc_combine_t<2> : k_mc_combine_t<1>;
   FS_LAUNCH(s, "advect_sl", (double)s->n * 32,
-            (tiles_per_cta(g) == 2 ? k_advect_sl_t<2> : k_advect_sl_t<1>)<<<tile_grid(g, tiles_per_cta(g)), kBlock, 0, s->stream>>>(u, v, fu, fv, g.nx, g.ny, cx, cy, s->mc_bounds, tu,
-                                                                  tv, tma, &s->dev->async_err));
+            forward<<<tile_grid(g, nt), kBlock, 0, s->stream>>>(u, v, fu, fv, g.nx, g.ny, cx, cy, s->mc_bounds, tu, tv,
+                                                                tma, &s->dev->async_err));
   FS_LAUNCH(s, "mc_combine", (double)s->n * 40,
-            launch_dependent(true, tiles_per_cta(g) == 2 ? k_mc_combine_t<2> : k_mc_combine_t<1>,
-                             tile_grid(g, tiles_per_cta(g)), kBlock, 0, s->stream, u, v, fu, fv, s->mc_bounds, ou, ov, g.nx, g.ny,
-                                                                   cx, cy, tu, tv, tfu, tfv, tma,
-                                                                   &s->dev->async_err));
+            launch_dependent(true, combine, tile_grid(g, nt), kBlock, 0, s->stream, u, v, fu, fv, s->mc_bounds, ou,
+                             ov, g.nx, g.ny, cx, cy, tu, tv, tfu, tfv, tma, &s->dev->async_err));
 }
 
 __device__ __forceinline__ void diffuse_body(const float* __restrict__ u, const float* __restrict__ v,
@@ -793,9 +797,11 @@ void launch_diffuse(Solver* s, const float* u, const float* v, float* ou, float*
   float b = (float)(s->prm.nu * dt / (g.dyd * g.dyd));
   FS_LAUNCH(s, "diffuse", (double)s->n * 16,
             if (g.nx % 4 == 0) {
-              launch_dependent(true, k_diffuse4, grid2d(g.nx / 4, g.ny, kBlock), kBlock, 0, s->stream, u, v, ou, ov, g.nx, g.ny, a, b);
+              launch_dependent(true, k_diffuse4, grid2d(g.nx / 4, g.ny, kBlock), kBlock, 0, s->stream, u, v, ou, ov,
+                               g.nx, g.ny, a, b);
             } else {
-              launch_dependent(true, k_diffuse, grid2d(g.nx, g.ny, kBlock), kBlock, 0, s->stream, u, v, ou, ov, g.nx, g.ny, a, b);
+              launch_dependent(true, k_diffuse, grid2d(g.nx, g.ny, kBlock), kBlock, 0, s->stream, u, v, ou, ov, g.nx,
+                               g.ny, a, b);
             });
 }
 
@@ -920,8 +926,9 @@ void launch_forcing(Solver* s, float* u, float* v, float dt) {
   float scale = (float)(s->amp * dt / sqrt((double)s->n_modes));
   float damp = (float)exp(-s->drag * dt);
   FS_LAUNCH(s, "forcing", (double)s->n * 16,
-            launch_dependent(true, k_forcing, dim3((g.nx + 31) / 32, (g.ny + kForceTY - 1) / kForceTY), kBlock, 0, s->stream, 
-                u, v, s->modes, s->n_modes, g.nx, g.ny, g.dx, g.dy, scale, damp, s->drift, s->dev));
+            launch_dependent(true, k_forcing, dim3((g.nx + 31) / 32, (g.ny + kForceTY - 1) / kForceTY), kBlock, 0,
+                             s->stream, u, v, s->modes, s->n_modes, g.nx, g.ny, g.dx, g.dy, scale, damp, s->drift,
+                             s->dev));
 }
 
 // Direct forcing of immersed disks (src/cpu/solid.js:165-233, shaders.js:587-653):
@@ -1114,7 +1121,8 @@ void launch_solids(Solver* s, float* u, float* v, float dt, bool record_impulse)
 __device__ __forceinline__ Home home_c() { return {0.5f, 0.f, 0.f, 0.5f}; }
 
 __global__ void __launch_bounds__(256) k_advect_dye(const float* u, const float* v, const float4* q,
-                                                    float4* __restrict__ out, int nx, int ny, float cx, float cy, float keep) {
+                                                    float4* __restrict__ out, int nx, int ny, float cx, float cy,
+                                                    float keep) {
   pdl_wait();
   int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
   if (i >= nx || j >= ny) return;
@@ -1138,9 +1146,9 @@ void launch_advect_dye(Solver* s, float dt) {
   const Grid& g = s->g;
   dim3 b(32, 8);
   FS_LAUNCH(s, "advect_dye", (double)s->n * 40,
-            launch_dependent(true, k_advect_dye, grid2d(g.nx, g.ny, b), b, 0, s->stream, 
-                s->u, s->v, static_cast<const float4*>(s->dye), static_cast<float4*>(s->dye2), g.nx, g.ny,
-                (float)(dt * g.idxd), (float)(dt * g.idyd), (float)(1.0 - s->prm.dye_fade)));
+            launch_dependent(true, k_advect_dye, grid2d(g.nx, g.ny, b), b, 0, s->stream, s->u, s->v,
+                             static_cast<const float4*>(s->dye), static_cast<float4*>(s->dye2), g.nx, g.ny,
+                             (float)(dt * g.idxd), (float)(dt * g.idyd), (float)(1.0 - s->prm.dye_fade)));
   // the next step reads s->dye again: copy back (a captured step cannot swap pointers)
   cudaMemcpyAsync(s->dye, s->dye2, (size_t)s->n * 16, cudaMemcpyDeviceToDevice, s->stream);
 }

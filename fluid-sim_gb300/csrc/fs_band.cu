@@ -334,13 +334,13 @@ void launch_band(Solver* s, float* u, float* v, float dt) {
   const float damp = b->drag > 0 ? (float)exp(-b->drag * (double)dt) : 1.f;
   const int nq = 2 * b->K + 1;
   FS_LAUNCH(s, "band_columns", (double)nq * g.nx * 32,
-            launch_dependent(true, k_band_columns, dim3((g.nx + 255) / 256, nq), dim3(256), 0, s->stream, 
-                b->kind, b->M, b->K, s->dev, b->seed, b->kf, b->width, scale, b->lattice, b->ex_u, b->ex_v, b->gu,
-                b->gv, g.nx));
+            launch_dependent(true, k_band_columns, dim3((g.nx + 255) / 256, nq), dim3(256), 0, s->stream, b->kind,
+                             b->M, b->K, s->dev, b->seed, b->kf, b->width, scale, b->lattice, b->ex_u, b->ex_v, b->gu,
+                             b->gv, g.nx));
   FS_LAUNCH(s, "band_apply", (double)s->n * 16,
             launch_dependent(true, k_band_apply, dim3((g.nx + kBandTX - 1) / kBandTX, (g.ny + kBandTY - 1) / kBandTY),
-                             dim3(32, 8), sizeof(BandStage), s->stream, 
-                u, v, g.nx, g.ny, b->K, b->gu, b->gv, b->ey_u, b->ey_v, damp, s->dev));
+                             dim3(32, 8), sizeof(BandStage), s->stream, u, v, g.nx, g.ny, b->K, b->gu, b->gv, b->ey_u,
+                             b->ey_v, damp, s->dev));
 }
 
 }  // namespace fs

@@ -534,7 +534,8 @@ struct Top {
   __device__ __forceinline__ void exchange(Edge& e, float (&below)[2], float (&above)[2]) {
     if (act) {
       e[buf][warp][0][lane] = make_float2(x[0][0], x[0][1]);
-      e[buf][warp][1][lane] = last ? make_float2(x[LAST - 1][0], x[LAST - 1][1]) : make_float2(x[RPW - 1][0], x[RPW - 1][1]);
+      e[buf][warp][1][lane] =
+          last ? make_float2(x[LAST - 1][0], x[LAST - 1][1]) : make_float2(x[RPW - 1][0], x[RPW - 1][1]);
     }
     __syncthreads();
     float2 b = make_float2(0.f, 0.f), a = b;
@@ -804,12 +805,12 @@ void launch_bottom(Solver* s, int lb, bool hx, float* acc_h, float* acc_l) {
   const double bytes = (double)nb * nb * (hx ? 12.0 : 8.0);
   const BottomH2 H = bottom_h2(s, lb);
   switch (bottom_chain(s, lb)) {
-#define FS_CASE(N0, NM)                                                                                          \
-  case N0:                                                                                                       \
-    FS_LAUNCH(s, "mg_bottom", bytes,                                                                             \
-              launch_dependent(true, k_mg_bottom_chain<N0, NM>, dim3(1), dim3(kBottomThreads), 0, s->stream,                                     \
-                  L[lb].rhs, L[lb].x, hx ? 1 : 0, H, P.mg_pre_smooth, P.mg_post_smooth, P.mg_coarse_sweeps,      \
-                  acc_h, acc_l));                                                                                \
+#define FS_CASE(N0, NM)                                                                                        \
+  case N0:                                                                                                     \
+    FS_LAUNCH(s, "mg_bottom", bytes,                                                                           \
+              launch_dependent(true, k_mg_bottom_chain<N0, NM>, dim3(1), dim3(kBottomThreads), 0, s->stream,   \
+                               L[lb].rhs, L[lb].x, hx ? 1 : 0, H, P.mg_pre_smooth, P.mg_post_smooth,           \
+                               P.mg_coarse_sweeps, acc_h, acc_l));                                             \
     return;
     FS_CHAINS(FS_CASE)
 #undef FS_CASE
@@ -818,8 +819,8 @@ void launch_bottom(Solver* s, int lb, bool hx, float* acc_h, float* acc_l) {
   const size_t smem = bottom_layout(s, &B);
   const int threads = std::min(1024, std::max(32, ((nb * nb / 4 + 31) / 32) * 32));
   FS_LAUNCH(s, "mg_bottom", bytes,
-            launch_dependent(true, k_mg_bottom, dim3(1), dim3(threads), smem, s->stream, L[lb].rhs, L[lb].x, hx ? 1 : 0, B, P.mg_pre_smooth,
-                                                         P.mg_post_smooth, P.mg_coarse_sweeps, acc_h, acc_l));
+            launch_dependent(true, k_mg_bottom, dim3(1), dim3(threads), smem, s->stream, L[lb].rhs, L[lb].x,
+                             hx ? 1 : 0, B, P.mg_pre_smooth, P.mg_post_smooth, P.mg_coarse_sweeps, acc_h, acc_l));
 }
 
 void launch_bottom_class(Solver* const* ms, int count, int lb, cudaStream_t st) {
@@ -836,8 +837,8 @@ void launch_bottom_class(Solver* const* ms, int count, int lb, cudaStream_t st) 
   switch (bottom_chain(s0, lb)) {
 #define FS_CASE(N0, NM)                                                                                        \
   case N0:                                                                                                     \
-    launch_dependent(true, k_mg_bottom_chain_class<N0, NM>, dim3(grid), dim3(kBottomThreads), 0, st, tab, H, P.mg_pre_smooth, P.mg_post_smooth, \
-                                                                     P.mg_coarse_sweeps, P.max_cycles);         \
+    launch_dependent(true, k_mg_bottom_chain_class<N0, NM>, dim3(grid), dim3(kBottomThreads), 0, st, tab, H,   \
+                     P.mg_pre_smooth, P.mg_post_smooth, P.mg_coarse_sweeps, P.max_cycles);                     \
     return;
     FS_CHAINS(FS_CASE)
 #undef FS_CASE
@@ -845,8 +846,8 @@ void launch_bottom_class(Solver* const* ms, int count, int lb, cudaStream_t st) 
   BottomLevels B;
   const size_t smem = bottom_layout(s0, &B);
   const int threads = std::min(1024, std::max(32, ((nb * nb / 4 + 31) / 32) * 32));
-  launch_dependent(true, k_mg_bottom_class, dim3(grid), dim3(threads), smem, st, tab, B, P.mg_pre_smooth, P.mg_post_smooth, P.mg_coarse_sweeps,
-                                                 P.max_cycles);
+  launch_dependent(true, k_mg_bottom_class, dim3(grid), dim3(threads), smem, st, tab, B, P.mg_pre_smooth,
+                   P.mg_post_smooth, P.mg_coarse_sweeps, P.max_cycles);
 }
 
 }  // namespace fs

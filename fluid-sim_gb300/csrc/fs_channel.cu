@@ -157,7 +157,8 @@ void launch_channel(Solver* s, float* u, float* v) {
   // algorithmic bytes: u, v read and written on the cells of the two bands
   const double cells = (double)b.nw * g.nx + (double)b.nf * (g.ny - b.nw);
   FS_LAUNCH(s, "channel", 16.0 * cells,
-            launch_dependent(true, k_channel, dim3(b.na + nb), dim3(32, 8), 0, s->stream, u, v, g.nx, g.ny, g.dx, g.dy, d, (float)w, b));
+            launch_dependent(true, k_channel, dim3(b.na + nb), dim3(32, 8), 0, s->stream, u, v, g.nx, g.ny, g.dx,
+                             g.dy, d, (float)w, b));
 }
 
 }  // namespace fs

@@ -95,7 +95,8 @@ struct Cfg {
   static constexpr int WTAP = KC * NS * 16;                  // bytes of one tap of this CTA's weights
   static constexpr int W_BYTES = align128(9 * WTAP);
   static constexpr int NACC = TY * NS;                       // columns of one accumulator set
-  static constexpr int NCOL = 2 * NACC <= 32 ? 32 : 2 * NACC <= 64 ? 64 : 2 * NACC <= 128 ? 128 : 2 * NACC <= 256 ? 256 : 512;
+  static constexpr int NCOL =
+      2 * NACC <= 32 ? 32 : 2 * NACC <= 64 ? 64 : 2 * NACC <= 128 ? 128 : 2 * NACC <= 256 ? 256 : 512;
   // + 128 bytes of barriers and the TMEM slot, and this CTA's biases (which the caller
   // aligns to a word only: the epilogue reads them four at a time from here)
   static constexpr int SMEM = RING + W_BYTES + 128 + align128(NS * 4);
@@ -160,7 +161,8 @@ struct Extra {
       for (int q = 0; q < 4; q++) {
         const int64_t fp = above(b, y, x, H, W, q);
         // fine and up may be one buffer (a pixel is read and written by one thread): a plain load
-        const uint4* sp = reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(o.fine) + fp * channels + c0);
+        const __nv_bfloat16* px = reinterpret_cast<const __nv_bfloat16*>(o.fine) + fp * channels + c0;
+        const uint4* sp = reinterpret_cast<const uint4*>(px);
         const uint4 s0 = sp[0], s1 = sp[1];
         fine[(F & kOutUp) ? q : 0] = Px16{{s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w}};
         if (F & kOutUpMask) up_mask[(F & kOutUpMask) ? q : 0] = load16(o.up_mask, fp, channels, c0);
@@ -210,7 +212,8 @@ __device__ __forceinline__ void pool16(const ConvOut& o, const Px16& r0, const P
     const uint32_t m0 = odd ? r0.w[k + 4] : r0.w[k], m1 = odd ? r1.w[k + 4] : r1.w[k];
     const float2 a = unpack_bf16(odd ? g0 : m0), c = unpack_bf16(odd ? m0 : g0);   // row y: left, right
     const float2 d = unpack_bf16(odd ? g1 : m1), e = unpack_bf16(odd ? m1 : g1);   // row y + 1
-    out[k] = pack_bf16((((0.f + a.x) + c.x) + d.x + e.x) * o.pool_scale, (((0.f + a.y) + c.y) + d.y + e.y) * o.pool_scale);
+    out[k] = pack_bf16((((0.f + a.x) + c.x) + d.x + e.x) * o.pool_scale,
+                       (((0.f + a.y) + c.y) + d.y + e.y) * o.pool_scale);
   }
   if (!store) return;
   const int64_t at = ((b * (H >> 1) + (y >> 1)) * (int64_t)(W >> 1) + (x >> 1)) * channels + c0 + 8 * odd;
@@ -425,7 +428,8 @@ __global__ void __launch_bounds__(kThreads, (Per<F, Cfg<CIN, COUT, TY, NS, D>>::
 #pragma unroll
             for (int j = 0; j < C::KC / 2; j++)
               tc::mma_bf16_warp(leader, d0 + r * NS, ay + 2 * j * (C::PLANE / 16) + dx,
-                                by + (dx * C::WTAP + 2 * j * NS * 16) / 16, IDESC, (dy > 0 || dx > 0 || j > 0) ? 1u : 0u);
+                                by + (dx * C::WTAP + 2 * j * NS * 16) / 16, IDESC,
+                                (dy > 0 || dx > 0 || j > 0) ? 1u : 0u);
         }
       }
       if (leader) {
@@ -578,7 +582,7 @@ static cudaError_t launch_t(const void* in, const void* w, const float* bias, co
   }
   // one strip per CTA where the images allow: as many vertical parts as there
   // are slots for (whole tiles each)
-  const int slots = 152 * Per<F, C>::SM / C::NSPLIT, nx = (W + kTX - 1) / kTX, rows = (H + TY - 1) / TY;
+  const int slots = kSMs * Per<F, C>::SM / C::NSPLIT, nx = (W + kTX - 1) / kTX, rows = (H + TY - 1) / TY;
   const int64_t columns = (int64_t)B * nx;
   const int parts = (int)(columns >= slots ? 1 : slots / columns < rows ? slots / columns : rows);
   const int per = (rows + parts - 1) / parts, nv = (rows + per - 1) / per;
@@ -596,8 +600,8 @@ static cudaError_t launch_t(const void* in, const void* w, const float* bias, co
   CASE(64, 32, 1, 32, 2) CASE(64, 128, 1, 64, 2) CASE(128, 64, 1, 32, 1)
 
 template <int F>
-static cudaError_t dispatch(int cin, int cout, const void* in, const void* w, const float* bias, const ConvOut& o, int B,
-                            int H, int W, int* err, cudaStream_t st, bool dependent) {
+static cudaError_t dispatch(int cin, int cout, const void* in, const void* w, const float* bias, const ConvOut& o,
+                            int B, int H, int W, int* err, cudaStream_t st, bool dependent) {
   // pooled layers widen or keep the channels, upsampled ones narrow them
   constexpr bool pool = (F & kOutPool) != 0, planar = (F & kOutPlanar) != 0, up = (F & kOutUp) != 0;
 #define FS_CASE(ci, co, ty, ns, d)                                                      \
@@ -668,7 +672,9 @@ extern "C" FS_API int fs_conv3x3_bf16(const void* d_in, const void* d_wpacked, c
     return conv_fail(FS_ERR_INVALID_ARGUMENT, "fs_conv3x3_bf16: buffers must be 16-byte aligned");
   conv::ConvOut o;
   o.out = d_out;
-  const int flags = epilogue == 0 ? conv::kOutStore : epilogue == 1 ? conv::kOutStore | conv::kOutRelu : conv::kOutPlanar;
+  const int flags = epilogue == 0   ? conv::kOutStore
+                    : epilogue == 1 ? conv::kOutStore | conv::kOutRelu
+                                    : conv::kOutPlanar;
   cudaError_t e = conv::conv3x3(c_in, c_out, flags, d_in, d_wpacked, d_bias, o, batch, h, w, d_err,
                                 static_cast<cudaStream_t>(stream));
   if (e != cudaSuccess) return conv_fail(FS_ERR_CUDA, std::string("fs_conv3x3_bf16: ") + cudaGetErrorString(e));

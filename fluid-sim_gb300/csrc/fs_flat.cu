@@ -20,8 +20,6 @@
 
 namespace fs {
 
-constexpr int kFlatSMs = 152;
-
 // Dynamic shared memory that leaves room for one CTA an SM only.  A launch of the
 // small region with at most one CTA an SM asks for it: its CTAs are placed while the
 // kernel ahead still holds some SMs, and where registers leave room for three an SM
@@ -58,7 +56,7 @@ static void flat_t(Solver* s, float** x, float** y, const float* d, int n, float
     cfg.gridDim = dim3((g.nx + F::TW - 1) / F::TW, (g.ny + F::RH - 2 * now - 1) / (F::RH - 2 * now));
     cfg.blockDim = dim3(NW * 32);
     cfg.stream = s->stream;
-    if (RPW == 4 && (int64_t)cfg.gridDim.x * cfg.gridDim.y <= kFlatSMs)
+    if (RPW == 4 && (int64_t)cfg.gridDim.x * cfg.gridDim.y <= kSMs)
       cfg.dynamicSmemBytes = flat_alone_bytes<CPL, RPW, NW, H, MODE>(s->device);
     cudaLaunchAttribute pdl = {};
     pdl.id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -88,7 +86,7 @@ constexpr int64_t kFlatLarge = 200000;
 // CTAs at 20); 440^2 33.9 / 44.2, 39.9 / 52.3, 46.6 / 65.9 (182 at 16).
 static bool flat_fits(const Solver* s, int n, int H) {
   const int launches = (n + H - 1) / H, k = (n + launches - 1) / launches, tw = 64 - 2 * H, th = 64 - 2 * k;
-  return (int64_t)((s->g.nx + tw - 1) / tw) * ((s->g.ny + th - 1) / th) <= kFlatSMs;
+  return (int64_t)((s->g.nx + tw - 1) / tw) * ((s->g.ny + th - 1) / th) <= kSMs;
 }
 
 template <int MODE>

@@ -62,8 +62,8 @@ struct FlatVec<4> {
 // (r + c) & 1 == Q.  Their neighbours are not written here, so the order of
 // the updates does not matter.
 template <int CPL, int RPW, int Q>
-__device__ __forceinline__ void flat_rb_rows(float (&p)[RPW][CPL], const float (&d)[RPW][CPL], const float (&below)[CPL],
-                                             const float (&above)[CPL], float h2, float w) {
+__device__ __forceinline__ void flat_rb_rows(float (&p)[RPW][CPL], const float (&d)[RPW][CPL],
+                                             const float (&below)[CPL], const float (&above)[CPL], float h2, float w) {
 #pragma unroll
   for (int r = 0; r < RPW; r++) {
     // column 0 is updated when (r + Q) is even, column CPL - 1 when it is odd:
@@ -83,8 +83,9 @@ __device__ __forceinline__ void flat_rb_rows(float (&p)[RPW][CPL], const float (
 
 // every cell (Jacobi), or those whose bit of `mask` is set, from the old values
 template <int CPL, int RPW, bool MASK>
-__device__ __forceinline__ void flat_all_rows(float (&p)[RPW][CPL], const float (&d)[RPW][CPL], const float (&below)[CPL],
-                                              const float (&above)[CPL], float h2, float w, uint32_t mask) {
+__device__ __forceinline__ void flat_all_rows(float (&p)[RPW][CPL], const float (&d)[RPW][CPL],
+                                              const float (&below)[CPL], const float (&above)[CPL], float h2, float w,
+                                              uint32_t mask) {
   float prev[CPL];
 #pragma unroll
   for (int c = 0; c < CPL; c++) prev[c] = below[c];

@@ -493,7 +493,7 @@ static cudaError_t wgrad_tc(const Ctx& c, int l, Buf xbuf, Buf gbuf, int B, int 
   // one wave: as many CTAs as the shared memory lets an SM hold, over the taps' groups
   constexpr int per_sm = C::SMEM <= 110 * 1024 ? 2 : 1;
   const int64_t ntiles = (int64_t)B * ((H + TY - 1) / TY) * ((W + PX - 1) / PX);
-  const int P = (int)std::max<int64_t>(1, std::min<int64_t>(ntiles, per_sm * 152 * NDX / 3));
+  const int P = (int)std::max<int64_t>(1, std::min<int64_t>(ntiles, per_sm * kSMs * NDX / 3));
   const int64_t nw = (int64_t)C::MROWS * COUT;
   CK(ensure_corr(g, (int64_t)P * (nw + COUT)));
   float* part = g->corr_part;
@@ -539,7 +539,7 @@ static cudaError_t backward(const Ctx& c, const float* target, int B, int H, int
   // rows of a strip: long ones read their two extra rows less often, short ones
   // give small images more warps
   const int64_t cols = (W + kLossCols - 1) / kLossCols;
-  const int rows = B * cols * (H / 32) >= 152 * 16 ? 32 : 8;
+  const int rows = B * cols * (H / 32) >= kSMs * 16 ? 32 : 8;
   const dim3 lb((unsigned)((cols * ((H + rows - 1) / rows) + kLossWarps - 1) / kLossWarps), B);
   if (with_res)
     GL(c, "guess_loss", npix * B * 12.0,

@@ -211,6 +211,8 @@ void prof_end(Solver* s, int slot, cudaEvent_t a);
     if ((S)->profiling) fs::prof_end((S), _slot, _ev);                   \
   } while (0)
 
+constexpr int kSMs = 152;  // of a GB300
+
 // Programmatic dependent launch: with dependent, a kernel may start while the one
 // ahead of it in the stream finishes, and calls pdl_wait before it reads or
 // overwrites anything of the step.  Every kernel waits first and lets the next

@@ -61,7 +61,8 @@ struct MgCells {
     __syncthreads();
     // beyond the region's edge: any value, the ring it reaches is not written
     *reinterpret_cast<V*>(below) = *reinterpret_cast<const V*>(&e[warp > 0 ? warp - 1 : 0][1][lane * R::CPL]);
-    *reinterpret_cast<V*>(above) = *reinterpret_cast<const V*>(&e[warp < R::NW - 1 ? warp + 1 : warp][0][lane * R::CPL]);
+    *reinterpret_cast<V*>(above) =
+        *reinterpret_cast<const V*>(&e[warp < R::NW - 1 ? warp + 1 : warp][0][lane * R::CPL]);
   }
   // half-sweep s (colour s & 1; the region's first column and row are even)
   __device__ __forceinline__ void half_sweep(Edge* e, int s, float h2, float w) {
@@ -147,7 +148,8 @@ __device__ __forceinline__ void mg_down_reg(const float* __restrict__ rhs, const
     float* co = crhs + (int64_t)((t.yl + r0) >> 1) * nc + (t.xl >> 1);
     float cv[CPL / 2];
 #pragma unroll
-    for (int q = 0; q < CPL / 2; q++) cv[q] = restrict4(res[0][2 * q], res[0][2 * q + 1], res[1][2 * q], res[1][2 * q + 1]);
+    for (int q = 0; q < CPL / 2; q++)
+      cv[q] = restrict4(res[0][2 * q], res[0][2 * q + 1], res[1][2 * q], res[1][2 * q + 1]);
     if (CPL == 4) *reinterpret_cast<float2*>(co) = make_float2(cv[0], cv[CPL / 2 - 1]);
     else *co = cv[0];  // the coarse level may be odd
   }

@@ -161,7 +161,7 @@ static std::string level_name(const Solver* s, const Level& L, const char* base)
 // two an SM ahead, on levels whose fields L2 does not hold (4096^2: 71 us with it, 75
 // without, the pressure fetched as well 77; the down kernel is not bound by its
 // loads; at 2048^2 it only costs, 563 against 560 us a step)
-constexpr int kAheadFrom = 2896;
+constexpr int kAheadFrom = 2896, kAhead = 2 * kSMs;
 
 template <class R>
 static dim3 region_grid(int n, int members = 1) {
@@ -179,10 +179,10 @@ static void down_t(Solver* s, Level& L, const Level& C, bool has_x, bool zero, i
   // a first cycle the host knows is profiled under its own name
   const std::string name = level_name(s, L, "mg_down") + (first >= 0 && !cyc ? "_first" : "");
   FS_LAUNCH(s, name.c_str(), bytes,
-            launch_dependent(true, k_mg_down<R>, region_grid<R>(L.n), dim3(R::THREADS), 0, s->stream, 
-                L.rhs, has_x && !zero ? L.x : nullptr, has_x ? L.x2 : L.x, C.rhs, L.n, L.h2, s->prm.mg_pre_smooth,
-                (float)s->prm.relax, cyc, first < s->prm.mg_pre_smooth ? first : s->prm.mg_pre_smooth,
-                x_unused ? 1 : 0));
+            launch_dependent(true, k_mg_down<R>, region_grid<R>(L.n), dim3(R::THREADS), 0, s->stream, L.rhs,
+                             has_x && !zero ? L.x : nullptr, has_x ? L.x2 : L.x, C.rhs, L.n, L.h2,
+                             s->prm.mg_pre_smooth, (float)s->prm.relax, cyc,
+                             first < s->prm.mg_pre_smooth ? first : s->prm.mg_pre_smooth, x_unused ? 1 : 0));
   if (has_x) std::swap(L.x, L.x2);
 }
 
@@ -200,19 +200,23 @@ static void up_t(Solver* s, Level& L, const Level& C, float* acc_h, float* acc_l
                  bool x_zero) {
   const int fp = first < s->prm.mg_post_smooth ? first : s->prm.mg_post_smooth;
   double bytes = (double)L.n * L.n * (acc_h ? 24.0 : 12.0) + (double)C.n * C.n * 4.0;
+  const bool ahead = L.n >= kAheadFrom && T == 64;
+  constexpr int AHEAD = T == 64 ? kAhead : 0;
   if (acc_h) {
     typedef typename RegionOf<T, H, true>::R R;
+    auto* kernel = ahead ? k_mg_up<R, true, AHEAD> : k_mg_up<R, true, 0>;
     FS_LAUNCH(s, first >= 0 && !cyc ? "mg_up_acc_first" : "mg_up_acc", bytes,
-              launch_dependent(true, (L.n >= kAheadFrom && T == 64 ? k_mg_up<R, true, T == 64 ? 304 : 0> : k_mg_up<R, true, 0>), region_grid<R>(L.n), dim3(R::THREADS), 0, s->stream, 
-                  L.rhs, L.x, nullptr, C.x, L.n, L.h2, s->prm.mg_post_smooth, (float)s->prm.relax, acc_h, acc_l, cyc,
-                  fp, x_zero ? 1 : 0));
+              launch_dependent(true, kernel, region_grid<R>(L.n), dim3(R::THREADS), 0, s->stream, L.rhs, L.x, nullptr,
+                               C.x, L.n, L.h2, s->prm.mg_post_smooth, (float)s->prm.relax, acc_h, acc_l, cyc, fp,
+                               x_zero ? 1 : 0));
     return;
   }
   typedef typename RegionOf<T, H>::R R;
+  auto* kernel = ahead ? k_mg_up<R, false, AHEAD> : k_mg_up<R, false, 0>;
   FS_LAUNCH(s, level_name(s, L, "mg_up").c_str(), bytes,
-            launch_dependent(true, (L.n >= kAheadFrom && T == 64 ? k_mg_up<R, false, T == 64 ? 304 : 0> : k_mg_up<R, false, 0>), region_grid<R>(L.n), dim3(R::THREADS), 0, s->stream, 
-                L.rhs, L.x, L.x2, C.x, L.n, L.h2, s->prm.mg_post_smooth, (float)s->prm.relax, nullptr, nullptr, cyc,
-                fp, x_zero ? 1 : 0));
+            launch_dependent(true, kernel, region_grid<R>(L.n), dim3(R::THREADS), 0, s->stream, L.rhs, L.x, L.x2, C.x,
+                             L.n, L.h2, s->prm.mg_post_smooth, (float)s->prm.relax, nullptr, nullptr, cyc, fp,
+                             x_zero ? 1 : 0));
   std::swap(L.x, L.x2);
 }
 
@@ -298,8 +302,8 @@ static void down_class_t(Solver* const* ms, int count, int l, cudaStream_t st) {
     Level& L = ms[i]->lev[l];
     tab.m[i] = {L.rhs, L.x, ms[i]->lev[l + 1].rhs, ms[i]->dev};
   }
-  launch_dependent(true, k_mg_down_class<R>, region_grid<R>(L0.n, count), dim3(R::THREADS), 0, st,
-      tab, L0.n, L0.h2, ms[0]->prm.mg_pre_smooth, (float)ms[0]->prm.relax, ms[0]->prm.max_cycles);
+  launch_dependent(true, k_mg_down_class<R>, region_grid<R>(L0.n, count), dim3(R::THREADS), 0, st, tab, L0.n, L0.h2,
+                   ms[0]->prm.mg_pre_smooth, (float)ms[0]->prm.relax, ms[0]->prm.max_cycles);
 }
 
 // tile side for a level of a class: an override of the class's members, else
@@ -334,11 +338,12 @@ static void up_class_t(Solver* const* ms, int count, int l, cudaStream_t st) {
   for (int i = 0; i < count; i++) {
     Solver* s = ms[i];
     Level& L = s->lev[l];
-    tab.m[i] = {L.rhs, L.x, ACC ? nullptr : L.x2, s->lev[l + 1].x, ACC ? s->ph : nullptr, ACC ? s->pl : nullptr, s->dev};
+    tab.m[i] = {L.rhs, L.x, ACC ? nullptr : L.x2, s->lev[l + 1].x, ACC ? s->ph : nullptr, ACC ? s->pl : nullptr,
+                s->dev};
     if (!ACC) std::swap(L.x, L.x2);
   }
-  launch_dependent(true, k_mg_up_class<R, ACC>, region_grid<R>(L0.n, count), dim3(R::THREADS), 0, st,
-      tab, L0.n, L0.h2, ms[0]->prm.mg_post_smooth, (float)ms[0]->prm.relax, ms[0]->prm.max_cycles);
+  launch_dependent(true, k_mg_up_class<R, ACC>, region_grid<R>(L0.n, count), dim3(R::THREADS), 0, st, tab, L0.n,
+                   L0.h2, ms[0]->prm.mg_post_smooth, (float)ms[0]->prm.relax, ms[0]->prm.max_cycles);
 }
 
 template <int H>

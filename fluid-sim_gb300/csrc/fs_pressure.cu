@@ -104,8 +104,8 @@ void launch_divergence(Solver* s, const TV* u, const TV* v, TD* d) {
   TD ix = sizeof(TD) == 8 ? (TD)g.idxd : (TD)g.idx;
   TD iy = sizeof(TD) == 8 ? (TD)g.idyd : (TD)g.idy;
   FS_LAUNCH(s, "divergence", (double)s->n * (2 * sizeof(TV) + sizeof(TD)),
-            launch_dependent(true, k_divergence<TV, TD>, grid2d(g.nx, g.ny, kBlock), kBlock, 0, s->stream, u, v, d, g.nx,
-                                                                                        g.ny, ix, iy));
+            launch_dependent(true, k_divergence<TV, TD>, grid2d(g.nx, g.ny, kBlock), kBlock, 0, s->stream, u, v, d,
+                             g.nx, g.ny, ix, iy));
 }
 template void launch_divergence<float, float>(Solver*, const float*, const float*, float*);
 
@@ -149,8 +149,8 @@ void launch_subtract_gradient_f32(Solver* s, const float* wu, const float* wv, c
                                   float* ou, float* ov, const StepFinish& fin) {
   const Grid& g = s->g;
   FS_LAUNCH(s, "subtract_gradient", (double)s->n * 20,
-            launch_dependent(true, k_subgrad_f32, grid2d(g.nx, g.ny, kBlock), kBlock, 0, s->stream, wu, wv, p, ou, ov, g.nx,
-                                                                                g.ny, g.idx, g.idy, fin));
+            launch_dependent(true, k_subgrad_f32, grid2d(g.nx, g.ny, kBlock), kBlock, 0, s->stream, wu, wv, p, ou, ov,
+                             g.nx, g.ny, g.idx, g.idy, fin));
 }
 // ----------------------------------------------------------------- smoothers
 // damped Jacobi, relaxation factor w (shaders.js:302-325)
@@ -450,8 +450,8 @@ void launch_div_df(Solver* s, const float* uh, const float* ul, const float* vh,
                    float* dl) {
   const Grid& g = s->g;
   FS_LAUNCH(s, "divergence", (double)s->n * ((ul ? 16 : 8) + 8),
-            launch_dependent(true, k_div_df, grid2d(g.nx, g.ny, kBlock), kBlock, 0, s->stream, 
-                uh, ul, vh, vl, dh, dl, g.nx, g.ny, df_host(g.idxd), df_host(g.idyd)));
+            launch_dependent(true, k_div_df, grid2d(g.nx, g.ny, kBlock), kBlock, 0, s->stream, uh, ul, vh, vl, dh, dl,
+                             g.nx, g.ny, df_host(g.idxd), df_host(g.idyd)));
 }
 
 // u = w - (p_i - p_{i-1})/dx, v = w - (p_j - p_{j-1})/dy in df; w lo planes optional
@@ -538,11 +538,11 @@ void launch_subgrad_df(Solver* s, const float* wuh, const float* wul, const floa
   const Grid& g = s->g;
   FS_LAUNCH(s, "subtract_gradient", (double)s->n * ((wul ? 16 : 8) + 8 + 16),
             if (g.nx % 4 == 0) {
-              launch_dependent(true, k_subgrad4_df, grid2d(g.nx / 4, g.ny, kBlock), kBlock, 0, s->stream, 
-                  wuh, wul, wvh, wvl, ph, pl, uh, ul, vh, vl, g.nx, g.ny, df_host(g.idxd), df_host(g.idyd), fin);
+              launch_dependent(true, k_subgrad4_df, grid2d(g.nx / 4, g.ny, kBlock), kBlock, 0, s->stream, wuh, wul,
+                               wvh, wvl, ph, pl, uh, ul, vh, vl, g.nx, g.ny, df_host(g.idxd), df_host(g.idyd), fin);
             } else {
-              launch_dependent(true, k_subgrad_df, grid2d(g.nx, g.ny, kBlock), kBlock, 0, s->stream, 
-                  wuh, wul, wvh, wvl, ph, pl, uh, ul, vh, vl, g.nx, g.ny, df_host(g.idxd), df_host(g.idyd), fin);
+              launch_dependent(true, k_subgrad_df, grid2d(g.nx, g.ny, kBlock), kBlock, 0, s->stream, wuh, wul, wvh,
+                               wvl, ph, pl, uh, ul, vh, vl, g.nx, g.ny, df_host(g.idxd), df_host(g.idyd), fin);
             });
 }
 
@@ -782,11 +782,11 @@ bool launch_refine_init(Solver* s, const float* dh, const float* dl, const float
                                      : CondFold{};
   FS_LAUNCH(s, "refine_init", (double)s->n * (zero_p ? 12 : 20),
             if (quad) {
-              launch_dependent(true, k_refine_init4, refine4_grid(s, g.nx / 4, g.ny), kBlock, 0, s->stream, 
-                  dh, dl, ph, pl, r32, g.nx, g.ny, lap_scale(g), red_ctx(s, s->red_out), cf);
+              launch_dependent(true, k_refine_init4, refine4_grid(s, g.nx / 4, g.ny), kBlock, 0, s->stream, dh, dl,
+                               ph, pl, r32, g.nx, g.ny, lap_scale(g), red_ctx(s, s->red_out), cf);
             } else {
-              launch_dependent(true, k_refine_init, red_grid2(g.nx, g.ny), kBlock, 0, s->stream, 
-                  dh, dl, ph, pl, r32, g.nx, g.ny, lap_scale(g), zero_p ? 1 : 0, red_ctx(s, s->red_out));
+              launch_dependent(true, k_refine_init, red_grid2(g.nx, g.ny), kBlock, 0, s->stream, dh, dl, ph, pl, r32,
+                               g.nx, g.ny, lap_scale(g), zero_p ? 1 : 0, red_ctx(s, s->red_out));
             });
   return cf.on != 0;
 }
@@ -796,8 +796,8 @@ void launch_diffuse_start(Solver* s, const float* u, const float* v, float* ou, 
   const Grid& g = s->g;
   const DiffuseOut o = {ou, ov, (float)(s->prm.nu * dt / (g.dxd * g.dxd)), (float)(s->prm.nu * dt / (g.dyd * g.dyd))};
   FS_LAUNCH(s, "diffuse_start", (double)s->n * 36,
-            launch_dependent(true, k_diffuse_start4, red_grid2(g.nx / 4, g.ny), kBlock, 0, s->stream, u, v, s->dh, s->dl,
-                             s->ph, s->pl, s->r32, g.nx, g.ny, df_host(g.idxd), df_host(g.idyd),
+            launch_dependent(true, k_diffuse_start4, red_grid2(g.nx / 4, g.ny), kBlock, 0, s->stream, u, v, s->dh,
+                             s->dl, s->ph, s->pl, s->r32, g.nx, g.ny, df_host(g.idxd), df_host(g.idyd),
                              red_ctx(s, s->red_out), o));
 }
 
@@ -813,9 +813,9 @@ void launch_div_start(Solver* s, const float* wu, const float* wv) {
     return;
   }
   FS_LAUNCH(s, "div_start", (double)s->n * 28,
-            launch_dependent(true, k_div_start4, red_grid2(g.nx / 4, g.ny), kBlock, 0, s->stream, 
-                wu, wv, s->dh, s->dl, s->ph, s->pl, s->r32, g.nx, g.ny, df_host(g.idxd), df_host(g.idyd),
-                red_ctx(s, s->red_out)));
+            launch_dependent(true, k_div_start4, red_grid2(g.nx / 4, g.ny), kBlock, 0, s->stream, wu, wv, s->dh,
+                             s->dl, s->ph, s->pl, s->r32, g.nx, g.ny, df_host(g.idxd), df_host(g.idyd),
+                             red_ctx(s, s->red_out)));
 }
 
 void launch_refine_update(Solver* s, const float* ph, const float* pl, const float* e, const float* dh,
@@ -988,14 +988,16 @@ void launch_refine_class(Solver* const* ms, int count, cudaStream_t st) {
   const bool quad = g.nx % 4 == 0;
   dim3 grid = quad ? red_grid2(g.nx / 4, g.ny) : red_grid2(g.nx, g.ny);
   grid.z = count;
-  launch_dependent(true, k_refine_class, grid, kBlock, 0, st, tab, g.nx, g.ny, lap_scale(g), s0->prm.max_cycles, quad ? 1 : 0);
+  launch_dependent(true, k_refine_class, grid, kBlock, 0, st, tab, g.nx, g.ny, lap_scale(g), s0->prm.max_cycles,
+                   quad ? 1 : 0);
 }
 
 void launch_cond_class(Solver* const* ms, int count, cudaStream_t st, cudaGraphConditionalHandle h, int init,
                        long long* iterations) {
   CondTab tab{};
   for (int i = 0; i < count; i++) tab.m[i] = {ms[i]->red_out, ms[i]->dev, dev_tol(ms[i])};
-  launch_dependent(true, k_cond_class, dim3(1), dim3(kClassMax), 0, st, tab, count, ms[0]->prm.max_cycles, h, init, iterations);
+  launch_dependent(true, k_cond_class, dim3(1), dim3(kClassMax), 0, st, tab, count, ms[0]->prm.max_cycles, h, init,
+                   iterations);
 }
 
 // ---- the rest of a plain class member's step, batched: the divergence of the

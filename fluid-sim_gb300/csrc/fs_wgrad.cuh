@@ -65,7 +65,8 @@ struct WgCfg {
   // the last M block reads groups up to here, inside the stage
   static_assert((16 * (MB - 1) + LAST_M / 8) * XP <= X_BYTES + G_BYTES, "A operand within the stage");
   static_assert(ACC_BYTES + kWgThreads * 32 <= 2 * STAGE, "sums and bias fold in the stages' words");
-  static_assert(COLS <= 512 && NN <= 256 && NN % 16 == 0 && COUT % 16 == 0 && CIN % 16 == 0 && PX % 16 == 0 && SMEM <= 227 * 1024, "shape");
+  static_assert(COLS <= 512 && NN <= 256 && NN % 16 == 0 && COUT % 16 == 0 && CIN % 16 == 0 && PX % 16 == 0, "shape");
+  static_assert(SMEM <= 227 * 1024, "shared memory of one CTA");
   static_assert(kWgThreads % OC == 0, "a bias thread keeps its channels");
 };
 
@@ -90,9 +91,10 @@ __device__ __forceinline__ int wg_wrap(int i, int n) {
 // warp 8 issues the MMAs; two stages, handed over by barriers: full[s] (the
 // staging threads' copies have landed) and done[s] (the MMAs that read them).
 template <int CIN, int COUT, int TY, int PX, int NDX>
-__global__ void __launch_bounds__(kWgThreads + 32, 1) k_wgrad_tc(const uint4* __restrict__ X, const uint4* __restrict__ G,
-                                                              int B, int H, int W, float* __restrict__ part,
-                                                              float* __restrict__ bpart, int* __restrict__ err) {
+__global__ void __launch_bounds__(kWgThreads + 32, 1) k_wgrad_tc(const uint4* __restrict__ X,
+                                                                 const uint4* __restrict__ G, int B, int H, int W,
+                                                                 float* __restrict__ part, float* __restrict__ bpart,
+                                                                 int* __restrict__ err) {
   using C = WgCfg<CIN, COUT, TY, PX, NDX>;
   extern __shared__ __align__(128) unsigned char smem[];
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + 2 * C::STAGE);
