@@ -112,6 +112,8 @@ __device__ __forceinline__ void lerp_rows(float a, float b, float c, float d, fl
       : "f"(a), "f"(b), "f"(c), "f"(d), "f"(fx));
 }
 
+// COMPLETE: the field was written before the launch ahead began (see pdl_wait)
+template <bool COMPLETE>
 struct TileView {
   const float* sm;  // kSH x kSW staged block
   int oi, oj;       // global (unwrapped) index of the block's element (0, 0)
@@ -135,7 +137,8 @@ struct TileView {
       const int i1 = i0 + 1 == nx ? 0 : i0 + 1;
       const int j1 = j0 + 1 == ny ? 0 : j0 + 1;
       const int64_t r0 = (int64_t)j0 * nx, r1 = (int64_t)j1 * nx;
-      a = g[r0 + i0]; b = g[r0 + i1]; c = g[r1 + i0]; d = g[r1 + i1];
+      auto at = [&](int64_t k) { return COMPLETE ? __ldg(g + k) : g[k]; };
+      a = at(r0 + i0); b = at(r0 + i1); c = at(r1 + i0); d = at(r1 + i1);
     }
     if (RANGE) {
       *lo = fminf(fminf(a, b), fminf(c, d));
@@ -148,7 +151,7 @@ struct TileView {
 };
 
 // RK2 midpoint backward trace (src/cpu/advect.js:46-54, shaders.js:117-122) in cells
-__device__ __forceinline__ void trace_t(const TileView& u, const TileView& v, int i, int j, Home h,
+__device__ __forceinline__ void trace_t(const TileView<true>& u, const TileView<true>& v, int i, int j, Home h,
                                         float cx, float cy, float& dX, float& dY) {
   const float u1 = u.sample(i, j, h.ux, h.uy);
   const float v1 = v.sample(i, j, h.vx, h.vy);
@@ -165,7 +168,7 @@ __device__ __forceinline__ void trace_t(const TileView& u, const TileView& v, in
 // every finite field, so it is passed in (own, read from the staged block)
 // instead of sampled.
 template <bool UFACE>
-__device__ __forceinline__ void trace_face(const TileView& u, const TileView& v, int i, int j,
+__device__ __forceinline__ void trace_face(const TileView<true>& u, const TileView<true>& v, int i, int j,
                                            float own, float cx, float cy, float& dX, float& dY) {
   const Home h = UFACE ? home_u() : home_v();
   const float u1 = UFACE ? own : u.sample(i, j, h.ux, h.uy);
@@ -179,8 +182,8 @@ __device__ __forceinline__ void trace_face(const TileView& u, const TileView& v,
 
 // Stage the kSH x kSW blocks of F fields whose (0, 0) is global (oi, oj),
 // wrapped, one row per warp at a time; returns max |value| of the first two
-// fields (the velocities), NaN counted as infinite.
-template <int F>
+// fields (the velocities), NaN counted as infinite.  COMPLETE as in TileView.
+template <int F, bool COMPLETE = false>
 __device__ __forceinline__ void stage_tiles(float* const (&sm)[F], const float* const (&f)[F], int oi, int oj,
                                             int nx, int ny, float& umax, float& vmax) {
   const int lane = threadIdx.x, warp = threadIdx.y, nwarp = blockDim.y;
@@ -194,7 +197,7 @@ __device__ __forceinline__ void stage_tiles(float* const (&sm)[F], const float* 
       const int k = lj * kSW + li;
 #pragma unroll
       for (int q = 0; q < F; q++) {
-        const float x = f[q][row + gi];
+        const float x = COMPLETE ? __ldg(f[q] + row + gi) : f[q][row + gi];
         sm[q][k] = x;
         if (q == 0) mu = max(mu, __float_as_uint(fabsf(x)));
         if (q == 1) mv = max(mv, __float_as_uint(fabsf(x)));
@@ -385,7 +388,7 @@ __device__ __forceinline__ void advect_pair(const float* su, const float* sv, fl
 // the four cells each sample read -- the limiter's range, src/cpu/advect.js
 // :104-111 -- are written too, planes (lo_u, hi_u, lo_v, hi_v), so the combine
 // pass does not trace forward again.
-__device__ __forceinline__ void advect_rows(const TileView& U, const TileView& V, float* __restrict__ ou,
+__device__ __forceinline__ void advect_rows(const TileView<true>& U, const TileView<true>& V, float* __restrict__ ou,
                                             float* __restrict__ ov, int nx, int ny, int ti, int tj, float cx,
                                             float cy, float* __restrict__ bounds) {
   const Home hu = home_u(), hv = home_v();
@@ -420,7 +423,7 @@ __device__ __forceinline__ void advect_rows(const TileView& U, const TileView& V
 // Tiles whose staged block lies inside the grid are staged by TMA when the
 // tensor maps are valid (tma != 0); the others by the wrapped loads.
 template <int NT>
-__global__ void __launch_bounds__(256) k_advect_sl_t(const float* u, const float* v,
+__global__ void __launch_bounds__(256) k_advect_sl_t(const float* __restrict__ u, const float* __restrict__ v,
                                                      float* __restrict__ ou, float* __restrict__ ov, int nx, int ny,
                                                      float cx, float cy, float* __restrict__ bounds,
                                                      const __grid_constant__ CUtensorMap tm_u,
@@ -451,12 +454,12 @@ __global__ void __launch_bounds__(256) k_advect_sl_t(const float* u, const float
     } else {
       float* const sm[2] = {su[t], sv[t]};
       const float* const f[2] = {u, v};
-      stage_tiles<2>(sm, f, oi, tj - kHalo, nx, ny, umax, vmax);
+      stage_tiles<2, true>(sm, f, oi, tj - kHalo, nx, ny, umax, vmax);
     }
     if (fast_tile(umax, vmax, cx, cy)) {
       advect_pair(su[t], sv[t], ou, ov, nx, ny, ti, tj, cx, cy, bounds);
     } else {
-      const TileView U{su[t], oi, tj - kHalo, u, nx, ny}, V{sv[t], oi, tj - kHalo, v, nx, ny};
+      const TileView<true> U{su[t], oi, tj - kHalo, u, nx, ny}, V{sv[t], oi, tj - kHalo, v, nx, ny};
       advect_rows(U, V, ou, ov, nx, ny, ti, tj, cx, cy, bounds);
     }
   }
@@ -465,8 +468,8 @@ __global__ void __launch_bounds__(256) k_advect_sl_t(const float* u, const float
 // MACCORMACK: the backward pass (ADVECT_FIELD_BY with -dt) is evaluated inside
 // the combine kernel at the single point it is needed, then the correction
 // limited to the forward pass's range (shaders.js:187-231, src/cpu/advect.js:149-185).
-__device__ __forceinline__ void combine_rows(const TileView& U, const TileView& V,
-                                             const TileView& FU, const TileView& FV,
+__device__ __forceinline__ void combine_rows(const TileView<true>& U, const TileView<true>& V,
+                                             const TileView<false>& FU, const TileView<false>& FV,
                                              const float* __restrict__ bounds, float* __restrict__ ou,
                                              float* __restrict__ ov, int nx, int ny, int ti, int tj, float cx,
                                              float cy) {
@@ -510,8 +513,6 @@ __device__ __forceinline__ void combine_pair(const float* su, const float* sv, c
 #pragma unroll
   for (int k = 0; k < 2; k++) {
     const float* b = bounds + 2 * k * n;
-    const float lo0 = b[c], hi0 = b[n + c];
-    const float lo1 = two ? b[c1] : 0.f, hi1 = two ? b[n + c1] : 0.f;
     const PairView& own = k == 0 ? U : V;
     const PairView F{(k == 0 ? sfu : sfv) + lc};
     F2 dx, dy;
@@ -520,6 +521,9 @@ __device__ __forceinline__ void combine_pair(const float* su, const float* sv, c
     else trace_pair<false>(U, V, -cx, -cy, dx, dy);
     float r0, r1;
     split(fma2(f2(0.5f), sub2(own.at(0), F.sample(dx, dy)), F.at(0)), r0, r1);
+    // the ranges, by now in L2 or on their way (asked for ahead of the sampling: 4096^2 149 -> 152 us)
+    const float lo0 = b[c], hi0 = b[n + c];
+    const float lo1 = two ? b[c1] : 0.f, hi1 = two ? b[n + c1] : 0.f;
     float* o = k == 0 ? ou : ov;
     o[c] = r0 < lo0 ? lo0 : r0 > hi0 ? hi0 : r0;
     if (two) o[c1] = r1 < lo1 ? lo1 : r1 > hi1 ? hi1 : r1;
@@ -573,8 +577,8 @@ __global__ void __launch_bounds__(256) k_mc_combine_t(const float* u, const floa
     if (fast_tile(umax, vmax, cx, cy)) {
       combine_pair(su[t], sv[t], sfu[t], sfv[t], bounds, ou, ov, nx, ny, ti, tj, cx, cy);
     } else {
-      const TileView U{su[t], oi, tj - kHalo, u, nx, ny}, V{sv[t], oi, tj - kHalo, v, nx, ny};
-      const TileView FU{sfu[t], oi, tj - kHalo, fu, nx, ny}, FV{sfv[t], oi, tj - kHalo, fv, nx, ny};
+      const TileView<true> U{su[t], oi, tj - kHalo, u, nx, ny}, V{sv[t], oi, tj - kHalo, v, nx, ny};
+      const TileView<false> FU{sfu[t], oi, tj - kHalo, fu, nx, ny}, FV{sfv[t], oi, tj - kHalo, fv, nx, ny};
       combine_rows(U, V, FU, FV, bounds, ou, ov, nx, ny, ti, tj, cx, cy);
     }
   }
@@ -618,12 +622,12 @@ __global__ void __launch_bounds__(256) k_advect_sl_class(const AdvTab tab, int n
   {
     float* const sm[2] = {su, sv};
     const float* const f[2] = {a.u, a.v};
-    stage_tiles<2>(sm, f, oi, oj, nx, ny, umax, vmax);
+    stage_tiles<2, true>(sm, f, oi, oj, nx, ny, umax, vmax);
   }
   if (fast_tile(umax, vmax, a.cx, a.cy)) {
     advect_pair(su, sv, a.ou, a.ov, nx, ny, ti, tj, a.cx, a.cy, a.bounds);
   } else {
-    const TileView U{su, oi, oj, a.u, nx, ny}, V{sv, oi, oj, a.v, nx, ny};
+    const TileView<true> U{su, oi, oj, a.u, nx, ny}, V{sv, oi, oj, a.v, nx, ny};
     advect_rows(U, V, a.ou, a.ov, nx, ny, ti, tj, a.cx, a.cy, a.bounds);
   }
 }
@@ -646,8 +650,8 @@ __global__ void __launch_bounds__(256) k_mc_combine_class(const AdvTab tab, int 
   if (fast_tile(umax, vmax, a.cx, a.cy)) {
     combine_pair(su, sv, sfu, sfv, a.bounds, a.ou, a.ov, nx, ny, ti, tj, a.cx, a.cy);
   } else {
-    const TileView U{su, oi, oj, a.u, nx, ny}, V{sv, oi, oj, a.v, nx, ny};
-    const TileView FU{sfu, oi, oj, a.fu, nx, ny}, FV{sfv, oi, oj, a.fv, nx, ny};
+    const TileView<true> U{su, oi, oj, a.u, nx, ny}, V{sv, oi, oj, a.v, nx, ny};
+    const TileView<false> FU{sfu, oi, oj, a.fu, nx, ny}, FV{sfv, oi, oj, a.fv, nx, ny};
     combine_rows(U, V, FU, FV, a.bounds, a.ou, a.ov, nx, ny, ti, tj, a.cx, a.cy);
   }
 }
@@ -779,7 +783,7 @@ __device__ __forceinline__ void diffuse4_body(const float* __restrict__ u, const
   diffuse4_one(v, ov, r, rm, rp, i0, il, ir, a, b);
 }
 
-__global__ void __launch_bounds__(256) k_diffuse4(const float* u, const float* v, float* __restrict__ ou,
+__global__ void __launch_bounds__(256, 8) k_diffuse4(const float* u, const float* v, float* __restrict__ ou,
                                                   float* __restrict__ ov, int nx, int ny, float a, float b) {
   pdl_wait();
   diffuse4_body(u, v, ou, ov, nx, ny, a, b);
@@ -805,7 +809,7 @@ void launch_diffuse(Solver* s, const float* u, const float* v, float* ou, float*
             });
 }
 
-__global__ void __launch_bounds__(256) k_diffuse_class(const DiffTab tab, int nx, int ny) {
+__global__ void __launch_bounds__(256, 8) k_diffuse_class(const DiffTab tab, int nx, int ny) {
   pdl_wait();
   const auto& a = tab.m[blockIdx.z];
   if ((nx & 3) == 0) diffuse4_body(a.u, a.v, a.ou, a.ov, nx, ny, a.a, a.b);

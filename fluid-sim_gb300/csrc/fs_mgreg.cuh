@@ -48,10 +48,14 @@ struct MgCells {
     yl = blockIdx.y * R::TH - R::HY + warp * R::RPW;
     gx = flat_wrap(xl, n);  // n is a multiple of CPL: a lane's columns do not straddle the wrap
   }
+  // COMPLETE: the field was written before the launch ahead began (see pdl_wait)
+  template <bool COMPLETE>
   __device__ __forceinline__ void load(float (&a)[R::RPW][R::CPL], const float* f, int n) const {
 #pragma unroll
-    for (int r = 0; r < R::RPW; r++)
-      *reinterpret_cast<V*>(a[r]) = *reinterpret_cast<const V*>(f + (int64_t)flat_wrap(yl + r, n) * n + gx);
+    for (int r = 0; r < R::RPW; r++) {
+      const V* at = reinterpret_cast<const V*>(f + (int64_t)flat_wrap(yl + r, n) * n + gx);
+      *reinterpret_cast<V*>(a[r]) = COMPLETE ? __ldg(at) : *at;
+    }
   }
   // the rows above and below the thread's, from the neighbouring warps
   typedef float Edge[R::NW][2][R::RW];
@@ -106,10 +110,10 @@ __device__ __forceinline__ void mg_down_reg(const float* __restrict__ rhs, const
   typedef typename MgCells<R>::V V;
   __shared__ __align__(16) typename MgCells<R>::Edge edge[2];
   MgCells<R> t(n);
-  t.load(t.d, rhs, n);
+  t.template load<false>(t.d, rhs, n);
   int s = 0;
   if (xin) {
-    t.load(t.p, xin, n);
+    t.template load<false>(t.p, xin, n);
   } else {
 #pragma unroll
     for (int r = 0; r < RPW; r++)
@@ -206,8 +210,8 @@ __device__ __forceinline__ void mg_up_reg(const float* __restrict__ rhs, const f
   const int nc = n >> 1, gc = t.gx >> 1, jc = (t.yl >> 1) - 1;
   // the iterate and the rhs were complete before the launch ahead of this one began
   if (!zero) {
-    t.load(t.p, xin, n);
-    t.load(t.d, rhs, n);
+    t.template load<true>(t.p, xin, n);
+    t.template load<true>(t.d, rhs, n);
   }
   pdl_wait();
   if (AHEAD > 0 && !zero) prefetch_region<R>(n, AHEAD, xin, rhs);
