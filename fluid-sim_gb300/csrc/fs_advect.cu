@@ -556,7 +556,8 @@ __global__ void __launch_bounds__(256) k_mc_combine_t(const float* u, const floa
     tma_issue<4, NT>(sm, tm, oi, oj, in, bar);
   }
   if (NT > 1) {
-    // large grids: the limiter's ranges into L2 meanwhile (4096^2 158 -> 154 us), a line a row, tile and plane
+    // large grids: the limiter's ranges into L2 meanwhile, a line a row, tile and plane
+    // (4096^2 158 -> 154 us, 149 with the ranges read late)
     const int k = threadIdx.y * 32 + threadIdx.x, q = k / (NT * kTY), j = blockIdx.y * NT * kTY + k % (NT * kTY);
     if (q < 4 && j < ny) prefetch_l2(bounds + (int64_t)q * nx * ny + (int64_t)j * nx + ti);
   }
@@ -664,9 +665,11 @@ static dim3 tile_grid(const Grid& g, int nt = 1) {
 
 // Tiles a CTA stages at once, one above the other: with two the copies of the
 // second are in flight while the first is worked on (4096^2: forward 151 -> 137
-// us, combine 174 -> 158; three 142 and 164).  Below 2048^2, where that leaves few
-// CTAs an SM, one is as fast (1024^2 303.4 us a step against 304.1) or faster
-// (512^2 110.7 against 118.9).
+// us, combine 174 -> 158; three 142 and 164).  On small grids, where that leaves few
+// CTAs an SM, one is faster (512^2 110.7 us a step against 118.9).  Steps with one
+// and two: 1024^2 272 / 275 us, 1280^2 349 / 351, 1536^2 402 / 409, 1792^2 521 / 515,
+// 2048^2 564 / 558, 2304^2 671 / 658, 3072^2 1049 / 1025: they cross between 1536^2
+// and 1792^2, a little below the line.
 static int tiles_per_cta(const Grid& g) { return (int64_t)g.nx * g.ny >= 4000000 ? 2 : 1; }
 
 // Tensor maps of the solver's f32 planes for the TMA-staged tiles' kSW x kSH boxes,

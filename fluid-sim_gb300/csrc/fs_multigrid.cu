@@ -160,7 +160,8 @@ static std::string level_name(const Solver* s, const Level& L, const char* base)
 // CTAs between the one whose region an up kernel's CTA fetches into L2 and itself:
 // two an SM ahead, on levels whose fields L2 does not hold (4096^2: 71 us with it, 75
 // without, the pressure fetched as well 77; the down kernel is not bound by its
-// loads; at 2048^2 it only costs, 563 against 560 us a step)
+// loads).  Steps with it and without: 2048^2 560 / 558 us, 2304^2 658 / 658, 2560^2 773 /
+// 774, 2816^2 894 / 905, 3072^2 1010 / 1025, 3584^2 1297 / 1324, 4096^2 1559 / 1587.
 constexpr int kAheadFrom = 2896, kAhead = 2 * kSMs;
 
 template <class R>
