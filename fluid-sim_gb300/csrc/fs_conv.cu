@@ -376,14 +376,15 @@ __global__ void __launch_bounds__(kThreads, (Per<F, Cfg<CIN, COUT, TY, NS, D>>::
         for (int r = R0; r < TY + 2; r++) {
           int q = t.ring + r;
           if (q >= C::NR) q -= C::NR;
-          src[r - R0] = in + (int64_t)(t.b * H + wrap_near(t.y - 1 + r, H)) * (W * C::KC);
+          src[r - R0] = in + ((int64_t)t.b * H + wrap_near(t.y - 1 + r, H)) * W * C::KC;
           dst[r - R0] = s0 + q * C::ROW;
         }
         for (int q = st; q < kTW * C::KC; q += kStage) {
           // 16 channels: a chunk of neighbouring pixels on neighbouring threads; more:
           // a pixel's chunks on neighbouring threads
           const int xx = C::KC == 2 ? q % kTW : q / C::KC, kc = C::KC == 2 ? q / kTW : q % C::KC;
-          const int col = wrap_near(t.x0 - 1 + xx, W) * C::KC + kc, off = kc * C::PLANE + xx * 16;
+          const int off = kc * C::PLANE + xx * 16;
+          const int64_t col = (int64_t)wrap_near(t.x0 - 1 + xx, W) * C::KC + kc;
 #pragma unroll
           for (int r = 0; r < TY + 2 - R0; r++) copy16(dst[r] + off, src[r] + col);
         }
