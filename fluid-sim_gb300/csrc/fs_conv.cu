@@ -448,6 +448,13 @@ __global__ void __launch_bounds__(kThreads, (Per<F, Cfg<CIN, COUT, TY, NS, D>>::
     const int r0 = C::BY_CHUNK ? 0 : group * C::EROWS;
     constexpr int CSTEP = C::BY_CHUNK ? 32 : 16;
     const int cfirst = C::BY_CHUNK ? 16 * group : 0;
+    // the biases of a thread's one chunk stay in registers (4 x 1024^2 gradient 1887 us with
+    // them read from shared memory for every pixel, 1846 us so); not where two CTAs an SM
+    // and the loads of a skip sum leave none for them
+    constexpr bool HELD = NS <= CSTEP && !(F & kOutPlanar) && !((F & kOutUp) && Per<F, C>::SM > 1);
+    float held[HELD ? 16 : 1];
+#pragma unroll
+    for (int e = 0; e < (HELD ? 16 : 1); e++) held[e] = sbias[HELD ? cfirst + e : 0];
     for (; !t.done() && !*failed; t.next()) {
       const int set = t.k & 1, x = t.x0 + p;
       const uint32_t d0 = taddr + set * C::NACC + ((uint32_t)(32 * quarter) << 16);
@@ -473,12 +480,14 @@ __global__ void __launch_bounds__(kThreads, (Per<F, Cfg<CIN, COUT, TY, NS, D>>::
             tc::mbar_arrive(&taken[set]);
           }
           if constexpr ((F & kOutPlanar) != 0) {
-            if (in_image) reinterpret_cast<float*>(o.out)[((int64_t)t.b * H + y) * W + x] = v[0] + sbias[0];
+            if (in_image) reinterpret_cast<float*>(o.out)[((int64_t)t.b * H + y) * W + x] = v[0] + held[0];
           } else {
             Px16 w;
 #pragma unroll
             for (int e = 0; e < 16; e += 4) {
-              const float4 bv = *reinterpret_cast<const float4*>(sbias + c0 + e);
+              float4 bv;
+              if constexpr (HELD) bv = make_float4(held[e], held[e + 1], held[e + 2], held[e + 3]);
+              else bv = *reinterpret_cast<const float4*>(sbias + c0 + e);
               v[e] += bv.x, v[e + 1] += bv.y, v[e + 2] += bv.z, v[e + 3] += bv.w;
             }
 #pragma unroll
