@@ -27,8 +27,8 @@
 // TMEM allocation, weight and tile staging, MMAs and epilogue (45% warps active,
 // tensor core 28% busy): 95 us for 16 -> 16 channels at 1024^2 x 4 against 56 us
 // here.  A 128 x 16 x 16 MMA takes 32 cycles however narrow it is, which makes 32 us
-// of those 56 (its math is 8 of the 32: the tensor pipe is 14% active, and what is
-// busiest is L1 and shared memory, 81%); the 268 MB are 40 us of HBM time.
+// of those 56 (its math is 8 of the 32: the tensor pipe is 16% active, and what is
+// busiest is L1 and shared memory, 72%); the 268 MB are 40 us of HBM time.
 // One 1024^2 forward pass, with the pooling and skip-sum passes it absorbs:
 // 323 -> 212 us.  Two CTAs an SM and eight epilogue warps each: the layers that
 // write the skip sum wait for the four finer pixels, which are therefore all
